@@ -11,31 +11,29 @@
 // Only x waits: the x warp copies a matmul's activations once every CTA has reported the matmuls it depends on
 // finished (a counter per matmul in global memory, read with acquire semantics; the host works out the dependences
 // from the buffer addresses, and matmuls that do not depend on one another overlap, two in flight at most). While
-// that report travels, the ring fills with the next weights.
+// that report travels, the ring fills with the next weights: 190 KB per SM, 28 MB in all, over 4 us of HBM.
 //
 // Decomposition ("stream-K"). A weight matrix is cut into sub-panels of 4 tile columns (one run of the streaming
 // layout). A unit is one tile row of one sub-panel. Units are numbered sub-panel by sub-panel and dealt out in
-// contiguous ranges to the CTAs (two per SM): equal shares of all CTAs, so every SM streams the same number of bytes
-// whatever the shape, or, where that keeps most CTAs busy, shares cut so that ranges end where sub-panels end. A
-// sub-panel that several CTAs share is finished by the CTA that holds its last tile row: the others write
-// their fp32 partial sums to scratch and bump a counter; the owner, which takes that sub-panel last, waits for the
-// counter (with a limit), adds the partials in CTA order, so results do not depend on timing, and runs the
-// epilogue. Contributors never wait, so the owner's wait always ends; it is bounded all the same.
+// contiguous ranges to the CTAs, one per SM: equal shares of all CTAs, so every SM streams the same number of bytes
+// whatever the shape, or, for small matmuls, whole sub-panels. A sub-panel that several CTAs share is finished by the
+// CTA that holds its last tile row: the others write their fp32 partial sums to scratch and bump a counter; the owner,
+// which takes that sub-panel last, waits for the counter (with a limit), adds the partials in CTA order, so results do
+// not depend on timing, and runs the epilogue. Contributors never wait, so the owner's wait always ends; it is bounded
+// all the same.
 //
-// Inside a CTA: warps 8 and 9 are the producers. Warp 8 waits for room in the ring, announces the stage's weight
-// bytes to the stage's mbarrier and issues one bulk copy per weight matrix; warp 9 does the same for the stage's x
-// tiles once the matmuls this one depends on are finished. Stages are as large as the matmul's kind wants and follow
-// one another through the ring's bytes; 16 mbarrier pairs go round with them. The 8 consumer
-// warps form a 2 x 4 grid: warp (ck, cc) takes column cc of the sub-panel; for one weight matrix ck picks every
-// other tile row of the stage (the two halves are added through shared memory when the sub-panel ends), for a
-// gate/up pair ck picks the matrix (the up half is handed to the gate warp for the epilogue). A weight tile is
+// Inside a CTA: two producer warps fill the ring, 16 consumer warps empty it. For one weight matrix a consumer warp has
+// one column of the sub-panel and every fourth tile row of a stage; for a gate/up pair one column of one of the two
+// matrices and every other tile row. When the CTA's part of a sub-panel ends the warps leave their sums in shared
+// memory and all 512 threads add them up and run the epilogue element by element. One CTA of 16 warps per SM rather
+// than two of 8: half the reports, polls and partial sums, and twice the bytes per copy. A weight tile is
 // four 16x16 faces; a face is one m16n8k16 MMA with the face's 16 output channels as the MMA's rows, 16 input
 // channels as its K and up to 8 tokens as its columns. The 16 weights of a face row share an exponent e; how the
-// packed bytes become exact bf16 weights times 2^(e - 197) is described at tile_mma; the epilogue multiplies the
-// sums by 2^64.
+// packed bytes become weights is described at tile_mma.
 #include "common.cuh"
 #include "ptx.cuh"
 #include "stream_layout.cuh"
+#include "tmap.cuh"
 #include <cstring>
 #include <mutex>
 
@@ -44,25 +42,24 @@ using namespace bt;
 namespace {
 
 constexpr int kWC = kPanel;                 // tile columns of a sub-panel = one run of the streaming layout
-constexpr int kCW = 8;                      // consumer warps per CTA
-constexpr int kThreads = (kCW + 2) * 32;    // plus the two producer warps
-constexpr int kOcc = 2;                     // CTAs per SM
+constexpr int kCW = 16;                     // consumer warps of the CTA; an SM holds one CTA
+constexpr int kConsumers = kCW * 32;
+constexpr int kThreads = (kCW + 3) * 32;    // plus two producer warps and a messenger
 constexpr int kBars = 16;                   // stages in the ring at most: mbarriers that go round with the stages
 constexpr int kMaxCtas = 320;
 constexpr int kMaxSubPanels = 16384;
 constexpr int kQueueMax = 32;               // matmuls per launch; longer lists take several launches
-constexpr uint32_t kSpinLimit = 1u << 14;   // attempts of up to 100 us each (mbarriers) or 32-64 ns polls x 32 (counters)
+constexpr uint32_t kSpinLimit = 1u << 14;   // attempts of up to 100 us each (mbarriers) or polls x 64 (counters)
 
-// Shared memory of a CTA.
+// Shared memory of a CTA: mbarriers and notes, the sums on their way through the CTA, then the ring.
 constexpr int kSmFull = 0, kSmEmpty = 128;  // mbarriers: a stage's weights and x have landed; it is free again
 constexpr int kSmHeld = 256;                // uint32[2][kBars]: ring bytes of each stage in the ring, as each producer warp noted them
-constexpr int kSmArgVal = 512;              // float[4][32]: best value per column warp and token
-constexpr int kSmArgIdx = 512 + 512;        // int[4][32]: and its channel
-constexpr int kSmRed = 1536;                // 4 KiB: 8 accumulators per lane handed from warps ck = 1 to warps ck = 0
-constexpr int kSmRing = kSmRed + 4096;
-constexpr int kSmemBytes = (228 * 1024 / kOcc - 1024) / 128 * 128;   // an SM's shared memory less the runtime's 1 KiB per CTA
-constexpr int kRingBytes = kSmemBytes - kSmRing;
-static_assert(kSmRing % 128 == 0 && kRingBytes % 128 == 0, "stages are 128-byte aligned");
+constexpr int kSmDead = 384;                // int: a wait on a stage gave up; nobody in this CTA waits for the ring any more
+constexpr int kSmStages = 512;              // Stage[kBars]: what the weight warp tells the consumers about each stage
+constexpr int kSmSums = 1024;               // float[k groups x matrices][tokens][kSumStride]
+constexpr int kSumStride = 132;             // floats from one token's 128 channels to the next: 4 past 128, so that the fragment stores meet no bank twice
+constexpr int sums_bytes(int tg) { return 4 * 8 * tg * kSumStride * 4; }
+constexpr int kSmemBytes = 227 * 1024;
 
 // Scratch layout (byte offsets into the caller's workspace). Two matmuls of a queue may be in flight at once, so
 // what a matmul uses while it runs exists twice (a set for even and one for odd positions in the queue).
@@ -73,7 +70,7 @@ constexpr size_t kSetPanelsDone = 0;                             // int: sub-pan
 constexpr size_t kSetKeys = 256;                                 // u64[32]: per token the best (value, column) so far (argmax epilogue)
 constexpr size_t kSetCounters = 512;                             // int[kMaxSubPanels]: CTAs arrived at a sub-panel
 constexpr size_t kSetPartials = kSetCounters + 4 * kMaxSubPanels;
-constexpr size_t kSlotFloatsMax = 8 * 32 * 32;                   // 8 warps x up to 32 accumulators x 32 lanes
+constexpr size_t kSlotFloatsMax = 32 * 2 * 128;                  // 32 tokens x up to two matrices x 128 channels
 constexpr size_t kSetBytes = kSetPartials + (size_t)kMaxCtas * kSlotFloatsMax * 4;
 constexpr int kSets = 2;                                         // matmuls of a queue in flight at most
 constexpr size_t kWsBytes = kWsSets + kSets * kSetBytes;
@@ -85,26 +82,28 @@ struct Geometry {
   int ups;       // units (tile rows) per stage
   int matrix;    // bytes of one matrix's part of a stage
   int w_bytes;   // all weights of a stage; the x tiles follow
-  int xb;        // bytes of an x tile staged: its first half (token rows 0-15) or all of it
+  int xb;        // bytes of an x tile staged: token rows 0-7, 0-15 or all
   int stage;     // bytes of a stage
 };
-__host__ __device__ constexpr int stage_rows_per_warp(int fmt, int tg) { return tg == 1 && fmt == BT_BFP4 ? 4 : 2; }
+// Large stages: a stage costs its waits, arrivals and copies whatever its size, about 430 cycles of a warp's time on an
+// 8192 x 28672 matmul, and a ring of three or four stages of 35-55 KB is enough to cover the latency of HBM.
+__host__ __device__ constexpr int stage_rows_per_warp(int fmt, int tg) { return fmt == BT_BFP4 && tg < 4 ? 4 : 2; }
 __host__ __device__ constexpr Geometry geometry(int fmt, bool pair, int tg) {
   Geometry g{};
   g.tb = tile_bytes(fmt), g.t = stage_rows_per_warp(fmt, tg);
-  g.ups = pair ? g.t : 2 * g.t;
+  g.ups = (pair ? 2 : 4) * g.t;
   g.matrix = g.ups * kWC * g.tb;
   g.w_bytes = (pair ? 2 : 1) * g.matrix;
-  g.xb = tg == 4 ? 2048 : 1024;
+  g.xb = 512 * tg;
   g.stage = g.w_bytes + g.ups * g.xb;
   return g;
 }
-static_assert(geometry(BT_BFP8, false, 1).stage % 128 == 0 && geometry(BT_BFP4, false, 4).stage % 128 == 0 && geometry(BT_BFP4, true, 4).stage % 128 == 0,
-              "stages keep the ring 128-byte aligned");
+static_assert(geometry(BT_BFP8, false, 1).w_bytes % 128 == 0 && geometry(BT_BFP4, false, 1).w_bytes % 128 == 0 && geometry(BT_BFP4, true, 4).w_bytes % 128 == 0,
+              "x tiles land on 128-byte boundaries");
 
 // One matmul of the queue, as the kernel sees it.
-struct GemvParams {
-  const uint8_t *x;
+struct alignas(64) GemvParams {
+  CUtensorMap xmap;           // x as (16-datum face rows of the staged tokens, faces, tile columns)
   const uint8_t *w[2];
   const uint16_t *add;
   void *out;
@@ -115,8 +114,22 @@ struct GemvParams {
   int fmt, pair, tg;
   int wait_for;               // the matmul of the launch that must be complete before this one starts; -1: none
   int turn;                   // CTA c takes the unit range (c + turn) % CTAs
-  int per;                    // units per range when ranges are cut to fit the sub-panels; 0: equal shares of all CTAs
+  int units;                  // tile rows of all sub-panels
+  int active;                 // CTAs with a range; range b starts at b * share + min(b, extra), the last one ends at units
+  int share, extra;
 };
+
+// Waits for a phase of a stage's mbarrier, with a limit. A wait that gives up marks the CTA: its sums are worthless from
+// there on (the error word says so), but every warp still goes through all of its pieces and barriers, without waiting
+// for the ring, so that the CTA ends.
+__device__ __forceinline__ bool stage_wait(uint32_t smem, uint32_t bar, uint32_t parity, int *error) {
+  if (mbar_try_wait(bar, parity, 100000u)) return true;
+  for (uint32_t i = 0; i < 2 * kSpinLimit && lds32(smem + kSmDead) == 0; i++)
+    if (mbar_try_wait(bar, parity, 100000u)) return true;
+  sts32(smem + kSmDead, 1);
+  atomicExch(error, 2);
+  return false;
+}
 
 // What a matmul uses while it runs: the count of finished sub-panels and the per-token best keys (argmax), the
 // arrivals per sub-panel (all zero before first use; the kernel leaves them zero) and one slot of partial sums per CTA.
@@ -129,195 +142,213 @@ struct Scratch {
 // What one launch gets: the matmuls and the scratch they share: a wait-gave-up flag, the counts of CTAs that
 // finished each matmul (zero before first use; the kernel leaves them zero) and one or two sets of running scratch.
 struct Queue {
+  GemvParams op[kQueueMax];
   int n;
   int sets;                   // kSets: matmuls take the sets in turn, and as many may be in flight; 1: one after the other
   int *error, *ops_done;
   Scratch set[kSets];
   int slot_floats;            // floats between two CTAs' slots of partial sums
-  GemvParams op[kQueueMax];
+  int ring;                   // where the ring starts in shared memory
+  int ring_bytes;
 };
 
+// A stage as the consumers see it, written by the weight warp ahead of its arrival on the stage's barrier: where a warp
+// goes next is worked out once per CTA, not by 16 warps.
+struct alignas(32) Stage {
+  uint32_t at;                // shared-memory address of its weights; the x tiles follow the matmul's w_bytes further
+  int rows, width;            // tile rows, and tile columns of the sub-panel
+  int last;                   // 1: the CTA's part of the sub-panel ends with it; 3: and so does its part of the matmul
+  int sp, first, cta, end;    // the sub-panel, the first range that shares it, this CTA's and the last one, the owner
+};
+static_assert(sizeof(Stage) * kBars <= kSmSums - kSmStages, "room for the stages' notes");
 
-// Where range b of `ctas` starts: equal shares, or with `per` > 0 shares of exactly `per` units (the last one shorter).
-__host__ __device__ __forceinline__ long long range_start(long long units, int b, int ctas, int per) {
-  return per > 0 ? min((long long)b * per, units) : units * b / ctas;
-}
+__device__ __forceinline__ int range_start(const GemvParams &p, int b) { return min(b * p.share + min(b, p.extra), p.units); }
 // The CTA whose (non-empty) range holds unit u.
-__device__ __forceinline__ int cta_of(long long u, long long units, int ctas, int per) {
-  if (per > 0) return (int)(u / per);
-  int b = (int)(u * ctas / units);
-  while (b + 1 < ctas && range_start(units, b + 1, ctas, 0) <= u) b++;
-  while (b > 0 && range_start(units, b, ctas, 0) > u) b--;
-  return b;
+__device__ __forceinline__ int cta_of(const GemvParams &p, int u) {
+  const int longer = p.extra * (p.share + 1);
+  return u < longer ? u / (p.share + 1) : p.extra + (u - longer) / p.share;
 }
-
 // One weight tile times the staged x tile. `tile`, `ex` and `xs` are shared-memory addresses that already include
 // the lane's own offsets: tile = tile base + 16 * lane; ex = tile base + 16 * t, where the lane's exponents are;
 // xs = x tile base + 32 * g + 8 * t (g = lane / 4, t = lane % 4).
 //
 // A weight byte (offset binary, see stream_layout.cuh) zero-extended into a 16-bit lane is the bf16 number
 // byte * 2^-133, so a mask (bytes 0 and 2 of a word: the lane's first k pair) or a byte-permute (bytes 1 and 3: its
-// second pair) makes a register of two weights, and one packed fused multiply-add with the face row's power of two
-// s = 2^(e - 64) and with -offset * 2^-133 * s turns it into the exact signed weights times 2^(e - 197); the
-// epilogue multiplies the sums by 2^64. An all-zero run has e = 0: both products underflow to zero, as they should.
+// second pair) makes a register of two weights. A face (16 k x 16 n) is one MMA, rows g and g + 8 of it the channels 2g
+// and 2g + 1; acc[fs][tg] collects face column fs. A bfp4 byte holds two channels of the same k: the masked low
+// nibble is channel 2g, the masked high nibble, 16 times its code, channel 2g + 1.
 //
-// bfp8: a face (16 k x 16 n) is one MMA, rows g and g + 8 of it the channels 2g and 2g + 1; acc[fs][tg] collects
-// face column fs. bfp4: a byte holds two channels of the same k, low and high nibble. The whole byte as a weight,
-// 16 * high + low, goes into one MMA ("both", acc[0]), the masked low nibble into another ("low", acc[1]); rows g of
-// these MMAs are the byte of channels (2g, 2g + 1) of face column 0, rows g + 8 that of face column 1. When a
-// sub-panel's sums are complete, 16 * high = both - low (settle below; a nibble q is worth 16 q). Sixteen registers of weights per tile either
-// way, for half as many loaded bytes.
-constexpr uint32_t kByteLanes = 0x00FF00FFu, kNibbleLanes = 0x000F000Fu, kOddBytes = 0x4341u;
+// Where the face row's power of two goes depends on how many tokens share it. Up to 16 tokens (TG 1 and 2) it goes to
+// x: the MMA's two x registers per 8 tokens are multiplied by 2^(e - 127), exactly unless the product with a weight
+// of that run leaves bf16's range, and the four weight registers take one multiply-add with constants that makes
+// them the signed integers times 2^-6, whatever the run; the sums are the results themselves. With 32 tokens eight x
+// registers would need it per face and the weights only four, so there the weights carry it: one packed
+// multiply-add with s = 2^(e - 64) and with -offset * 2^-133 * s makes them the weights times 2^-64, which the epilogue
+// undoes. On shared-memory data alone, 16 warps, an SM does a tile in 23 (8 tokens), 32 (16) and 47-50 cycles
+// (32); weights that carry the scale take 24 / 27 (bfp8 / bfp4) for 8 tokens, and x that carries it 52 for 32, where
+// the MMAs themselves (about 10 cycles each per scheduler) are the bound. Subtracting the offset with a second MMA
+// instead of the multiply-adds was slower (26-28 cycles for 8 tokens) for the same reason.
+constexpr uint32_t kByteLanes = 0x00FF00FFu, kNibbleLanes = 0x000F000Fu, kHighLanes = 0x00F000F0u, kOddBytes = 0x4341u;
 constexpr uint32_t kMinus128 = 0x80808080u;   // two bf16 lanes of -128 * 2^-133 = -2^-126
-constexpr uint32_t kMinus136 = 0x80888088u;   // -(128 + 8) * 2^-133: offset of a byte made of two offset nibbles
 constexpr uint32_t kMinus8 = 0x80088008u;     // -8 * 2^-133
+constexpr uint32_t kTimes16 = 0x41804180u;
+constexpr uint32_t kTo6 = 0x7F007F00u, kHighTo6 = 0x7D007D00u;         // 2^127: code * 2^-133 to code * 2^-6; 2^123: the same for 16 * code
+constexpr uint32_t kOff128 = 0xC000C000u, kOff8 = 0xBE00BE00u;         // -128 * 2^-6 and -8 * 2^-6
+__host__ __device__ constexpr bool scale_on_x(int tg) { return tg <= 2; }
+// what turns the sums of a format and token group count into results (bfp4: a nibble q is worth 16 q)
+__host__ __device__ constexpr float unscale_of(int fmt, int tg) { return scale_on_x(tg) ? (fmt == BT_BFP4 ? 16.f : 1.f) : 18446744073709551616.f; }   // 2^64
 template <int FMT, int TG>
 __device__ __forceinline__ void tile_mma(uint32_t tile, uint32_t ex, uint32_t xs, float (&acc)[2][TG][4]) {
+  constexpr bool SX = TG <= 2;
   const uint4 ev = lds128(ex);
   const uint32_t ee[4] = {ev.x, ev.y, ev.z, ev.w};
   uint2 bx[2][TG];
 #pragma unroll
   for (int h = 0; h < 2; h++) {
 #pragma unroll
-    for (int tg = 0; tg < TG; tg++) bx[h][tg] = lds64(xs + (tg >> 1) * 1024 + h * 512 + (tg & 1) * 256);
+    for (int tg = 0; tg < TG; tg++) bx[h][tg] = lds64(xs + (TG == 1 ? h * 256 : (tg >> 1) * 1024 + h * 512 + (tg & 1) * 256));
   }
   uint4 wv[2];
-  if (FMT == BT_BFP8) wv[0] = lds128(tile + 64), wv[1] = lds128(tile + 64 + 512);
-  else wv[0] = lds128(tile + 64), wv[1] = wv[0];
-  uint32_t s[4][2];   // scales of face 2h + fs, first and second k pair
-#pragma unroll
-  for (int f = 0; f < 4; f++) s[f][0] = scale_pair<0>(ee[f]), s[f][1] = scale_pair<1>(ee[f]);
+  wv[0] = lds128(tile + 64);
+  if (FMT == BT_BFP8) wv[1] = lds128(tile + 64 + 512);
 #pragma unroll
   for (int h = 0; h < 2; h++) {
-    if (FMT == BT_BFP8) {
-#pragma unroll
-      for (int fs = 0; fs < 2; fs++) {
-        const int f = 2 * h + fs;
-        const uint32_t w0 = fs ? wv[h].z : wv[h].x, w1 = fs ? wv[h].w : wv[h].y;   // channels 2g and 2g + 1
-        const uint32_t n01 = mul_bf16x2(s[f][0], kMinus128), n23 = mul_bf16x2(s[f][1], kMinus128);
-        const uint32_t a0 = fma_bf16x2(w0 & kByteLanes, s[f][0], n01), a1 = fma_bf16x2(w1 & kByteLanes, s[f][0], n01);
-        const uint32_t a2 = fma_bf16x2(prmt(w0, 0u, kOddBytes), s[f][1], n23), a3 = fma_bf16x2(prmt(w1, 0u, kOddBytes), s[f][1], n23);
-#pragma unroll
-        for (int tg = 0; tg < TG; tg++) mma_bf16(acc[fs][tg], a0, a1, a2, a3, bx[h][tg].x, bx[h][tg].y);
-      }
-    } else {
-      const uint32_t w0 = h ? wv[0].z : wv[0].x, w1 = h ? wv[0].w : wv[0].y;       // face columns 0 and 1
-      const uint32_t b0 = w0 & kByteLanes, b1 = w1 & kByteLanes, b2 = prmt(w0, 0u, kOddBytes), b3 = prmt(w1, 0u, kOddBytes);
-      const uint32_t s0 = s[2 * h][0], s1 = s[2 * h + 1][0], s2 = s[2 * h][1], s3 = s[2 * h + 1][1];
-      {
-        const uint32_t a0 = fma_bf16x2(b0, s0, mul_bf16x2(s0, kMinus136)), a1 = fma_bf16x2(b1, s1, mul_bf16x2(s1, kMinus136));
-        const uint32_t a2 = fma_bf16x2(b2, s2, mul_bf16x2(s2, kMinus136)), a3 = fma_bf16x2(b3, s3, mul_bf16x2(s3, kMinus136));
-#pragma unroll
-        for (int tg = 0; tg < TG; tg++) mma_bf16(acc[0][tg], a0, a1, a2, a3, bx[h][tg].x, bx[h][tg].y);
-      }
-      {
-        const uint32_t a0 = fma_bf16x2(w0 & kNibbleLanes, s0, mul_bf16x2(s0, kMinus8)), a1 = fma_bf16x2(w1 & kNibbleLanes, s1, mul_bf16x2(s1, kMinus8));
-        const uint32_t a2 = fma_bf16x2(b2 & kNibbleLanes, s2, mul_bf16x2(s2, kMinus8)), a3 = fma_bf16x2(b3 & kNibbleLanes, s3, mul_bf16x2(s3, kMinus8));
-#pragma unroll
-        for (int tg = 0; tg < TG; tg++) mma_bf16(acc[1][tg], a0, a1, a2, a3, bx[h][tg].x, bx[h][tg].y);
-      }
-    }
-  }
-}
-
-// bfp4: from ("both", "low") sums to the arrangement the rest of the kernel uses, acc[face column][tg][j] for
-// channel 2g and [2 + j] for channel 2g + 1. "both" and "low" hold face column 0 in [0], [1] and face column 1 in
-// [2], [3]. Linear, so it may run on partial sums.
-template <int FMT, int TG>
-__device__ __forceinline__ void settle(float (&acc)[2][TG][4]) {
-  if (FMT != BT_BFP4) return;
-#pragma unroll
-  for (int tg = 0; tg < TG; tg++) {
-    float both[4], low[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) both[i] = acc[0][tg][i], low[i] = acc[1][tg][i];
 #pragma unroll
     for (int fs = 0; fs < 2; fs++) {
+      const uint32_t e = ee[2 * h + fs];
+      const uint32_t s01 = SX ? (e << 7) & 0x7F807F80u : scale_pair<0>(e), s23 = SX ? (e >> 1) & 0x7F807F80u : scale_pair<1>(e);
+      uint32_t a0, a1, a2, a3;
+      if (FMT == BT_BFP8) {
+        const uint32_t w0 = fs ? wv[h].z : wv[h].x, w1 = fs ? wv[h].w : wv[h].y;   // channels 2g and 2g + 1
+        const uint32_t m01 = SX ? kTo6 : s01, m23 = SX ? kTo6 : s23, n01 = SX ? kOff128 : mul_bf16x2(s01, kMinus128), n23 = SX ? kOff128 : mul_bf16x2(s23, kMinus128);
+        a0 = fma_bf16x2(w0 & kByteLanes, m01, n01), a1 = fma_bf16x2(w1 & kByteLanes, m01, n01);
+        a2 = fma_bf16x2(prmt(w0, 0u, kOddBytes), m23, n23), a3 = fma_bf16x2(prmt(w1, 0u, kOddBytes), m23, n23);
+      } else {
+        const uint32_t w = h ? (fs ? wv[0].w : wv[0].z) : (fs ? wv[0].y : wv[0].x), wo = w >> 8;
+        // a nibble q is worth 16 q: a high nibble stands in its byte at 16 times its code, a low one takes 16 times the factor
+        const uint32_t l01 = SX ? kTo6 : mul_bf16x2(s01, kTimes16), l23 = SX ? kTo6 : mul_bf16x2(s23, kTimes16);
+        const uint32_t h01 = SX ? kHighTo6 : s01, h23 = SX ? kHighTo6 : s23;
+        const uint32_t n01 = SX ? kOff8 : mul_bf16x2(l01, kMinus8), n23 = SX ? kOff8 : mul_bf16x2(l23, kMinus8);
+        a0 = fma_bf16x2(w & kNibbleLanes, l01, n01), a1 = fma_bf16x2(w & kHighLanes, h01, n01);
+        a2 = fma_bf16x2(wo & kNibbleLanes, l23, n23), a3 = fma_bf16x2(wo & kHighLanes, h23, n23);
+      }
 #pragma unroll
-      for (int j = 0; j < 2; j++) acc[fs][tg][j] = 16.f * low[2 * fs + j], acc[fs][tg][2 + j] = both[2 * fs + j] - low[2 * fs + j];
+      for (int tg = 0; tg < TG; tg++) {
+        const uint32_t b0 = SX ? mul_bf16x2(bx[h][tg].x, s01) : bx[h][tg].x, b1 = SX ? mul_bf16x2(bx[h][tg].y, s23) : bx[h][tg].y;
+        mma_bf16(acc[fs][tg], a0, a1, a2, a3, b0, b1);
+      }
     }
   }
 }
 
 __device__ __forceinline__ float silu(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 __device__ __forceinline__ uint32_t bf16_half_up(float v) { return (__float_as_uint(v) + 0x8000u) >> 16; }
-__device__ __forceinline__ float bf16_value(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
-// a beats b: larger value, or the same value at a lower column; -0 equals 0; a NaN never wins
-__device__ __forceinline__ bool beats(float av, int ai, float bv, int bi) { return av > bv || (av == bv && ai < bi); }
-// (value, column) as one number whose order is `beats`: larger value first, then the lower column. Zero is reserved
-// for "nothing yet"; no value maps to it, since a NaN is never offered and -inf maps to 0x007FFFFF in the upper half.
+// (value, column) as one number whose order is the pick's: larger value first, of equal values (-0 equals 0) the lower
+// column. Zero is "nothing": a NaN, which never wins, maps to it, and no other value does (-inf maps to 0x007FFFFF in
+// the upper half).
 __device__ __forceinline__ unsigned long long pick_key(float v, int column) {
+  if (v != v) return 0ull;
   uint32_t b = __float_as_uint(v == 0.f ? 0.f : v);
   b ^= b >> 31 ? 0xFFFFFFFFu : 0x80000000u;
   return (unsigned long long)b << 32 | (0xFFFFFFFFu - (uint32_t)column);
 }
 
-
-// The epilogue of one finished tile column. Lane (g, t) holds, for each channel group ng and token group tg,
-// tokens 8 tg + 2t + j (j = 0, 1) and channels 16 ng + 2g + {0, 1}: acc[ng][tg][j] and [2 + j].
-// For a gate/up pair `acc` holds the gate sums and `up` the up sums in the same arrangement.
-template <int TG, bool PAIR>
-__device__ __forceinline__ void finish_column(const GemvParams &p, const float (&acc)[2][TG][4], const float (&up)[2][TG][4], int col, int cc,
-                                              int lane, float *arg_v, int *arg_i) {
-  const int g = lane >> 2, t = lane & 3;
-  const float unscale = 18446744073709551616.f * p.alpha;  // 2^64: the weights entered the MMA scaled by 2^-64
-  float best_v[TG][2];
-  int best_i[TG][2];
+// ---- a sub-panel's end: the CTA's warps, then the CTAs that share it ---------------------------------------------
+// The warps have left their sums in shared memory, [k group][matrix][token][channel]. Every consumer thread takes
+// one pair of neighbouring channels and every eighth token, adds the k groups in order and either stores the sums
+// in the CTA's slot of partial sums (a contributor) or adds the contributors' slots in CTA order, so that results do
+// not depend on timing, and runs the epilogue (the sub-panel's owner). Elementwise over all 512 threads: one small
+// piece of code for every kind of matmul. It runs once per sub-panel on warps that have nothing else to do, so its time is its
+// chain of dependent instructions: no loops over the k groups, parameters fetched up front, loads in flight together (as
+// plain loops over groups, contributors and all 32 rows it took 3000-5000 cycles).
+struct Piece {
+  int sp;                  // the sub-panel
+  int first, last, me;     // the ranges that share it, and this CTA's
+  int toks;                // tokens whose sums are in shared memory: M rounded up to whole groups of 8
+};
+// One token's sums of the channel pair: the k groups of one matrix, or of gate and up, added in order.
+__device__ __forceinline__ void sum_groups(const float *sums, bool pair, int toks, int tok, int pr, float2 &v, float2 &u) {
+  float2 s[4];
 #pragma unroll
-  for (int tg = 0; tg < TG; tg++) best_v[tg][0] = best_v[tg][1] = -INFINITY, best_i[tg][0] = best_i[tg][1] = 0x7FFFFFFF;
-#pragma unroll
-  for (int ng = 0; ng < 2; ng++) {
-#pragma unroll
-    for (int tg = 0; tg < 4; tg++) {
-      constexpr int kLast = TG - 1;
-      const int tgs = tg < TG ? tg : 0;  // a one-row result repeats across its tile: every row shows token 0
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
-        const int m = 8 * tg + 2 * t + j, at = ((m >> 4) * 2 + ng) * 256 + (m & 15) * 16 + 2 * g;
-        const bool valid = p.M == 1 || (tg <= kLast && m < p.M);
-        float v0 = acc[ng][tgs][j] * unscale, v1 = acc[ng][tgs][2 + j] * unscale;
-        if (p.add) {
-          const uint32_t a = *reinterpret_cast<const uint32_t *>(p.add + (size_t)col * 1024 + at);
-          v0 += bf16_value((uint16_t)a), v1 += bf16_value((uint16_t)(a >> 16));
-        }
-        if (p.epi == BT_EPI_RELU) v0 = fmaxf(v0, 0.f), v1 = fmaxf(v1, 0.f);
-        else if (p.epi == BT_EPI_SILU) v0 = silu(v0), v1 = silu(v1);
-        else if (PAIR) v0 = silu(v0) * (up[ng][tgs][j] * unscale), v1 = silu(v1) * (up[ng][tgs][2 + j] * unscale);
-        if (p.epi == BT_EPI_ARGMAX) {
-          if (tg <= kLast && m < p.M) {
-            const int n0 = col * 32 + 16 * ng + 2 * g;
-            if (beats(v0, n0, best_v[tgs][j], best_i[tgs][j])) best_v[tgs][j] = v0, best_i[tgs][j] = n0;
-            if (beats(v1, n0 + 1, best_v[tgs][j], best_i[tgs][j])) best_v[tgs][j] = v1, best_i[tgs][j] = n0 + 1;
-          }
-          continue;
-        }
-        if (p.out_fp32 == 2) {
-          // row-major fp32, only the rows there are: partial sums on their way to an all-reduce
-          if (tg <= kLast && m < p.M) *reinterpret_cast<float2 *>(static_cast<float *>(p.out) + (size_t)m * (p.TC * 32) + col * 32 + 16 * ng + 2 * g) = make_float2(v0, v1);
-          continue;
-        }
-        if (!valid) v0 = v1 = 0.f;
-        if (p.out_fp32) *reinterpret_cast<float2 *>(static_cast<float *>(p.out) + (size_t)col * 1024 + at) = make_float2(v0, v1);
-        else *reinterpret_cast<uint32_t *>(static_cast<uint16_t *>(p.out) + (size_t)col * 1024 + at) = bf16_half_up(v0) | bf16_half_up(v1) << 16;
-      }
-    }
+  for (int j = 0; j < 4; j++) s[j] = *reinterpret_cast<const float2 *>(sums + (j * toks + tok) * kSumStride + 2 * pr);
+  u = make_float2(s[1].x + s[3].x, s[1].y + s[3].y);
+  v = make_float2(s[0].x + s[2].x, s[0].y + s[2].y);
+  if (!pair) v.x += u.x, v.y += u.y;
+}
+__device__ __forceinline__ void contribute(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc) {
+  const int pr = threadIdx.x & 63, M = p.M;
+  const bool pair = p.pair;
+  float *slot = sc.partials + (size_t)pc.me * slot_floats + 2 * pr;
+  for (int tok = threadIdx.x >> 6; tok < M; tok += kConsumers / 64) {
+    float2 v, u;
+    sum_groups(sums, pair, pc.toks, tok, pr, v, u);
+    float2 *to = reinterpret_cast<float2 *>(slot + (pair ? 2 * tok : tok) * 128);
+    *to = v;
+    if (pair) to[64] = u;
   }
-  if (p.epi == BT_EPI_ARGMAX) {
-    // best over this column's 32 channels: combine the lanes that hold the same tokens (same t)
+}
+// The rows past M of an owner's tiles are zeros; they need no sums, so the messenger writes them while it waits.
+__device__ __forceinline__ void zero_rows(const GemvParams &p, int sp) {
+  const int M = p.M, lane = threadIdx.x & 31;
+  if (M == 1 || p.epi == BT_EPI_ARGMAX || p.out_fp32 == 2) return;
+  const int per_row = p.out_fp32 ? 4 : 2, first = sp * kWC;                         // 16-byte words of a face row
+  for (int face = 0; face < 4 * min(kWC, p.TC - first); face++) {                   // two lower and two upper faces of each tile
+    uint4 *rows = static_cast<uint4 *>(p.out) + ((size_t)first * 4 + face) * 16 * per_row;
+    for (int i = max(M - (face & 2) * 8, 0) * per_row + lane; i < 16 * per_row; i += 32) rows[i] = make_uint4(0, 0, 0, 0);
+  }
+}
+__device__ __forceinline__ void finish(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc) {
+  const int pr = threadIdx.x & 63, M = p.M, epi = p.epi, fp32 = p.out_fp32, first = pc.first, last = pc.last;
+  const bool pair = p.pair;
+  const int tcol = pc.sp * kWC + (pr >> 4), n0 = pc.sp * kWC * 32 + 2 * pr;           // tile column and first channel of the pair
+  const bool inside = tcol < p.TC;
+  const float unscale = unscale_of(p.fmt, p.tg) * p.alpha;
+  const uint16_t *add = p.add;
+  char *out = static_cast<char *>(p.out);
+  // a one-row result repeats across its tile: each of the eight groups of 64 threads works it out and writes four rows
+  for (int row = threadIdx.x >> 6; row < (M == 1 && epi != BT_EPI_ARGMAX ? kConsumers / 64 : M); row += kConsumers / 64) {
+    const int tok = M == 1 ? 0 : row;
+    const int at = tcol * 1024 + ((row >> 4) * 2 + ((pr >> 3) & 1)) * 256 + (row & 15) * 16 + (2 * pr & 15);
+    float2 v, u;
+    // everything that comes from L2 in flight together: the addend and the contributors' sums, four at a time
+    uint32_t a = 0;
+    if (add && inside) a = *reinterpret_cast<const uint32_t *>(add + at);
+    const float *slots = sc.partials + (size_t)first * slot_floats + (pair ? 2 * tok : tok) * 128 + 2 * pr;
+    float2 w[4], x[4];
+    for (int c0 = first, once = 1; once || c0 < last; c0 += 4, once = 0, slots += 4 * (size_t)slot_floats) {
 #pragma unroll
-    for (int tg = 0; tg < 4; tg++) {
+      for (int j = 0; j < 4; j++) {
+        w[j] = x[j] = make_float2(0.f, 0.f);
+        if (c0 + j < last) w[j] = __ldcg(reinterpret_cast<const float2 *>(slots + (size_t)j * slot_floats));
+        if (pair && c0 + j < last) x[j] = __ldcg(reinterpret_cast<const float2 *>(slots + (size_t)j * slot_floats + 128));
+      }
+      if (once) sum_groups(sums, pair, pc.toks, tok, pr, v, u);
 #pragma unroll
-      for (int j = 0; j < 2; j++) {
-        float v = -INFINITY;
-        int i = 0x7FFFFFFF;
-        if (tg < TG) v = best_v[tg < TG ? tg : 0][j], i = best_i[tg < TG ? tg : 0][j];
+      for (int j = 0; j < 4; j++) v.x += w[j].x, v.y += w[j].y, u.x += x[j].x, u.y += x[j].y;
+    }
+    v.x = v.x * unscale + __uint_as_float(a << 16), v.y = v.y * unscale + __uint_as_float(a & 0xFFFF0000u);
+    if (epi == BT_EPI_RELU) v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f);
+    if (epi == BT_EPI_SILU || pair) v.x = silu(v.x), v.y = silu(v.y);
+    if (pair) v.x *= u.x * unscale, v.y *= u.y * unscale;
+    if (epi == BT_EPI_ARGMAX) {
+      unsigned long long key = inside ? max(pick_key(v.x, n0), pick_key(v.y, n0 + 1)) : 0ull;
 #pragma unroll
-        for (int d = 4; d < 32; d <<= 1) {
-          const float ov = __shfl_xor_sync(0xFFFFFFFFu, v, d);
-          const int oi = __shfl_xor_sync(0xFFFFFFFFu, i, d);
-          if (beats(ov, oi, v, i)) v = ov, i = oi;
-        }
-        if (g == 0) arg_v[cc * 32 + 8 * tg + 2 * t + j] = v, arg_i[cc * 32 + 8 * tg + 2 * t + j] = i;
+      for (int d = 1; d < 32; d <<= 1) key = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, d));
+      // a maximum over all sub-panels whatever the order they finish in, so the last one to finish has the answer at hand
+      if ((threadIdx.x & 31) == 0 && key) atomicMax(sc.keys + row, key);
+    } else if (inside) {
+      const uint32_t both = bf16_half_up(v.x) | bf16_half_up(v.y) << 16;
+      // row-major fp32, only the rows there are: partial sums on their way to an all-reduce
+      if (fp32 == 2) {
+        if (row < M) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + n0)) = v;
+      } else {
+#pragma unroll
+        for (int r = 0; r < 4; r++)                                                   // rows row, + 8, + 16, + 24 of a one-row result
+          if (r == 0 || M == 1) {
+            const size_t to = at + (r >> 1) * 512 + (r & 1) * 128;
+            if (fp32) *reinterpret_cast<float2 *>(out + 4 * to) = v;
+            else *reinterpret_cast<uint32_t *>(out + 2 * to) = both;
+          }
       }
     }
   }
@@ -327,375 +358,277 @@ __device__ __forceinline__ void finish_column(const GemvParams &p, const float (
 // that holds its last tile row (its owner); the others hand it their partial sums through global memory. So a CTA
 // first takes the sub-panel its range ends in (it is that one's first contributor, and the owner will not need the
 // sums for a while), then the sub-panels it has whole, and last the sub-panel its range starts in, which it owns:
-// by then the other contributors have long signalled, or are finishing at the same moment.
-struct Segments {
-  long long a[3], b[3];
-  int n;
+// by then the other contributors have long signalled, or are finishing at the same moment. `walk` below goes through
+// these pieces sub-panel by sub-panel; everything is a scalar with a fixed place, so it lives in registers.
+struct Walk {
+  int KT, segs;                      // segments left, the one at hand included
+  int a, b, a1, b1, a2, b2;          // units [a, b) of this segment, and the segments after it
+  __device__ __forceinline__ void start(const GemvParams &p, int range) {
+    const int u0 = range_start(p, range), u1 = range_start(p, range + 1);
+    KT = p.KT, segs = 0;
+    a = b = a1 = b1 = a2 = b2 = 0;
+    const int head_end = min(u1, (u0 / KT + 1) * KT);                  // end of the sub-panel the range starts in
+    const bool head_partial = u0 % KT != 0 || head_end - u0 < KT;
+    const int tail_start = u1 / KT * KT;                               // start of the sub-panel the range ends in
+    const bool tail_partial = u1 % KT != 0 && tail_start >= head_end;  // a tail that is not the head itself
+    const int mid_a = head_partial ? head_end : u0, mid_b = tail_partial ? tail_start : u1;
+    if (head_partial) push(u0, head_end);
+    if (mid_b > mid_a) push(mid_a, mid_b);
+    if (tail_partial) push(tail_start, u1);
+  }
+  __device__ __forceinline__ void push(int from, int to) { a2 = a1, b2 = b1, a1 = a, b1 = b, a = from, b = to, segs++; }
+  __device__ __forceinline__ bool more() const { return segs > 0; }
+  // the next piece: up to the end of a sub-panel or of the segment
+  __device__ __forceinline__ void next(int &sp, int &kt, int &rows) {
+    sp = a / KT, kt = a - sp * KT, rows = min(KT - kt, b - a);
+    a += rows;
+    if (a == b) segs--, a = a1, b = b1, a1 = a2, b1 = b2;
+  }
 };
-__device__ __forceinline__ Segments segments_of(long long u0, long long u1, int KT) {
-  Segments s;
-  s.n = 0;
-  for (int i = 0; i < 3; i++) s.a[i] = s.b[i] = 0;
-  if (u0 >= u1) return s;
-  const long long head_end = min(u1, (u0 / KT + 1) * KT);            // end of the sub-panel the range starts in
-  const bool head_partial = u0 % KT != 0 || head_end - u0 < KT;
-  const long long tail_start = (u1 / KT) * KT;                       // start of the sub-panel the range ends in
-  const bool tail_partial = u1 % KT != 0 && tail_start >= head_end;  // a tail that is not the head itself
-  long long mid_a = head_partial ? head_end : u0, mid_b = tail_partial ? tail_start : u1;
-  if (tail_partial) s.a[s.n] = tail_start, s.b[s.n++] = u1;
-  if (mid_b > mid_a) s.a[s.n] = mid_a, s.b[s.n++] = mid_b;
-  if (head_partial) s.a[s.n] = u0, s.b[s.n++] = head_end;
-  return s;
-}
 
-// Where the next stage goes, kept in step by the three parties of a CTA: stages follow one another through the
-// ring's bytes (a stage that would run past the end starts over at 0) and through the kBars mbarrier pairs.
+// Where the next stage goes, kept in step by the two producers: stages follow one another through the ring's bytes (a
+// stage that would run past the end starts over at 0).
 struct Ring {
   uint32_t off;     // where the next stage would start
-  uint32_t bar;     // byte offset of its mbarriers among their kind: 8 * (stages so far % kBars)
-  uint32_t parity;  // the phase to wait for: (stages so far / kBars) & 1
-  __device__ __forceinline__ uint32_t place(uint32_t bytes) {       // byte offset of the next stage
-    if (off + bytes > kRingBytes) off = 0;
+  __device__ __forceinline__ uint32_t place(uint32_t bytes, uint32_t ring_bytes) {       // byte offset of the next stage
+    if (off + bytes > ring_bytes) off = 0;
     const uint32_t at = off;
     off += bytes;
     return at;
   }
-  __device__ __forceinline__ void advance() {
-    bar = (bar + 8) & (8 * kBars - 1);
-    if (bar == 0) parity ^= 1;
-  }
-};
-
-// A CTA's stages of one matmul, in order: sub-panel, first tile row and number of tile rows of each. Everything
-// is a scalar with a fixed place, so the walk lives in registers.
-struct Walk {
-  int KT, ups, segs;                       // segments left, this one included
-  int sp, kt, left;                        // where the next stage starts, and the tile rows left in this segment
-  int sp1, kt1, left1, sp2, kt2, left2;    // the segments after this one
-  __device__ __forceinline__ void start(const Segments &s, int kt_count, int units_per_stage) {
-    KT = kt_count, ups = units_per_stage, segs = s.n;
-    sp = (int)(s.a[0] / KT), kt = (int)(s.a[0] % KT), left = (int)(s.b[0] - s.a[0]);
-    sp1 = (int)(s.a[1] / KT), kt1 = (int)(s.a[1] % KT), left1 = (int)(s.b[1] - s.a[1]);
-    sp2 = (int)(s.a[2] / KT), kt2 = (int)(s.a[2] % KT), left2 = (int)(s.b[2] - s.a[2]);
-  }
-  __device__ __forceinline__ bool more() const { return segs > 0; }
-  __device__ __forceinline__ int rows() const { return min(min(ups, left), KT - kt); }
-  // past `n` tile rows that end at the sub-panel's end or at the segment's
-  __device__ __forceinline__ void skip(int n) { next(n); }
-  __device__ __forceinline__ void next(int n) {
-    left -= n, kt += n;
-    if (kt == KT) kt = 0, sp++;
-    if (left == 0) segs--, sp = sp1, kt = kt1, left = left1, sp1 = sp2, kt1 = kt2, left1 = left2;
-  }
 };
 
 // ---- producers: two warps walk the whole queue ---------------------------------------------------------------
-// Warp 8 copies weights, warp 9 copies x. Both follow the same stages through the ring and wait for the same room
+// One warp copies weights, the other x. Both follow the same stages through the ring and wait for the same room
 // (the oldest stage in the ring freed by the consumers), each keeping its own books, so neither waits for the other.
-// Weights never depend on an earlier matmul: their copies go out as soon as the ring has room, lane 0 announcing
-// the bytes and lanes 0 and 1 issuing one bulk copy per weight matrix. x is the result of an earlier matmul: the x
-// warp waits (with a limit) until every CTA has reported the matmuls it depends on finished, then copies each stage's
-// x tiles: whole with one bulk copy for more than 16 token rows, else the first half of each tile (token rows 0-15),
-// one copy per tile issued from as many lanes at once (an asynchronous copy costs its issuer some 250 cycles
-// whatever its size, which rules out copying row by row). While the x warp waits, the weight warp fills the ring.
+// Weights never depend on an earlier matmul: their copies go out as soon as the ring has room, one bulk copy per
+// weight matrix and stage. x is the result of an earlier matmul: the x warp waits (with a limit) until every CTA has
+// reported the matmuls it depends on finished, then copies each stage's x tiles with ONE tiled TMA copy, which picks
+// the token rows that are there out of every tile (8 rows: 256 bytes of each of two faces). An asynchronous copy costs
+// its issuer and the copy engine the same whatever its size: with two plain copies of 256 bytes per tile the x
+// warp alone held an 8192 x 28672 bfp4 matmul at 46 us, with one of 1 KB at 35, where the weights take 31.
+// x may be the result of the launch before this one, or of an earlier matmul of this one: the host has worked out the
+// last matmul this one must see finished, by every CTA. False: gave up.
+__device__ __forceinline__ bool await_turn(const Queue &q, const GemvParams &p, int ctas) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");     // returns when the previous launch is complete and visible
+  if (p.wait_for >= 0) {
+    uint32_t spins = 0;
+    while (ld_acquire_gpu(q.ops_done + p.wait_for) < ctas)
+      if (++spins > kSpinLimit * 64) return false;
+  }
+  return true;
+}
+
 template <bool WEIGHTS>
 __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t sbase, int cta, int ctas) {
-  const uint32_t full0 = sbase + kSmFull, empty0 = sbase + kSmEmpty, ring0 = sbase + kSmRing;
+  const uint32_t full0 = sbase + kSmFull, empty0 = sbase + kSmEmpty, ring0 = sbase + q.ring, ring_bytes = q.ring_bytes;
   volatile uint32_t *held = reinterpret_cast<volatile uint32_t *>(smem + kSmHeld) + (WEIGHTS ? 0 : kBars);   // ring bytes of each stage in the ring
   const int lane = threadIdx.x & 31;
-  Ring ring{0, 0, 0};
+  if (!WEIGHTS && lane < q.n) tensormap_prefetch(&q.op[lane].xmap);
+  Ring ring{0};
   uint32_t count = 0, oldest = 0, used = 0;   // stages placed; first stage not yet known to be free; ring bytes held from there on
   for (int i = 0; i < q.n; i++) {
     const GemvParams &p = q.op[i];
     const Geometry g = geometry(p.fmt, p.pair != 0, p.tg);
-    const int KT = p.KT, nw = p.pair ? 2 : 1;
-    const long long units = (long long)((p.TC + kWC - 1) / kWC) * KT;
-    const int active = p.per > 0 ? (int)((units + p.per - 1) / p.per) : (int)min((long long)ctas, units);   // the other ranges are empty
     const int me = (cta + p.turn) % ctas;                    // the range this CTA takes in this matmul
-    if (me >= active) continue;
-    Walk walk;
-    walk.start(segments_of(range_start(units, me, active, p.per), range_start(units, me + 1, active, p.per), KT), KT, g.ups);
+    if (me >= p.active) continue;
+    const int KT = p.KT, TC = p.TC, nw = p.pair ? 2 : 1;
     const uint8_t *w = p.w[lane < nw ? lane : 0];
+    Walk walk;
+    walk.start(p, me);
     bool gate = !WEIGHTS;                 // the x warp has yet to wait for the matmul before this one
-    for (int stage_no = 0; walk.more(); stage_no++) {
-      const int n = walk.rows(), sp = walk.sp, kt = walk.kt;
-      walk.next(n);
-      // room: the stage's bytes plus what is skipped when it starts over at the ring's beginning
-      const uint32_t need = g.stage + (ring.off + g.stage > kRingBytes ? kRingBytes - ring.off : 0);
-      for (uint32_t spins = 0; used + need > kRingBytes || count - oldest == kBars;) {
-        // looking in a loop rather than sleeping in the instruction: a sleeper is woken some hundreds of ns late, and
-        // this latency is on the ring's critical path; the two producer warps are 2 of 20, so the polls are cheap
-        int ok = 0;
-        if (lane == 0) ok = mbar_test(empty0 + 8 * (oldest % kBars), (oldest / kBars) & 1);
-        if (__shfl_sync(0xFFFFFFFFu, ok, 0)) {
+    while (walk.more()) {
+      int sp, kt, rows;
+      walk.next(sp, kt, rows);
+      const int width = min(kWC, TC - sp * kWC), ends = walk.more() ? 1 : 3;
+      const int first = WEIGHTS ? cta_of(p, sp * KT) : 0, end = WEIGHTS ? cta_of(p, (sp + 1) * KT - 1) : 0;
+      for (; rows > 0; rows -= g.ups, kt += g.ups) {
+        const int n = min(g.ups, rows);
+        // room: the stage's bytes plus what is skipped when it starts over at the ring's beginning
+        const uint32_t need = g.stage + (ring.off + g.stage > ring_bytes ? ring_bytes - ring.off : 0);
+        while (used + need > ring_bytes || count - oldest == kBars) {
+          // asleep in the instruction: a polling loop takes issue slots from the consumers, and the ring is deep enough to
+          // hide a late wake-up
+          if (!stage_wait(sbase, empty0 + 8 * (oldest % kBars), (oldest / kBars) & 1, q.error)) {
+            // the copies in flight land before the CTA may end (with a limit: some of these stages may never get their x)
+            for (; oldest != count; oldest++) mbar_wait(full0 + 8 * (oldest % kBars), (oldest / kBars) & 1, 100);
+            return;
+          }
           used -= held[oldest % kBars], oldest++;
-        } else if (++spins > kSpinLimit * 4096) {
-          if (lane == 0) atomicExch(q.error, 1);
-          break;
         }
-      }
-      const uint32_t b = count % kBars, stage = ring0 + ring.place(g.stage);
-      if (lane == 0) held[b] = need;
-      if (WEIGHTS) {
-        const int width = min(kWC, p.TC - sp * kWC);
-        const uint32_t bytes = n * width * g.tb;
-        if (lane == 0) mbar_expect_tx(full0 + 8 * b, nw * bytes);
-        __syncwarp();
-        if (lane < nw) bulk_g2s(stage + lane * g.matrix, w + ((size_t)sp * kWC * KT + (size_t)kt * width) * g.tb, bytes, full0 + 8 * b);
-      } else {
-        if (gate) {
-          // x may be the result of the launch before this one, or of an earlier matmul of this one: the host has
-          // worked out the last matmul this one must see finished, by every CTA
-          int ok = 1;
+        const uint32_t bar = full0 + 8 * (count % kBars), stage = ring0 + ring.place(g.stage, ring_bytes);
+        if (lane == 0) held[count % kBars] = need;
+        if (WEIGHTS) {
+          const uint32_t bytes = n * width * g.tb;
           if (lane == 0) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");     // returns when the previous launch is complete and visible
-            if (p.wait_for >= 0) {
-              uint32_t spins = 0;
-              while (ld_acquire_gpu(q.ops_done + p.wait_for) < ctas) {
-                if (++spins > kSpinLimit * 32) { ok = 0; break; }
-                __nanosleep(32);
-              }
-            }
+            uint4 *note = reinterpret_cast<uint4 *>(smem + kSmStages) + 2 * (count % kBars);
+            note[0] = make_uint4(stage, n, width, rows <= g.ups ? ends : 0), note[1] = make_uint4(sp, first, me, end);
+            mbar_expect_tx(bar, nw * bytes);
           }
-          if (!__shfl_sync(0xFFFFFFFFu, ok, 0) && lane == 0) atomicExch(q.error, 5);
-          // x was written with ordinary stores (by other CTAs of this launch, or by the launch before) and is about to
-          // be read by bulk copies: order what the acquire made visible before the asynchronous proxy's reads
-          fence_proxy_async();
-          gate = false;
-        }
-        if (p.tg == 4) {
-          if (lane == 0) {
-            mbar_expect_tx(full0 + 8 * b, n * 2048);
-            bulk_g2s(stage + g.w_bytes, p.x + (size_t)kt * 2048, n * 2048, full0 + 8 * b);
-          }
-        } else {
-          // up to 16 token rows: the first half of each x tile, one copy per tile from as many lanes
-          if (lane == 0) mbar_expect_tx(full0 + 8 * b, n * 1024);
           __syncwarp();
-          if (lane < n) bulk_g2s(stage + g.w_bytes + lane * 1024, p.x + (size_t)(kt + lane) * 2048, 1024, full0 + 8 * b);
-        }
-      }
-      used += need, count++;
-    }
-  }
-}
-
-// ---- consumers: one matmul of the queue -------------------------------------------------------------------------
-template <int FMT, int TG, bool PAIR>
-__device__ __forceinline__ void consume(const Queue &q, const GemvParams &p, const Scratch &sc, Ring &ring, uint8_t *smem, uint32_t sbase, int cta, int ctas) {
-  constexpr Geometry G = geometry(FMT, PAIR, TG);
-  constexpr int ACC = 8 * TG;                                  // accumulator floats per lane
-  const uint32_t full0 = sbase + kSmFull, empty0 = sbase + kSmEmpty;
-  float *arg_v = reinterpret_cast<float *>(smem + kSmArgVal);
-  int *arg_i = reinterpret_cast<int *>(smem + kSmArgIdx);
-  float *red = reinterpret_cast<float *>(smem + kSmRed);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ck = warp >> 2, cc = warp & 3, tl = lane & 3;
-  const int KT = p.KT, subpanels = (p.TC + kWC - 1) / kWC;
-  const long long units = (long long)subpanels * KT;
-  const int active = p.per > 0 ? (int)((units + p.per - 1) / p.per) : (int)min((long long)ctas, units);   // the other ranges are empty
-  // The ranges go round the CTAs from matmul to matmul: the CTAs that finish shared sub-panels have more to do than
-  // the others, and it should not be the same ones every time.
-  const int me = (cta + p.turn) % ctas;
-  if (me >= active) return;
-  Walk walk;
-  walk.start(segments_of(range_start(units, me, active, p.per), range_start(units, me + 1, active, p.per), KT), KT, G.ups);
-
-  float acc[2][TG][4];
-// accumulator i of the lane, with i a compile-time constant after unrolling, so that acc stays in registers
-#define ACC_OF(a, i) a[(i) / (4 * TG)][(i) / 4 % TG][(i) % 4]
-#pragma unroll
-  for (int i = 0; i < ACC; i++) ACC_OF(acc, i) = 0.f;
-
-  // shared-memory addresses of this lane's pieces, relative to a stage: its 16 bytes of a tile's values, its exponents
-  // and its rows of an x tile
-  const uint32_t matrix0 = sbase + kSmRing + (PAIR ? ck * G.matrix : 0);
-  const uint32_t lane_tile = matrix0 + lane * 16, lane_ex = matrix0 + tl * 16, lane_x = sbase + kSmRing + G.w_bytes + lane * 8;
-  const bool mine = PAIR || ck == 0;       // this warp holds sums when a sub-panel ends
-  const int slab = PAIR ? warp : cc;       // and this is their place in a slot of partial sums
-  bool first_stage = true;
-  int stage_no = 0;
-  const int TC = p.TC;
-  uint32_t slot = 0;
-  // A stage: find its place in the ring and wait for its weights and x; when done with it, free it.
-  auto stage_begin = [&]() {
-    slot = ring.place(G.stage);
-    if (!mbar_wait(full0 + ring.bar, ring.parity, kSpinLimit)) atomicExch(q.error, 2);
-    first_stage = false;
-  };
-  auto stage_end = [&]() {
-    __syncwarp();
-    mbar_arrive_if(empty0 + ring.bar, lane == 0);
-    ring.advance();
-    stage_no++;
-  };
-  while (walk.more()) {
-    // one piece: the rest of this sub-panel's share of the range, as whole stages and then what is left
-    const int sp = walk.sp, col = sp * kWC + cc, done_sp = sp, width = min(kWC, TC - sp * kWC);
-    int todo = min(walk.left, KT - walk.kt);
-    walk.skip(todo);
-    const bool last_stage = !walk.more();
-    {
-      if (width == kWC) {
-        // full stages of a full run: every offset is a compile-time constant
-        for (; todo >= G.ups; todo -= G.ups) {
-          stage_begin();
-#pragma unroll
-          for (int j = 0; j < G.t; j++) {
-            const uint32_t row = PAIR ? j : 2 * j + ck, o = slot + (row * kWC + cc) * G.tb;
-            tile_mma<FMT, TG>(lane_tile + o, lane_ex + o, lane_x + slot + row * G.xb, acc);
-          }
-          stage_end();
-        }
-      }
-      while (todo > 0) {
-        const int n = min(G.ups, todo);
-        todo -= n;
-        stage_begin();
-        if (col < TC) {
-#pragma unroll
-          for (int j = 0; j < G.t; j++) {
-            const int row = PAIR ? j : 2 * j + ck;
-            if (row < n) {
-              const uint32_t o = slot + (row * width + cc) * G.tb;
-              tile_mma<FMT, TG>(lane_tile + o, lane_ex + o, lane_x + slot + row * G.xb, acc);
-            }
-          }
-        }
-        stage_end();
-      }
-
-      // ---- this CTA is done with sub-panel done_sp: add the k halves, combine with other CTAs, run the epilogue ----
-      settle<FMT, TG>(acc);
-      if (!PAIR) {
-        // eight accumulators per lane at a time go through the 4 KiB buffer
-#pragma unroll
-        for (int r = 0; r < TG; r++) {
-          if (r > 0) named_barrier(1, kCW * 32);
-          if (ck == 1) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) red[(cc * 8 + i) * 32 + lane] = ACC_OF(acc, 8 * r + i);
-          }
-          named_barrier(1, kCW * 32);
-          if (ck == 0) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) ACC_OF(acc, 8 * r + i) += red[(cc * 8 + i) * 32 + lane];
-          }
-        }
-      }
-      const int first = cta_of((long long)done_sp * KT, units, active, p.per), last = cta_of((long long)(done_sp + 1) * KT - 1, units, active, p.per);
-      const bool finish = me == last;         // the owner finishes the sub-panel; the others only contribute
-      if (first != last) {
-        int *counter = sc.counters + done_sp;
-        if (!finish) {
-          // a contributor has one shared sub-panel that it does not own, so one slot per CTA is enough
-          if (mine) {
-            float4 *slot = reinterpret_cast<float4 *>(sc.partials + (size_t)me * q.slot_floats) + (size_t)slab * (ACC / 4) * 32;
-#pragma unroll
-            for (int i = 0; i < ACC / 4; i++)
-              slot[i * 32 + lane] = make_float4(ACC_OF(acc, 4 * i), ACC_OF(acc, 4 * i + 1), ACC_OF(acc, 4 * i + 2), ACC_OF(acc, 4 * i + 3));
-          }
-          // the barrier orders every warp's stores before thread 0's fence, which releases them with the count
-          named_barrier(1, kCW * 32);
-          if (threadIdx.x == 0) {
-            fence_gpu();
-            atomicAdd(counter, 1);
-          }
+          if (lane < nw) bulk_g2s(stage + lane * g.matrix, w + ((size_t)sp * kWC * KT + (size_t)kt * width) * g.tb, bytes, bar);
         } else {
-          // wait, with a limit, until the last - first other contributors have signalled
-          if (threadIdx.x == 0) {
-            uint32_t spins = 0;
-            while (*reinterpret_cast<volatile int *>(counter) < last - first) {
-              if (++spins > kSpinLimit * 32) { atomicExch(q.error, 3); break; }
-              __nanosleep(64);
-            }
-            *counter = 0;                      // ready for the next matmul
-            fence_gpu();                       // what follows the barrier, in any warp, sees the contributors' sums
+          if (gate) {
+            int ok = 1;
+            if (lane == 0) ok = await_turn(q, p, ctas);
+            if (!__shfl_sync(0xFFFFFFFFu, ok, 0) && lane == 0) atomicExch(q.error, 5);
+            // x was written with ordinary stores (by other CTAs of this launch, or by the launch before) and is about to
+            // be read by TMA copies: order what the acquire made visible before the asynchronous proxy's reads
+            fence_proxy_async();
+            gate = false;
           }
-          named_barrier(1, kCW * 32);
-          if (mine) {
-            // this CTA's own sums first, then the others' in CTA order: the result does not depend on timing
-            constexpr int BATCH = ACC <= 8 ? 5 : ACC <= 16 ? 3 : 2;   // contributors whose loads are in flight together
-            for (int c0 = first; c0 < last; c0 += BATCH) {
-              float4 v[BATCH][ACC / 4];
-#pragma unroll
-              for (int j = 0; j < BATCH; j++) {
-                const float4 *slot = reinterpret_cast<const float4 *>(sc.partials + (size_t)(c0 + j) * q.slot_floats) + (size_t)slab * (ACC / 4) * 32;
-#pragma unroll
-                for (int i = 0; i < ACC / 4; i++) v[j][i] = c0 + j < last ? __ldcg(slot + i * 32 + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-              }
-#pragma unroll
-              for (int j = 0; j < BATCH; j++) {
-#pragma unroll
-                for (int i = 0; i < ACC / 4; i++)
-                  ACC_OF(acc, 4 * i) += v[j][i].x, ACC_OF(acc, 4 * i + 1) += v[j][i].y, ACC_OF(acc, 4 * i + 2) += v[j][i].z, ACC_OF(acc, 4 * i + 3) += v[j][i].w;
-              }
-            }
+          // always a whole stage's box: tile columns past K come as zeros, those past the piece are not looked at
+          if (lane == 0) {
+            mbar_expect_tx(bar, g.ups * g.xb);
+            tma_load_3d(stage + g.w_bytes, &p.xmap, 0, 0, kt, bar);
           }
         }
+        __syncwarp();
+        used += need, count++;
       }
-      if (finish) {
-        if (PAIR) {
-          // the up warp hands its sums to the gate warp of the same column
-          float up[2][TG][4];
-#pragma unroll
-          for (int r = 0; r < TG; r++) {        // eight accumulators per lane at a time
-            if (r > 0) named_barrier(1, kCW * 32);
-            if (ck == 1) {
-#pragma unroll
-              for (int i = 0; i < 8; i++) red[(cc * 8 + i) * 32 + lane] = ACC_OF(acc, 8 * r + i);
-            }
-            named_barrier(1, kCW * 32);
-#pragma unroll
-            for (int i = 0; i < 8; i++) ACC_OF(up, 8 * r + i) = red[(cc * 8 + i) * 32 + lane];
-          }
-          if (ck == 0 && col < TC) finish_column<TG, true>(p, acc, up, col, cc, lane, arg_v, arg_i);
-        } else if (ck == 0 && col < TC) {
-          finish_column<TG, false>(p, acc, acc, col, cc, lane, arg_v, arg_i);
-        }
-        if (!PAIR && p.epi == BT_EPI_ARGMAX) {
-          // the sub-panel's best per token, then, in the last sub-panel to finish, the best over all sub-panels in order
-          named_barrier(1, kCW * 32);
-          const int wcols = min(kWC, TC - done_sp * kWC);
-          if (warp == 0) {
-            float v = arg_v[lane];
-            int i = arg_i[lane];
-            for (int c = 1; c < wcols; c++)
-              if (beats(arg_v[c * 32 + lane], arg_i[c * 32 + lane], v, i)) v = arg_v[c * 32 + lane], i = arg_i[c * 32 + lane];
-            // offer it to the token's key: a maximum over all sub-panels whatever the order they finish in, so the last
-            // one to finish has the answer at hand instead of a pass over every sub-panel's candidates
-            if (lane < p.M && i != 0x7FFFFFFF) atomicMax(sc.keys + lane, pick_key(v, i));
-            __syncwarp();
-            int is_last = 0;
-            if (lane == 0) {
-              fence_gpu();
-              is_last = atomicAdd(sc.panels_done, 1) == subpanels - 1;
-            }
-            is_last = __shfl_sync(0xFFFFFFFFu, is_last, 0);
-            if (is_last) {
-              // turns the keys into the answer and leaves the scratch as it found it
-              fence_gpu();
-              if (lane < p.M) {
-                const unsigned long long key = atomicExch(sc.keys + lane, 0ull);
-                uint32_t b = (uint32_t)(key >> 32);
-                b ^= b >> 31 ? 0x80000000u : 0xFFFFFFFFu;
-                p.arg_val[lane] = key ? __uint_as_float(b) : -INFINITY;
-                p.arg_idx[lane] = (key ? (int)(0xFFFFFFFFu - (uint32_t)key) : 0x7FFFFFFF) + p.arg_base;
-              }
-              if (lane == 0) *sc.panels_done = 0;
-            }
-          }
-        }
-      }
-      // the next sub-panel must not overwrite `red` or the argmax staging while a slower warp still reads them
-      named_barrier(1, kCW * 32);
-#pragma unroll
-      for (int i = 0; i < ACC; i++) ACC_OF(acc, i) = 0.f;
     }
   }
-#undef ACC_OF
 }
 
-__global__ void __launch_bounds__(kThreads, kOcc) gemv_queue_kernel(const __grid_constant__ Queue q) {
+// ---- consumers --------------------------------------------------------------------------------------------------
+// A warp's part of one piece: `rows` tile rows of a sub-panel, of which the warp takes every `groups`-th from `ck` on in
+// one column, stage by stage; then its sums go to shared memory. What does not depend on the format and the token
+// count lives in the kernel itself, once, where the matmul's parameters are read from the constant bank (passed on by
+// reference they were fetched through global memory, and a sub-panel's end took 4-6 us).
+struct Place {
+  uint32_t smem;                     // shared memory
+  uint32_t bar, parity;              // the next stage's mbarriers (8 * its number among kBars) and their phase
+  int cc, ck, mat, groups;           // this warp's column, first tile row, weight matrix; warps that share a column
+  int lane;
+};
+template <int FMT, int TG>
+__device__ __forceinline__ uint4 stream_rows(Place &w, float *sums, int *error) {
+  constexpr int TB = tile_bytes(FMT), T = stage_rows_per_warp(FMT, TG), XB = 512 * TG;
+  const int lane = w.lane, groups = w.groups, ck = w.ck, cc = w.cc;
+  const uint32_t x_step = groups * XB, x0 = 4 * T * kWC * TB + ck * XB + lane * 8, matrix0 = w.mat * (groups * T * kWC * TB);
+  float acc[2][TG][4];
+#pragma unroll
+  for (int i = 0; i < 8 * TG; i++) acc[i / (4 * TG)][i / 4 % TG][i % 4] = 0.f;
+  uint4 piece = make_uint4(0, 0, 0, 0);
+  for (int last = 0; !last;) {
+    if (!stage_wait(w.smem, w.smem + kSmFull + w.bar, w.parity, error)) break;
+    const uint4 stage = lds128(w.smem + kSmStages + 4 * w.bar);        // at, rows, width, last
+    const int width = stage.z;
+    uint32_t tile = stage.x + matrix0 + (ck * width + cc) * TB, xs = stage.x + x0;
+    const uint32_t tile_step = groups * width * TB;
+    last = stage.w;
+    if (last) piece = lds128(w.smem + kSmStages + 4 * w.bar + 16), piece.x |= (uint32_t)last << 30;
+    if (cc < width) {
+      if ((int)stage.y == groups * T) {
+#pragma unroll
+        for (int j = 0; j < T; j++, tile += tile_step, xs += x_step) tile_mma<FMT, TG>(tile + lane * 16, tile + (lane & 3) * 16, xs, acc);
+      } else {
+#pragma unroll 1
+        for (int row = ck; row < (int)stage.y; row += groups, tile += tile_step, xs += x_step) tile_mma<FMT, TG>(tile + lane * 16, tile + (lane & 3) * 16, xs, acc);
+      }
+    }
+    __syncwarp();
+    mbar_arrive_if(w.smem + kSmEmpty + w.bar, lane == 0);
+    w.bar = (w.bar + 8) & (8 * kBars - 1);
+    if (w.bar == 0) w.parity ^= 1;
+  }
+  // fragments to [k group][matrix][token][channel]: lane (g, t) holds tokens 8 tg + 2 t + j and channels 16 fs + 2 g + {0, 1}
+  const int t = lane & 3, g = lane >> 2;
+  float *to = sums + ((ck * (4 / groups) + w.mat) * 8 * TG + 2 * t) * kSumStride + cc * 32 + 2 * g;
+#pragma unroll
+  for (int fs = 0; fs < 2; fs++)
+#pragma unroll
+    for (int tg = 0; tg < TG; tg++)
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+        *reinterpret_cast<float2 *>(to + (8 * tg + j) * kSumStride + 16 * fs) = make_float2(acc[fs][tg][j], acc[fs][tg][2 + j]);
+  return piece;
+}
+
+// ---- the messenger: one warp tells other CTAs and hears from them ------------------------------------------------
+// It goes through the CTA's pieces beside the consumers and meets them at two barriers: the first it reaches when, for a
+// sub-panel this CTA owns, every contributor has signalled (a wait with a limit); after the second the consumers have
+// stored what they had, and it signals. A release takes 1000 to 3000 cycles under load; a consumer warp that did it
+// was that much behind the others at the next barrier.
+__device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
+  const int lane = threadIdx.x & 31;
+  for (int i = 0; i < q.n; i++) {
+    const GemvParams &p = q.op[i];
+    const Scratch &sc = q.set[i % q.sets];
+    const int me = (cta + p.turn) % ctas, M = p.M;
+    Walk walk{};
+    if (me < p.active) {
+      walk.start(p, me);
+      // the counters and the result are this matmul's only when the ones before it that it must not overtake are done
+      if (lane == 0 && !await_turn(q, p, ctas)) atomicExch(q.error, 5);
+      __syncwarp();
+    }
+    while (walk.more()) {
+      int sp, kt, rows;
+      walk.next(sp, kt, rows);
+      const int first = cta_of(p, sp * p.KT), last = cta_of(p, (sp + 1) * p.KT - 1);
+      int *counter = sc.counters + sp;
+      if (me == last) zero_rows(p, sp);
+      if (me == last && first != last && lane == 0) {
+        uint32_t spins = 0;
+        while (ld_acquire_gpu(counter) < last - first) {
+          if (++spins > kSpinLimit * 32) { atomicExch(q.error, 3); break; }
+          __nanosleep(40);
+        }
+        *counter = 0;                          // ready for the next matmul
+      }
+      __syncwarp();
+      named_barrier(1, kConsumers + 32);
+      named_barrier(2, kConsumers + 32);
+      if (me != last) {
+        if (lane == 0) red_release_gpu(counter, 1);
+      } else if (p.epi == BT_EPI_ARGMAX) {
+        // the last sub-panel to finish turns the keys into the answer and leaves the scratch as it found it
+        int is_last = 0;
+        if (lane == 0) {
+          fence_gpu();
+          is_last = atomicAdd(sc.panels_done, 1) == (p.TC + kWC - 1) / kWC - 1;
+        }
+        if (__shfl_sync(0xFFFFFFFFu, is_last, 0)) {
+          fence_gpu();
+          if (lane < M) {
+            const unsigned long long key = atomicExch(sc.keys + lane, 0ull);
+            uint32_t b = (uint32_t)(key >> 32);
+            b ^= b >> 31 ? 0x80000000u : 0xFFFFFFFFu;
+            p.arg_val[lane] = key ? __uint_as_float(b) : -INFINITY;
+            p.arg_idx[lane] = (key ? (int)(0xFFFFFFFFu - (uint32_t)key) : 0x7FFFFFFF) + p.arg_base;
+          }
+          if (lane == 0) *sc.panels_done = 0;
+        }
+        __syncwarp();
+      }
+    }
+    // Report this CTA done with matmul i: its results and partial sums are visible to the whole GPU before the count
+    // moves. A CTA without work in a matmul reports at once, which is harmless: the count of matmul i is complete only
+    // when the CTAs that do have work got their x, that is when matmul i - 1 was complete. The last report of the last
+    // matmul finds every producer past its last look at the counts, and zeroes them for the next launch. The counts are
+    // shared with the launch before this one, which may still be running (this launch may start early): a CTA without
+    // work in the first matmul must not report before that launch is complete.
+    if (lane == 0) {
+      fence_gpu();
+      if (i == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (atomicAdd(q.ops_done + i, 1) == ctas - 1 && i == q.n - 1)
+        for (int j = 0; j < q.n; j++) q.ops_done[j] = 0;
+    }
+    __syncwarp();
+  }
+}
+
+// Piece `n` of range `me` as a stage's note has it: (sub-panel | what ends with it << 30, first range, this one, last one).
+__device__ __noinline__ uint4 piece_at(const GemvParams &p, int me, int n) {
+  int sp = 0, kt, rows;
+  Walk walk;
+  walk.start(p, me);
+  for (int i = 0; i <= n; i++) walk.next(sp, kt, rows);
+  return make_uint4(sp | (walk.more() ? 1u : 3u) << 30, cta_of(p, sp * p.KT), me, cta_of(p, (sp + 1) * p.KT - 1));
+}
+
+__global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_constant__ Queue q) {
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const int warp = threadIdx.x >> 5, cta = blockIdx.x, ctas = gridDim.x;
@@ -703,6 +636,7 @@ __global__ void __launch_bounds__(kThreads, kOcc) gemv_queue_kernel(const __grid
   // griddepcontrol.wait (set up, prefetch weights) does not depend on this launch.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
+    sts32(sbase + kSmDead, 0);
     for (int s = 0; s < kBars; s++) {
       mbar_init(sbase + kSmFull + 8 * s, 2);        // the announcements of the weight bytes and of the x bytes
       mbar_init(sbase + kSmEmpty + 8 * s, kCW);
@@ -712,40 +646,40 @@ __global__ void __launch_bounds__(kThreads, kOcc) gemv_queue_kernel(const __grid
   __syncthreads();
   if (warp >= kCW) {
     if (warp == kCW) produce<true>(q, smem, sbase, cta, ctas);
-    else produce<false>(q, smem, sbase, cta, ctas);
+    else if (warp == kCW + 1) produce<false>(q, smem, sbase, cta, ctas);
+    else carry(q, cta, ctas);
     return;
   }
-  Ring ring{0, 0, 0};
+  float *sums = reinterpret_cast<float *>(smem + kSmSums);
+  Place w;
+  w.smem = sbase, w.bar = 0, w.parity = 0, w.lane = threadIdx.x & 31, w.cc = warp & 3;
   for (int i = 0; i < q.n; i++) {
     const GemvParams &p = q.op[i];
     const Scratch &sc = q.set[i % q.sets];
-    const int kind = (p.fmt == BT_BFP4 ? 6 : 0) + (p.pair ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2);
-    switch (kind) {
-      case 0: consume<BT_BFP8, 1, false>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 1: consume<BT_BFP8, 2, false>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 2: consume<BT_BFP8, 4, false>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 3: consume<BT_BFP8, 1, true>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 4: consume<BT_BFP8, 2, true>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 5: consume<BT_BFP8, 4, true>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 6: consume<BT_BFP4, 1, false>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 7: consume<BT_BFP4, 2, false>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 8: consume<BT_BFP4, 4, false>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 9: consume<BT_BFP4, 1, true>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      case 10: consume<BT_BFP4, 2, true>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-      default: consume<BT_BFP4, 4, true>(q, p, sc, ring, smem, sbase, cta, ctas); break;
-    }
-    // Report this CTA done with matmul i: its results and partial sums are visible to the whole GPU before the count
-    // moves. A CTA without work in a matmul reports at once, which is harmless: the count of matmul i is complete
-    // only when the CTAs that do have work got their x, that is when matmul i - 1 was complete. The last report of
-    // the last matmul finds every producer past its last look at the counts, and zeroes them for the next launch.
-    // The counts are shared with the launch before this one, which may still be running (this launch may start
-    // early): a CTA without work in the first matmul must not report before that launch is complete.
-    named_barrier(1, kCW * 32);
-    if (threadIdx.x == 0) {
-      fence_gpu();
-      if (i == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
-      if (atomicAdd(q.ops_done + i, 1) == ctas - 1 && i == q.n - 1)
-        for (int j = 0; j < q.n; j++) q.ops_done[j] = 0;
+    // for one weight matrix a column's tile rows go round four warps, for a pair round two, and the others have the second matrix
+    w.mat = p.pair ? warp >> 2 & 1 : 0, w.groups = p.pair ? 2 : 4, w.ck = p.pair ? warp >> 3 : warp >> 2;
+    // The ranges go round the CTAs from matmul to matmul: the CTAs that finish shared sub-panels have more to do than
+    // the others, and it should not be the same ones every time.
+    const int me = (cta + p.turn) % ctas;
+    int pieces = 0;
+    for (bool more = me < p.active; more; pieces++) {
+      uint4 piece;
+      switch ((p.fmt == BT_BFP4 ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2)) {
+        case 0: piece = stream_rows<BT_BFP8, 1>(w, sums, q.error); break;
+        case 1: piece = stream_rows<BT_BFP8, 2>(w, sums, q.error); break;
+        case 2: piece = stream_rows<BT_BFP8, 4>(w, sums, q.error); break;
+        case 3: piece = stream_rows<BT_BFP4, 1>(w, sums, q.error); break;
+        case 4: piece = stream_rows<BT_BFP4, 2>(w, sums, q.error); break;
+        default: piece = stream_rows<BT_BFP4, 4>(w, sums, q.error); break;
+      }
+      // ---- this CTA is done with its part of the sub-panel ----
+      if (lds32(sbase + kSmDead)) piece = piece_at(p, me, pieces);       // not from the ring's notes
+      more = piece.x >> 30 != 3;
+      const Piece pc = {(int)(piece.x & 0x3FFFFFFF), (int)piece.y, (int)piece.w, (int)piece.z, 8 * p.tg};
+      named_barrier(1, kConsumers + 32);       // every warp's sums are in place and, for an owner, the contributors' too
+      if (pc.me == pc.last) finish(p, sc, q.slot_floats, sums, pc);
+      else contribute(p, sc, q.slot_floats, sums, pc);
+      named_barrier(2, kConsumers + 32);       // the messenger may tell; the sums may be overwritten
     }
   }
 }
@@ -808,24 +742,30 @@ int wait_for(const bt_gemv_op *ops, int i, int sets) {
   return w < 0 ? -1 : w;
 }
 
-// Units per CTA such that range boundaries fall on sub-panel boundaries (a share that divides a sub-panel's K tiles,
-// or a whole number of sub-panels), when that keeps enough of the CTAs busy; else 0: equal shares of all CTAs, whose
-// ranges straddle sub-panels. With fitted shares a CTA has one piece per matmul instead of up to three, and a
-// sub-panel's partial sums come from fewer CTAs. That is worth idle CTAs only while ranges are short and the hand-over
-// of partial sums weighs against the streaming: up to kShortRange units per CTA a fitted share is taken if it keeps
-// 70 % of the CTAs busy (inside a queue the CTAs left without a share go on to the next matmul), beyond that only if it
-// keeps 97 % busy. The choice depends on the shape only, never on a matmul's place in a queue: the way the sums are
-// grouped, and with it the last bit of a result, must not change with how matmuls are batched.
-constexpr int kShortRange = 96;
-int aligned_share(int KT, int subpanels, int ctas, int least_busy_percent) {
-  const long long units = (long long)subpanels * KT;
-  const int least = (int)((units + ctas - 1) / ctas);
-  for (int d = least; d <= 4 * least && d <= units; d++) {
-    if (KT % d != 0 && d % KT != 0) continue;
-    const long long busy = (units + d - 1) / d;
-    return busy * 100 >= (long long)(least <= kShortRange ? least_busy_percent : 97) * ctas ? d : 0;
+// The ranges of a matmul's units: how many CTAs get one, and how large. Equal shares of all CTAs, so every SM streams
+// the same number of bytes whatever the shape, except where a matmul is so small that handing partial sums from CTA to
+// CTA (about 2 us: a store, a release, an acquire, a load) costs more than streaming the rest of a sub-panel: then a
+// share is a whole number of sub-panels. The choice depends on the shape only, never on a matmul's place in a queue:
+// the way the sums are grouped, and with it the last bit of a result, must not change with how matmuls are batched.
+constexpr int kWholePanel = 24;             // tile rows an SM streams in about the time of a hand-over
+void deal_units(GemvParams &p, int ctas) {
+  const int panels = (p.TC + kWC - 1) / kWC;
+  p.units = panels * p.KT;
+  const int equal = (p.units + ctas - 1) / ctas;
+  if (p.KT <= equal + kWholePanel && (panels + ctas - 1) / ctas * p.KT <= equal + kWholePanel) {
+    p.share = (panels + ctas - 1) / ctas * p.KT, p.extra = 0, p.active = (p.units + p.share - 1) / p.share;
+  } else {
+    p.active = min(ctas, p.units), p.share = p.units / p.active, p.extra = p.units % p.active;
   }
-  return 0;
+}
+
+// The tensor map of a matmul's x (one tile row of bf16 tiles): the staged token rows of each face are contiguous, a tile
+// has its faces 512 bytes apart, and a copy takes the tile columns of one stage.
+int map_x(GemvParams &p, uint64_t x) {
+  const Geometry g = geometry(p.fmt, p.pair != 0, p.tg);
+  const uint32_t box[3] = {p.tg == 1 ? 128u : 256u, p.tg == 4 ? 4u : 2u, (uint32_t)g.ups};
+  const uint64_t dims[3] = {box[0], box[1], (uint64_t)p.KT}, strides[2] = {512, 2048};
+  return make_tmap(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, as_ptr<void>(x), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 // Whether the last thing this library queued, on any stream, before the current entry-point call was a matmul launch
@@ -861,23 +801,27 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
     int per_sm = 0;
     BT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemv_queue_kernel, kThreads, kSmemBytes));
     if (per_sm < 1) return fail(BT_DEVICE, "%s: the matmul kernel does not fit an SM of device %d", who, device);
-    resident[device & 63] = min(per_sm, kOcc);
+    resident[device & 63] = 1;
   }
-  const int ctas = min(sms * resident[device & 63], kMaxCtas);
+  const int ctas = min(sms, kMaxCtas);
   for (int base = 0; base < n; base += kQueueMax) {
     Queue q = scratch;
     q.n = min(kQueueMax, n - base);
+    int tg_max = 1;
     for (int i = 0; i < q.n; i++) {
       const bt_gemv_op &o = ops[base + i];
       GemvParams &p = q.op[i];
-      p.x = as_ptr<uint8_t>(o.x), p.w[0] = as_ptr<uint8_t>(o.w), p.w[1] = as_ptr<uint8_t>(o.w2), p.add = as_ptr<uint16_t>(o.add);
+      p.w[0] = as_ptr<uint8_t>(o.w), p.w[1] = as_ptr<uint8_t>(o.w2), p.add = as_ptr<uint16_t>(o.add);
       p.out = as_ptr<void>(o.out), p.arg_val = as_ptr<float>(o.arg_val), p.arg_idx = as_ptr<int>(o.arg_idx);
       p.alpha = o.alpha, p.arg_base = o.arg_base, p.M = o.M, p.KT = o.K / 32, p.TC = o.N / 32, p.epi = o.epilogue, p.out_fp32 = o.out_dtype == BT_FP32 ? 1 : o.out_dtype == BT_FP32_ROWS ? 2 : 0;
       p.fmt = o.fmt, p.pair = o.epilogue == BT_EPI_GLU, p.tg = o.M <= 8 ? 1 : o.M <= 16 ? 2 : 4;
       p.wait_for = wait_for(ops + base, i, scratch.sets);
       p.turn = (int)(((long long)(base + i) * 101) % ctas);
-      p.per = aligned_share(p.KT, (p.TC + kWC - 1) / kWC, ctas, 70);
+      deal_units(p, ctas);
+      if (int s = map_x(p, o.x)) return s;
+      tg_max = max(tg_max, p.tg);
     }
+    q.ring = kSmSums + sums_bytes(tg_max), q.ring_bytes = (kSmemBytes - q.ring) / 128 * 128;
     // Programmatic dependent launch: this grid may begin while the previous launch of the stream is still finishing.
     // It only sets up and prefetches weights until its x warps pass griddepcontrol.wait. Weights read that early must
     // be in place, so the launch overlaps its predecessor only when that was a matmul launch of this file too (which

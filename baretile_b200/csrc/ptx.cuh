@@ -66,6 +66,9 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
                : "memory");
 }
 
+// Bring a tensor map into the cache it is read from by TMA, ahead of its first use.
+__device__ __forceinline__ void tensormap_prefetch(const void *tmap) { asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory"); }
+
 // Tiled TMA load of one box of a rank-3 tensor map into shared memory (128-byte aligned), completing on the
 // mbarrier with the box's full byte count. No multicast.
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void *tmap, int c0, int c1, int c2, uint32_t bar) {
@@ -84,6 +87,13 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
   asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
   return v;
 }
+
+__device__ __forceinline__ int lds32(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void sts32(uint32_t addr, int v) { asm volatile("st.shared.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   uint32_t d;
@@ -175,6 +185,10 @@ __device__ __forceinline__ int ld_acquire_gpu(const int *p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
+}
+// Adds to a counter behind everything this thread wrote or observed so far, which whoever acquires the sum then sees.
+__device__ __forceinline__ void red_release_gpu(int *p, int v) {
+  asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // Orders this thread's earlier (observed) generic-proxy accesses before its later asynchronous-proxy ones (TMA and
 // bulk copies), here: global data another CTA wrote, about to be fetched by a bulk copy.

@@ -29,7 +29,7 @@ inline int encode_fn(EncodeTiledFn *out) {
 // the byte stride of dimension i + 1 (a multiple of 16); box[] is the tile a copy moves.
 inline int make_tmap(CUtensorMap *map, CUtensorMapDataType dtype, int rank, const void *base, const uint64_t *dims,
                      const uint64_t *strides, const uint32_t *box, CUtensorMapSwizzle swizzle) {
-  EncodeTiledFn encode;
+  EncodeTiledFn encode = nullptr;
   if (int s = encode_fn(&encode)) return s;
   cuuint64_t d[5], st[4];
   cuuint32_t b[5], es[5];

@@ -441,3 +441,24 @@ def test_lm_head_pick_full_size(rt, m):
   top2 = np.sort(logits, -1)[:, -2:]
   near = top2[:, 1] - top2[:, 0] <= 2.0 ** -8 * (np.abs(xf).sum(1) @ np.abs(wd)).max(-1)
   assert np.array_equal(got_ids[~near], o.argmax(logits)[~near]), ("near ties at rows", np.nonzero(near)[0].tolist())
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+@pytest.mark.parametrize("m,k,n", [(1, 32, 32), (3, 32, 4128), (8, 96, 160), (9, 544, 96), (16, 800, 1056), (17, 8192, 128), (32, 1184, 2080), (5, 14336, 352)])
+def test_edges_of_stages_ranges_and_panels(rt, fmt, m, k, n):
+  # one tile row, part of a stage, sub-panels narrower than four columns, whole sub-panels per CTA and sub-panels shared
+  # by more CTAs than the owner adds at a time; one matrix with every kind of result, and a pair
+  rng = np.random.default_rng(m * k + n)
+  x, w, w2 = acts(rng, m, k), weights(rng, k, n), weights(rng, k, n)
+  got, ref = run(rt, x, w, fmt, dtype="fp32", add=bf16(rng.normal(0, 1, (m, n))), alpha=0.5)
+  check_matmul(got, x, None, ref, TOL_FP32)
+  got, ref = run(rt, x, w, fmt, "glu", w2)
+  check_matmul(got, x, None, ref, TOL_BF16)
+  # exact integers pin the offset coding, the shared exponents on x and the order of rows and columns
+  xi, wi = rng.integers(-3, 4, (m, k)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32)
+  got, _ = run(rt, xi, wi, fmt, dtype="fp32")
+  assert np.array_equal(got, xi @ wi)
+  if m > 8: return
+  values, ids = (upload(rt, x) @ upload(rt, w).cast(fmt).columns()).topk(1)
+  full = upload(rt, x).matmul(upload(rt, w).cast(fmt).columns(), dtype="fp32").numpy()
+  assert np.array_equal(np.array(ids.tolist())[:, 0], o.argmax(full)) and np.array_equal(np.array(values.tolist())[:, 0], full.max(-1))
