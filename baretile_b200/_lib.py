@@ -36,6 +36,10 @@ SIGNATURES = {
   "bt_d2h": [i32, vp, u64, size_t, u64],
   "bt_d2d": [i32, u64, u64, size_t, u64],
   "bt_memset": [i32, u64, i32, size_t, u64],
+  "bt_stage_create": [i32, ctypes.POINTER(u64)],
+  "bt_stage_destroy": [u64],
+  "bt_stage_upload": [u64, u64, vp, size_t, u64],
+  "bt_stage_download": [u64, vp, u64, size_t, u64],
   "bt_event_create": [i32, ctypes.POINTER(u64)],
   "bt_event_destroy": [i32, u64],
   "bt_event_record": [i32, u64, u64],

@@ -11,7 +11,23 @@ from baretile_b200 import _lib
 
 ALIGN = 256            # allocation granularity in bytes
 ARENA = 1 << 30        # device memory is taken from the driver in pieces of at least this size
+LARGE = 256 << 10      # host copies from this size on go through page-locked staging buffers; below, their set-up costs more than it saves
 TIMES = 1024           # launches whose timing records are kept (baretile/runtime.py: TIMES)
+
+
+class _Buffer(ctypes.Structure):
+  """A Py_buffer: the memory behind any object with the buffer protocol, read-only ones too, without a copy."""
+  _fields_ = [("buf", ctypes.c_void_p), ("obj", ctypes.c_void_p), ("len", ctypes.c_ssize_t), ("itemsize", ctypes.c_ssize_t), ("readonly", ctypes.c_int),
+              ("ndim", ctypes.c_int), ("format", ctypes.c_char_p), ("shape", ctypes.c_void_p), ("strides", ctypes.c_void_p), ("suboffsets", ctypes.c_void_p),
+              ("internal", ctypes.c_void_p)]
+  def __init__(self, data):
+    super().__init__()
+    ctypes.pythonapi.PyObject_GetBuffer(ctypes.py_object(data), ctypes.byref(self), 0)   # contiguous bytes, or BufferError
+  def release(self): ctypes.pythonapi.PyBuffer_Release(ctypes.byref(self))
+
+
+_new_bytes = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_void_p, ctypes.c_ssize_t)(("PyBytes_FromStringAndSize", ctypes.pythonapi))
+_bytes_at = ctypes.PYFUNCTYPE(ctypes.c_void_p, ctypes.py_object)(("PyBytes_AsString", ctypes.pythonapi))
 
 
 class Bound(int):
@@ -186,6 +202,7 @@ class Runtime:
     self.pending = None      # matmuls collected for one queue launch (a list while queueing)
     self.recording = None    # the Recording in progress, which keeps what is freed meanwhile
     self.sides, self.unjoined, self.side = [], [], None   # (stream, fork event, done event) of beside blocks; their done events not yet joined; the own stream while a block is open
+    self.stage = 0           # staging buffers for large copies from and to pageable memory
     self.stream = ctypes.c_uint64()
     for other in list(chip.taken.values()): other.close()
     _lib.call("bt_stream_create", self.device, ctypes.byref(self.stream))
@@ -225,6 +242,8 @@ class Runtime:
       _lib.lib().bt_stream_destroy(self.device, stream)
       for e in (fork, done): _lib.lib().bt_event_destroy(self.device, e)
     self.sides, self.unjoined = [], []
+    if self.stage: _lib.lib().bt_stage_destroy(self.stage)
+    self.stage = 0
     for ptr in getattr(self, "pinned", []): _lib.lib().bt_host_free(ptr)
     self.pinned = []
     for addr, _ in self.arenas: _lib.lib().bt_free(self.device, addr)
@@ -407,19 +426,33 @@ class Runtime:
     self.launch("bt_tilize_many" if tilize else "bt_untilize_many", (itemsize, n, src, dst, rows, cols), name="upload" if tilize else "readback")
 
   def upload(self, addr, data):
-    """Copy host bytes to device memory at addr, in order with the queued launches."""
+    """Copy host bytes to device memory at addr, in order with the queued launches. Returns when `data` has been read."""
     self.check()
-    data = bytes(data) if not isinstance(data, (bytes, bytearray)) else data
-    buf = (ctypes.c_char * len(data)).from_buffer_copy(data)
-    self.flush()
-    _lib.call("bt_h2d", self.device, addr, ctypes.cast(buf, ctypes.c_void_p), len(data), self.stream)
-    _lib.call("bt_stream_sync", self.device, self.stream, -1)   # buf is pageable and short-lived
+    if self.recording is not None: raise RuntimeError("an upload of host bytes cannot be recorded: use upload_async from page-locked memory")
+    try: src = _Buffer(data)
+    except (TypeError, ValueError, BufferError): src = _Buffer(bytes(data))
+    try:
+      self.flush()
+      if src.len >= LARGE: _lib.call("bt_stage_upload", self._staging(), addr, src.buf, src.len, self.stream)
+      elif src.len: _lib.call("bt_h2d", self.device, addr, src.buf, src.len, self.stream)   # from pageable memory: returns when it has been read
+    finally: src.release()
 
   def download(self, addr, n):
     """n bytes of device memory at addr, after the queued launches."""
     self.check()
-    buf = ctypes.create_string_buffer(n)
+    if self.recording is not None: raise RuntimeError("a read-back cannot be recorded: use download_async into page-locked memory")
+    out = _new_bytes(None, n)
     self.flush()
-    _lib.call("bt_d2h", self.device, ctypes.cast(buf, ctypes.c_void_p), addr, n, self.stream)
-    _lib.call("bt_stream_sync", self.device, self.stream, -1)
-    return buf.raw
+    if n >= LARGE: _lib.call("bt_stage_download", self._staging(), _bytes_at(out), addr, n, self.stream)
+    else:
+      _lib.call("bt_d2h", self.device, _bytes_at(out), addr, n, self.stream)
+      _lib.call("bt_stream_sync", self.device, self.stream, -1)
+    return out
+
+  def _staging(self):
+    """The runtime's page-locked staging buffers, made at the first large copy and kept until close()."""
+    if not self.stage:
+      stage = ctypes.c_uint64()
+      _lib.call("bt_stage_create", self.device, ctypes.byref(stage))
+      self.stage = stage.value
+    return self.stage

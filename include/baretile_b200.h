@@ -58,6 +58,14 @@ int bt_h2d(int device, uint64_t dst, const void *src, size_t bytes, uint64_t str
 int bt_d2h(int device, void *dst, uint64_t src, size_t bytes, uint64_t stream);       /* Chip.read / readback_kernel */
 int bt_d2d(int device, uint64_t dst, uint64_t src, size_t bytes, uint64_t stream);    /* copy_kernel (kernels.py:1051) */
 int bt_memset(int device, uint64_t dst, int value, size_t bytes, uint64_t stream);    /* zeros_kernel (kernels.py:1439) */
+/* Large copies from and to pageable host memory: several threads copy through page-locked buffers while the bus moves
+ * the others' (host DMA pages, runtime.py:548-600). A staging object holds up to 16 MB of page-locked memory and 7
+ * threads until it is destroyed; calls on one object take turns. bt_stage_upload returns when src has been read (the
+ * copy itself is queued on the stream like bt_h2d), bt_stage_download when dst is complete. Not for recording. */
+int bt_stage_create(int device, uint64_t *stage);
+int bt_stage_destroy(uint64_t stage);
+int bt_stage_upload(uint64_t stage, uint64_t dst, const void *src, size_t bytes, uint64_t stream);
+int bt_stage_download(uint64_t stage, void *dst, uint64_t src, size_t bytes, uint64_t stream);
 int bt_event_create(int device, uint64_t *event);      /* dispatcher timestamps (runtime.py:773-786) */
 int bt_event_destroy(int device, uint64_t event);
 int bt_event_record(int device, uint64_t event, uint64_t stream);

@@ -256,3 +256,22 @@ def test_copies_beside_a_recorded_step(rt):
   finally:
     for g, _ in pipe: g.close()
     for addr in stage_in + stage_out: rt.dram_free(addr)
+
+
+@pytest.mark.parametrize("size", [1, 255, (256 << 10) - 1, 256 << 10, (1 << 20) + 1, (2 << 20) + 7, 16 << 20, (37 << 20) - 3])
+def test_host_copies_of_every_size(rt, size):
+  # below and above where copies go through the staging buffers, one thread's chunk and more, a ragged last chunk; any
+  # object with the buffer protocol; and a copy that overwrites what an earlier one still has on its way
+  rng = np.random.default_rng(size)
+  a, b = (rng.integers(0, 256, size, dtype=np.uint8) for _ in range(2))
+  addr = rt.dram_alloc(size)
+  try:
+    rt.upload(addr, a.tobytes())
+    assert rt.download(addr, size) == a.tobytes()
+    rt.upload(addr, a)
+    rt.upload(addr, memoryview(bytearray(b.tobytes())))
+    assert rt.download(addr, size) == b.tobytes()
+    with pytest.raises(RuntimeError, match="recorded"):
+      with rt.record(): rt.upload(addr, a)
+    rt.wait()
+  finally: rt.dram_free(addr)
