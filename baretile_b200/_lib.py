@@ -105,4 +105,6 @@ def check(status):
   if status: raise ERRORS.get(status, RuntimeError)(lib().bt_last_error().decode(errors="replace"))
 
 
-def call(name, *args): check(getattr(lib(), name)(*args))
+def call(name, *args):
+  status = getattr(_lib or lib(), name)(*args)
+  if status: check(status)

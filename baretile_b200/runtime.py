@@ -6,7 +6,7 @@ asynchronously; `wait` blocks), device memory comes from arenas carved by the sa
 (64-byte granularity there, 256 here), and timing records are CUDA events. Frees need no deferral: every access
 to device memory is queued on the runtime's stream, so memory released now is reused only by work queued later.
 """
-import collections, ctypes, time
+import bisect, collections, ctypes, time
 from baretile_b200 import _lib
 
 ALIGN = 256            # allocation granularity in bytes
@@ -58,6 +58,26 @@ def _merge_holes(holes, starts=()):
   holes[:] = merged
 
 
+def _add_hole(holes, addr, size, arenas):
+  """Put one hole into the sorted list, joined with its neighbours (as _merge_holes joins them)."""
+  i = bisect.bisect_left(holes, (addr,))
+  if i < len(holes) and holes[i][0] == addr + size and all(a != addr + size for a, _ in arenas): size += holes.pop(i)[1]
+  if i and holes[i - 1][0] + holes[i - 1][1] == addr and all(a != addr for a, _ in arenas): holes[i - 1] = (holes[i - 1][0], holes[i - 1][1] + size)
+  else: holes.insert(i, (addr, size))
+
+
+# where bt_gemv_bfp's arguments (after the device) go in a bt_gemv_op; its scratch belongs to the call, not to the matmul
+GEMV_FIELDS = ("fmt", "epilogue", "M", "K", "N", "x", "w", "w2", "add", "alpha", "out", "out_dtype", "arg_val", "arg_idx", "arg_base")
+
+def _queue_of(ops):
+  """bt_gemv_bfp argument tuples as an array for bt_gemv_queue."""
+  arr = (_lib.GemvOp * len(ops))()
+  for o, (fmt, epi, m, k, n, x, w, w2, add, alpha, out, out_dtype, arg_val, arg_idx, arg_base, _work, _bytes) in zip(arr, ops):
+    o.fmt, o.epilogue, o.M, o.K, o.N, o.out_dtype, o.arg_base, o.alpha = fmt, epi, m, k, n, out_dtype, arg_base, getattr(alpha, "value", alpha)
+    o.x, o.w, o.w2, o.add, o.out, o.arg_val, o.arg_idx = x, w, w2, add, out, arg_val, arg_idx
+  return arr
+
+
 class Recording:
   """Launches recorded once and replayed with one call: the reference's Recording / tensor.jit
   (baretile/tensor.py:1171-1293), which replays a block of commands with one doorbell write. Here the block is a
@@ -69,7 +89,7 @@ class Recording:
       with rt.record() as step: y = (x @ w).relu().realize()      # runs once, like any launches
       step.replay()                                                # and again
   """
-  def __init__(self, rt): self.rt, self.graph, self.count, self.held, self.launches = rt, None, 0, [], None
+  def __init__(self, rt): self.rt, self.graph, self.count, self.held, self.launches, self.steps = rt, None, 0, [], None, None
   def __enter__(self):
     self.rt.check()
     if self.rt.recording is not None: raise RuntimeError("a recording is already in progress on this runtime")
@@ -114,9 +134,37 @@ class Recording:
       _lib.call("bt_graph_launch", self.rt.device, self.graph, self.rt.stream)
       self.rt.launches += self.count
       return
-    with self.rt.queue():
-      for kernel, args, units, name in self.launches:
-        self.rt.launch(kernel, tuple(a.rebind(binding) if isinstance(a, Bound) else a for a in args), units, name)
+    rt = self.rt
+    if rt.pending is not None or rt.side is not None or rt.log is not None or rt.timing:    # part of something larger: one by one
+      with rt.queue():
+        for kernel, args, units, name in self.launches:
+          rt.launch(kernel, tuple(a.rebind(binding) if isinstance(a, Bound) else a for a in args), units, name)
+      return
+    if self.steps is None: self.steps = self._steps()
+    for kernel, args, bound, names in self.steps:
+      if kernel == "bt_gemv_queue":
+        for o, field, a in bound: setattr(o, field, a.rebind(binding))
+        _lib.call(kernel, rt.device, len(args), args, rt.work, rt.work_bytes, rt.stream)
+      else: _lib.call(kernel, rt.device, *(a.rebind(binding) if isinstance(a, Bound) else a for a in args), rt.stream)
+      for name in names: rt._count(name, 0, 0)
+  def _steps(self):
+    """The recorded launches as the calls a replay with a binding makes, worked out once: consecutive matmuls are one
+    bt_gemv_queue whose array is kept, and a replay writes only the Bound fields (with 90 matmuls of a small model,
+    going through every launch again took longer than the GPU did)."""
+    steps, ops = [], []
+    def matmuls():
+      if not ops: return
+      arr = _queue_of([args for _, args, _, _ in ops])
+      bound = [(o, field, a) for o, (_, args, _, _) in zip(arr, ops) for field, a in zip(GEMV_FIELDS, args) if isinstance(a, Bound)]
+      steps.append(("bt_gemv_queue", arr, bound, [name or kernel for kernel, _, _, name in ops]))
+      ops.clear()
+    for launch in self.launches:
+      if launch[0] == "bt_gemv_bfp": ops.append(launch)
+      else:
+        matmuls()
+        steps.append((launch[0], launch[1], None, [launch[3] or launch[0]]))
+    matmuls()
+    return steps
   send = replay                          # the reference's name for it
   def close(self):
     """Drop the recording and hand the memory it kept back to the allocator."""
@@ -265,7 +313,7 @@ class Runtime:
     """Queue a kernel: here `kernel` is the name of a C-ABI entry point and `args` its arguments after the device
     and before the stream (reference: a compiled kernel image and its words, baretile/runtime.py:680-697). `units`
     is accepted for parity; the entry point sizes its own grid."""
-    self.check()
+    if not self.active: self.check()
     if units is not None and not 1 <= int(units) < 2**32: raise ValueError("launch units must be in [1, 2**32 - 1]")
     if self.side is not None and kernel in ("bt_gemv_bfp", "bt_gemv_queue", "bt_gemm_bfp"):
       raise RuntimeError("a matmul uses the runtime's scratch and runs on its own stream, not in a beside block")
@@ -274,24 +322,24 @@ class Runtime:
       self.pending.append(args)
       self._count(name or kernel, 0, 0)
       return
-    self.flush()
-    start = end = 0
-    if self.timing:
-      start, end = ctypes.c_uint64(), ctypes.c_uint64()
-      _lib.call("bt_event_create", self.device, ctypes.byref(start))
-      _lib.call("bt_event_create", self.device, ctypes.byref(end))
-      start, end = start.value, end.value
-      _lib.call("bt_event_record", self.device, start, self.stream)
+    if self.pending: self.flush()
+    if not self.timing:
+      _lib.call(kernel, self.device, *args, self.stream)
+      return self._count(name or kernel, 0, 0)
+    start, end = ctypes.c_uint64(), ctypes.c_uint64()
+    _lib.call("bt_event_create", self.device, ctypes.byref(start))
+    _lib.call("bt_event_create", self.device, ctypes.byref(end))
+    start, end = start.value, end.value
+    _lib.call("bt_event_record", self.device, start, self.stream)
     _lib.call(kernel, self.device, *args, self.stream)
-    if self.timing: _lib.call("bt_event_record", self.device, end, self.stream)
+    _lib.call("bt_event_record", self.device, end, self.stream)
     self._count(name or kernel, start, end)
 
   def _count(self, name, start, end):
     self.launches += 1
-    old = self.sent.pop(self.launches % TIMES, None)
-    if old:
-      for e in old[1:]:
-        if e: _lib.lib().bt_event_destroy(self.device, e)
+    old = self.sent.get(self.launches % TIMES)
+    if old is not None and old[1]:
+      for e in old[1:]: _lib.lib().bt_event_destroy(self.device, e)
     self.sent[self.launches % TIMES] = (name, start, end)
 
   def queue(self): return Queue(self)
@@ -317,11 +365,7 @@ class Runtime:
     """Send the matmuls collected so far as one queue launch."""
     if not self.pending: return
     ops, self.pending = self.pending, []
-    arr = (_lib.GemvOp * len(ops))()
-    for o, (fmt, epi, m, k, n, x, w, w2, add, alpha, out, out_dtype, arg_val, arg_idx, arg_base, _work, _bytes) in zip(arr, ops):
-      o.fmt, o.epilogue, o.M, o.K, o.N, o.out_dtype, o.arg_base, o.alpha = fmt, epi, m, k, n, out_dtype, arg_base, getattr(alpha, "value", alpha)
-      o.x, o.w, o.w2, o.add, o.out, o.arg_val, o.arg_idx = x, w, w2, add, out, arg_val, arg_idx
-    _lib.call("bt_gemv_queue", self.device, len(ops), arr, self.work, self.work_bytes, self.stream)
+    _lib.call("bt_gemv_queue", self.device, len(ops), _queue_of(ops), self.work, self.work_bytes, self.stream)
 
   def wait(self, timeout=60, launch=None):
     """Block until the queued launches are done (baretile/runtime.py:858-880). On timeout raise TimeoutError; the
@@ -363,7 +407,7 @@ class Runtime:
   # ---- device memory ----
   def dram_alloc(self, size):
     """First free hole that is big enough (baretile/runtime.py:791-812); a new arena from the driver when none is."""
-    self.check()
+    if not self.active: self.check()
     size = max(ALIGN, -(-size // ALIGN) * ALIGN)
     for attempt in range(2):
       for i, (addr, room) in enumerate(self.holes):
@@ -376,7 +420,7 @@ class Runtime:
       try: _lib.call("bt_malloc", self.device, arena, ctypes.byref(addr))
       except MemoryError: raise MemoryError(f"no {size} bytes free in DRAM") from None
       self.arenas.append((addr.value, arena))
-      self.holes.append((addr.value, arena))
+      _add_hole(self.holes, addr.value, arena, self.arenas)
     raise MemoryError(f"no {size} bytes free in DRAM")
 
   def dram_free(self, addr):
@@ -388,8 +432,7 @@ class Runtime:
     if self.recording is not None:   # a replay will use this memory again
       self.recording.held.append((addr, size))
       return
-    self.holes.append((addr, size))
-    _merge_holes(self.holes, {a for a, _ in self.arenas})
+    _add_hole(self.holes, addr, size, self.arenas)
 
   def record(self): return Recording(self)
 
