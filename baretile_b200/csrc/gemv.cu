@@ -8,8 +8,8 @@
 // unless the next weights are already on their way. The kernel therefore takes a list of matmuls (up to kQueueMax
 // per launch) and runs them in order with the same persistent CTAs. The weight warp of a CTA walks the whole list:
 // weight copies depend on nothing and go out as soon as the ring has room, across the boundary between two matmuls.
-// Only x waits: the x warp copies a matmul's activations once every CTA has reported the matmuls it depends on
-// finished (a counter per matmul in global memory, read with acquire semantics; the host works out the dependences
+// Only x waits: the x warp copies a matmul's activations once every sub-panel of the matmuls it depends on is
+// reported finished (a counter per matmul in global memory, read with acquire semantics; the host works out the dependences
 // from the buffer addresses, and matmuls that do not depend on one another overlap, two in flight at most). While
 // that report travels, the ring fills with the next weights: 190 KB per SM, 28 MB in all, over 4 us of HBM.
 //
@@ -64,7 +64,8 @@ constexpr int kSmemBytes = 227 * 1024;
 // Scratch layout (byte offsets into the caller's workspace). Two matmuls of a queue may be in flight at once, so
 // what a matmul uses while it runs exists twice (a set for even and one for odd positions in the queue).
 constexpr size_t kWsError = 0;                                   // int: set to nonzero when a wait gave up
-constexpr size_t kWsOpsDone = 8;                                 // int[kQueueMax]: CTAs that finished each matmul of the launch
+constexpr size_t kWsOpsDone = 8;                                 // int[kQueueMax]: finished sub-panels of each matmul of the launch
+constexpr size_t kWsAllDone = 144;                               // int: and of all of them
 constexpr size_t kWsSets = 256;                                  // the sets start here
 constexpr size_t kSetPanelsDone = 0;                             // int: sub-panels finished (argmax epilogue)
 constexpr size_t kSetKeys = 256;                                 // u64[32]: per token the best (value, column) so far (argmax epilogue)
@@ -112,11 +113,12 @@ struct alignas(64) GemvParams {
   float alpha;
   int arg_base, M, KT, TC, epi, out_fp32;
   int fmt, pair, tg;
-  int wait_for;               // the matmul of the launch that must be complete before this one starts; -1: none
+  int wait_for, wait_panels;  // the matmul of the launch that must be complete before this one starts (-1: none), and its sub-panels
   int turn;                   // CTA c takes the unit range (c + turn) % CTAs
   int units;                  // tile rows of all sub-panels
-  int active;                 // CTAs with a range; range b starts at b * share + min(b, extra), the last one ends at units
-  int share, extra;
+  int active;                 // CTAs with a range
+  int parts;                  // > 0: every sub-panel is cut into so many ranges; 0: ranges of equal size whatever they straddle,
+  int share, extra;           // range b then starts at b * share + min(b, extra), and the last one ends at units
 };
 
 // Waits for a phase of a stage's mbarrier, with a limit. A wait that gives up marks the CTA: its sums are worthless from
@@ -139,13 +141,14 @@ struct Scratch {
   float *partials;
 };
 
-// What one launch gets: the matmuls and the scratch they share: a wait-gave-up flag, the counts of CTAs that
-// finished each matmul (zero before first use; the kernel leaves them zero) and one or two sets of running scratch.
+// What one launch gets: the matmuls and the scratch they share: a wait-gave-up flag, the counts of finished sub-panels of
+// each matmul and of the launch (zero before first use; the kernel leaves them zero) and one or two sets of running scratch.
 struct Queue {
   GemvParams op[kQueueMax];
   int n;
   int sets;                   // kSets: matmuls take the sets in turn, and as many may be in flight; 1: one after the other
-  int *error, *ops_done;
+  int *error, *ops_done, *all_done;
+  int panels;                 // sub-panels of all matmuls
   Scratch set[kSets];
   int slot_floats;            // floats between two CTAs' slots of partial sums
   int ring;                   // where the ring starts in shared memory
@@ -157,17 +160,22 @@ struct Queue {
 struct alignas(32) Stage {
   uint32_t at;                // shared-memory address of its weights; the x tiles follow the matmul's w_bytes further
   int rows, width;            // tile rows, and tile columns of the sub-panel
-  int last;                   // 1: the CTA's part of the sub-panel ends with it; 3: and so does its part of the matmul
+  int ends;                   // bits 0-1: 1, the CTA's part of the sub-panel ends with it; 3, and so does its part of the matmul; bit 2: all rows, four columns
   int sp, first, cta, end;    // the sub-panel, the first range that shares it, this CTA's and the last one, the owner
 };
 static_assert(sizeof(Stage) * kBars <= kSmSums - kSmStages, "room for the stages' notes");
 
-__device__ __forceinline__ int range_start(const GemvParams &p, int b) { return min(b * p.share + min(b, p.extra), p.units); }
+__device__ __forceinline__ int range_start(const GemvParams &p, int b) {
+  if (p.parts > 0) return b / p.parts * p.KT + b % p.parts * p.KT / p.parts;
+  return min(b * p.share + min(b, p.extra), p.units);
+}
 // The CTA whose (non-empty) range holds unit u.
 __device__ __forceinline__ int cta_of(const GemvParams &p, int u) {
+  if (p.parts > 0) return u / p.KT * p.parts + ((u % p.KT + 1) * p.parts - 1) / p.KT;
   const int longer = p.extra * (p.share + 1);
   return u < longer ? u / (p.share + 1) : p.extra + (u - longer) / p.share;
 }
+
 // One weight tile times the staged x tile. `tile`, `ex` and `xs` are shared-memory addresses that already include
 // the lane's own offsets: tile = tile base + 16 * lane; ex = tile base + 16 * t, where the lane's exponents are;
 // xs = x tile base + 32 * g + 8 * t (g = lane / 4, t = lane % 4).
@@ -175,31 +183,31 @@ __device__ __forceinline__ int cta_of(const GemvParams &p, int u) {
 // A weight byte (offset binary, see stream_layout.cuh) zero-extended into a 16-bit lane is the bf16 number
 // byte * 2^-133, so a mask (bytes 0 and 2 of a word: the lane's first k pair) or a byte-permute (bytes 1 and 3: its
 // second pair) makes a register of two weights. A face (16 k x 16 n) is one MMA, rows g and g + 8 of it the channels 2g
-// and 2g + 1; acc[fs][tg] collects face column fs. A bfp4 byte holds two channels of the same k: the masked low
-// nibble is channel 2g, the masked high nibble, 16 times its code, channel 2g + 1.
+// and 2g + 1; acc[fs][tg] collects face column fs. A bfp4 byte holds two channels of the
+// same k: rows g of its MMA are the whole byte, 16 * high + low, rows g + 8 the masked low nibble, and the high channel
+// is the difference, taken once per sub-panel (one mask less per word than two masked nibbles).
 //
 // Where the face row's power of two goes depends on how many tokens share it. Up to 16 tokens (TG 1 and 2) it goes to
 // x: the MMA's two x registers per 8 tokens are multiplied by 2^(e - 127), exactly unless the product with a weight
 // of that run leaves bf16's range, and the four weight registers take one multiply-add with constants that makes
-// them the signed integers times 2^-6, whatever the run; the sums are the results themselves. With 32 tokens eight x
+// them the signed integers times 2^-6, whatever the run. With 32 tokens eight x
 // registers would need it per face and the weights only four, so there the weights carry it: one packed
 // multiply-add with s = 2^(e - 64) and with -offset * 2^-133 * s makes them the weights times 2^-64, which the epilogue
 // undoes. On shared-memory data alone, 16 warps, an SM does a tile in 23 (8 tokens), 32 (16) and 47-50 cycles
-// (32); weights that carry the scale take 24 / 27 (bfp8 / bfp4) for 8 tokens, and x that carries it 52 for 32, where
-// the MMAs themselves (about 10 cycles each per scheduler) are the bound. Subtracting the offset with a second MMA
-// instead of the multiply-adds was slower (26-28 cycles for 8 tokens) for the same reason.
-constexpr uint32_t kByteLanes = 0x00FF00FFu, kNibbleLanes = 0x000F000Fu, kHighLanes = 0x00F000F0u, kOddBytes = 0x4341u;
+// (32): 68 instructions, of which an MMA holds the tensor pipe for about 10 cycles, so the bound is instructions. Weights
+// that carry the scale take 24 / 27 (bfp8 / bfp4) for 8 tokens, x that carries it 52 for 32, and subtracting the offset
+// with a second MMA instead of the multiply-adds 26-28 for 8.
+constexpr uint32_t kByteLanes = 0x00FF00FFu, kNibbleLanes = 0x000F000Fu, kOddBytes = 0x4341u;
 constexpr uint32_t kMinus128 = 0x80808080u;   // two bf16 lanes of -128 * 2^-133 = -2^-126
+constexpr uint32_t kMinus136 = 0x80888088u;   // -(128 + 8) * 2^-133: offset of a byte made of two offset nibbles
 constexpr uint32_t kMinus8 = 0x80088008u;     // -8 * 2^-133
-constexpr uint32_t kTimes16 = 0x41804180u;
-constexpr uint32_t kTo6 = 0x7F007F00u, kHighTo6 = 0x7D007D00u;         // 2^127: code * 2^-133 to code * 2^-6; 2^123: the same for 16 * code
-constexpr uint32_t kOff128 = 0xC000C000u, kOff8 = 0xBE00BE00u;         // -128 * 2^-6 and -8 * 2^-6
+constexpr uint32_t kTo6 = 0x7F007F00u;                                              // 2^127: code * 2^-133 to code * 2^-6
+constexpr uint32_t kOff128 = 0xC000C000u, kOff136 = 0xC008C008u, kOff8 = 0xBE00BE00u;   // the same offsets times 2^-6
 __host__ __device__ constexpr bool scale_on_x(int tg) { return tg <= 2; }
-// what turns the sums of a format and token group count into results (bfp4: a nibble q is worth 16 q)
-__host__ __device__ constexpr float unscale_of(int fmt, int tg) { return scale_on_x(tg) ? (fmt == BT_BFP4 ? 16.f : 1.f) : 18446744073709551616.f; }   // 2^64
+__host__ __device__ constexpr float unscale_of(int tg) { return scale_on_x(tg) ? 1.f : 18446744073709551616.f; }   // 2^64
 template <int FMT, int TG>
 __device__ __forceinline__ void tile_mma(uint32_t tile, uint32_t ex, uint32_t xs, float (&acc)[2][TG][4]) {
-  constexpr bool SX = TG <= 2;
+  constexpr bool SX = scale_on_x(TG);
   const uint4 ev = lds128(ex);
   const uint32_t ee[4] = {ev.x, ev.y, ev.z, ev.w};
   uint2 bx[2][TG];
@@ -224,13 +232,10 @@ __device__ __forceinline__ void tile_mma(uint32_t tile, uint32_t ex, uint32_t xs
         a0 = fma_bf16x2(w0 & kByteLanes, m01, n01), a1 = fma_bf16x2(w1 & kByteLanes, m01, n01);
         a2 = fma_bf16x2(prmt(w0, 0u, kOddBytes), m23, n23), a3 = fma_bf16x2(prmt(w1, 0u, kOddBytes), m23, n23);
       } else {
-        const uint32_t w = h ? (fs ? wv[0].w : wv[0].z) : (fs ? wv[0].y : wv[0].x), wo = w >> 8;
-        // a nibble q is worth 16 q: a high nibble stands in its byte at 16 times its code, a low one takes 16 times the factor
-        const uint32_t l01 = SX ? kTo6 : mul_bf16x2(s01, kTimes16), l23 = SX ? kTo6 : mul_bf16x2(s23, kTimes16);
-        const uint32_t h01 = SX ? kHighTo6 : s01, h23 = SX ? kHighTo6 : s23;
-        const uint32_t n01 = SX ? kOff8 : mul_bf16x2(l01, kMinus8), n23 = SX ? kOff8 : mul_bf16x2(l23, kMinus8);
-        a0 = fma_bf16x2(w & kNibbleLanes, l01, n01), a1 = fma_bf16x2(w & kHighLanes, h01, n01);
-        a2 = fma_bf16x2(wo & kNibbleLanes, l23, n23), a3 = fma_bf16x2(wo & kHighLanes, h23, n23);
+        const uint32_t w = h ? (fs ? wv[0].w : wv[0].z) : (fs ? wv[0].y : wv[0].x), w01 = w & kByteLanes, w23 = prmt(w, 0u, kOddBytes);
+        const uint32_t m01 = SX ? kTo6 : s01, m23 = SX ? kTo6 : s23;
+        a0 = fma_bf16x2(w01, m01, SX ? kOff136 : mul_bf16x2(s01, kMinus136)), a1 = fma_bf16x2(w01 & kNibbleLanes, m01, SX ? kOff8 : mul_bf16x2(s01, kMinus8));
+        a2 = fma_bf16x2(w23, m23, SX ? kOff136 : mul_bf16x2(s23, kMinus136)), a3 = fma_bf16x2(w23 & kNibbleLanes, m23, SX ? kOff8 : mul_bf16x2(s23, kMinus8));
       }
 #pragma unroll
       for (int tg = 0; tg < TG; tg++) {
@@ -257,37 +262,42 @@ __device__ __forceinline__ unsigned long long pick_key(float v, int column) {
 // The warps have left their sums in shared memory, [k group][matrix][token][channel]. Every consumer thread takes
 // one pair of neighbouring channels and every eighth token, adds the k groups in order and either stores the sums
 // in the CTA's slot of partial sums (a contributor) or adds the contributors' slots in CTA order, so that results do
-// not depend on timing, and runs the epilogue (the sub-panel's owner). Elementwise over all 512 threads: one small
-// piece of code for every kind of matmul. It runs once per sub-panel on warps that have nothing else to do, so its time is its
-// chain of dependent instructions: no loops over the k groups, parameters fetched up front, loads in flight together (as
-// plain loops over groups, contributors and all 32 rows it took 3000-5000 cycles).
+// not depend on timing, and runs the epilogue (the sub-panel's owner). Elementwise over 512 threads: one small piece of
+// code for every kind of matmul. Everybody waits for it, so what counts is its chain of dependent steps and the
+// instructions that 16 warps issue (as plain loops over groups, contributors and all 32 rows it took 3000-5000 cycles).
+//
+// Partial sums carry their own signal: a word of a slot is zero until it is there (a zero sum is sent as -0, and the
+// reader adds +0 at the end), the owner's threads poll the words they need and put zeros back. A counter released by
+// the contributor and acquired by the owner took about 1.2 us more.
 struct Piece {
   int sp;                  // the sub-panel
   int first, last, me;     // the ranges that share it, and this CTA's
   int toks;                // tokens whose sums are in shared memory: M rounded up to whole groups of 8
 };
-// One token's sums of the channel pair: the k groups of one matrix, or of gate and up, added in order.
-__device__ __forceinline__ void sum_groups(const float *sums, bool pair, int toks, int tok, int pr, float2 &v, float2 &u) {
-  float2 s[4];
+constexpr int kSlots = 4;  // contributors whose words are in flight together
+struct Slots {
+  uint2 w[kSlots];
+  __device__ __forceinline__ void load(const float *at, int slot_floats, int n) {
 #pragma unroll
-  for (int j = 0; j < 4; j++) s[j] = *reinterpret_cast<const float2 *>(sums + (j * toks + tok) * kSumStride + 2 * pr);
-  u = make_float2(s[1].x + s[3].x, s[1].y + s[3].y);
-  v = make_float2(s[0].x + s[2].x, s[0].y + s[2].y);
-  if (!pair) v.x += u.x, v.y += u.y;
-}
-__device__ __forceinline__ void contribute(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc) {
-  const int pr = threadIdx.x & 63, M = p.M;
-  const bool pair = p.pair;
-  float *slot = sc.partials + (size_t)pc.me * slot_floats + 2 * pr;
-  for (int tok = threadIdx.x >> 6; tok < M; tok += kConsumers / 64) {
-    float2 v, u;
-    sum_groups(sums, pair, pc.toks, tok, pr, v, u);
-    float2 *to = reinterpret_cast<float2 *>(slot + (pair ? 2 * tok : tok) * 128);
-    *to = v;
-    if (pair) to[64] = u;
+    for (int j = 0; j < kSlots; j++)
+      if (j < n) w[j] = ld_relaxed2(at + (size_t)j * slot_floats);
   }
+  __device__ __forceinline__ void add_to(float2 &v, float *at, int slot_floats, int n, uint32_t &patience) {
+#pragma unroll
+    for (int j = 0; j < kSlots; j++)
+      if (j < n) {
+        float *from = at + (size_t)j * slot_floats;
+        while ((w[j].x == 0 || w[j].y == 0) && patience) w[j] = ld_relaxed2(from), patience--;
+        st_relaxed2(from, make_uint2(0, 0));
+        v.x += __uint_as_float(w[j].x), v.y += __uint_as_float(w[j].y);
+      }
+  }
+};
+__device__ __forceinline__ void send(float *to, float2 v) {
+  const uint32_t x = __float_as_uint(v.x), y = __float_as_uint(v.y);
+  st_relaxed2(to, make_uint2(x ? x : 0x80000000u, y ? y : 0x80000000u));
 }
-// The rows past M of an owner's tiles are zeros; they need no sums, so the messenger writes them while it waits.
+// The rows past M of an owner's tiles are zeros; they need no sums, so the messenger writes them while the others work.
 __device__ __forceinline__ void zero_rows(const GemvParams &p, int sp) {
   const int M = p.M, lane = threadIdx.x & 31;
   if (M == 1 || p.epi == BT_EPI_ARGMAX || p.out_fp32 == 2) return;
@@ -297,60 +307,79 @@ __device__ __forceinline__ void zero_rows(const GemvParams &p, int sp) {
     for (int i = max(M - (face & 2) * 8, 0) * per_row + lane; i < 16 * per_row; i += 32) rows[i] = make_uint4(0, 0, 0, 0);
   }
 }
-__device__ __forceinline__ void finish(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc) {
-  const int pr = threadIdx.x & 63, M = p.M, epi = p.epi, fp32 = p.out_fp32, first = pc.first, last = pc.last;
-  const bool pair = p.pair;
+__device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc, uint32_t smem, int *error) {
+  const int pr = threadIdx.x & 63, M = p.M, epi = p.epi, fp32 = p.out_fp32, step = p.pair ? 256 : 128;
+  const bool pair = p.pair, owner = pc.me == pc.last;
+  const int others = owner ? pc.last - pc.first : 0;                                  // contributors whose sums are to be added
   const int tcol = pc.sp * kWC + (pr >> 4), n0 = pc.sp * kWC * 32 + 2 * pr;           // tile column and first channel of the pair
   const bool inside = tcol < p.TC;
-  const float unscale = unscale_of(p.fmt, p.tg) * p.alpha;
-  const uint16_t *add = p.add;
+  const float unscale = unscale_of(p.tg) * p.alpha;
+  const uint16_t *add = owner && inside ? p.add : nullptr;
   char *out = static_cast<char *>(p.out);
-  // a one-row result repeats across its tile: each of the eight groups of 64 threads works it out and writes four rows
-  for (int row = threadIdx.x >> 6; row < (M == 1 && epi != BT_EPI_ARGMAX ? kConsumers / 64 : M); row += kConsumers / 64) {
-    const int tok = M == 1 ? 0 : row;
-    const int at = tcol * 1024 + ((row >> 4) * 2 + ((pr >> 3) & 1)) * 256 + (row & 15) * 16 + (2 * pr & 15);
-    float2 v, u;
-    // everything that comes from L2 in flight together: the addend and the contributors' sums, four at a time
-    uint32_t a = 0;
-    if (add && inside) a = *reinterpret_cast<const uint32_t *>(add + at);
-    const float *slots = sc.partials + (size_t)first * slot_floats + (pair ? 2 * tok : tok) * 128 + 2 * pr;
-    float2 w[4], x[4];
-    for (int c0 = first, once = 1; once || c0 < last; c0 += 4, once = 0, slots += 4 * (size_t)slot_floats) {
+  float *slots = sc.partials + (size_t)(owner ? pc.first : pc.me) * slot_floats + 2 * pr;
+  int row = threadIdx.x >> 6;
+  // datum index of (row, channel pair) in the result's tiles, and in an addend's
+  auto place = [&](int r) { return tcol * 1024 + ((r >> 4) * 2 + ((pr >> 3) & 1)) * 256 + (r & 15) * 16 + (2 * pr & 15); };
+  auto addend = [&](int r) { return add && r < M ? __ldcg(reinterpret_cast<const uint32_t *>(add + place(r))) : 0u; };
+  uint32_t a = addend(row);
+  named_barrier(1, kConsumers);                                                       // every warp's sums are in place
+  uint32_t patience = others && lds32(smem + kSmDead) ? 1 : kSpinLimit * 64;
+  for (; row < M; row += kConsumers / 64) {
+    float2 s[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        w[j] = x[j] = make_float2(0.f, 0.f);
-        if (c0 + j < last) w[j] = __ldcg(reinterpret_cast<const float2 *>(slots + (size_t)j * slot_floats));
-        if (pair && c0 + j < last) x[j] = __ldcg(reinterpret_cast<const float2 *>(slots + (size_t)j * slot_floats + 128));
-      }
-      if (once) sum_groups(sums, pair, pc.toks, tok, pr, v, u);
-#pragma unroll
-      for (int j = 0; j < 4; j++) v.x += w[j].x, v.y += w[j].y, u.x += x[j].x, u.y += x[j].y;
+    for (int j = 0; j < 4; j++) s[j] = *reinterpret_cast<const float2 *>(sums + (j * pc.toks + row) * kSumStride + 2 * pr);
+    float2 u = make_float2(s[1].x + s[3].x, s[1].y + s[3].y), v = make_float2(s[0].x + s[2].x, s[0].y + s[2].y);
+    if (!pair) v.x += u.x, v.y += u.y;
+    float *slot = slots + row * step;
+    if (!owner) {
+      send(slot, v);
+      if (pair) send(slot + 128, u);
+      continue;
+    }
+    for (int c = 0; c < others; c += kSlots, slot += kSlots * (size_t)slot_floats) {
+      Slots w, x;
+      w.load(slot, slot_floats, others - c);
+      if (pair) x.load(slot + 128, slot_floats, others - c);
+      w.add_to(v, slot, slot_floats, others - c, patience);
+      if (pair) x.add_to(u, slot + 128, slot_floats, others - c, patience);
     }
     v.x = v.x * unscale + __uint_as_float(a << 16), v.y = v.y * unscale + __uint_as_float(a & 0xFFFF0000u);
+    a = addend(row + kConsumers / 64);
     if (epi == BT_EPI_RELU) v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f);
     if (epi == BT_EPI_SILU || pair) v.x = silu(v.x), v.y = silu(v.y);
-    if (pair) v.x *= u.x * unscale, v.y *= u.y * unscale;
+    if (pair) v.x *= (u.x + 0.f) * unscale, v.y *= (u.y + 0.f) * unscale;
     if (epi == BT_EPI_ARGMAX) {
       unsigned long long key = inside ? max(pick_key(v.x, n0), pick_key(v.y, n0 + 1)) : 0ull;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) key = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, d));
       // a maximum over all sub-panels whatever the order they finish in, so the last one to finish has the answer at hand
       if ((threadIdx.x & 31) == 0 && key) atomicMax(sc.keys + row, key);
-    } else if (inside) {
-      const uint32_t both = bf16_half_up(v.x) | bf16_half_up(v.y) << 16;
+      continue;
+    }
+    const uint32_t both = bf16_half_up(v.x) | bf16_half_up(v.y) << 16;
+    if (fp32 == 2) {
       // row-major fp32, only the rows there are: partial sums on their way to an all-reduce
-      if (fp32 == 2) {
-        if (row < M) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + n0)) = v;
-      } else {
+      if (inside) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + n0)) = v;
+    } else if (M > 1) {
+      if (inside && fp32) *reinterpret_cast<float2 *>(out + 4 * (size_t)place(row)) = v;
+      else if (inside) *reinterpret_cast<uint32_t *>(out + 2 * (size_t)place(row)) = both;
+    } else if (fp32) {
+      // a one-row result repeats across its tile
+      for (int r = 0; inside && r < 32; r++) *reinterpret_cast<float2 *>(out + 4 * (size_t)place(r)) = v;
+    } else {
+      // the same: four lanes put half a face row together, and each of them writes it to eight of the rows
+      uint4 half;
+      half.x = __shfl_sync(0xFFFFFFFFu, both, 0, 4), half.y = __shfl_sync(0xFFFFFFFFu, both, 1, 4);
+      half.z = __shfl_sync(0xFFFFFFFFu, both, 2, 4), half.w = __shfl_sync(0xFFFFFFFFu, both, 3, 4);
+      if (inside) {
 #pragma unroll
-        for (int r = 0; r < 4; r++)                                                   // rows row, + 8, + 16, + 24 of a one-row result
-          if (r == 0 || M == 1) {
-            const size_t to = at + (r >> 1) * 512 + (r & 1) * 128;
-            if (fp32) *reinterpret_cast<float2 *>(out + 4 * to) = v;
-            else *reinterpret_cast<uint32_t *>(out + 2 * to) = both;
-          }
+        for (int r = 0; r < 32; r += 4) *reinterpret_cast<uint4 *>(out + 2 * (size_t)(place(r + (pr & 3)) - 2 * (pr & 3))) = half;
       }
     }
+  }
+  if (!patience) {
+    sts32(smem + kSmDead, 1);
+    atomicExch(error, 3);
   }
 }
 
@@ -402,19 +431,21 @@ struct Ring {
 // One warp copies weights, the other x. Both follow the same stages through the ring and wait for the same room
 // (the oldest stage in the ring freed by the consumers), each keeping its own books, so neither waits for the other.
 // Weights never depend on an earlier matmul: their copies go out as soon as the ring has room, one bulk copy per
-// weight matrix and stage. x is the result of an earlier matmul: the x warp waits (with a limit) until every CTA has
-// reported the matmuls it depends on finished, then copies each stage's x tiles with ONE tiled TMA copy, which picks
+// weight matrix and stage. x is the result of an earlier matmul: the x warp waits (with a limit) until all sub-panels of
+// the matmul it depends on are reported finished, then copies each stage's x tiles with ONE tiled TMA copy, which picks
 // the token rows that are there out of every tile (8 rows: 256 bytes of each of two faces). An asynchronous copy costs
 // its issuer and the copy engine the same whatever its size: with two plain copies of 256 bytes per tile the x
 // warp alone held an 8192 x 28672 bfp4 matmul at 46 us, with one of 1 KB at 35, where the weights take 31.
 // x may be the result of the launch before this one, or of an earlier matmul of this one: the host has worked out the
-// last matmul this one must see finished, by every CTA. False: gave up.
-__device__ __forceinline__ bool await_turn(const Queue &q, const GemvParams &p, int ctas) {
+// last matmul this one must see finished, all of its sub-panels. False: gave up.
+__device__ __forceinline__ bool await_turn(const Queue &q, const GemvParams &p, int pause_ns) {
   asm volatile("griddepcontrol.wait;" ::: "memory");     // returns when the previous launch is complete and visible
   if (p.wait_for >= 0) {
     uint32_t spins = 0;
-    while (ld_acquire_gpu(q.ops_done + p.wait_for) < ctas)
+    while (ld_acquire_gpu(q.ops_done + p.wait_for) < p.wait_panels) {
       if (++spins > kSpinLimit * 64) return false;
+      if (pause_ns) __nanosleep(pause_ns);
+    }
   }
   return true;
 }
@@ -462,7 +493,7 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
           const uint32_t bytes = n * width * g.tb;
           if (lane == 0) {
             uint4 *note = reinterpret_cast<uint4 *>(smem + kSmStages) + 2 * (count % kBars);
-            note[0] = make_uint4(stage, n, width, rows <= g.ups ? ends : 0), note[1] = make_uint4(sp, first, me, end);
+            note[0] = make_uint4(stage, n, width, (rows <= g.ups ? ends : 0) | (n == g.ups && width == kWC ? 4 : 0)), note[1] = make_uint4(sp, first, me, end);
             mbar_expect_tx(bar, nw * bytes);
           }
           __syncwarp();
@@ -470,7 +501,7 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
         } else {
           if (gate) {
             int ok = 1;
-            if (lane == 0) ok = await_turn(q, p, ctas);
+            if (lane == 0) ok = await_turn(q, p, 0);
             if (!__shfl_sync(0xFFFFFFFFu, ok, 0) && lane == 0) atomicExch(q.error, 5);
             // x was written with ordinary stores (by other CTAs of this launch, or by the launch before) and is about to
             // be read by TMA copies: order what the acquire made visible before the asynchronous proxy's reads
@@ -491,65 +522,63 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
 }
 
 // ---- consumers --------------------------------------------------------------------------------------------------
-// A warp's part of one piece: `rows` tile rows of a sub-panel, of which the warp takes every `groups`-th from `ck` on in
-// one column, stage by stage; then its sums go to shared memory. What does not depend on the format and the token
-// count lives in the kernel itself, once, where the matmul's parameters are read from the constant bank (passed on by
-// reference they were fetched through global memory, and a sub-panel's end took 4-6 us).
+// A warp's part of one piece: tile rows of a sub-panel, of which the warp takes every second or fourth from `ck` on in
+// one column, stage by stage; then its sums go to shared memory. What does not depend on the kind of matmul lives in the
+// kernel itself, once, where the matmul's parameters are read from the constant bank (passed on by reference they were
+// fetched through global memory, and a sub-panel's end took 4-6 us).
 struct Place {
   uint32_t smem;                     // shared memory
-  uint32_t bar, parity;              // the next stage's mbarriers (8 * its number among kBars) and their phase
-  int cc, ck, mat, groups;           // this warp's column, first tile row, weight matrix; warps that share a column
+  uint32_t count;                    // stages so far
+  int cc, ck, mat;                   // this warp's column, first tile row, weight matrix
   int lane;
 };
-template <int FMT, int TG>
+template <int FMT, int TG, bool PAIR>
 __device__ __forceinline__ uint4 stream_rows(Place &w, float *sums, int *error) {
-  constexpr int TB = tile_bytes(FMT), T = stage_rows_per_warp(FMT, TG), XB = 512 * TG;
-  const int lane = w.lane, groups = w.groups, ck = w.ck, cc = w.cc;
-  const uint32_t x_step = groups * XB, x0 = 4 * T * kWC * TB + ck * XB + lane * 8, matrix0 = w.mat * (groups * T * kWC * TB);
+  constexpr int TB = tile_bytes(FMT), T = stage_rows_per_warp(FMT, TG), XB = 512 * TG, GROUPS = PAIR ? 2 : 4;   // warps that share a column
+  const int lane = w.lane, ck = w.ck, cc = w.cc;
+  const uint32_t matrix0 = w.mat * (GROUPS * T * kWC * TB), x0 = 4 * T * kWC * TB + ck * XB + lane * 8, tile0 = matrix0 + (ck * kWC + cc) * TB;
   float acc[2][TG][4];
 #pragma unroll
   for (int i = 0; i < 8 * TG; i++) acc[i / (4 * TG)][i / 4 % TG][i % 4] = 0.f;
   uint4 piece = make_uint4(0, 0, 0, 0);
   for (int last = 0; !last;) {
-    if (!stage_wait(w.smem, w.smem + kSmFull + w.bar, w.parity, error)) break;
-    const uint4 stage = lds128(w.smem + kSmStages + 4 * w.bar);        // at, rows, width, last
-    const int width = stage.z;
-    uint32_t tile = stage.x + matrix0 + (ck * width + cc) * TB, xs = stage.x + x0;
-    const uint32_t tile_step = groups * width * TB;
-    last = stage.w;
-    if (last) piece = lds128(w.smem + kSmStages + 4 * w.bar + 16), piece.x |= (uint32_t)last << 30;
-    if (cc < width) {
-      if ((int)stage.y == groups * T) {
+    const uint32_t slot = w.count & (kBars - 1), bar = w.smem + 8 * slot, note = w.smem + kSmStages + 32 * slot;
+    if (!stage_wait(w.smem, bar + kSmFull, w.count / kBars & 1, error)) break;
+    const uint4 stage = lds128(note);                                  // at, rows, width, ends
+    last = stage.w & 3;
+    if (last) piece = lds128(note + 16), piece.x |= (uint32_t)last << 30;
+    if (stage.w & 4) {
+      // a whole stage of four columns: every offset is a constant
+      const uint32_t tile = stage.x + tile0 + lane * 16, ex = stage.x + tile0 + (lane & 3) * 16, xs = stage.x + x0;
 #pragma unroll
-        for (int j = 0; j < T; j++, tile += tile_step, xs += x_step) tile_mma<FMT, TG>(tile + lane * 16, tile + (lane & 3) * 16, xs, acc);
-      } else {
+      for (int j = 0; j < T; j++) tile_mma<FMT, TG>(tile + j * (GROUPS * kWC * TB), ex + j * (GROUPS * kWC * TB), xs + j * (GROUPS * XB), acc);
+    } else if (cc < (int)stage.z) {
+      uint32_t tile = stage.x + matrix0 + (ck * stage.z + cc) * TB, xs = stage.x + x0;
 #pragma unroll 1
-        for (int row = ck; row < (int)stage.y; row += groups, tile += tile_step, xs += x_step) tile_mma<FMT, TG>(tile + lane * 16, tile + (lane & 3) * 16, xs, acc);
-      }
+      for (int row = ck; row < (int)stage.y; row += GROUPS, tile += GROUPS * stage.z * TB, xs += GROUPS * XB)
+        tile_mma<FMT, TG>(tile + lane * 16, tile + (lane & 3) * 16, xs, acc);
     }
     __syncwarp();
-    mbar_arrive_if(w.smem + kSmEmpty + w.bar, lane == 0);
-    w.bar = (w.bar + 8) & (8 * kBars - 1);
-    if (w.bar == 0) w.parity ^= 1;
+    mbar_arrive_if(bar + kSmEmpty, lane == 0);
+    w.count++;
   }
   // fragments to [k group][matrix][token][channel]: lane (g, t) holds tokens 8 tg + 2 t + j and channels 16 fs + 2 g + {0, 1}
   const int t = lane & 3, g = lane >> 2;
-  float *to = sums + ((ck * (4 / groups) + w.mat) * 8 * TG + 2 * t) * kSumStride + cc * 32 + 2 * g;
+  float *to = sums + ((PAIR ? 2 * ck + w.mat : ck) * 8 * TG + 2 * t) * kSumStride + cc * 32 + 2 * g;
 #pragma unroll
   for (int fs = 0; fs < 2; fs++)
 #pragma unroll
     for (int tg = 0; tg < TG; tg++)
 #pragma unroll
       for (int j = 0; j < 2; j++)
-        *reinterpret_cast<float2 *>(to + (8 * tg + j) * kSumStride + 16 * fs) = make_float2(acc[fs][tg][j], acc[fs][tg][2 + j]);
+        *reinterpret_cast<float2 *>(to + (8 * tg + j) * kSumStride + 16 * fs) =
+            FMT == BT_BFP8 ? make_float2(acc[fs][tg][j], acc[fs][tg][2 + j]) : make_float2(16.f * acc[fs][tg][2 + j], acc[fs][tg][j] - acc[fs][tg][2 + j]);
   return piece;
 }
 
 // ---- the messenger: one warp tells other CTAs and hears from them ------------------------------------------------
-// It goes through the CTA's pieces beside the consumers and meets them at two barriers: the first it reaches when, for a
-// sub-panel this CTA owns, every contributor has signalled (a wait with a limit); after the second the consumers have
-// stored what they had, and it signals. A release takes 1000 to 3000 cycles under load; a consumer warp that did it
-// was that much behind the others at the next barrier.
+// It goes through the CTA's pieces beside the consumers and meets them when they have stored what they had. A release
+// takes 1000 to 3000 cycles under load; a consumer warp that did it was that much behind the others at the next barrier.
 __device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
   const int lane = threadIdx.x & 31;
   for (int i = 0; i < q.n; i++) {
@@ -560,7 +589,7 @@ __device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
     if (me < p.active) {
       walk.start(p, me);
       // the counters and the result are this matmul's only when the ones before it that it must not overtake are done
-      if (lane == 0 && !await_turn(q, p, ctas)) atomicExch(q.error, 5);
+      if (lane == 0 && !await_turn(q, p, 100)) atomicExch(q.error, 5);
       __syncwarp();
     }
     while (walk.more()) {
@@ -569,20 +598,20 @@ __device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
       const int first = cta_of(p, sp * p.KT), last = cta_of(p, (sp + 1) * p.KT - 1);
       int *counter = sc.counters + sp;
       if (me == last) zero_rows(p, sp);
-      if (me == last && first != last && lane == 0) {
-        uint32_t spins = 0;
-        while (ld_acquire_gpu(counter) < last - first) {
-          if (++spins > kSpinLimit * 32) { atomicExch(q.error, 3); break; }
-          __nanosleep(40);
-        }
-        *counter = 0;                          // ready for the next matmul
-      }
-      __syncwarp();
-      named_barrier(1, kConsumers + 32);
       named_barrier(2, kConsumers + 32);
       if (me != last) {
-        if (lane == 0) red_release_gpu(counter, 1);
-      } else if (p.epi == BT_EPI_ARGMAX) {
+        if (lane == 0) atomicAdd(counter, 1);    // the sums themselves say that they are there
+        continue;
+      }
+      // every contributor is past its last look at the counts of this launch
+      if (first != last && lane == 0) {
+        uint32_t spins = 0;
+        while (ld_acquire_gpu(counter) < last - first)
+          if (++spins > kSpinLimit * 64) { atomicExch(q.error, 3); break; }
+        *counter = 0;                            // ready for the next matmul
+      }
+      __syncwarp();
+      if (p.epi == BT_EPI_ARGMAX) {
         // the last sub-panel to finish turns the keys into the answer and leaves the scratch as it found it
         int is_last = 0;
         if (lane == 0) {
@@ -602,20 +631,19 @@ __device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
         }
         __syncwarp();
       }
+      // Report the sub-panel: its results are visible to the whole GPU before the count moves. A matmul is complete when all
+      // its sub-panels are: by then every CTA with a part in it has read its x, and is past its look at the counts. (Counting
+      // the CTAs instead, idle ones too, took 148 reports to one address where a small matmul has 5 sub-panels.) The last
+      // report of the launch therefore finds nobody looking any more, and zeroes the counts for the next launch.
+      if (lane == 0) {
+        red_release_gpu(q.ops_done + i, 1);
+        if (atom_add_acq_rel_gpu(q.all_done, 1) == q.panels - 1) {
+          for (int j = 0; j < q.n; j++) q.ops_done[j] = 0;
+          *q.all_done = 0;
+        }
+      }
+      __syncwarp();
     }
-    // Report this CTA done with matmul i: its results and partial sums are visible to the whole GPU before the count
-    // moves. A CTA without work in a matmul reports at once, which is harmless: the count of matmul i is complete only
-    // when the CTAs that do have work got their x, that is when matmul i - 1 was complete. The last report of the last
-    // matmul finds every producer past its last look at the counts, and zeroes them for the next launch. The counts are
-    // shared with the launch before this one, which may still be running (this launch may start early): a CTA without
-    // work in the first matmul must not report before that launch is complete.
-    if (lane == 0) {
-      fence_gpu();
-      if (i == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
-      if (atomicAdd(q.ops_done + i, 1) == ctas - 1 && i == q.n - 1)
-        for (int j = 0; j < q.n; j++) q.ops_done[j] = 0;
-    }
-    __syncwarp();
   }
 }
 
@@ -652,33 +680,37 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
   }
   float *sums = reinterpret_cast<float *>(smem + kSmSums);
   Place w;
-  w.smem = sbase, w.bar = 0, w.parity = 0, w.lane = threadIdx.x & 31, w.cc = warp & 3;
+  w.smem = sbase, w.count = 0, w.lane = threadIdx.x & 31, w.cc = warp & 3;
   for (int i = 0; i < q.n; i++) {
     const GemvParams &p = q.op[i];
     const Scratch &sc = q.set[i % q.sets];
     // for one weight matrix a column's tile rows go round four warps, for a pair round two, and the others have the second matrix
-    w.mat = p.pair ? warp >> 2 & 1 : 0, w.groups = p.pair ? 2 : 4, w.ck = p.pair ? warp >> 3 : warp >> 2;
+    w.mat = p.pair ? warp >> 2 & 1 : 0, w.ck = p.pair ? warp >> 3 : warp >> 2;
     // The ranges go round the CTAs from matmul to matmul: the CTAs that finish shared sub-panels have more to do than
     // the others, and it should not be the same ones every time.
     const int me = (cta + p.turn) % ctas;
     int pieces = 0;
     for (bool more = me < p.active; more; pieces++) {
       uint4 piece;
-      switch ((p.fmt == BT_BFP4 ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2)) {
-        case 0: piece = stream_rows<BT_BFP8, 1>(w, sums, q.error); break;
-        case 1: piece = stream_rows<BT_BFP8, 2>(w, sums, q.error); break;
-        case 2: piece = stream_rows<BT_BFP8, 4>(w, sums, q.error); break;
-        case 3: piece = stream_rows<BT_BFP4, 1>(w, sums, q.error); break;
-        case 4: piece = stream_rows<BT_BFP4, 2>(w, sums, q.error); break;
-        default: piece = stream_rows<BT_BFP4, 4>(w, sums, q.error); break;
+      switch ((p.fmt == BT_BFP4 ? 6 : 0) + (p.pair ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2)) {
+        case 0: piece = stream_rows<BT_BFP8, 1, false>(w, sums, q.error); break;
+        case 1: piece = stream_rows<BT_BFP8, 2, false>(w, sums, q.error); break;
+        case 2: piece = stream_rows<BT_BFP8, 4, false>(w, sums, q.error); break;
+        case 3: piece = stream_rows<BT_BFP8, 1, true>(w, sums, q.error); break;
+        case 4: piece = stream_rows<BT_BFP8, 2, true>(w, sums, q.error); break;
+        case 5: piece = stream_rows<BT_BFP8, 4, true>(w, sums, q.error); break;
+        case 6: piece = stream_rows<BT_BFP4, 1, false>(w, sums, q.error); break;
+        case 7: piece = stream_rows<BT_BFP4, 2, false>(w, sums, q.error); break;
+        case 8: piece = stream_rows<BT_BFP4, 4, false>(w, sums, q.error); break;
+        case 9: piece = stream_rows<BT_BFP4, 1, true>(w, sums, q.error); break;
+        case 10: piece = stream_rows<BT_BFP4, 2, true>(w, sums, q.error); break;
+        default: piece = stream_rows<BT_BFP4, 4, true>(w, sums, q.error); break;
       }
       // ---- this CTA is done with its part of the sub-panel ----
       if (lds32(sbase + kSmDead)) piece = piece_at(p, me, pieces);       // not from the ring's notes
       more = piece.x >> 30 != 3;
       const Piece pc = {(int)(piece.x & 0x3FFFFFFF), (int)piece.y, (int)piece.w, (int)piece.z, 8 * p.tg};
-      named_barrier(1, kConsumers + 32);       // every warp's sums are in place and, for an owner, the contributors' too
-      if (pc.me == pc.last) finish(p, sc, q.slot_floats, sums, pc);
-      else contribute(p, sc, q.slot_floats, sums, pc);
+      end_piece(p, sc, q.slot_floats, sums, pc, sbase, q.error);
       named_barrier(2, kConsumers + 32);       // the messenger may tell; the sums may be overwritten
     }
   }
@@ -742,20 +774,35 @@ int wait_for(const bt_gemv_op *ops, int i, int sets) {
   return w < 0 ? -1 : w;
 }
 
-// The ranges of a matmul's units: how many CTAs get one, and how large. Equal shares of all CTAs, so every SM streams
-// the same number of bytes whatever the shape, except where a matmul is so small that handing partial sums from CTA to
-// CTA (about 2 us: a store, a release, an acquire, a load) costs more than streaming the rest of a sub-panel: then a
-// share is a whole number of sub-panels. The choice depends on the shape only, never on a matmul's place in a queue:
-// the way the sums are grouped, and with it the last bit of a result, must not change with how matmuls are batched.
-constexpr int kWholePanel = 24;             // tile rows an SM streams in about the time of a hand-over
+// The ranges of a matmul's units. Sharing a sub-panel costs a hand-over of partial sums, a range that straddles sub-panels
+// a second pass through a sub-panel's end, and fewer CTAs than SMs cost time only while the busy ones cannot take in what
+// HBM delivers. So the candidates are: every sub-panel cut into 1, 2, ... ranges, as many as there are SMs for; whole
+// sub-panels, several to a CTA, when there are more of them than SMs; equal shares of all SMs that straddle. The one
+// with the least estimated time is taken, from the rates measured on 8192 x 28672 in steady state: HBM 6.3 TB/s, 50 GB/s
+// into one SM, and an SM's time for a tile row of four tiles (row_us). In ranges that straddle, a sub-panel shared by two or
+// three CTAs is handed over early: its contributors take it first. 4096 x 4096 is cut 4 ways (128 CTAs), 4096 x 14336 not
+// at all (112 CTAs), 576 x 1536 not at all, 1536 x 576 8 ways; a gate/up pair of 4096 x 14336 and 8192 x 28672 go in
+// equal shares. The choice depends on the shape only, never on a matmul's place in a queue: the way the sums are grouped,
+// and with it the last bit of a result, must not change with how matmuls are batched.
+constexpr float kHbmBytesPerUs = 6.3e6f, kSmBytesPerUs = 50e3f, kHandOverUs = 2.f, kEarlyUs = 1.2f, kFourSlotsUs = 0.4f, kStraddleUs = 1.f;
+float row_us(int tg) { return tg == 1 ? 0.07f : tg == 2 ? 0.1f : 0.145f; }
 void deal_units(GemvParams &p, int ctas) {
-  const int panels = (p.TC + kWC - 1) / kWC;
+  const int panels = (p.TC + kWC - 1) / kWC, matrices = p.pair ? 2 : 1;
   p.units = panels * p.KT;
-  const int equal = (p.units + ctas - 1) / ctas;
-  if (p.KT <= equal + kWholePanel && (panels + ctas - 1) / ctas * p.KT <= equal + kWholePanel) {
-    p.share = (panels + ctas - 1) / ctas * p.KT, p.extra = 0, p.active = (p.units + p.share - 1) / p.share;
-  } else {
-    p.active = min(ctas, p.units), p.share = p.units / p.active, p.extra = p.units % p.active;
+  const float hbm = (float)p.KT * p.TC * tile_bytes(p.fmt) * matrices / kHbmBytesPerUs;
+  const float row = max(row_us(p.tg) * matrices, kWC * tile_bytes(p.fmt) * matrices / kSmBytesPerUs);   // us per tile row, an SM on its own
+  auto stream = [&](float rows) { return max(hbm, rows * row); };
+  auto shared = [&](int ranges) { return ranges > 1 ? kHandOverUs + kFourSlotsUs * ((ranges - 1 + kSlots - 1) / kSlots) : 0.f; };
+  const int each = (panels + ctas - 1) / ctas;
+  // whole sub-panels, or equal shares that straddle
+  float best = stream((float)each * p.KT);
+  p.parts = 0, p.share = each * p.KT, p.extra = 0, p.active = (p.units + p.share - 1) / p.share;
+  const int busy = min(ctas, p.units), equal = p.units / busy;
+  const float straddling = stream((float)p.units / busy) + kStraddleUs + (p.KT <= 2 * equal ? kEarlyUs : shared(p.KT / equal + 2));
+  if (straddling < best) best = straddling, p.active = busy, p.share = equal, p.extra = p.units % busy;
+  for (int parts = 2; parts <= p.KT && parts * panels <= ctas; parts++) {
+    const float t = stream((float)((p.KT + parts - 1) / parts)) + shared(parts);
+    if (t < best) best = t, p.parts = parts, p.active = parts * panels;
   }
 }
 
@@ -807,6 +854,7 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
   for (int base = 0; base < n; base += kQueueMax) {
     Queue q = scratch;
     q.n = min(kQueueMax, n - base);
+    q.panels = 0;
     int tg_max = 1;
     for (int i = 0; i < q.n; i++) {
       const bt_gemv_op &o = ops[base + i];
@@ -817,6 +865,8 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       p.fmt = o.fmt, p.pair = o.epilogue == BT_EPI_GLU, p.tg = o.M <= 8 ? 1 : o.M <= 16 ? 2 : 4;
       p.wait_for = wait_for(ops + base, i, scratch.sets);
       p.turn = (int)(((long long)(base + i) * 101) % ctas);
+      if (p.wait_for >= 0) p.wait_panels = (q.op[p.wait_for].TC + kWC - 1) / kWC;
+      q.panels += (p.TC + kWC - 1) / kWC;
       deal_units(p, ctas);
       if (int s = map_x(p, o.x)) return s;
       tg_max = max(tg_max, p.tg);
@@ -850,7 +900,7 @@ Scratch scratch_at(unsigned char *set) {
 Queue workspace_scratch(uint64_t work) {
   Queue q{};
   unsigned char *base = as_ptr<unsigned char>(work);
-  q.error = reinterpret_cast<int *>(base + kWsError), q.ops_done = reinterpret_cast<int *>(base + kWsOpsDone);
+  q.error = reinterpret_cast<int *>(base + kWsError), q.ops_done = reinterpret_cast<int *>(base + kWsOpsDone), q.all_done = reinterpret_cast<int *>(base + kWsAllDone);
   q.sets = kSets;
   for (int s = 0; s < kSets; s++) q.set[s] = scratch_at(base + kWsSets + s * kSetBytes);
   q.slot_floats = (int)kSlotFloatsMax;
@@ -939,7 +989,7 @@ int bt_gemv_bfp_static(int device, int fmt, int epilogue, int M, int K, int N, u
   // its start is left alone, so that it stays until bt_gemv_check(device, 0, ...) reads it.
   BT_CUDA(cudaMemsetAsync(base + kWsOpsDone, 0, kStControlBytes - kWsOpsDone, as_stream(stream)));
   Queue scratch{};
-  scratch.error = reinterpret_cast<int *>(base + kWsError), scratch.ops_done = reinterpret_cast<int *>(base + kWsOpsDone);
+  scratch.error = reinterpret_cast<int *>(base + kWsError), scratch.ops_done = reinterpret_cast<int *>(base + kWsOpsDone), scratch.all_done = reinterpret_cast<int *>(base + kWsAllDone);
   scratch.sets = 1;
   scratch.set[0].panels_done = reinterpret_cast<int *>(base + 192), scratch.set[0].counters = reinterpret_cast<int *>(base + kStCounters);
   scratch.set[0].keys = reinterpret_cast<unsigned long long *>(base + kStKeys);
@@ -962,12 +1012,7 @@ int bt_gemv_check(int device, uint64_t work, uint64_t stream, int *error) {
   BT_CUDA(cudaMemcpyAsync(error, base + kWsError, 4, cudaMemcpyDeviceToHost, as_stream(stream)));
   BT_CUDA(cudaStreamSynchronize(as_stream(stream)));
   if (*error) {
-    if (!work) BT_CUDA(cudaMemsetAsync(base, 0, kStControlBytes, as_stream(stream)));
-    else {
-      BT_CUDA(cudaMemsetAsync(base, 0, kWsSets, as_stream(stream)));
-      for (int s = 0; s < kSets; s++)
-        BT_CUDA(cudaMemsetAsync(base + kWsSets + s * kSetBytes, 0, kSetCounters + 4 * (size_t)kMaxSubPanels, as_stream(stream)));
-    }
+    BT_CUDA(cudaMemsetAsync(base, 0, work ? kWsBytes : kStaticBytes, as_stream(stream)));
   }
   return BT_OK;
 }

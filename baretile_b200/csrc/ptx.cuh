@@ -190,6 +190,21 @@ __device__ __forceinline__ int ld_acquire_gpu(const int *p) {
 __device__ __forceinline__ void red_release_gpu(int *p, int v) {
   asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// The same, returning what the counter was, and seeing what everybody who added to it had done by then.
+__device__ __forceinline__ int atom_add_acq_rel_gpu(int *p, int v) {
+  int was;
+  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(was) : "l"(p), "r"(v) : "memory");
+  return was;
+}
+// Loads and stores of two words that other SMs store and load meanwhile: each word on its own is whole, nothing is ordered.
+__device__ __forceinline__ uint2 ld_relaxed2(const void *p) {
+  uint2 v;
+  asm volatile("ld.relaxed.gpu.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed2(void *p, uint2 v) {
+  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
+}
 // Orders this thread's earlier (observed) generic-proxy accesses before its later asynchronous-proxy ones (TMA and
 // bulk copies), here: global data another CTA wrote, about to be fetched by a bulk copy.
 __device__ __forceinline__ void fence_proxy_async() {
