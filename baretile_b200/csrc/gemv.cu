@@ -275,24 +275,6 @@ struct Piece {
   int toks;                // tokens whose sums are in shared memory: M rounded up to whole groups of 8
 };
 constexpr int kSlots = 4;  // contributors whose words are in flight together
-struct Slots {
-  uint2 w[kSlots];
-  __device__ __forceinline__ void load(const float *at, int slot_floats, int n) {
-#pragma unroll
-    for (int j = 0; j < kSlots; j++)
-      if (j < n) w[j] = ld_relaxed2(at + (size_t)j * slot_floats);
-  }
-  __device__ __forceinline__ void add_to(float2 &v, float *at, int slot_floats, int n, uint32_t &patience) {
-#pragma unroll
-    for (int j = 0; j < kSlots; j++)
-      if (j < n) {
-        float *from = at + (size_t)j * slot_floats;
-        while ((w[j].x == 0 || w[j].y == 0) && patience) w[j] = ld_relaxed2(from), patience--;
-        st_relaxed2(from, make_uint2(0, 0));
-        v.x += __uint_as_float(w[j].x), v.y += __uint_as_float(w[j].y);
-      }
-  }
-};
 __device__ __forceinline__ void send(float *to, float2 v) {
   const uint32_t x = __float_as_uint(v.x), y = __float_as_uint(v.y);
   st_relaxed2(to, make_uint2(x ? x : 0x80000000u, y ? y : 0x80000000u));
@@ -337,11 +319,30 @@ __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc
       continue;
     }
     for (int c = 0; c < others; c += kSlots, slot += kSlots * (size_t)slot_floats) {
-      Slots w, x;
-      w.load(slot, slot_floats, others - c);
-      if (pair) x.load(slot + 128, slot_floats, others - c);
-      w.add_to(v, slot, slot_floats, others - c, patience);
-      if (pair) x.add_to(u, slot + 128, slot_floats, others - c, patience);
+      uint2 w[kSlots], x[kSlots];
+      bool missing;
+      do {                                                                            // all of them in flight together, again until all are there
+        missing = false;
+#pragma unroll
+        for (int j = 0; j < kSlots; j++)
+          if (c + j < others) {
+            w[j] = ld_relaxed2(slot + (size_t)j * slot_floats);
+            if (pair) x[j] = ld_relaxed2(slot + (size_t)j * slot_floats + 128);
+          }
+#pragma unroll
+        for (int j = 0; j < kSlots; j++)
+          if (c + j < others) missing |= w[j].x == 0 || w[j].y == 0 || (pair && (x[j].x == 0 || x[j].y == 0));
+      } while (missing && patience && --patience);
+#pragma unroll
+      for (int j = 0; j < kSlots; j++)
+        if (c + j < others) {
+          st_relaxed2(slot + (size_t)j * slot_floats, make_uint2(0, 0));
+          v.x += __uint_as_float(w[j].x), v.y += __uint_as_float(w[j].y);
+          if (pair) {
+            st_relaxed2(slot + (size_t)j * slot_floats + 128, make_uint2(0, 0));
+            u.x += __uint_as_float(x[j].x), u.y += __uint_as_float(x[j].y);
+          }
+        }
     }
     v.x = v.x * unscale + __uint_as_float(a << 16), v.y = v.y * unscale + __uint_as_float(a & 0xFFFF0000u);
     a = addend(row + kConsumers / 64);
@@ -598,19 +599,21 @@ __device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
       const int first = cta_of(p, sp * p.KT), last = cta_of(p, (sp + 1) * p.KT - 1);
       int *counter = sc.counters + sp;
       if (me == last) zero_rows(p, sp);
+      // every contributor is past its last look at the counts of this launch
+      if (me == last && first != last && lane == 0) {
+        uint32_t spins = 0;
+        while (ld_acquire_gpu(counter) < last - first) {
+          if (++spins > kSpinLimit * 32) { atomicExch(q.error, 3); break; }
+          __nanosleep(100);
+        }
+        *counter = 0;                            // ready for the next matmul
+      }
+      __syncwarp();
       named_barrier(2, kConsumers + 32);
       if (me != last) {
         if (lane == 0) atomicAdd(counter, 1);    // the sums themselves say that they are there
         continue;
       }
-      // every contributor is past its last look at the counts of this launch
-      if (first != last && lane == 0) {
-        uint32_t spins = 0;
-        while (ld_acquire_gpu(counter) < last - first)
-          if (++spins > kSpinLimit * 64) { atomicExch(q.error, 3); break; }
-        *counter = 0;                            // ready for the next matmul
-      }
-      __syncwarp();
       if (p.epi == BT_EPI_ARGMAX) {
         // the last sub-panel to finish turns the keys into the answer and leaves the scratch as it found it
         int is_last = 0;
