@@ -58,7 +58,10 @@ struct GemmParams {
   int *error;
   float alpha;
   int M, KT, TC, epi, out_fp32, pair;
-  int row_blocks;            // blocks of 512 rows
+  int row_blocks;            // blocks of 512 rows, or of 256 where `half`
+  int half;                  // every pair takes 256 rows
+  int splits;                // pairs of CTAs that share a block, each with its part of K; their sums meet in `part`
+  float *part;               // [split][gate, up][tile_rows * 32][TC * 32] fp32, where splits > 1
   int whole;                 // pairs of CTAs that take a whole block of 512 rows x 256 MMA columns; the pairs after them
 };                           // take half a block (256 rows) each, so that the last wave of the grid is a short one
 
@@ -135,10 +138,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
   const uint32_t rank = cluster_ctarank();                          // 0: the leader, which issues the MMAs
   const int KB = (p.KT + 1) / 2;                                    // K blocks of 64; the last may hold one tile row
   const int pair_id = blockIdx.x >> 1;
-  const int block = pair_id < p.whole ? pair_id : p.whole + ((pair_id - p.whole) >> 1);   // blocks go down the rows first
+  const int split = pair_id % p.splits, kb0 = KB * split / p.splits, kbs = KB * (split + 1) / p.splits - kb0;   // this pair's K blocks
+  const int block = p.splits > 1 ? pair_id / p.splits : pair_id < p.whole ? pair_id : p.whole + ((pair_id - p.whole) >> 1);   // blocks go down the rows first
   const int bc = block / p.row_blocks;                              // block column: 128 output columns (pair) or 256
-  const int pair_m0 = (block % p.row_blocks) * 512 + (pair_id < p.whole ? 0 : ((pair_id - p.whole) & 1) * 256);   // first row of the pair's rows
-  const int MH = pair_id < p.whole && pair_m0 + 256 < p.M ? 2 : 1;  // halves of 256 rows this pair computes
+  const bool all_rows = !p.half && (p.splits > 1 || pair_id < p.whole);
+  const int pair_m0 = (block % p.row_blocks) * (p.half ? 256 : 512) + (p.half || all_rows ? 0 : ((pair_id - p.whole) & 1) * 256);   // first row of the pair's rows
+  const int MH = all_rows && pair_m0 + 256 < p.M ? 2 : 1;           // halves of 256 rows this pair computes
   if (pair_m0 >= p.M) return;                                       // (both CTAs of the pair: nothing here)
   const int run = p.pair ? bc : 2 * bc + (int)rank;                 // this CTA's run of 4 tile columns
   const int width = min(kPanel, p.TC - run * kPanel);               // tile columns it really has; <= 0: none
@@ -168,36 +173,36 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
     // ---- producer ----
     if (lane == 0) {
       const uint32_t leader_full = map_to_cta(full0, 0);
-      auto packed = [&](int kb) {           // the K block's packed tiles of this CTA's run: up to 2 tile rows x 4 tiles
+      auto packed = [&](int i) {            // the i-th K block's packed tiles of this CTA's run: up to 2 tile rows x 4 tiles
         if (width <= 0) return;
-        const int ps = kb % kStagesP, rows = min(2, p.KT - 2 * kb);
-        if (kb >= kStagesP) wait(pempty0 + 8 * ps, (kb / kStagesP - 1) & 1, 11);
+        const int kb = kb0 + i, ps = i % kStagesP, rows = min(2, p.KT - 2 * kb);
+        if (i >= kStagesP) wait(pempty0 + 8 * ps, (i / kStagesP - 1) & 1, 11);
         mbar_expect_tx(pfull0 + 8 * ps, rows * width * L::TB);
         const uint8_t *src = wsrc + (size_t)(2 * kb) * width * L::TB;
         if (width == kPanel) bulk_g2s(p_stage(ps), src, rows * kPanel * L::TB, pfull0 + 8 * ps);
         else
           for (int j = 0; j < rows; j++) bulk_g2s(p_stage(ps) + j * kPanel * L::TB, src + (size_t)j * width * L::TB, width * L::TB, pfull0 + 8 * ps);
       };
-      for (int kb = 0; kb < min(KB, kStagesP - 1); kb++) packed(kb);
-      for (int kb = 0; kb < KB; kb++) {
-        if (kb + kStagesP - 1 < KB) packed(kb + kStagesP - 1);
-        const int s = kb % kStagesAB;
-        if (kb >= kStagesAB) wait(empty0 + 8 * s, (kb / kStagesAB - 1) & 1, 12);
+      for (int i = 0; i < min(kbs, kStagesP - 1); i++) packed(i);
+      for (int i = 0; i < kbs; i++) {
+        if (i + kStagesP - 1 < kbs) packed(i + kStagesP - 1);
+        const int s = i % kStagesAB;
+        if (i >= kStagesAB) wait(empty0 + 8 * s, (i / kStagesAB - 1) & 1, 12);
         // the x tiles of BOTH CTAs complete on the leader's barrier, which the leader arms for all of them
         if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * MH * kABytes);
-        for (int mh = 0; mh < MH; mh++) tma_load_2d_pair(a_tile(s, mh), &amap, kb * kBK, row0(mh), leader_full + 8 * s);   // past M or K: zeros
+        for (int mh = 0; mh < MH; mh++) tma_load_2d_pair(a_tile(s, mh), &amap, (kb0 + i) * kBK, row0(mh), leader_full + 8 * s);   // past M or K: zeros
       }
     }
   } else if (warp == 1) {
     // ---- MMA issuer: the leader CTA alone ----
     if (lane == 0 && rank == 0) {
-      for (int kb = 0; kb < KB; kb++) {
-        const int s = kb % kStagesAB, steps = 2 * min(2, p.KT - 2 * kb);       // 16-deep MMAs in this K block
-        wait(full0 + 8 * s, (kb / kStagesAB) & 1, 13);
+      for (int i = 0; i < kbs; i++) {
+        const int s = i % kStagesAB, steps = 2 * min(2, p.KT - 2 * (kb0 + i));   // 16-deep MMAs in this K block
+        wait(full0 + 8 * s, (i / kStagesAB) & 1, 13);
         tc_fence_after();
         for (int mh = 0; mh < MH; mh++)
           for (int kk = 0; kk < steps; kk++)
-            umma_bf16_pair(tmem + mh * 256, smem_desc(a_tile(s, mh) + kk * 32), smem_desc(b_tile(s) + kk * 32), kIdesc, (kb | kk) != 0);
+            umma_bf16_pair(tmem + mh * 256, smem_desc(a_tile(s, mh) + kk * 32), smem_desc(b_tile(s) + kk * 32), kIdesc, (i | kk) != 0);
         umma_commit_pair(empty0 + 8 * s);
       }
       umma_commit_pair(acc_full);
@@ -206,12 +211,12 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
     // ---- dequant warps, then the epilogue ----
     const int d = warp - 2, c = d & 3, j = d >> 2;                  // this warp's tile column and tile row in a K block
     const uint32_t leader_full0 = map_to_cta(full0, 0);
-    for (int kb = 0; kb < KB; kb++) {
-      const int ps = kb % kStagesP, s = kb % kStagesAB;
-      if (width > 0) wait(pfull0 + 8 * ps, (kb / kStagesP) & 1, 14);
-      if (kb >= kStagesAB) wait(empty0 + 8 * s, (kb / kStagesAB - 1) & 1, 15);
+    for (int i = 0; i < kbs; i++) {
+      const int ps = i % kStagesP, s = i % kStagesAB;
+      if (width > 0) wait(pfull0 + 8 * ps, (i / kStagesP) & 1, 14);
+      if (i >= kStagesAB) wait(empty0 + 8 * s, (i / kStagesAB - 1) & 1, 15);
       tc_fence_after();
-      if (c < width && 2 * kb + j < p.KT) expand_tile<FMT>(p_stage(ps) + (j * kPanel + c) * L::TB, b_tile(s), c, j, lane);
+      if (c < width && 2 * (kb0 + i) + j < p.KT) expand_tile<FMT>(p_stage(ps) + (j * kPanel + c) * L::TB, b_tile(s), c, j, lane);
       fence_async_shared();
       __syncwarp();
       if (lane == 0) {
@@ -238,6 +243,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
         tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + mh * 256 + col, v);
         if (p.pair) tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + mh * 256 + 128 + col, u);
         tmem_ld_wait();
+        if (p.splits > 1) {
+          // sums of a part of K, as they are: reduce_kernel adds the parts
+          if (row < p.M) {
+            const size_t cols = (size_t)p.TC * 32, plane = (size_t)tile_rows * 32 * cols;
+            float *o = p.part + (size_t)split * (p.pair ? 2 : 1) * plane + (size_t)row * cols + tcol * 32;
+#pragma unroll
+            for (int i = 0; i < 8; i++) reinterpret_cast<uint4 *>(o)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            if (p.pair) {
+#pragma unroll
+              for (int i = 0; i < 8; i++) reinterpret_cast<uint4 *>(o + plane)[i] = make_uint4(u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
+            }
+          }
+          continue;
+        }
         const int in_tile = ((row >> 4) & 1) * 512 + (row & 15) * 16;    // datum index of (row, 0) in the tile
         float f[32];
         if (p.add) {
@@ -290,20 +309,91 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
   if (warp == 1) tmem_dealloc_pair(tmem, 512);
 }
 
-}  // namespace
+// The parts of K added in order, and the epilogue: one thread to four neighbouring columns of a row, 16 bytes of each part
+// (which L2 still holds) and 8 or 16 bytes of the result.
+__global__ void __launch_bounds__(256) reduce_kernel(const GemmParams p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int quads = p.TC * 8, tile_rows = (p.M + 31) / 32;
+  const unsigned i = blockIdx.x * 256u + threadIdx.x;
+  if (i >= (unsigned)tile_rows * 32 * quads) return;
+  const int row = i / quads, col = (i - row * quads) * 4, tcol = col >> 5, tr = row >> 5;
+  const size_t cols = (size_t)p.TC * 32, plane = (size_t)tile_rows * 32 * cols;
+  const float unscale = 18446744073709551616.f * p.alpha;           // 2^64: the weights were expanded times 2^-64
+  float f[4] = {0.f, 0.f, 0.f, 0.f}, g[4] = {0.f, 0.f, 0.f, 0.f};
+  const int at = ((row >> 4) & 1) * 512 + (row & 15) * 16 + ((col >> 4) & 1) * 256 + (col & 15);   // datum index in the tile
+  if (row < p.M) {
+    const float *from = p.part + (size_t)row * cols + col;
+    for (int s = 0; s < p.splits; s++) {
+      const float4 a = __ldcg(reinterpret_cast<const float4 *>(from));
+      f[0] += a.x, f[1] += a.y, f[2] += a.z, f[3] += a.w;
+      if (p.pair) {
+        const float4 b = __ldcg(reinterpret_cast<const float4 *>(from + plane));
+        g[0] += b.x, g[1] += b.y, g[2] += b.z, g[3] += b.w;
+      }
+      from += (p.pair ? 2 : 1) * plane;
+    }
+    uint2 a = make_uint2(0, 0);
+    if (p.add) a = *reinterpret_cast<const uint2 *>(p.add + (size_t)tr * p.add_row_stride + (size_t)tcol * 1024 + (p.add_row_stride ? at : ((col >> 4) & 1) * 256 + (col & 15)));
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t w = k < 2 ? a.x : a.y;
+      float x = f[k] * unscale;
+      if (p.add) x += __uint_as_float(k % 2 ? w & 0xFFFF0000u : w << 16);
+      if (p.pair) x = silu(x) * (g[k] * unscale);
+      else if (p.epi == BT_EPI_RELU) x = fmaxf(x, 0.f);
+      else if (p.epi == BT_EPI_SILU) x = silu(x);
+      f[k] = x;
+    }
+  }
+  const size_t o = ((size_t)tr * p.TC + tcol) * 1024 + at;
+  if (p.out_fp32) *reinterpret_cast<float4 *>(static_cast<float *>(p.out) + o) = make_float4(f[0], f[1], f[2], f[3]);
+  else *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(p.out) + o) = make_uint2(bf16_half_up(f[0]) | bf16_half_up(f[1]) << 16, bf16_half_up(f[2]) | bf16_half_up(f[3]) << 16);
+}
 
-extern "C" {
+// How the blocks of a matmul are dealt out to the `slots` pairs of CTAs that fit on the GPU at once: pairs, and in `p` what
+// they do. With at least as many blocks as slots the pairs take whole blocks, and when they do not fill the last wave, the
+// blocks of that wave are cut in two, so that it takes half as long (as long as the halves still fit in one wave). With
+// fewer, which is what prompts of some hundred rows and few columns have, blocks of 256 rows and blocks whose K is shared
+// by several pairs keep more of the GPU busy, at the price of fp32 parts written and read once more. The estimate: a pair
+// takes kBlockUs for a K block of 256 rows and kFixedUs for everything else; the parts move at 3 TB/s and cost another
+// launch. 2048 rows of 14336 x 4096 stay as they are (64 blocks), 77 rows of 5632 x 2048 (8 blocks of 88 K blocks) go in 9
+// parts.
+constexpr float kBlockUs = 0.42f, kFixedUs = 5.f, kReduceUs = 3.f, kPartBytesPerUs = 3e6f;
+int deal_blocks(GemmParams &p, int slots, size_t part_bytes) {
+  const int runs = (p.TC + kPanel - 1) / kPanel, columns = p.pair ? runs : (runs + 1) / 2, KB = (p.KT + 1) / 2, tile_rows = (p.M + 31) / 32;
+  p.row_blocks = (p.M + 511) / 512, p.half = 0, p.splits = 1;
+  const int blocks = p.row_blocks * columns;
+  p.whole = blocks;
+  if (blocks >= slots) {
+    const int last = blocks % slots;
+    if (last > 0 && 2 * last <= slots && p.M > 256) p.whole = blocks - last;
+    return p.whole + 2 * (blocks - p.whole);
+  }
+  float best = 1e30f;
+  int pairs = blocks;
+  const float plane = (float)tile_rows * 32 * p.TC * 32 * 4 * (p.pair ? 2 : 1);
+  for (int half = 0; half <= (p.M > 256 ? 1 : 0); half++) {
+    const int rows = half ? (p.M + 255) / 256 : p.row_blocks, b = rows * columns, height = half || p.M <= 256 ? 1 : 2;
+    for (int splits = 1; splits == 1 || (b * splits <= slots && splits <= KB && splits * (double)plane <= part_bytes); splits++) {
+      const int waves = (b * splits + slots - 1) / slots;
+      const float us = waves * (kFixedUs + (KB + splits - 1) / splits * kBlockUs * height) + (splits > 1 ? kReduceUs + 2 * splits * plane / kPartBytesPerUs : 0.f);
+      if (us < best) best = us, pairs = b * splits, p.half = half, p.splits = splits, p.row_blocks = rows, p.whole = b;
+    }
+  }
+  return pairs;
+}
 
-int bt_gemm_bfp(int device, int fmt, int epilogue, int M, int K, int N, uint64_t a, uint64_t w, uint64_t w2, uint64_t add, int add_rows,
-                float alpha, uint64_t out, int out_dtype, uint64_t work, uint64_t stream) {
-  BT_REQUIRE(fmt == BT_BFP8 || fmt == BT_BFP4, "bt_gemm_bfp: weights must be bfp8 (8) or bfp4 (4), not %d", fmt);
-  BT_REQUIRE(epilogue >= BT_EPI_NONE && epilogue <= BT_EPI_GLU, "bt_gemm_bfp: the epilogue is none, relu, silu or glu, not %d", epilogue);
+// Argument checks and launches of both entry points.
+int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N, uint64_t a, uint64_t w, uint64_t w2, uint64_t add, int add_rows, float alpha,
+         uint64_t out, int out_dtype, uint64_t part, size_t part_bytes, uint64_t work, uint64_t stream) {
+  BT_REQUIRE(fmt == BT_BFP8 || fmt == BT_BFP4, "%s: weights must be bfp8 (8) or bfp4 (4), not %d", who, fmt);
+  BT_REQUIRE(epilogue >= BT_EPI_NONE && epilogue <= BT_EPI_GLU, "%s: the epilogue is none, relu, silu or glu, not %d", who, epilogue);
   const bool pair = epilogue == BT_EPI_GLU;
-  BT_REQUIRE(M >= 1 && K > 0 && N > 0 && K % 32 == 0, "bt_gemm_bfp: needs M >= 1, N >= 1 and K a positive multiple of 32: %d x %d x %d", M, K, N);
-  BT_REQUIRE(a && w && out && work && a % 16 == 0 && w % 16 == 0 && out % 16 == 0, "bt_gemm_bfp: needs 16-byte aligned device addresses");
-  BT_REQUIRE(pair == (w2 != 0) && w2 % 16 == 0, "bt_gemm_bfp: w2 goes with the GLU epilogue, and only with it");
-  BT_REQUIRE(add % 16 == 0 && (!add || add_rows == 1 || add_rows == M), "bt_gemm_bfp: the addend is 16-byte aligned and has 1 or M rows, not %d", add_rows);
-  BT_REQUIRE(out_dtype == BT_BF16 || out_dtype == BT_FP32, "bt_gemm_bfp: results are bf16 or fp32");
+  BT_REQUIRE(M >= 1 && K > 0 && N > 0 && K % 32 == 0, "%s: needs M >= 1, N >= 1 and K a positive multiple of 32: %d x %d x %d", who, M, K, N);
+  BT_REQUIRE(a && w && out && work && a % 16 == 0 && w % 16 == 0 && out % 16 == 0, "%s: needs 16-byte aligned device addresses", who);
+  BT_REQUIRE(pair == (w2 != 0) && w2 % 16 == 0, "%s: w2 goes with the GLU epilogue, and only with it", who);
+  BT_REQUIRE(add % 16 == 0 && (!add || add_rows == 1 || add_rows == M), "%s: the addend is 16-byte aligned and has 1 or M rows, not %d", who, add_rows);
+  BT_REQUIRE(out_dtype == BT_BF16 || out_dtype == BT_FP32, "%s: results are bf16 or fp32", who);
   if (int s = use_device(device)) return s;
   alignas(64) CUtensorMap amap;
   const uint64_t dims[2] = {(uint64_t)K, (uint64_t)M}, strides[1] = {(uint64_t)K * 2};
@@ -313,15 +403,10 @@ int bt_gemm_bfp(int device, int fmt, int epilogue, int M, int K, int N, uint64_t
   p.w[0] = as_ptr<uint8_t>(w), p.w[1] = as_ptr<uint8_t>(w2), p.add = as_ptr<uint16_t>(add), p.out = as_ptr<void>(out), p.error = as_ptr<int>(work);
   p.alpha = alpha, p.M = M, p.KT = K / 32, p.TC = (N + 31) / 32, p.epi = epilogue, p.out_fp32 = out_dtype == BT_FP32, p.pair = pair;
   p.add_row_stride = add && add_rows > 1 ? (size_t)p.TC * 1024 : 0;
-  const int runs = (p.TC + kPanel - 1) / kPanel, columns = pair ? runs : (runs + 1) / 2;
-  p.row_blocks = (M + 511) / 512;
-  // One pair of CTAs per pair of SMs is resident. When the blocks do not fill the last wave, the blocks of that wave
-  // are cut in two, so that it takes half as long (as long as the halves still fit in one wave).
+  p.part = as_ptr<float>(part);
   int sms = 0;
   BT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  const int blocks = p.row_blocks * columns, slots = sms / 2 > 0 ? sms / 2 : 1, last = blocks % slots;
-  p.whole = blocks >= slots && last > 0 && 2 * last <= slots && M > 256 ? blocks - last : blocks;
-  const int pairs = p.whole + 2 * (blocks - p.whole);
+  const int pairs = deal_blocks(p, sms / 2 > 0 ? sms / 2 : 1, part_bytes);
   static bool configured[64] = {};
   if (!configured[device & 63]) {
     BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP8>::BYTES + 1024));
@@ -339,7 +424,34 @@ int bt_gemm_bfp(int device, int fmt, int epilogue, int M, int K, int N, uint64_t
   cfg.attrs = attr, cfg.numAttrs = 1;
   if (fmt == BT_BFP8) BT_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP8>, p, amap));
   else BT_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP4>, p, amap));
-  return launched("gemm_kernel");
+  if (int s = launched("gemm_kernel")) return s;
+  if (p.splits == 1) return BT_OK;
+  // its blocks come up while the last of gemm_kernel drain, and wait there until that is complete
+  cudaLaunchConfig_t add_up{};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  add_up.gridDim = dim3((unsigned)(((size_t)(M + 31) / 32 * 32 * p.TC * 8 + 255) / 256)), add_up.blockDim = dim3(256), add_up.stream = as_stream(stream);
+  add_up.attrs = attr, add_up.numAttrs = 1;
+  BT_CUDA(cudaLaunchKernelEx(&add_up, reduce_kernel, p));
+  return launched("reduce_kernel");
+}
+
+}  // namespace
+
+extern "C" {
+
+int bt_gemm_bfp(int device, int fmt, int epilogue, int M, int K, int N, uint64_t a, uint64_t w, uint64_t w2, uint64_t add, int add_rows,
+                float alpha, uint64_t out, int out_dtype, uint64_t work, uint64_t stream) {
+  return gemm("bt_gemm_bfp", device, fmt, epilogue, M, K, N, a, w, w2, add, add_rows, alpha, out, out_dtype, 0, 0, work, stream);
+}
+
+int bt_gemm_tiles(int device, int fmt, int epilogue, int M, int K, int N, uint64_t x, uint64_t w, uint64_t w2, uint64_t add, int add_rows,
+                  float alpha, uint64_t out, int out_dtype, uint64_t scratch, size_t scratch_bytes, uint64_t work, uint64_t stream) {
+  BT_REQUIRE(M >= 1 && K > 0 && K % 32 == 0, "bt_gemm_tiles: needs M >= 1 and K a positive multiple of 32: %d x %d", M, K);
+  const size_t rows = ((size_t)M * K * 2 + 255) / 256 * 256;
+  BT_REQUIRE(x && x % 16 == 0 && scratch && scratch % 256 == 0 && scratch_bytes >= rows, "bt_gemm_tiles: needs x and at least %zu bytes of 256-byte aligned scratch, got %zu", rows, scratch_bytes);
+  if (int s = bt_untilize(device, 2, x, scratch, 1, M, K, stream)) return s;
+  return gemm("bt_gemm_tiles", device, fmt, epilogue, M, K, N, scratch, w, w2, add, add_rows, alpha, out, out_dtype, scratch + rows, scratch_bytes - rows, work, stream);
 }
 
 }  // extern "C"

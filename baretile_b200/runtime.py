@@ -315,7 +315,7 @@ class Runtime:
     is accepted for parity; the entry point sizes its own grid."""
     if not self.active: self.check()
     if units is not None and not 1 <= int(units) < 2**32: raise ValueError("launch units must be in [1, 2**32 - 1]")
-    if self.side is not None and kernel in ("bt_gemv_bfp", "bt_gemv_queue", "bt_gemm_bfp"):
+    if self.side is not None and kernel in ("bt_gemv_bfp", "bt_gemv_queue", "bt_gemm_bfp", "bt_gemm_tiles"):
       raise RuntimeError("a matmul uses the runtime's scratch and runs on its own stream, not in a beside block")
     if self.log is not None: self.log.append((kernel, args, units, name))
     if self.pending is not None and kernel == "bt_gemv_bfp":

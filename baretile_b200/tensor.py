@@ -16,6 +16,7 @@ from baretile_b200 import _lib
 from baretile_b200.tensix import BFP, FMT_CODE, ITEMSIZE, tile_bytes
 
 DIMS = 5
+PARTS = 48 << 20   # bytes at most that a matmul of many rows borrows for sums of parts of K
 FIDELITY = 4   # accepted for parity; products are always exact here (baretile/tensor.py:12)
 EPILOGUE = {"none": 0, "relu": 1, "silu": 2, "glu": 3, "argmax": 4}
 NAMES = {(dtype, epilogue): f"matmul {dtype} {epilogue}" for dtype in BFP for epilogue in EPILOGUE}
@@ -387,13 +388,13 @@ def _launch_matmul(rt, e, epilogue, out, rows, arg=(0, 0), arg_base=0):
     if rows > 32: raise ValueError("the fused pick takes up to 32 rows")
   out_dtype = FMT_CODE[out.dtype] if out is not None else 0
   if rows > 32:
-    # many rows: the tensor-core kernel, which reads x row-major, whole tiles wide
-    flat = rt.dram_alloc(2 * rows * K)
+    # many rows: the tensor-core kernel, which lays x out by rows in scratch lent to it, and adds up parts of K there
+    size = 2 * rows * K + 256 + min(PARTS, 16 * 4 * out.tiles * 1024 * (2 if w2 else 1))
+    scratch = rt.dram_alloc(size)
     try:
-      rt.launch("bt_untilize", (2, x.addr, flat, 1, rows, K), name="rows")
-      rt.launch("bt_gemm_bfp", (fmt, code, rows, K, w.cols, flat, w.addr, w2.addr if w2 else 0, add.addr if add else 0,
-                                add.rows if add else 0, alpha, out.addr, out_dtype, rt.work), name=f"prefill {w.dtype} {epilogue}")
-    finally: rt.dram_free(flat)
+      rt.launch("bt_gemm_tiles", (fmt, code, rows, K, w.cols, x.addr, w.addr, w2.addr if w2 else 0, add.addr if add else 0,
+                                  add.rows if add else 0, alpha, out.addr, out_dtype, scratch, size, rt.work), name=f"prefill {w.dtype} {epilogue}")
+    finally: rt.dram_free(scratch)
     return
   rt.launch("bt_gemv_bfp", (fmt, code, rows, K, w.tc * 32, x.addr, w.addr, w2.addr if w2 else 0, add.addr if add else 0, alpha,
                             out.addr if out is not None else 0, out_dtype, arg[0], arg[1], arg_base, rt.work, rt.work_bytes), name=NAMES[w.dtype, epilogue])

@@ -129,3 +129,22 @@ def test_results_stay_inside_their_tiles(rt):
   tiles = raw_tiles(rt, y).view(np.uint16).reshape(3, 5, 1024)
   full = o.untilize(tiles.reshape(15, 1024), 1, 96, 160)[0]
   assert not full[70:].any() and not full[:, 130:].any()            # rows past M and columns past N are zero
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+@pytest.mark.parametrize("m,k,n", [(33, 64, 32), (33, 4096, 64), (77, 2080, 330), (256, 1024, 128), (257, 2112, 96), (300, 8192, 288), (520, 1536, 1000)])
+def test_shared_k_and_half_blocks(rt, fmt, m, k, n):
+  # few blocks: their K is shared by several pairs of CTAs (one K block each at the least, an odd last tile row in the last
+  # part), blocks of 256 rows; every epilogue of the kernel that adds the parts up
+  rng = np.random.default_rng(m + k + n)
+  xi, wi = rng.integers(-2, 3, (m, k)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32)
+  got, _ = run(rt, xi, wi, fmt, dtype="fp32")
+  assert np.array_equal(got, xi @ wi)
+  x, w, w2 = acts(rng, m, k), weights(rng, k, n, stress=False), weights(rng, k, n, stress=False)
+  for add in (bf16(rng.normal(0, 1, (1, n))), bf16(rng.normal(0, 1, (m, n)))):
+    got, ref = run(rt, x, w, fmt, "relu", add=add, alpha=0.5)
+    check_matmul(got, x, None, ref, 1e-2)
+  got, ref = run(rt, x, w, fmt, "silu", dtype="fp32")
+  check_matmul(got, x, None, ref, 1e-4)
+  got, ref = run(rt, x, w, fmt, "glu", w2)
+  check_matmul(got, x, None, ref, 1e-2)
