@@ -11,6 +11,7 @@ from baretile_b200 import _lib
 
 ALIGN = 256            # allocation granularity in bytes
 ARENA = 1 << 30        # device memory is taken from the driver in pieces of at least this size
+KEPT = 32              # freed pieces of device memory kept by size before they join the holes around them
 LARGE = 256 << 10      # host copies from this size on go through page-locked staging buffers; below, their set-up costs more than it saves
 TIMES = 1024           # launches whose timing records are kept (baretile/runtime.py: TIMES)
 
@@ -244,6 +245,7 @@ class Runtime:
     self.start, self.end = start or self.cores[0], end or self.cores[-1]
     self.active, self.timing = False, timing
     self.holes, self.used, self.arenas = [], {}, []
+    self.kept, self.kept_count = {}, 0               # size -> addresses freed lately and not yet joined with the holes around them
     self.sent = {}                                   # launch number % TIMES -> (name, start event, end event)
     self.numbers = {}                                # 1 x 1 tensors of Python numbers, made once
     self.log = None
@@ -295,7 +297,7 @@ class Runtime:
     for ptr in getattr(self, "pinned", []): _lib.lib().bt_host_free(ptr)
     self.pinned = []
     for addr, _ in self.arenas: _lib.lib().bt_free(self.device, addr)
-    self.arenas, self.holes = [], []
+    self.arenas, self.holes, self.kept, self.kept_count = [], [], {}, 0
     self.used.clear()
     _lib.lib().bt_stream_destroy(self.device, self.stream)
     self.chip.taken.pop(id(self), None)
@@ -409,6 +411,13 @@ class Runtime:
     """First free hole that is big enough (baretile/runtime.py:791-812); a new arena from the driver when none is."""
     if not self.active: self.check()
     size = max(ALIGN, -(-size // ALIGN) * ALIGN)
+    kept = self.kept.get(size)
+    if kept:                                         # a step frees and takes the same sizes again and again
+      addr = kept.pop()
+      self.kept_count -= 1
+      self.used[addr] = size
+      return addr
+    if self.kept_count and not any(room >= size for _, room in self.holes): self._join_kept()
     for attempt in range(2):
       for i, (addr, room) in enumerate(self.holes):
         if room >= size:
@@ -432,7 +441,14 @@ class Runtime:
     if self.recording is not None:   # a replay will use this memory again
       self.recording.held.append((addr, size))
       return
-    _add_hole(self.holes, addr, size, self.arenas)
+    self.kept.setdefault(size, []).append(addr)
+    self.kept_count += 1
+    if self.kept_count > KEPT: self._join_kept()
+
+  def _join_kept(self):
+    for size, addrs in self.kept.items():
+      for addr in addrs: _add_hole(self.holes, addr, size, self.arenas)
+    self.kept, self.kept_count = {}, 0
 
   def record(self): return Recording(self)
 

@@ -221,18 +221,22 @@ class Tensor:
 
   # ---- expressions ----
   def _node(self, op, srcs, rows=None, cols=None, dtype=None):
-    # an expression's shape and operands are its sources', which were checked when they were made
-    t, rows, cols, batch = Tensor.__new__(Tensor), rows or self.rows, cols or self.cols, self.batch
-    tr, tc = rows + 31 >> 5, cols + 31 >> 5
-    t.__dict__ = {"rt": self.rt, "rows": rows, "cols": cols, "batch": batch, "op": op, "srcs": srcs, "dtype": dtype or self.dtype, "lead": (batch,),
-                  "tr": tr, "tc": tc, "tiles": batch * tr * tc}
+    # an expression's shape and operands are its sources', which were checked when they were made; most expressions are
+    # only parts of others, so what storage they would take is worked out when it is asked for (__getattr__)
+    t = Tensor.__new__(Tensor)
+    t.__dict__ = {"rt": self.rt, "rows": rows or self.rows, "cols": cols or self.cols, "batch": self.batch, "op": op, "srcs": srcs, "dtype": dtype or self.dtype}
     return t
+  def __getattr__(self, name):
+    if name not in ("tr", "tc", "tiles", "lead") or "rows" not in self.__dict__: raise AttributeError(f"{type(self).__name__!r} object has no attribute {name!r}")
+    self.lead, self.tr, self.tc = (self.batch,), self.rows + 31 >> 5, self.cols + 31 >> 5
+    self.tiles = self.batch * self.tr * self.tc
+    return self.__dict__[name]
   def relu(self): return self._node("relu", (self,))
   def silu(self): return self._node("silu", (self,))
   def __mul__(self, x):
     if isinstance(x, (int, float)): return self._node("scale", (self, float(x)))
     self._same_runtime(x)
-    if x.shape != self.shape: raise ValueError(f"cannot broadcast {self.shape} with {x.shape}")
+    if (x.rows, x.cols, x.batch) != (self.rows, self.cols, self.batch): raise ValueError(f"cannot broadcast {self.shape} with {x.shape}")
     return self._node("mul", (self, x))
   __rmul__ = __mul__
   def __add__(self, x):
@@ -361,7 +365,7 @@ def _plan(t):
     for a, b in (t.srcs, t.srcs[::-1]):
       if a.op == "silu" and a.srcs[0].op == "matmul" and b.op == "matmul":
         (x, wg), (y, wu) = a.srcs[0].srcs, b.srcs
-        if x is y and wg.dtype == wu.dtype and wg.shape == wu.shape: return "glu", (x, wg, wu, 1.0, None)
+        if x is y and (wg.dtype, wg.rows, wg.cols, wg.batch) == (wu.dtype, wu.rows, wu.cols, wu.batch): return "glu", (x, wg, wu, 1.0, None)
     return None
   e = _linear(t)
   return None if e is None else ("none", e)
