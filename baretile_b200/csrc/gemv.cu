@@ -41,7 +41,7 @@ using namespace bt;
 
 namespace {
 
-constexpr int kWC = kPanel;                 // tile columns of a sub-panel = one run of the streaming layout
+constexpr int kWC = kPanel;                 // tile columns of a run of the streaming layout, and of a sub-panel but for small matmuls
 constexpr int kCW = 16;                     // consumer warps of the CTA; an SM holds one CTA
 constexpr int kConsumers = kCW * 32;
 constexpr int kThreads = (kCW + 3) * 32;    // plus two producer warps and a messenger
@@ -56,9 +56,11 @@ constexpr int kSmFull = 0, kSmEmpty = 128;  // mbarriers: a stage's weights and 
 constexpr int kSmHeld = 256;                // uint32[2][kBars]: ring bytes of each stage in the ring, as each producer warp noted them
 constexpr int kSmDead = 384;                // int: a wait on a stage gave up; nobody in this CTA waits for the ring any more
 constexpr int kSmStages = 512;              // Stage[kBars]: what the weight warp tells the consumers about each stage
-constexpr int kSmSums = 1024;               // float[k groups x matrices][tokens][kSumStride]
-constexpr int kSumStride = 132;             // floats from one token's 128 channels to the next: 4 past 128, so that the fragment stores meet no bank twice
-constexpr int sums_bytes(int tg) { return 4 * 8 * tg * kSumStride * 4; }
+constexpr int kSmSums = 1024;               // float[k groups x matrices, or tile rows x matrices][tokens][channels of a sub-panel + 4]
+// Floats from one token's channels to the next: 4 past the channels, so that the fragment stores meet no bank twice.
+__host__ __device__ constexpr int sum_stride(int lw) { return (32 << lw) + 4; }
+constexpr int sums_bytes(int tg) { return 4 * 8 * tg * sum_stride(2) * 4; }
+constexpr int kSmallSums = 84 * 1024;       // bytes at most that the sums of a small matmul's tile rows take of the ring
 constexpr int kSmemBytes = 227 * 1024;
 
 // Scratch layout (byte offsets into the caller's workspace). Two matmuls of a queue may be in flight at once, so
@@ -76,35 +78,39 @@ constexpr size_t kSetBytes = kSetPartials + (size_t)kMaxCtas * kSlotFloatsMax * 
 constexpr int kSets = 2;                                         // matmuls of a queue in flight at most
 constexpr size_t kWsBytes = kWsSets + kSets * kSetBytes;
 
-// The shape of a stage for one kind of matmul: format, one matrix or a gate/up pair, token groups of 8 rows.
+// The shape of a stage for one kind of matmul: format, one matrix or a gate/up pair, token groups of 8 rows, columns of a
+// sub-panel (1 << lw).
 struct Geometry {
   int tb;        // bytes of a packed tile
-  int t;         // tile rows a warp takes per stage
   int ups;       // units (tile rows) per stage
   int matrix;    // bytes of one matrix's part of a stage
   int w_bytes;   // all weights of a stage; the x tiles follow
   int xb;        // bytes of an x tile staged: token rows 0-7, 0-15 or all
   int stage;     // bytes of a stage
 };
-// Large stages: a stage costs its waits, arrivals and copies whatever its size, about 430 cycles of a warp's time on an
-// 8192 x 28672 matmul, and a ring of three or four stages of 35-55 KB is enough to cover the latency of HBM.
-__host__ __device__ constexpr int stage_rows_per_warp(int fmt, int tg) { return fmt == BT_BFP4 && tg < 4 ? 4 : 2; }
-__host__ __device__ constexpr Geometry geometry(int fmt, bool pair, int tg) {
+// Tile rows a warp takes per stage. Large stages: a stage costs its waits, arrivals and copies whatever its size, about
+// 430 cycles of a warp's time on an 8192 x 28672 matmul, and a ring of three or four stages of 35-55 KB is enough to cover
+// the latency of HBM. In narrow sub-panels, whose rows go round more warps, x would outgrow the weights.
+__host__ __device__ constexpr int stage_rows_per_warp(int fmt, int tg, int lw) {
+  return lw == 2 ? (fmt == BT_BFP4 && tg < 4 ? 4 : 2) : lw == 1 ? (tg == 4 ? 1 : 2) : tg == 1 ? 2 : 1;
+}
+__host__ __device__ constexpr Geometry geometry(int fmt, bool pair, int tg, int lw) {
   Geometry g{};
-  g.tb = tile_bytes(fmt), g.t = stage_rows_per_warp(fmt, tg);
-  g.ups = (pair ? 2 : 4) * g.t;
-  g.matrix = g.ups * kWC * g.tb;
+  g.tb = tile_bytes(fmt);
+  g.ups = (kCW >> lw >> (pair ? 1 : 0)) * stage_rows_per_warp(fmt, tg, lw);
+  g.matrix = (g.ups << lw) * g.tb;
   g.w_bytes = (pair ? 2 : 1) * g.matrix;
   g.xb = 512 * tg;
   g.stage = g.w_bytes + g.ups * g.xb;
   return g;
 }
-static_assert(geometry(BT_BFP8, false, 1).w_bytes % 128 == 0 && geometry(BT_BFP4, false, 1).w_bytes % 128 == 0 && geometry(BT_BFP4, true, 4).w_bytes % 128 == 0,
-              "x tiles land on 128-byte boundaries");
+static_assert(geometry(BT_BFP8, false, 1, 2).w_bytes % 128 == 0 && geometry(BT_BFP4, true, 4, 2).matrix % 128 == 0 && geometry(BT_BFP4, true, 2, 0).matrix % 128 == 0 &&
+              geometry(BT_BFP8, true, 4, 1).matrix % 128 == 0 && geometry(BT_BFP4, true, 4, 0).matrix % 128 == 0, "tiled copies land on 128-byte boundaries");
 
 // One matmul of the queue, as the kernel sees it.
 struct alignas(64) GemvParams {
   CUtensorMap xmap;           // x as (16-datum face rows of the staged tokens, faces, tile columns)
+  CUtensorMap wmap[2];        // for sub-panels narrower than a run: the weights as (a tile's bytes, the four tiles of a run's tile row, tile rows)
   const uint8_t *w[2];
   const uint16_t *add;
   void *out;
@@ -115,10 +121,22 @@ struct alignas(64) GemvParams {
   int fmt, pair, tg;
   int wait_for, wait_panels;  // the matmul of the launch that must be complete before this one starts (-1: none), and its sub-panels
   int turn;                   // CTA c takes the unit range (c + turn) % CTAs
+  int lw, panels;             // tile columns of a sub-panel are 1 << lw, and there are so many sub-panels
+  int tiled;                  // wmap is used
+  int small;                  // every tile row's sums are kept apart and added in order at the end
   int units;                  // tile rows of all sub-panels
   int active;                 // CTAs with a range
   int parts;                  // > 0: every sub-panel is cut into so many ranges; 0: ranges of equal size whatever they straddle,
   int share, extra;           // range b then starts at b * share + min(b, extra), and the last one ends at units
+};
+
+// Where sub-panel `sp` lies: 1 << lw tile columns from `col` on, fewer at the end of a matrix, part of a run of `run_width`.
+struct Columns {
+  int run, run_width, col, width;
+  __device__ __forceinline__ Columns(const GemvParams &p, int sp) {
+    run = sp >> (2 - p.lw), col = run * kWC + ((sp & ((1 << (2 - p.lw)) - 1)) << p.lw);
+    run_width = min(kWC, p.TC - run * kWC), width = min(1 << p.lw, p.TC - col);
+  }
 };
 
 // Waits for a phase of a stage's mbarrier, with a limit. A wait that gives up marks the CTA: its sums are worthless from
@@ -160,7 +178,8 @@ struct Queue {
 struct alignas(32) Stage {
   uint32_t at;                // shared-memory address of its weights; the x tiles follow the matmul's w_bytes further
   int rows, width;            // tile rows, and tile columns of the sub-panel
-  int ends;                   // bits 0-1: 1, the CTA's part of the sub-panel ends with it; 3, and so does its part of the matmul; bit 2: all rows, four columns
+  int ends;                   // bits 0-1: 1, the CTA's part of the sub-panel ends with it; 3, and so does its part of the matmul; bit 2: all rows,
+                              // four columns; from bit 3 on the first tile row
   int sp, first, cta, end;    // the sub-panel, the first range that shares it, this CTA's and the last one, the owner
 };
 static_assert(sizeof(Stage) * kBars <= kSmSums - kSmStages, "room for the stages' notes");
@@ -260,7 +279,7 @@ __device__ __forceinline__ unsigned long long pick_key(float v, int column) {
 
 // ---- a sub-panel's end: the CTA's warps, then the CTAs that share it ---------------------------------------------
 // The warps have left their sums in shared memory, [k group][matrix][token][channel]. Every consumer thread takes
-// one pair of neighbouring channels and every eighth token, adds the k groups in order and either stores the sums
+// one pair of neighbouring channels and every eighth token (or sixteenth, or thirty-second), adds the k groups in order and either stores the sums
 // in the CTA's slot of partial sums (a contributor) or adds the contributors' slots in CTA order, so that results do
 // not depend on timing, and runs the epilogue (the sub-panel's owner). Elementwise over 512 threads: one small piece of
 // code for every kind of matmul. Everybody waits for it, so what counts is its chain of dependent steps and the
@@ -274,7 +293,7 @@ struct Piece {
   int first, last, me;     // the ranges that share it, and this CTA's
   int toks;                // tokens whose sums are in shared memory: M rounded up to whole groups of 8
 };
-constexpr int kSlots = 4;  // contributors whose words are in flight together
+constexpr int kSlots = 4;  // words of contributors' slots that a thread has in flight together
 __device__ __forceinline__ void send(float *to, float2 v) {
   const uint32_t x = __float_as_uint(v.x), y = __float_as_uint(v.y);
   st_relaxed2(to, make_uint2(x ? x : 0x80000000u, y ? y : 0x80000000u));
@@ -283,96 +302,116 @@ __device__ __forceinline__ void send(float *to, float2 v) {
 __device__ __forceinline__ void zero_rows(const GemvParams &p, int sp) {
   const int M = p.M, lane = threadIdx.x & 31;
   if (M == 1 || p.epi == BT_EPI_ARGMAX || p.out_fp32 == 2) return;
-  const int per_row = p.out_fp32 ? 4 : 2, first = sp * kWC;                         // 16-byte words of a face row
-  for (int face = 0; face < 4 * min(kWC, p.TC - first); face++) {                   // two lower and two upper faces of each tile
-    uint4 *rows = static_cast<uint4 *>(p.out) + ((size_t)first * 4 + face) * 16 * per_row;
+  const Columns at(p, sp);
+  const int per_row = p.out_fp32 ? 4 : 2;                                           // 16-byte words of a face row
+  for (int face = 0; face < 4 * at.width; face++) {                                 // two lower and two upper faces of each tile
+    uint4 *rows = static_cast<uint4 *>(p.out) + ((size_t)at.col * 4 + face) * 16 * per_row;
     for (int i = max(M - (face & 2) * 8, 0) * per_row + lane; i < 16 * per_row; i += 32) rows[i] = make_uint4(0, 0, 0, 0);
   }
 }
 __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc, uint32_t smem, int *error) {
-  const int pr = threadIdx.x & 63, M = p.M, epi = p.epi, fp32 = p.out_fp32, step = p.pair ? 256 : 128;
+  const Columns at(p, pc.sp);
+  const int lw = p.lw, pairs = 16 << lw, pr = threadIdx.x & (pairs - 1), M = p.M, epi = p.epi, fp32 = p.out_fp32;
   const bool pair = p.pair, owner = pc.me == pc.last;
   const int others = owner ? pc.last - pc.first : 0;                                  // contributors whose sums are to be added
-  const int tcol = pc.sp * kWC + (pr >> 4), n0 = pc.sp * kWC * 32 + 2 * pr;           // tile column and first channel of the pair
-  const bool inside = tcol < p.TC;
+  const int tcol = at.col + (pr >> 4), n0 = at.col * 32 + 2 * pr;                     // tile column and first channel of the pair
+  const bool inside = (pr >> 4) < at.width;
   const float unscale = unscale_of(p.tg) * p.alpha;
   const uint16_t *add = owner && inside ? p.add : nullptr;
   char *out = static_cast<char *>(p.out);
   float *slots = sc.partials + (size_t)(owner ? pc.first : pc.me) * slot_floats + 2 * pr;
-  int row = threadIdx.x >> 6;
+  const int rows = kConsumers >> (4 + lw), mine = threadIdx.x >> (4 + lw);            // rows at a time, and this thread's among them
   // datum index of (row, channel pair) in the result's tiles, and in an addend's
   auto place = [&](int r) { return tcol * 1024 + ((r >> 4) * 2 + ((pr >> 3) & 1)) * 256 + (r & 15) * 16 + (2 * pr & 15); };
   auto addend = [&](int r) { return add && r < M ? __ldcg(reinterpret_cast<const uint32_t *>(add + place(r))) : 0u; };
-  uint32_t a = addend(row);
+  uint32_t a = addend(mine);
   named_barrier(1, kConsumers);                                                       // every warp's sums are in place
   uint32_t patience = others && lds32(smem + kSmDead) ? 1 : kSpinLimit * 64;
-  for (; row < M; row += kConsumers / 64) {
-    float2 s[4];
+  for (int row0 = 0; row0 < M; row0 += rows) {
+    const int row = row0 + mine;
+    const bool live = row < M;
+    float2 v = make_float2(0.f, 0.f), u = v;
+    if (p.small) {
+      // one slab of sums per tile row (and matrix): the last row's, then the others' in order, as if every row were a CTA's
+      // share: how a matmul is spread over CTAs and warps then has no say in the last bit of a result
+      const int step = M * sum_stride(lw), next = pair ? 2 * step : step, KT = p.KT;
+      const float *from = sums + (live ? row : 0) * sum_stride(lw) + 2 * pr, *last = from + (KT - 1) * next;
+      v = *reinterpret_cast<const float2 *>(last);
+      if (pair) u = *reinterpret_cast<const float2 *>(last + step);
+#pragma unroll 4
+      for (int k = 0; k < KT - 1; k++, from += next) {
+        const float2 w = *reinterpret_cast<const float2 *>(from);
+        v.x += w.x, v.y += w.y;
+        if (pair) {
+          const float2 x = *reinterpret_cast<const float2 *>(from + step);
+          u.x += x.x, u.y += x.y;
+        }
+      }
+    } else if (live) {
+      // four slabs: k groups of one matrix, or two of gate and of up by turns
+      float2 s[4];
 #pragma unroll
-    for (int j = 0; j < 4; j++) s[j] = *reinterpret_cast<const float2 *>(sums + (j * pc.toks + row) * kSumStride + 2 * pr);
-    float2 u = make_float2(s[1].x + s[3].x, s[1].y + s[3].y), v = make_float2(s[0].x + s[2].x, s[0].y + s[2].y);
-    if (!pair) v.x += u.x, v.y += u.y;
-    float *slot = slots + row * step;
+      for (int j = 0; j < 4; j++) s[j] = *reinterpret_cast<const float2 *>(sums + (j * pc.toks + row) * sum_stride(2) + 2 * pr);
+      u = make_float2(s[1].x + s[3].x, s[1].y + s[3].y), v = make_float2(s[0].x + s[2].x, s[0].y + s[2].y);
+      if (!pair) v.x += u.x, v.y += u.y;
+    }
+    float *slot = slots + (pair ? 2 * row : row) * 128;
     if (!owner) {
-      send(slot, v);
-      if (pair) send(slot + 128, u);
+      if (live) send(slot, v);
+      if (live && pair) send(slot + 128, u);
       continue;
     }
-    for (int c = 0; c < others; c += kSlots, slot += kSlots * (size_t)slot_floats) {
-      uint2 w[kSlots], x[kSlots];
+    const int per = pair ? kSlots / 2 : kSlots;                                       // contributors at a time: words of gate and up by turns, or of one matrix
+    for (int c = live ? 0 : others; c < others; c += per, slot += per * (size_t)slot_floats) {
+      uint2 w[kSlots];
+      auto there = [&](int j) { return c + (pair ? j / 2 : j) < others; };
+      auto at_slot = [&](int j) { return slot + (size_t)(pair ? j / 2 : j) * slot_floats + (pair ? j % 2 * 128 : 0); };
       bool missing;
       do {                                                                            // all of them in flight together, again until all are there
         missing = false;
 #pragma unroll
         for (int j = 0; j < kSlots; j++)
-          if (c + j < others) {
-            w[j] = ld_relaxed2(slot + (size_t)j * slot_floats);
-            if (pair) x[j] = ld_relaxed2(slot + (size_t)j * slot_floats + 128);
-          }
+          if (there(j)) w[j] = ld_relaxed2(at_slot(j));
 #pragma unroll
         for (int j = 0; j < kSlots; j++)
-          if (c + j < others) missing |= w[j].x == 0 || w[j].y == 0 || (pair && (x[j].x == 0 || x[j].y == 0));
+          if (there(j)) missing |= w[j].x == 0 || w[j].y == 0;
       } while (missing && patience && --patience);
 #pragma unroll
       for (int j = 0; j < kSlots; j++)
-        if (c + j < others) {
-          st_relaxed2(slot + (size_t)j * slot_floats, make_uint2(0, 0));
-          v.x += __uint_as_float(w[j].x), v.y += __uint_as_float(w[j].y);
-          if (pair) {
-            st_relaxed2(slot + (size_t)j * slot_floats + 128, make_uint2(0, 0));
-            u.x += __uint_as_float(x[j].x), u.y += __uint_as_float(x[j].y);
-          }
+        if (there(j)) {
+          st_relaxed2(at_slot(j), make_uint2(0, 0));
+          if (pair && j % 2) u.x += __uint_as_float(w[j].x), u.y += __uint_as_float(w[j].y);
+          else v.x += __uint_as_float(w[j].x), v.y += __uint_as_float(w[j].y);
         }
     }
     v.x = v.x * unscale + __uint_as_float(a << 16), v.y = v.y * unscale + __uint_as_float(a & 0xFFFF0000u);
-    a = addend(row + kConsumers / 64);
+    a = addend(row + rows);
     if (epi == BT_EPI_RELU) v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f);
     if (epi == BT_EPI_SILU || pair) v.x = silu(v.x), v.y = silu(v.y);
     if (pair) v.x *= (u.x + 0.f) * unscale, v.y *= (u.y + 0.f) * unscale;
     if (epi == BT_EPI_ARGMAX) {
-      unsigned long long key = inside ? max(pick_key(v.x, n0), pick_key(v.y, n0 + 1)) : 0ull;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) key = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, d));
+      unsigned long long key = inside && live ? max(pick_key(v.x, n0), pick_key(v.y, n0 + 1)) : 0ull;
+      for (int d = 1; d < min(pairs, 32); d <<= 1) key = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, d));
       // a maximum over all sub-panels whatever the order they finish in, so the last one to finish has the answer at hand
-      if ((threadIdx.x & 31) == 0 && key) atomicMax(sc.keys + row, key);
+      if ((threadIdx.x & (min(pairs, 32) - 1)) == 0 && key) atomicMax(sc.keys + row, key);
       continue;
     }
     const uint32_t both = bf16_half_up(v.x) | bf16_half_up(v.y) << 16;
     if (fp32 == 2) {
       // row-major fp32, only the rows there are: partial sums on their way to an all-reduce
-      if (inside) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + n0)) = v;
+      if (inside && live) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + n0)) = v;
     } else if (M > 1) {
-      if (inside && fp32) *reinterpret_cast<float2 *>(out + 4 * (size_t)place(row)) = v;
-      else if (inside) *reinterpret_cast<uint32_t *>(out + 2 * (size_t)place(row)) = both;
+      if (inside && live && fp32) *reinterpret_cast<float2 *>(out + 4 * (size_t)place(row)) = v;
+      else if (inside && live) *reinterpret_cast<uint32_t *>(out + 2 * (size_t)place(row)) = both;
     } else if (fp32) {
       // a one-row result repeats across its tile
-      for (int r = 0; inside && r < 32; r++) *reinterpret_cast<float2 *>(out + 4 * (size_t)place(r)) = v;
+      for (int r = 0; inside && live && r < 32; r++) *reinterpret_cast<float2 *>(out + 4 * (size_t)place(r)) = v;
     } else {
       // the same: four lanes put half a face row together, and each of them writes it to eight of the rows
       uint4 half;
       half.x = __shfl_sync(0xFFFFFFFFu, both, 0, 4), half.y = __shfl_sync(0xFFFFFFFFu, both, 1, 4);
       half.z = __shfl_sync(0xFFFFFFFFu, both, 2, 4), half.w = __shfl_sync(0xFFFFFFFFu, both, 3, 4);
-      if (inside) {
+      if (inside && live) {
 #pragma unroll
         for (int r = 0; r < 32; r += 4) *reinterpret_cast<uint4 *>(out + 2 * (size_t)(place(r + (pr & 3)) - 2 * (pr & 3))) = half;
       }
@@ -457,14 +496,18 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
   volatile uint32_t *held = reinterpret_cast<volatile uint32_t *>(smem + kSmHeld) + (WEIGHTS ? 0 : kBars);   // ring bytes of each stage in the ring
   const int lane = threadIdx.x & 31;
   if (!WEIGHTS && lane < q.n) tensormap_prefetch(&q.op[lane].xmap);
+  if (WEIGHTS && lane < q.n && q.op[lane].tiled) {
+    tensormap_prefetch(&q.op[lane].wmap[0]);
+    if (q.op[lane].pair) tensormap_prefetch(&q.op[lane].wmap[1]);
+  }
   Ring ring{0};
   uint32_t count = 0, oldest = 0, used = 0;   // stages placed; first stage not yet known to be free; ring bytes held from there on
   for (int i = 0; i < q.n; i++) {
     const GemvParams &p = q.op[i];
-    const Geometry g = geometry(p.fmt, p.pair != 0, p.tg);
+    const Geometry g = geometry(p.fmt, p.pair != 0, p.tg, p.lw);
     const int me = (cta + p.turn) % ctas;                    // the range this CTA takes in this matmul
     if (me >= p.active) continue;
-    const int KT = p.KT, TC = p.TC, nw = p.pair ? 2 : 1;
+    const int KT = p.KT, nw = p.pair ? 2 : 1;
     const uint8_t *w = p.w[lane < nw ? lane : 0];
     Walk walk;
     walk.start(p, me);
@@ -472,7 +515,8 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
     while (walk.more()) {
       int sp, kt, rows;
       walk.next(sp, kt, rows);
-      const int width = min(kWC, TC - sp * kWC), ends = walk.more() ? 1 : 3;
+      const Columns at(p, sp);
+      const int width = at.width, ends = walk.more() ? 1 : 3;
       const int first = WEIGHTS ? cta_of(p, sp * KT) : 0, end = WEIGHTS ? cta_of(p, (sp + 1) * KT - 1) : 0;
       for (; rows > 0; rows -= g.ups, kt += g.ups) {
         const int n = min(g.ups, rows);
@@ -494,11 +538,23 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
           const uint32_t bytes = n * width * g.tb;
           if (lane == 0) {
             uint4 *note = reinterpret_cast<uint4 *>(smem + kSmStages) + 2 * (count % kBars);
-            note[0] = make_uint4(stage, n, width, (rows <= g.ups ? ends : 0) | (n == g.ups && width == kWC ? 4 : 0)), note[1] = make_uint4(sp, first, me, end);
+            note[0] = make_uint4(stage, n, width, (rows <= g.ups ? ends : 0) | (n == g.ups && width == kWC ? 4 : 0) | kt << 3), note[1] = make_uint4(sp, first, me, end);
             mbar_expect_tx(bar, nw * bytes);
           }
           __syncwarp();
-          if (lane < nw) bulk_g2s(stage + lane * g.matrix, w + ((size_t)sp * kWC * KT + (size_t)kt * width) * g.tb, bytes, bar);
+          if (width == at.run_width) {
+            // one contiguous range of each matrix
+            if (lane < nw) bulk_g2s(stage + lane * g.matrix, w + ((size_t)at.run * kWC * KT + (size_t)kt * width) * g.tb, bytes, bar);
+          } else if (n == g.ups && at.run_width == kWC) {
+            // some columns of a run: a tiled copy of each matrix
+            if (lane < nw) tma_load_3d(stage + lane * g.matrix, &p.wmap[lane], 0, at.col & 3, at.run * KT + kt, bar);
+          } else {
+            // the last, shorter stage of such a piece, or a run shorter than four: a copy per tile row
+            for (int j = lane; j < nw * n; j += 32) {
+              const int m = j >= n, row = j - m * n;
+              bulk_g2s(stage + m * g.matrix + row * width * g.tb, p.w[m] + ((size_t)at.run * kWC * KT + (size_t)(kt + row) * at.run_width + (at.col & 3)) * g.tb, width * g.tb, bar);
+            }
+          }
         } else {
           if (gate) {
             int ok = 1;
@@ -533,9 +589,25 @@ struct Place {
   int cc, ck, mat;                   // this warp's column, first tile row, weight matrix
   int lane;
 };
+// Fragments to [k group][matrix][token][channel]: lane (g, t) holds tokens 8 tg + 2 t + j and channels 16 fs + 2 g + {0, 1}.
+// Tokens from `tokens` on are left out.
+template <int FMT, int TG>
+__device__ __forceinline__ void leave_sums(const float (&acc)[2][TG][4], float *to, int stride, int tokens, int cc, int lane) {
+  const int t = lane & 3, g = lane >> 2;
+  to += 2 * t * stride + cc * 32 + 2 * g;
+#pragma unroll
+  for (int fs = 0; fs < 2; fs++)
+#pragma unroll
+    for (int tg = 0; tg < TG; tg++)
+#pragma unroll
+      for (int j = 0; j < 2; j++)
+        if (8 * tg + 2 * t + j < tokens)
+          *reinterpret_cast<float2 *>(to + (8 * tg + j) * stride + 16 * fs) =
+              FMT == BT_BFP8 ? make_float2(acc[fs][tg][j], acc[fs][tg][2 + j]) : make_float2(16.f * acc[fs][tg][2 + j], acc[fs][tg][j] - acc[fs][tg][2 + j]);
+}
 template <int FMT, int TG, bool PAIR>
 __device__ __forceinline__ uint4 stream_rows(Place &w, float *sums, int *error) {
-  constexpr int TB = tile_bytes(FMT), T = stage_rows_per_warp(FMT, TG), XB = 512 * TG, GROUPS = PAIR ? 2 : 4;   // warps that share a column
+  constexpr int TB = tile_bytes(FMT), T = stage_rows_per_warp(FMT, TG, 2), XB = 512 * TG, GROUPS = PAIR ? 2 : 4;   // warps that share a column
   const int lane = w.lane, ck = w.ck, cc = w.cc;
   const uint32_t matrix0 = w.mat * (GROUPS * T * kWC * TB), x0 = 4 * T * kWC * TB + ck * XB + lane * 8, tile0 = matrix0 + (ck * kWC + cc) * TB;
   float acc[2][TG][4];
@@ -563,17 +635,38 @@ __device__ __forceinline__ uint4 stream_rows(Place &w, float *sums, int *error) 
     mbar_arrive_if(bar + kSmEmpty, lane == 0);
     w.count++;
   }
-  // fragments to [k group][matrix][token][channel]: lane (g, t) holds tokens 8 tg + 2 t + j and channels 16 fs + 2 g + {0, 1}
-  const int t = lane & 3, g = lane >> 2;
-  float *to = sums + ((PAIR ? 2 * ck + w.mat : ck) * 8 * TG + 2 * t) * kSumStride + cc * 32 + 2 * g;
+  leave_sums<FMT, TG>(acc, sums + (PAIR ? 2 * ck + w.mat : ck) * 8 * TG * sum_stride(2), sum_stride(2), 8 * TG, cc, lane);
+  return piece;
+}
+// The same for small matmuls, whose sub-panels have one, two or four columns and whose tile rows go round up to 16 warps: a
+// warp has a few tiles in all, and leaves the sums of each by itself.
+template <int FMT, int TG>
+__device__ __forceinline__ uint4 stream_small(Place &w, float *sums, int *error, const GemvParams &p) {
+  constexpr int TB = tile_bytes(FMT), XB = 512 * TG;
+  const int lw = p.lw, M = p.M, matrices = p.pair ? 2 : 1, lane = w.lane, groups = kCW >> lw >> (matrices - 1);
+  const Geometry g = geometry(FMT, matrices == 2, TG, lw);
+  uint4 piece = make_uint4(0, 0, 0, 0);
+  for (int last = 0; !last;) {
+    const uint32_t slot = w.count & (kBars - 1), bar = w.smem + 8 * slot, note = w.smem + kSmStages + 32 * slot;
+    if (!stage_wait(w.smem, bar + kSmFull, w.count / kBars & 1, error)) break;
+    const uint4 stage = lds128(note);
+    last = stage.w & 3;
+    if (last) piece = lds128(note + 16), piece.x |= (uint32_t)last << 30;
+    if (w.cc < (int)stage.z) {
+      uint32_t tile = stage.x + w.mat * g.matrix + (w.ck * stage.z + w.cc) * TB, xs = stage.x + g.w_bytes + w.ck * XB + lane * 8;
+#pragma unroll 1
+      for (int row = w.ck; row < (int)stage.y; row += groups, tile += groups * stage.z * TB, xs += groups * XB) {
+        float acc[2][TG][4];
 #pragma unroll
-  for (int fs = 0; fs < 2; fs++)
-#pragma unroll
-    for (int tg = 0; tg < TG; tg++)
-#pragma unroll
-      for (int j = 0; j < 2; j++)
-        *reinterpret_cast<float2 *>(to + (8 * tg + j) * kSumStride + 16 * fs) =
-            FMT == BT_BFP8 ? make_float2(acc[fs][tg][j], acc[fs][tg][2 + j]) : make_float2(16.f * acc[fs][tg][2 + j], acc[fs][tg][j] - acc[fs][tg][2 + j]);
+        for (int i = 0; i < 8 * TG; i++) acc[i / (4 * TG)][i / 4 % TG][i % 4] = 0.f;
+        tile_mma<FMT, TG>(tile + lane * 16, tile + (lane & 3) * 16, xs, acc);
+        leave_sums<FMT, TG>(acc, sums + ((((int)stage.w >> 3) + row) * matrices + w.mat) * M * sum_stride(lw), sum_stride(lw), M, w.cc, lane);
+      }
+    }
+    __syncwarp();
+    mbar_arrive_if(bar + kSmEmpty, lane == 0);
+    w.count++;
+  }
   return piece;
 }
 
@@ -619,7 +712,7 @@ __device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
         int is_last = 0;
         if (lane == 0) {
           fence_gpu();
-          is_last = atomicAdd(sc.panels_done, 1) == (p.TC + kWC - 1) / kWC - 1;
+          is_last = atomicAdd(sc.panels_done, 1) == p.panels - 1;
         }
         if (__shfl_sync(0xFFFFFFFFu, is_last, 0)) {
           fence_gpu();
@@ -687,15 +780,23 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
   for (int i = 0; i < q.n; i++) {
     const GemvParams &p = q.op[i];
     const Scratch &sc = q.set[i % q.sets];
-    // for one weight matrix a column's tile rows go round four warps, for a pair round two, and the others have the second matrix
-    w.mat = p.pair ? warp >> 2 & 1 : 0, w.ck = p.pair ? warp >> 3 : warp >> 2;
+    // a column's tile rows go round the warps that a sub-panel's columns and matrices leave for it: 4 of them for four columns of one matrix
+    const int rest = warp >> p.lw;
+    w.cc = warp & ((1 << p.lw) - 1), w.mat = p.pair ? rest & 1 : 0, w.ck = p.pair ? rest >> 1 : rest;
     // The ranges go round the CTAs from matmul to matmul: the CTAs that finish shared sub-panels have more to do than
     // the others, and it should not be the same ones every time.
     const int me = (cta + p.turn) % ctas;
     int pieces = 0;
     for (bool more = me < p.active; more; pieces++) {
       uint4 piece;
-      switch ((p.fmt == BT_BFP4 ? 6 : 0) + (p.pair ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2)) {
+      if (p.small) switch ((p.fmt == BT_BFP4 ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2)) {
+        case 0: piece = stream_small<BT_BFP8, 1>(w, sums, q.error, p); break;
+        case 1: piece = stream_small<BT_BFP8, 2>(w, sums, q.error, p); break;
+        case 2: piece = stream_small<BT_BFP8, 4>(w, sums, q.error, p); break;
+        case 3: piece = stream_small<BT_BFP4, 1>(w, sums, q.error, p); break;
+        case 4: piece = stream_small<BT_BFP4, 2>(w, sums, q.error, p); break;
+        default: piece = stream_small<BT_BFP4, 4>(w, sums, q.error, p); break;
+      } else switch ((p.fmt == BT_BFP4 ? 6 : 0) + (p.pair ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2)) {
         case 0: piece = stream_rows<BT_BFP8, 1, false>(w, sums, q.error); break;
         case 1: piece = stream_rows<BT_BFP8, 2, false>(w, sums, q.error); break;
         case 2: piece = stream_rows<BT_BFP8, 4, false>(w, sums, q.error); break;
@@ -789,9 +890,26 @@ int wait_for(const bt_gemv_op *ops, int i, int sets) {
 // and with it the last bit of a result, must not change with how matmuls are batched.
 constexpr float kHbmBytesPerUs = 6.3e6f, kSmBytesPerUs = 50e3f, kHandOverUs = 2.f, kEarlyUs = 1.2f, kFourSlotsUs = 0.4f, kStraddleUs = 1.f;
 float row_us(int tg) { return tg == 1 ? 0.07f : tg == 2 ? 0.1f : 0.145f; }
+// Small matmuls: up to two tile rows of four-column sub-panels per SM. What they cost is the chain from x to the report, so
+// nothing is handed over: sub-panels are as narrow as there are SMs for, whole, and their tile rows go round all warps.
+// Every tile row's sums are added by themselves (see end_piece), as far as they fit: 84 KB.
+bool deal_small(GemvParams &p, int ctas) {
+  const int runs = p.TC / kWC, rest = p.TC % kWC, matrices = p.pair ? 2 : 1;
+  if (p.units > 2 * ctas) return false;
+  for (int lw = 0; lw <= 2; lw++) {
+    const int w = 1 << lw, panels = (runs << (2 - lw)) + (rest + w - 1) / w, each = (panels + ctas - 1) / ctas;
+    if (each > 1 && lw < 2) continue;
+    if (p.KT * matrices * p.M * sum_stride(lw) * 4 > kSmallSums) continue;
+    p.lw = lw, p.panels = panels, p.units = panels * p.KT, p.small = 1;
+    p.parts = 0, p.share = each * p.KT, p.extra = 0, p.active = (panels + each - 1) / each;
+    return true;
+  }
+  return false;
+}
 void deal_units(GemvParams &p, int ctas) {
   const int panels = (p.TC + kWC - 1) / kWC, matrices = p.pair ? 2 : 1;
-  p.units = panels * p.KT;
+  p.units = panels * p.KT, p.panels = panels, p.lw = 2, p.small = 0;
+  if (deal_small(p, ctas)) return;
   const float hbm = (float)p.KT * p.TC * tile_bytes(p.fmt) * matrices / kHbmBytesPerUs;
   const float row = max(row_us(p.tg) * matrices, kWC * tile_bytes(p.fmt) * matrices / kSmBytesPerUs);   // us per tile row, an SM on its own
   auto stream = [&](float rows) { return max(hbm, rows * row); };
@@ -810,12 +928,21 @@ void deal_units(GemvParams &p, int ctas) {
 }
 
 // The tensor map of a matmul's x (one tile row of bf16 tiles): the staged token rows of each face are contiguous, a tile
-// has its faces 512 bytes apart, and a copy takes the tile columns of one stage.
-int map_x(GemvParams &p, uint64_t x) {
-  const Geometry g = geometry(p.fmt, p.pair != 0, p.tg);
+// has its faces 512 bytes apart, and a copy takes the tile columns of one stage. And those of its weights, if sub-panels are
+// narrower than the runs of the streaming layout.
+int make_maps(GemvParams &p, uint64_t x) {
+  const Geometry g = geometry(p.fmt, p.pair != 0, p.tg, p.lw);
   const uint32_t box[3] = {p.tg == 1 ? 128u : 256u, p.tg == 4 ? 4u : 2u, (uint32_t)g.ups};
   const uint64_t dims[3] = {box[0], box[1], (uint64_t)p.KT}, strides[2] = {512, 2048};
-  return make_tmap(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, as_ptr<void>(x), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+  if (int s = make_tmap(&p.xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, as_ptr<void>(x), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE)) return s;
+  p.tiled = p.lw < 2 && p.TC >= kWC && p.KT >= g.ups;                 // else contiguous, or never a whole stage
+  if (!p.tiled) return BT_OK;
+  // weights in 8-byte elements: a tile is 136 or 72 of them
+  const uint32_t wbox[3] = {(uint32_t)g.tb / 8, 1u << p.lw, (uint32_t)g.ups};
+  const uint64_t wdims[3] = {wbox[0], kWC, (uint64_t)(p.TC / kWC) * p.KT}, wstrides[2] = {(uint64_t)g.tb, (uint64_t)kWC * g.tb};
+  for (int m = 0; m < (p.pair ? 2 : 1); m++)
+    if (int s = make_tmap(&p.wmap[m], CU_TENSOR_MAP_DATA_TYPE_UINT64, 3, p.w[m], wdims, wstrides, wbox, CU_TENSOR_MAP_SWIZZLE_NONE)) return s;
+  return BT_OK;
 }
 
 // Whether the last thing this library queued, on any stream, before the current entry-point call was a matmul launch
@@ -858,7 +985,7 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
     Queue q = scratch;
     q.n = min(kQueueMax, n - base);
     q.panels = 0;
-    int tg_max = 1;
+    int sums = 0;
     for (int i = 0; i < q.n; i++) {
       const bt_gemv_op &o = ops[base + i];
       GemvParams &p = q.op[i];
@@ -868,13 +995,13 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       p.fmt = o.fmt, p.pair = o.epilogue == BT_EPI_GLU, p.tg = o.M <= 8 ? 1 : o.M <= 16 ? 2 : 4;
       p.wait_for = wait_for(ops + base, i, scratch.sets);
       p.turn = (int)(((long long)(base + i) * 101) % ctas);
-      if (p.wait_for >= 0) p.wait_panels = (q.op[p.wait_for].TC + kWC - 1) / kWC;
-      q.panels += (p.TC + kWC - 1) / kWC;
+      if (p.wait_for >= 0) p.wait_panels = q.op[p.wait_for].panels;
       deal_units(p, ctas);
-      if (int s = map_x(p, o.x)) return s;
-      tg_max = max(tg_max, p.tg);
+      q.panels += p.panels;
+      if (int s = make_maps(p, o.x)) return s;
+      sums = max(sums, p.small ? p.KT * (p.pair ? 2 : 1) * p.M * sum_stride(p.lw) * 4 : sums_bytes(p.tg));
     }
-    q.ring = kSmSums + sums_bytes(tg_max), q.ring_bytes = (kSmemBytes - q.ring) / 128 * 128;
+    q.ring = kSmSums + (sums + 127) / 128 * 128, q.ring_bytes = (kSmemBytes - q.ring) / 128 * 128;
     // Programmatic dependent launch: this grid may begin while the previous launch of the stream is still finishing.
     // It only sets up and prefetches weights until its x warps pass griddepcontrol.wait. Weights read that early must
     // be in place, so the launch overlaps its predecessor only when that was a matmul launch of this file too (which
