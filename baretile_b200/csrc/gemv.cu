@@ -325,6 +325,10 @@ __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc
   auto place = [&](int r) { return tcol * 1024 + ((r >> 4) * 2 + ((pr >> 3) & 1)) * 256 + (r & 15) * 16 + (2 * pr & 15); };
   auto addend = [&](int r) { return add && r < M ? __ldcg(reinterpret_cast<const uint32_t *>(add + place(r))) : 0u; };
   uint32_t a = addend(mine);
+  // what the barrier is waited with is worked out and fetched already
+  int KT = p.KT, next = M * sum_stride(lw) * (pair ? 2 : 1);
+  float scale = unscale;
+  asm volatile("" : "+r"(KT), "+r"(next), "+f"(scale), "+l"(out), "+l"(slots) :: "memory");
   named_barrier(1, kConsumers);                                                       // every warp's sums are in place
   uint32_t patience = others && lds32(smem + kSmDead) ? 1 : kSpinLimit * 64;
   for (int row0 = 0; row0 < M; row0 += rows) {
@@ -334,17 +338,22 @@ __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc
     if (p.small) {
       // one slab of sums per tile row (and matrix): the last row's, then the others' in order, as if every row were a CTA's
       // share: how a matmul is spread over CTAs and warps then has no say in the last bit of a result
-      const int step = M * sum_stride(lw), next = pair ? 2 * step : step, KT = p.KT;
-      const float *from = sums + (live ? row : 0) * sum_stride(lw) + 2 * pr, *last = from + (KT - 1) * next;
-      v = *reinterpret_cast<const float2 *>(last);
-      if (pair) u = *reinterpret_cast<const float2 *>(last + step);
+      if (live) {
+        const float *from = sums + row * sum_stride(lw) + 2 * pr, *last = from + (KT - 1) * next;
+        v = *reinterpret_cast<const float2 *>(last);
+        if (!pair) {
 #pragma unroll 4
-      for (int k = 0; k < KT - 1; k++, from += next) {
-        const float2 w = *reinterpret_cast<const float2 *>(from);
-        v.x += w.x, v.y += w.y;
-        if (pair) {
-          const float2 x = *reinterpret_cast<const float2 *>(from + step);
-          u.x += x.x, u.y += x.y;
+          for (int k = 0; k < KT - 1; k++, from += next) {
+            const float2 w = *reinterpret_cast<const float2 *>(from);
+            v.x += w.x, v.y += w.y;
+          }
+        } else {
+          u = *reinterpret_cast<const float2 *>(last + next / 2);
+#pragma unroll 4
+          for (int k = 0; k < KT - 1; k++, from += next) {
+            const float2 w = *reinterpret_cast<const float2 *>(from), x = *reinterpret_cast<const float2 *>(from + next / 2);
+            v.x += w.x, v.y += w.y, u.x += x.x, u.y += x.y;
+          }
         }
       }
     } else if (live) {
@@ -384,11 +393,11 @@ __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc
           else v.x += __uint_as_float(w[j].x), v.y += __uint_as_float(w[j].y);
         }
     }
-    v.x = v.x * unscale + __uint_as_float(a << 16), v.y = v.y * unscale + __uint_as_float(a & 0xFFFF0000u);
+    v.x = v.x * scale + __uint_as_float(a << 16), v.y = v.y * scale + __uint_as_float(a & 0xFFFF0000u);
     a = addend(row + rows);
     if (epi == BT_EPI_RELU) v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f);
     if (epi == BT_EPI_SILU || pair) v.x = silu(v.x), v.y = silu(v.y);
-    if (pair) v.x *= (u.x + 0.f) * unscale, v.y *= (u.y + 0.f) * unscale;
+    if (pair) v.x *= (u.x + 0.f) * scale, v.y *= (u.y + 0.f) * scale;
     if (epi == BT_EPI_ARGMAX) {
       unsigned long long key = inside && live ? max(pick_key(v.x, n0), pick_key(v.y, n0 + 1)) : 0ull;
       for (int d = 1; d < min(pairs, 32); d <<= 1) key = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, d));
