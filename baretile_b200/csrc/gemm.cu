@@ -127,7 +127,9 @@ __device__ __forceinline__ void expand_tile(uint32_t tile, uint32_t b, int c, in
   }
 }
 
-template <int FMT>
+// SPLIT: the pairs share K. A kernel of its own, since whole blocks lose 2 % to the K block a pair starts at and the sums that
+// go out as they are.
+template <int FMT, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap) {
   using L = Layout<FMT>;
   extern __shared__ uint8_t smem_raw[];
@@ -138,10 +140,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
   const uint32_t rank = cluster_ctarank();                          // 0: the leader, which issues the MMAs
   const int KB = (p.KT + 1) / 2;                                    // K blocks of 64; the last may hold one tile row
   const int pair_id = blockIdx.x >> 1;
-  const int split = pair_id % p.splits, kb0 = KB * split / p.splits, kbs = KB * (split + 1) / p.splits - kb0;   // this pair's K blocks
-  const int block = p.splits > 1 ? pair_id / p.splits : pair_id < p.whole ? pair_id : p.whole + ((pair_id - p.whole) >> 1);   // blocks go down the rows first
+  const int split = SPLIT ? pair_id % p.splits : 0, kb0 = SPLIT ? KB * split / p.splits : 0, kbs = SPLIT ? KB * (split + 1) / p.splits - kb0 : KB;   // this pair's K blocks
+  const int block = SPLIT ? pair_id / p.splits : pair_id < p.whole ? pair_id : p.whole + ((pair_id - p.whole) >> 1);   // blocks go down the rows first
   const int bc = block / p.row_blocks;                              // block column: 128 output columns (pair) or 256
-  const bool all_rows = !p.half && (p.splits > 1 || pair_id < p.whole);
+  const bool all_rows = !p.half && (SPLIT || pair_id < p.whole);
   const int pair_m0 = (block % p.row_blocks) * (p.half ? 256 : 512) + (p.half || all_rows ? 0 : ((pair_id - p.whole) & 1) * 256);   // first row of the pair's rows
   const int MH = all_rows && pair_m0 + 256 < p.M ? 2 : 1;           // halves of 256 rows this pair computes
   if (pair_m0 >= p.M) return;                                       // (both CTAs of the pair: nothing here)
@@ -243,7 +245,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
         tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + mh * 256 + col, v);
         if (p.pair) tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + mh * 256 + 128 + col, u);
         tmem_ld_wait();
-        if (p.splits > 1) {
+        if (SPLIT) {
           // sums of a part of K, as they are: reduce_kernel adds the parts
           if (row < p.M) {
             const size_t cols = (size_t)p.TC * 32, plane = (size_t)tile_rows * 32 * cols;
@@ -409,8 +411,10 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
   const int pairs = deal_blocks(p, sms / 2 > 0 ? sms / 2 : 1, part_bytes);
   static bool configured[64] = {};
   if (!configured[device & 63]) {
-    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP8>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP8>::BYTES + 1024));
-    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP4>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP4>::BYTES + 1024));
+    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP8>::BYTES + 1024));
+    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP8>::BYTES + 1024));
+    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP4>::BYTES + 1024));
+    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP4>::BYTES + 1024));
     configured[device & 63] = true;
   }
   cudaLaunchConfig_t cfg{};
@@ -422,8 +426,9 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
   cfg.dynamicSmemBytes = (fmt == BT_BFP8 ? Layout<BT_BFP8>::BYTES : Layout<BT_BFP4>::BYTES) + 1024;
   cfg.stream = as_stream(stream);
   cfg.attrs = attr, cfg.numAttrs = 1;
-  if (fmt == BT_BFP8) BT_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP8>, p, amap));
-  else BT_CUDA(cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP4>, p, amap));
+  const bool split = p.splits > 1;
+  if (fmt == BT_BFP8) BT_CUDA(split ? cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP8, true>, p, amap) : cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP8, false>, p, amap));
+  else BT_CUDA(split ? cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP4, true>, p, amap) : cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP4, false>, p, amap));
   if (int s = launched("gemm_kernel")) return s;
   if (p.splits == 1) return BT_OK;
   // its blocks come up while the last of gemm_kernel drain, and wait there until that is complete
