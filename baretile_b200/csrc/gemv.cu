@@ -34,6 +34,7 @@
 #include "ptx.cuh"
 #include "stream_layout.cuh"
 #include "tmap.cuh"
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -130,12 +131,17 @@ struct alignas(64) GemvParams {
   int share, extra;           // range b then starts at b * share + min(b, extra), and the last one ends at units
 };
 
+// The kernel exists twice: for lists with a small matmul in them, and for lists without one, which is spared all that sub-panels
+// of other widths than four take (as one kernel it cost lists of large matmuls 2-3 %).
+template <bool SMALL> __device__ __forceinline__ int lw_of(const GemvParams &p) { return SMALL ? p.lw : 2; }
+
 // Where sub-panel `sp` lies: 1 << lw tile columns from `col` on, fewer at the end of a matrix, part of a run of `run_width`.
-struct Columns {
+template <bool SMALL> struct Columns {
   int run, run_width, col, width;
   __device__ __forceinline__ Columns(const GemvParams &p, int sp) {
-    run = sp >> (2 - p.lw), col = run * kWC + ((sp & ((1 << (2 - p.lw)) - 1)) << p.lw);
-    run_width = min(kWC, p.TC - run * kWC), width = min(1 << p.lw, p.TC - col);
+    const int lw = lw_of<SMALL>(p);
+    run = sp >> (2 - lw), col = run * kWC + ((sp & ((1 << (2 - lw)) - 1)) << lw);
+    run_width = min(kWC, p.TC - run * kWC), width = min(1 << lw, p.TC - col);
   }
 };
 
@@ -161,8 +167,7 @@ struct Scratch {
 
 // What one launch gets: the matmuls and the scratch they share: a wait-gave-up flag, the counts of finished sub-panels of
 // each matmul and of the launch (zero before first use; the kernel leaves them zero) and one or two sets of running scratch.
-struct Queue {
-  GemvParams op[kQueueMax];
+struct QueueHead {
   int n;
   int sets;                   // kSets: matmuls take the sets in turn, and as many may be in flight; 1: one after the other
   int *error, *ops_done, *all_done;
@@ -171,6 +176,11 @@ struct Queue {
   int slot_floats;            // floats between two CTAs' slots of partial sums
   int ring;                   // where the ring starts in shared memory
   int ring_bytes;
+};
+// A launch's parameters travel with it, and 16 KB of them cost it about a microsecond, so short lists have a kernel of their own.
+constexpr int kQueueShort = 8;
+template <int OPS> struct Queue : QueueHead {
+  GemvParams op[OPS];
 };
 
 // A stage as the consumers see it, written by the weight warp ahead of its arrival on the stage's barrier: where a warp
@@ -299,19 +309,19 @@ __device__ __forceinline__ void send(float *to, float2 v) {
   st_relaxed2(to, make_uint2(x ? x : 0x80000000u, y ? y : 0x80000000u));
 }
 // The rows past M of an owner's tiles are zeros; they need no sums, so the messenger writes them while the others work.
-__device__ __forceinline__ void zero_rows(const GemvParams &p, int sp) {
+template <bool SMALL> __device__ __forceinline__ void zero_rows(const GemvParams &p, int sp) {
   const int M = p.M, lane = threadIdx.x & 31;
   if (M == 1 || p.epi == BT_EPI_ARGMAX || p.out_fp32 == 2) return;
-  const Columns at(p, sp);
+  const Columns<SMALL> at(p, sp);
   const int per_row = p.out_fp32 ? 4 : 2;                                           // 16-byte words of a face row
   for (int face = 0; face < 4 * at.width; face++) {                                 // two lower and two upper faces of each tile
     uint4 *rows = static_cast<uint4 *>(p.out) + ((size_t)at.col * 4 + face) * 16 * per_row;
     for (int i = max(M - (face & 2) * 8, 0) * per_row + lane; i < 16 * per_row; i += 32) rows[i] = make_uint4(0, 0, 0, 0);
   }
 }
-__device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc, uint32_t smem, int *error) {
-  const Columns at(p, pc.sp);
-  const int lw = p.lw, pairs = 16 << lw, pr = threadIdx.x & (pairs - 1), M = p.M, epi = p.epi, fp32 = p.out_fp32;
+template <bool SMALL> __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc, uint32_t smem, int *error) {
+  const Columns<SMALL> at(p, pc.sp);
+  const int lw = lw_of<SMALL>(p), pairs = 16 << lw, pr = threadIdx.x & (pairs - 1), M = p.M, epi = p.epi, fp32 = p.out_fp32;
   const bool pair = p.pair, owner = pc.me == pc.last;
   const int others = owner ? pc.last - pc.first : 0;                                  // contributors whose sums are to be added
   const int tcol = at.col + (pr >> 4), n0 = at.col * 32 + 2 * pr;                     // tile column and first channel of the pair
@@ -335,7 +345,7 @@ __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc
     const int row = row0 + mine;
     const bool live = row < M;
     float2 v = make_float2(0.f, 0.f), u = v;
-    if (p.small) {
+    if (SMALL && p.small) {
       // one slab of sums per tile row (and matrix): the last row's, then the others' in order, as if every row were a CTA's
       // share: how a matmul is spread over CTAs and warps then has no say in the last bit of a result
       if (live) {
@@ -487,7 +497,7 @@ struct Ring {
 // warp alone held an 8192 x 28672 bfp4 matmul at 46 us, with one of 1 KB at 35, where the weights take 31.
 // x may be the result of the launch before this one, or of an earlier matmul of this one: the host has worked out the
 // last matmul this one must see finished, all of its sub-panels. False: gave up.
-__device__ __forceinline__ bool await_turn(const Queue &q, const GemvParams &p, int pause_ns) {
+__device__ __forceinline__ bool await_turn(const QueueHead &q, const GemvParams &p, int pause_ns) {
   asm volatile("griddepcontrol.wait;" ::: "memory");     // returns when the previous launch is complete and visible
   if (p.wait_for >= 0) {
     uint32_t spins = 0;
@@ -499,13 +509,13 @@ __device__ __forceinline__ bool await_turn(const Queue &q, const GemvParams &p, 
   return true;
 }
 
-template <bool WEIGHTS>
-__device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t sbase, int cta, int ctas) {
+template <bool WEIGHTS, bool SMALL, class Q>
+__device__ __forceinline__ void produce(const Q &q, uint8_t *smem, uint32_t sbase, int cta, int ctas) {
   const uint32_t full0 = sbase + kSmFull, empty0 = sbase + kSmEmpty, ring0 = sbase + q.ring, ring_bytes = q.ring_bytes;
   volatile uint32_t *held = reinterpret_cast<volatile uint32_t *>(smem + kSmHeld) + (WEIGHTS ? 0 : kBars);   // ring bytes of each stage in the ring
   const int lane = threadIdx.x & 31;
   if (!WEIGHTS && lane < q.n) tensormap_prefetch(&q.op[lane].xmap);
-  if (WEIGHTS && lane < q.n && q.op[lane].tiled) {
+  if (WEIGHTS && SMALL && lane < q.n && q.op[lane].tiled) {
     tensormap_prefetch(&q.op[lane].wmap[0]);
     if (q.op[lane].pair) tensormap_prefetch(&q.op[lane].wmap[1]);
   }
@@ -513,7 +523,7 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
   uint32_t count = 0, oldest = 0, used = 0;   // stages placed; first stage not yet known to be free; ring bytes held from there on
   for (int i = 0; i < q.n; i++) {
     const GemvParams &p = q.op[i];
-    const Geometry g = geometry(p.fmt, p.pair != 0, p.tg, p.lw);
+    const Geometry g = geometry(p.fmt, p.pair != 0, p.tg, lw_of<SMALL>(p));
     const int me = (cta + p.turn) % ctas;                    // the range this CTA takes in this matmul
     if (me >= p.active) continue;
     const int KT = p.KT, nw = p.pair ? 2 : 1;
@@ -524,7 +534,7 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
     while (walk.more()) {
       int sp, kt, rows;
       walk.next(sp, kt, rows);
-      const Columns at(p, sp);
+      const Columns<SMALL> at(p, sp);
       const int width = at.width, ends = walk.more() ? 1 : 3;
       const int first = WEIGHTS ? cta_of(p, sp * KT) : 0, end = WEIGHTS ? cta_of(p, (sp + 1) * KT - 1) : 0;
       for (; rows > 0; rows -= g.ups, kt += g.ups) {
@@ -551,7 +561,7 @@ __device__ __forceinline__ void produce(const Queue &q, uint8_t *smem, uint32_t 
             mbar_expect_tx(bar, nw * bytes);
           }
           __syncwarp();
-          if (width == at.run_width) {
+          if (!SMALL || width == at.run_width) {
             // one contiguous range of each matrix
             if (lane < nw) bulk_g2s(stage + lane * g.matrix, w + ((size_t)at.run * kWC * KT + (size_t)kt * width) * g.tb, bytes, bar);
           } else if (n == g.ups && at.run_width == kWC) {
@@ -682,7 +692,7 @@ __device__ __forceinline__ uint4 stream_small(Place &w, float *sums, int *error,
 // ---- the messenger: one warp tells other CTAs and hears from them ------------------------------------------------
 // It goes through the CTA's pieces beside the consumers and meets them when they have stored what they had. A release
 // takes 1000 to 3000 cycles under load; a consumer warp that did it was that much behind the others at the next barrier.
-__device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
+template <bool SMALL, class Q> __device__ __forceinline__ void carry(const Q &q, int cta, int ctas) {
   const int lane = threadIdx.x & 31;
   for (int i = 0; i < q.n; i++) {
     const GemvParams &p = q.op[i];
@@ -700,7 +710,7 @@ __device__ __forceinline__ void carry(const Queue &q, int cta, int ctas) {
       walk.next(sp, kt, rows);
       const int first = cta_of(p, sp * p.KT), last = cta_of(p, (sp + 1) * p.KT - 1);
       int *counter = sc.counters + sp;
-      if (me == last) zero_rows(p, sp);
+      if (me == last) zero_rows<SMALL>(p, sp);
       // every contributor is past its last look at the counts of this launch
       if (me == last && first != last && lane == 0) {
         uint32_t spins = 0;
@@ -761,7 +771,8 @@ __device__ __noinline__ uint4 piece_at(const GemvParams &p, int me, int n) {
   return make_uint4(sp | (walk.more() ? 1u : 3u) << 30, cta_of(p, sp * p.KT), me, cta_of(p, (sp + 1) * p.KT - 1));
 }
 
-__global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_constant__ Queue q) {
+template <bool SMALL, int OPS>
+__global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_constant__ Queue<OPS> q) {
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   const int warp = threadIdx.x >> 5, cta = blockIdx.x, ctas = gridDim.x;
@@ -778,9 +789,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
   }
   __syncthreads();
   if (warp >= kCW) {
-    if (warp == kCW) produce<true>(q, smem, sbase, cta, ctas);
-    else if (warp == kCW + 1) produce<false>(q, smem, sbase, cta, ctas);
-    else carry(q, cta, ctas);
+    if (warp == kCW) produce<true, SMALL>(q, smem, sbase, cta, ctas);
+    else if (warp == kCW + 1) produce<false, SMALL>(q, smem, sbase, cta, ctas);
+    else carry<SMALL>(q, cta, ctas);
     return;
   }
   float *sums = reinterpret_cast<float *>(smem + kSmSums);
@@ -790,15 +801,15 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
     const GemvParams &p = q.op[i];
     const Scratch &sc = q.set[i % q.sets];
     // a column's tile rows go round the warps that a sub-panel's columns and matrices leave for it: 4 of them for four columns of one matrix
-    const int rest = warp >> p.lw;
-    w.cc = warp & ((1 << p.lw) - 1), w.mat = p.pair ? rest & 1 : 0, w.ck = p.pair ? rest >> 1 : rest;
+    const int lw = lw_of<SMALL>(p), rest = warp >> lw;
+    w.cc = warp & ((1 << lw) - 1), w.mat = p.pair ? rest & 1 : 0, w.ck = p.pair ? rest >> 1 : rest;
     // The ranges go round the CTAs from matmul to matmul: the CTAs that finish shared sub-panels have more to do than
     // the others, and it should not be the same ones every time.
     const int me = (cta + p.turn) % ctas;
     int pieces = 0;
     for (bool more = me < p.active; more; pieces++) {
       uint4 piece;
-      if (p.small) switch ((p.fmt == BT_BFP4 ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2)) {
+      if (SMALL && p.small) switch ((p.fmt == BT_BFP4 ? 3 : 0) + (p.tg == 1 ? 0 : p.tg == 2 ? 1 : 2)) {
         case 0: piece = stream_small<BT_BFP8, 1>(w, sums, q.error, p); break;
         case 1: piece = stream_small<BT_BFP8, 2>(w, sums, q.error, p); break;
         case 2: piece = stream_small<BT_BFP8, 4>(w, sums, q.error, p); break;
@@ -823,7 +834,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
       if (lds32(sbase + kSmDead)) piece = piece_at(p, me, pieces);       // not from the ring's notes
       more = piece.x >> 30 != 3;
       const Piece pc = {(int)(piece.x & 0x3FFFFFFF), (int)piece.y, (int)piece.w, (int)piece.z, 8 * p.tg};
-      end_piece(p, sc, q.slot_floats, sums, pc, sbase, q.error);
+      end_piece<SMALL>(p, sc, q.slot_floats, sums, pc, sbase, q.error);
       named_barrier(2, kConsumers + 32);       // the messenger may tell; the sums may be overwritten
     }
   }
@@ -973,7 +984,7 @@ bool follows_matmul(uint64_t stream) {
 }
 
 // Argument checks and the launches shared by the entry points. `scratch` carries the scratch pointers.
-int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Queue &scratch, uint64_t stream) {
+int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const QueueHead &scratch, uint64_t stream) {
   BT_REQUIRE(n >= 1 && ops, "%s: needs at least one matmul", who);
   for (int i = 0; i < n; i++)
     if (int s = check_op(who, i, ops[i])) return s;
@@ -983,18 +994,27 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
   // The CTAs of a launch wait for one another, so all of them must fit on the GPU at once.
   static int resident[64] = {};
   if (!resident[device & 63]) {
-    BT_CUDA(cudaFuncSetAttribute(gemv_queue_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-    int per_sm = 0;
-    BT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemv_queue_kernel, kThreads, kSmemBytes));
-    if (per_sm < 1) return fail(BT_DEVICE, "%s: the matmul kernel does not fit an SM of device %d", who, device);
+    auto fits = [&](auto *kernel) -> int {
+      BT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+      int per_sm = 0;
+      BT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, kSmemBytes));
+      if (per_sm < 1) return fail(BT_DEVICE, "%s: the matmul kernel does not fit an SM of device %d", who, device);
+      return BT_OK;
+    };
+    if (int s = fits(gemv_queue_kernel<true, kQueueShort>)) return s;
+    if (int s = fits(gemv_queue_kernel<true, kQueueMax>)) return s;
+    if (int s = fits(gemv_queue_kernel<false, kQueueShort>)) return s;
+    if (int s = fits(gemv_queue_kernel<false, kQueueMax>)) return s;
     resident[device & 63] = 1;
   }
   const int ctas = min(sms, kMaxCtas);
   for (int base = 0; base < n; base += kQueueMax) {
-    Queue q = scratch;
+    Queue<kQueueMax> q;
+    static_cast<QueueHead &>(q) = scratch;
     q.n = min(kQueueMax, n - base);
     q.panels = 0;
     int sums = 0;
+    bool small = false;
     for (int i = 0; i < q.n; i++) {
       const bt_gemv_op &o = ops[base + i];
       GemvParams &p = q.op[i];
@@ -1007,6 +1027,7 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       if (p.wait_for >= 0) p.wait_panels = q.op[p.wait_for].panels;
       deal_units(p, ctas);
       q.panels += p.panels;
+      small |= p.small;
       if (int s = make_maps(p, o.x)) return s;
       sums = max(sums, p.small ? p.KT * (p.pair ? 2 : 1) * p.M * sum_stride(p.lw) * 4 : sums_bytes(p.tg));
     }
@@ -1022,7 +1043,12 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr, cfg.numAttrs = base > 0 || follows_matmul(stream) ? 1 : 0;
-    BT_CUDA(cudaLaunchKernelEx(&cfg, gemv_queue_kernel, q));
+    if (q.n <= kQueueShort) {
+      Queue<kQueueShort> s;
+      static_cast<QueueHead &>(s) = q;
+      std::copy(q.op, q.op + q.n, s.op);
+      BT_CUDA(small ? cudaLaunchKernelEx(&cfg, gemv_queue_kernel<true, kQueueShort>, s) : cudaLaunchKernelEx(&cfg, gemv_queue_kernel<false, kQueueShort>, s));
+    } else BT_CUDA(small ? cudaLaunchKernelEx(&cfg, gemv_queue_kernel<true, kQueueMax>, q) : cudaLaunchKernelEx(&cfg, gemv_queue_kernel<false, kQueueMax>, q));
     if (int st = launched("gemv_queue_kernel")) return st;
   }
   return BT_OK;
@@ -1036,8 +1062,8 @@ Scratch scratch_at(unsigned char *set) {
   return s;
 }
 
-Queue workspace_scratch(uint64_t work) {
-  Queue q{};
+QueueHead workspace_scratch(uint64_t work) {
+  QueueHead q{};
   unsigned char *base = as_ptr<unsigned char>(work);
   q.error = reinterpret_cast<int *>(base + kWsError), q.ops_done = reinterpret_cast<int *>(base + kWsOpsDone), q.all_done = reinterpret_cast<int *>(base + kWsAllDone);
   q.sets = kSets;
@@ -1127,7 +1153,7 @@ int bt_gemv_bfp_static(int device, int fmt, int epilogue, int M, int K, int N, u
   // the array keeps whatever the last call left: the arrival counters must start at zero. The wait-gave-up word at
   // its start is left alone, so that it stays until bt_gemv_check(device, 0, ...) reads it.
   BT_CUDA(cudaMemsetAsync(base + kWsOpsDone, 0, kStControlBytes - kWsOpsDone, as_stream(stream)));
-  Queue scratch{};
+  QueueHead scratch{};
   scratch.error = reinterpret_cast<int *>(base + kWsError), scratch.ops_done = reinterpret_cast<int *>(base + kWsOpsDone), scratch.all_done = reinterpret_cast<int *>(base + kWsAllDone);
   scratch.sets = 1;
   scratch.set[0].panels_done = reinterpret_cast<int *>(base + 192), scratch.set[0].counters = reinterpret_cast<int *>(base + kStCounters);
