@@ -315,14 +315,6 @@ __global__ void put_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict_
   auto place = [&](int r) { return ids[(size_t)(r / 32) * 1024 + (r % 32 / 16) * 256 + r % 16]; };
   const int p = place(i);
   if (p < 0 || p / 32 >= dst_tr) return;
-  if (last) {
-    if (last[single ? 0 : p] != i) return;
-  } else {
-    for (int later = i + 1; later < n; later++) {
-      const int q = place(later);
-      if (single ? (unsigned)q < 32u : q == p) return;
-    }
-  }
   constexpr int ITEM = FMT < 0 ? -FMT : 2;                                    // bytes of a datum of x
   const size_t at_x = (size_t)((i % 32 / 16) * 2 + f) * 256 + (i % 16) * 16;  // first datum of the run in x's tile
   const uint8_t *src = x + (((size_t)b * x_tr + i / 32) * tc + j) * (1024 * ITEM) + at_x * ITEM;
@@ -337,6 +329,20 @@ __global__ void put_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict_
     const uint4 lo = reinterpret_cast<const uint4 *>(src)[0], hi = reinterpret_cast<const uint4 *>(src)[1];
     const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
     top = pack_run<BFP>(w, v);
+  }
+  // the places after this one are looked at while the run is on its way, eight at a time
+  if (last) {
+    if (last[single ? 0 : p] != i) return;
+  } else {
+    bool again = false;
+    for (int later = i + 1; later < n; later += 8) {
+      int q[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) q[k] = place(min(later + k, n - 1));
+#pragma unroll
+      for (int k = 0; k < 8; k++) again |= later + k < n && (single ? (unsigned)q[k] < 32u : q[k] == p);
+    }
+    if (again) return;
   }
   for (int r = single ? 0 : p % 32, end = single ? 32 : r + 1; r < end; r++) {
     const int run = ((r / 16) * 2 + f) * 16 + r % 16;                         // which of the destination tile's 64 runs
@@ -363,9 +369,9 @@ __device__ __forceinline__ uint32_t decode_bfp(uint32_t x, uint32_t e) {
   return (x >> 7) << 15 | ((e - s) & 255u) << 7 | ((m << s) & 0x7Eu);
 }
 
-// One run: the exponent byte e and the 16 value bytes in xb, four to a word (bfp4: each nibble moved to the top of a
-// byte of its own), to 16 bf16 values in o, two to a word.
-__device__ __forceinline__ void unpack_run(uint32_t e, const uint32_t (&xb)[4], uint32_t (&o)[8]) {
+// Half a run: the exponent byte e and 8 value bytes in xb, four to a word (bfp4: each nibble moved to the top of a
+// byte of its own), to 8 bf16 values in o, two to a word.
+__device__ __forceinline__ void unpack_half(uint32_t e, const uint32_t (&xb)[2], uint32_t (&o)[4]) {
   if (e >= 7u && e <= 247u) {
     // The same values on the multiply-add pipe: a magnitude of up to 7 bits times 2^(e - 133) is exact in fp32 and needs
     // no rounding to bf16, so its upper half IS the normalised bf16 the integer formula builds (equal for every byte
@@ -378,7 +384,7 @@ __device__ __forceinline__ void unpack_run(uint32_t e, const uint32_t (&xb)[4], 
     // never writes, and filling in only then, was slower: the branch costs more than the operations it saves.)
     const float scale = __uint_as_float((e - 6u) << 23);
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < 4; k++) {
       const uint32_t x = xb[k / 2], mags = x & 0x7F7F7F7Fu;
       const uint32_t low = x & ~(mags + 0x7F7F7F7Fu) & 0x80808080u, top = (x & 0x80808080u) | (low - (low >> 7));
       const uint32_t a = k % 2 ? __byte_perm(mags, 0x4B000000u, 0x7442) : __byte_perm(mags, 0x4B000000u, 0x7440);
@@ -389,38 +395,44 @@ __device__ __forceinline__ void unpack_run(uint32_t e, const uint32_t (&xb)[4], 
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
+    for (int k = 0; k < 4; k++) {
       const uint32_t lo = xb[k / 2] >> (16 * (k % 2)) & 255u, hi = xb[k / 2] >> (16 * (k % 2) + 8) & 255u;
       o[k] = decode_bfp(lo, e) | decode_bfp(hi, e) << 16;
     }
   }
 }
 
-// A thread unpacks one run: 64 consecutive bytes of a warp's output per store instruction pair (two runs to a thread,
-// which serves the packer well, spreads a warp's stores over twice the lines and was slower here).
+// A thread unpacks half a run at a time, 16 bytes of the result, so that a warp's store is 512 bytes in one piece and every
+// 32-byte sector goes to L2 whole; four of them, a block's width apart, so that enough loads are in flight.
+constexpr int kHalves = 4;
 template <int FMT>
-__global__ void unpack_kernel(const uint8_t *__restrict__ src, uint4 *__restrict__ dst, size_t runs) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= runs) return;
+__global__ void __launch_bounds__(kThreads) unpack_kernel(const uint8_t *__restrict__ src, uint4 *__restrict__ dst, size_t halves) {
   constexpr size_t TB = tile_bytes(FMT);
-  const uint8_t *tile = src + i / 64 * TB;
-  int r = (int)(i % 64);
-  uint32_t e = tile[r], xb[4], o[8];
-  if (FMT == BT_BFP8) {
-    uint4 v = *reinterpret_cast<const uint4 *>(tile + 64 + r * 16);
-    xb[0] = v.x, xb[1] = v.y, xb[2] = v.z, xb[3] = v.w;
-  } else {
-    uint2 v = *reinterpret_cast<const uint2 *>(tile + 64 + r * 8);
-    const uint32_t w[2] = {v.x, v.y};
+  const size_t first = (size_t)blockIdx.x * (kThreads * kHalves) + threadIdx.x;
+  uint32_t e[kHalves];
+  uint2 v[kHalves];
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-      const uint32_t even = (w[k] & 0x0F0F0F0Fu) << 4, odd = w[k] & 0xF0F0F0F0u;
-      xb[2 * k] = __byte_perm(even, odd, 0x5140), xb[2 * k + 1] = __byte_perm(even, odd, 0x7362);
-    }
+  for (int u = 0; u < kHalves; u++) {
+    const size_t i = first + u * kThreads;
+    if (i >= halves) break;
+    const uint8_t *tile = src + i / 128 * TB;
+    const int in = (int)(i % 128);
+    e[u] = tile[in / 2];
+    if (FMT == BT_BFP8) v[u] = *reinterpret_cast<const uint2 *>(tile + 64 + in * 8);
+    else v[u].x = *reinterpret_cast<const uint32_t *>(tile + 64 + in * 4);
   }
-  unpack_run(e, xb, o);
-  dst[2 * i] = make_uint4(o[0], o[1], o[2], o[3]);
-  dst[2 * i + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+#pragma unroll
+  for (int u = 0; u < kHalves; u++) {
+    const size_t i = first + u * kThreads;
+    if (i >= halves) break;
+    uint32_t xb[2] = {v[u].x, v[u].y}, o[4];
+    if (FMT == BT_BFP4) {
+      const uint32_t even = (v[u].x & 0x0F0F0F0Fu) << 4, odd = v[u].x & 0xF0F0F0F0u;
+      xb[0] = __byte_perm(even, odd, 0x5140), xb[1] = __byte_perm(even, odd, 0x7362);
+    }
+    unpack_half(e[u], xb, o);
+    dst[i] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
 }
 
 // ---- canonical <-> streaming layout ---------------------------------------------------------------------------
@@ -671,9 +683,10 @@ int bt_unpack_bfp(int device, int fmt, uint64_t src, uint64_t dst, size_t ntiles
   BT_REQUIRE(src && dst && ntiles, "bt_unpack_bfp: null device address or zero tiles");
   BT_REQUIRE(src % 16 == 0 && dst % 16 == 0, "bt_unpack_bfp: tiles must be 16-byte aligned");
   if (int s = use_device(device)) return s;
-  size_t runs = ntiles * 64;
-  if (fmt == BT_BFP8) unpack_kernel<BT_BFP8><<<blocks_for(runs), kThreads, 0, as_stream(stream)>>>(as_ptr<uint8_t>(src), as_ptr<uint4>(dst), runs);
-  else unpack_kernel<BT_BFP4><<<blocks_for(runs), kThreads, 0, as_stream(stream)>>>(as_ptr<uint8_t>(src), as_ptr<uint4>(dst), runs);
+  const size_t halves = ntiles * 128;
+  const unsigned blocks = blocks_for(ntiles * (128 / kHalves));
+  if (fmt == BT_BFP8) unpack_kernel<BT_BFP8><<<blocks, kThreads, 0, as_stream(stream)>>>(as_ptr<uint8_t>(src), as_ptr<uint4>(dst), halves);
+  else unpack_kernel<BT_BFP4><<<blocks, kThreads, 0, as_stream(stream)>>>(as_ptr<uint8_t>(src), as_ptr<uint4>(dst), halves);
   return launched("unpack_kernel");
 }
 
