@@ -19,6 +19,7 @@ DIMS = 5
 PARTS = 48 << 20   # bytes at most that a matmul of many rows borrows for sums of parts of K
 FIDELITY = 4   # accepted for parity; products are always exact here (baretile/tensor.py:12)
 EPILOGUE = {"none": 0, "relu": 1, "silu": 2, "glu": 3, "argmax": 4}
+DTYPES = (*ITEMSIZE, *BFP)
 NAMES = {(dtype, epilogue): f"matmul {dtype} {epilogue}" for dtype in BFP for epilogue in EPILOGUE}
 
 
@@ -36,10 +37,10 @@ class Tensor:
   addr, op, srcs, owner, runs = None, None, (), None, None
   _stream = None               # this block-float matrix in streaming layout, made on first use as a matmul's B
   def __init__(self, rt, rows, cols, op=None, srcs=(), batch=1, dtype="bf16"):
-    batch, rows, cols = _shape((batch, rows, cols))
-    if dtype not in (*ITEMSIZE, *BFP): raise ValueError(f"unknown tensor dtype: {dtype}")
-    if any(s.rt is not rt for s in srcs if isinstance(s, Tensor)): raise ValueError("tensor operands must use the same runtime")
-    rt.check()
+    if not (type(batch) is type(rows) is type(cols) is int and batch > 0 and rows > 0 and cols > 0): batch, rows, cols = _shape((batch, rows, cols))
+    if dtype not in DTYPES: raise ValueError(f"unknown tensor dtype: {dtype}")
+    if srcs and any(s.rt is not rt for s in srcs if isinstance(s, Tensor)): raise ValueError("tensor operands must use the same runtime")
+    if not rt.active: rt.check()
     self.rt, self.rows, self.cols, self.batch, self.op, self.srcs, self.dtype = rt, rows, cols, batch, op, srcs, dtype
     self.lead = (batch,)
     self.tr, self.tc = -(-rows // 32), -(-cols // 32)
@@ -153,7 +154,7 @@ class Tensor:
   def cast(self, dtype):
     """Convert storage format (baretile/tensor.py:581-596). bf16 -> bfp8 / bfp4 packs each run of 16 values along a
     row around its largest exponent; a block float -> bf16 decodes exactly."""
-    if dtype not in (*ITEMSIZE, *BFP): raise ValueError(f"unknown tensor dtype: {dtype}")
+    if dtype not in DTYPES: raise ValueError(f"unknown tensor dtype: {dtype}")
     if dtype == self.dtype and not self.runs: return self
     x = self.realize()
     if self.dtype in BFP:
@@ -164,7 +165,7 @@ class Tensor:
         src = held
       self.rt.launch("bt_unpack_bfp", (FMT_CODE[self.dtype], src, out.addr, self.tiles), name="storage")
       if held is not None: self.rt.dram_free(held)
-      return out.cast(dtype)
+      return out if dtype == "bf16" else out.cast(dtype)
     if dtype in BFP:
       if self.dtype != "bf16": raise ValueError(f"a block float is cast from bf16, not {self.dtype}")
       out = Tensor(self.rt, self.rows, self.cols, batch=self.batch, dtype=dtype)
@@ -280,7 +281,7 @@ class Tensor:
 
   def realize(self, into=None):
     """Compute an unrealized expression with one launch and keep the result (baretile/tensor.py:466-524)."""
-    self.rt.check()
+    if not self.rt.active: self.rt.check()
     if self.op is None: return self
     if into is not None: raise ValueError("realize(into=) is not on this backend's path")
     plan = _plan(self)
