@@ -10,21 +10,26 @@ namespace {
 constexpr int kThreads = 256;
 inline unsigned blocks_for(size_t items) { return (unsigned)((items + kThreads - 1) / kThreads); }
 
-// Launches a kernel whose blocks may come up while the launch before it drains; they wait for it in in_turn(), ahead of everything
-// else. For short kernels that follow one another, a cache's rows and its decoding: the launch itself is a fifth of their time.
+// Every kernel of this file is launched so that its blocks may come up while the launch before it drains, and waits for that one
+// in in_turn(), ahead of anything it reads or writes: these kernels are short and follow one another, and a launch's start
+// was a fifth of their time (a cache's rows and its decoding together 25.1 us, this way 21.2). The pointers that are read from go
+// through in_turn() so that no load of theirs can be moved ahead of it.
 template <typename... P, typename... A>
-int launch_early(const char *name, void (*kernel)(P...), unsigned blocks, uint64_t stream, A... args) {
+int launch_early(const char *name, void (*kernel)(P...), dim3 grid, uint64_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3(blocks), cfg.blockDim = dim3(kThreads), cfg.stream = as_stream(stream), cfg.attrs = attr, cfg.numAttrs = 1;
+  cfg.gridDim = grid, cfg.blockDim = dim3(kThreads), cfg.stream = as_stream(stream), cfg.attrs = attr, cfg.numAttrs = 1;
   BT_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
   return launched(name);
 }
-__device__ __forceinline__ void in_turn() {
+template <typename P> __device__ __forceinline__ void behind_wait(P &p) { asm volatile("" : "+l"(p)::"memory"); }
+template <typename... P>
+__device__ __forceinline__ void in_turn(P &...read) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  (behind_wait(read), ...);
 }
 
 // ---- tilize / untilize ------------------------------------------------------------------------------------
@@ -34,6 +39,7 @@ __device__ __forceinline__ void in_turn() {
 // move as whole 16-byte words.
 template <typename T, bool WIDE>
 __global__ void tilize_kernel(const T *__restrict__ src, T *__restrict__ dst, int batch, int rows, int cols, int tr, int tc) {
+  in_turn(src);
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;          // half-run index in the tiled image
   size_t total = (size_t)batch * tr * tc * 128;
   if (i >= total) return;
@@ -62,6 +68,7 @@ __global__ void tilize_kernel(const T *__restrict__ src, T *__restrict__ dst, in
 
 template <typename T, bool WIDE>
 __global__ void untilize_kernel(const T *__restrict__ src, T *__restrict__ dst, int batch, int rows, int cols, int tr, int tc) {
+  in_turn(src);
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   size_t total = (size_t)batch * tr * tc * 128;
   if (i >= total) return;
@@ -92,6 +99,7 @@ __global__ void untilize_kernel(const T *__restrict__ src, T *__restrict__ dst, 
 // threadIdx.x, k = 0..3, the half run within the tile row.
 template <typename T, bool TILIZE>
 __global__ void __launch_bounds__(kThreads) tile_wide_kernel(const T *__restrict__ src, T *__restrict__ dst, int batch, int rows, int cols, int tr, int tc) {
+  in_turn(src);
   constexpr int W = (int)sizeof(T) * 8 / 16;                           // 16-byte words of a half run
   const int ti = blockIdx.x;
   for (int b = blockIdx.z; b < batch; b += gridDim.z)
@@ -125,9 +133,9 @@ __global__ void __launch_bounds__(kThreads) tile_wide_kernel(const T *__restrict
     }
 }
 template <typename T, bool TILIZE>
-void launch_tile_wide(const T *src, T *dst, int batch, int rows, int cols, int tr, int tc, cudaStream_t st) {
+int launch_tile_wide(uint64_t src, uint64_t dst, int batch, int rows, int cols, int tr, int tc, uint64_t stream) {
   const dim3 grid((unsigned)tr, (unsigned)min((tc * 128 + 1023) / 1024, 65535), (unsigned)min(batch, 65535));
-  tile_wide_kernel<T, TILIZE><<<grid, kThreads, 0, st>>>(src, dst, batch, rows, cols, tr, tc);
+  return launch_early("tile_wide_kernel", tile_wide_kernel<T, TILIZE>, grid, stream, as_ptr<T>(src), as_ptr<T>(dst), batch, rows, cols, tr, tc);
 }
 
 // Many small matrices in one launch (a decode step's inputs on their way in, its results on their way out): the table
@@ -143,6 +151,7 @@ struct ManyArgs {
 };
 template <typename T, bool TILIZE>
 __global__ void many_kernel(const ManyArgs a) {
+  in_turn();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.first[a.n]) return;
   int k = 0;
@@ -193,6 +202,7 @@ __global__ void many_kernel(const ManyArgs a) {
 
 // fp32 bits -> bf16 bits, round to nearest even; a NaN keeps a quiet payload.
 __global__ void round_bf16_kernel(const uint32_t *__restrict__ src, uint16_t *__restrict__ dst, size_t n) {
+  in_turn(src);
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint32_t b = src[i];
@@ -281,6 +291,7 @@ __device__ __forceinline__ uint32_t pack_run(const uint32_t (&w)[8], uint32_t (&
 // the values as 32 (bfp8) or 16 (bfp4) bytes. (A tile has 64 runs, so a pair never straddles two tiles.)
 template <int FMT>
 __global__ void pack_kernel(const uint4 *__restrict__ src, uint8_t *__restrict__ dst, size_t pairs) {
+  in_turn(src);
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= pairs) return;
   uint4 q[4];
@@ -316,6 +327,7 @@ __global__ void pack_kernel(const uint4 *__restrict__ src, uint8_t *__restrict__
 // place), so a caller may lend an int per row of the destination's tile rows: a first pass leaves there, for each
 // place, the last row of x that goes to it (the array starts at -1), and the copy compares instead of searching.
 __global__ void put_last_kernel(const int *__restrict__ ids, int n, int dst_tr, int single, int *__restrict__ last) {
+  in_turn(ids);
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int p = ids[(size_t)(i / 32) * 1024 + (i % 32 / 16) * 256 + i % 16];
@@ -326,7 +338,7 @@ __global__ void put_last_kernel(const int *__restrict__ ids, int n, int dst_tr, 
 template <int FMT>   // BT_BFP8, BT_BFP4, or an item size in bytes (2, 4 coded as -2, -4) for a plain copy
 __global__ void put_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict__ x, const int *__restrict__ ids, int batch, int n, int tc,
                            int dst_tr, int x_tr, int single, const int *__restrict__ last) {
-  in_turn();
+  in_turn(x, ids, last);
   const size_t unit = (size_t)blockIdx.x * blockDim.x + threadIdx.x;          // ((b * n + i) * tc + j) * 2 + f
   if (unit >= (size_t)batch * n * tc * 2) return;
   const int f = (int)(unit % 2), j = (int)(unit / 2 % tc), i = (int)(unit / 2 / tc % n), b = (int)(unit / 2 / tc / n);
@@ -425,7 +437,7 @@ __device__ __forceinline__ void unpack_half(uint32_t e, const uint32_t (&xb)[2],
 constexpr int kHalves = 4;
 template <int FMT>
 __global__ void __launch_bounds__(kThreads) unpack_kernel(const uint8_t *__restrict__ src, uint4 *__restrict__ dst, size_t halves) {
-  in_turn();
+  in_turn(src);
   constexpr size_t TB = tile_bytes(FMT);
   const size_t first = (size_t)blockIdx.x * (kThreads * kHalves) + threadIdx.x;
   uint32_t e[kHalves];
@@ -464,6 +476,7 @@ __global__ void __launch_bounds__(kThreads) unpack_kernel(const uint8_t *__restr
 // in the order 0, 2, 1, 3. blockIdx.y is the run of tile columns; a thread's unit is (tile of the run, h, t).
 template <int FMT>
 __global__ void __launch_bounds__(256) to_stream_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int tr, int tc) {
+  in_turn(src);
   constexpr int TB = tile_bytes(FMT), UNITS = FMT == BT_BFP8 ? 8 : 4;
   const int run = blockIdx.y, tj0 = run * kPanel, width = min(kPanel, tc - tj0);
   const unsigned long long u = (unsigned long long)blockIdx.x * 256 + threadIdx.x;
@@ -529,6 +542,7 @@ __global__ void __launch_bounds__(256) to_stream_kernel(const uint8_t *__restric
 // at a time, undoes the transposition and writes the datum rows 4t..4t+3 (and the exponent words of t).
 template <int FMT>
 __global__ void __launch_bounds__(256) from_stream_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int tr, int tc) {
+  in_turn(src);
   constexpr int TB = tile_bytes(FMT), UNITS = FMT == BT_BFP8 ? 8 : 4;
   const int run = blockIdx.y, tj0 = run * kPanel, width = min(kPanel, tc - tj0);
   const unsigned long long u = (unsigned long long)blockIdx.x * 256 + threadIdx.x;
@@ -600,20 +614,9 @@ int bt_tilize(int device, int itemsize, uint64_t src, uint64_t dst, int batch, i
   size_t items = (size_t)batch * tr * tc * 128;
   const bool wide = cols % 8 == 0 && src % 16 == 0 && dst % 16 == 0;
   const unsigned blocks = blocks_for(items);
-  cudaStream_t st = as_stream(stream);
-  if (wide && tc >= 8) {
-    if (itemsize == 2) launch_tile_wide<uint16_t, true>(as_ptr<uint16_t>(src), as_ptr<uint16_t>(dst), batch, rows, cols, tr, tc, st);
-    else launch_tile_wide<uint32_t, true>(as_ptr<uint32_t>(src), as_ptr<uint32_t>(dst), batch, rows, cols, tr, tc, st);
-    return launched("tile_wide_kernel");
-  }
-  if (itemsize == 2) {
-    if (wide) tilize_kernel<uint16_t, true><<<blocks, kThreads, 0, st>>>(as_ptr<uint16_t>(src), as_ptr<uint16_t>(dst), batch, rows, cols, tr, tc);
-    else tilize_kernel<uint16_t, false><<<blocks, kThreads, 0, st>>>(as_ptr<uint16_t>(src), as_ptr<uint16_t>(dst), batch, rows, cols, tr, tc);
-  } else {
-    if (wide) tilize_kernel<uint32_t, true><<<blocks, kThreads, 0, st>>>(as_ptr<uint32_t>(src), as_ptr<uint32_t>(dst), batch, rows, cols, tr, tc);
-    else tilize_kernel<uint32_t, false><<<blocks, kThreads, 0, st>>>(as_ptr<uint32_t>(src), as_ptr<uint32_t>(dst), batch, rows, cols, tr, tc);
-  }
-  return launched("tilize_kernel");
+  if (wide && tc >= 8) return itemsize == 2 ? launch_tile_wide<uint16_t, true>(src, dst, batch, rows, cols, tr, tc, stream) : launch_tile_wide<uint32_t, true>(src, dst, batch, rows, cols, tr, tc, stream);
+  if (itemsize == 2) return launch_early("tilize_kernel", wide ? tilize_kernel<uint16_t, true> : tilize_kernel<uint16_t, false>, blocks, stream, as_ptr<uint16_t>(src), as_ptr<uint16_t>(dst), batch, rows, cols, tr, tc);
+  return launch_early("tilize_kernel", wide ? tilize_kernel<uint32_t, true> : tilize_kernel<uint32_t, false>, blocks, stream, as_ptr<uint32_t>(src), as_ptr<uint32_t>(dst), batch, rows, cols, tr, tc);
 }
 
 int bt_untilize(int device, int itemsize, uint64_t src, uint64_t dst, int batch, int rows, int cols, uint64_t stream) {
@@ -625,20 +628,9 @@ int bt_untilize(int device, int itemsize, uint64_t src, uint64_t dst, int batch,
   size_t items = (size_t)batch * tr * tc * 128;
   const bool wide = cols % 8 == 0 && src % 16 == 0 && dst % 16 == 0;
   const unsigned blocks = blocks_for(items);
-  cudaStream_t st = as_stream(stream);
-  if (wide && tc >= 8) {
-    if (itemsize == 2) launch_tile_wide<uint16_t, false>(as_ptr<uint16_t>(src), as_ptr<uint16_t>(dst), batch, rows, cols, tr, tc, st);
-    else launch_tile_wide<uint32_t, false>(as_ptr<uint32_t>(src), as_ptr<uint32_t>(dst), batch, rows, cols, tr, tc, st);
-    return launched("tile_wide_kernel");
-  }
-  if (itemsize == 2) {
-    if (wide) untilize_kernel<uint16_t, true><<<blocks, kThreads, 0, st>>>(as_ptr<uint16_t>(src), as_ptr<uint16_t>(dst), batch, rows, cols, tr, tc);
-    else untilize_kernel<uint16_t, false><<<blocks, kThreads, 0, st>>>(as_ptr<uint16_t>(src), as_ptr<uint16_t>(dst), batch, rows, cols, tr, tc);
-  } else {
-    if (wide) untilize_kernel<uint32_t, true><<<blocks, kThreads, 0, st>>>(as_ptr<uint32_t>(src), as_ptr<uint32_t>(dst), batch, rows, cols, tr, tc);
-    else untilize_kernel<uint32_t, false><<<blocks, kThreads, 0, st>>>(as_ptr<uint32_t>(src), as_ptr<uint32_t>(dst), batch, rows, cols, tr, tc);
-  }
-  return launched("untilize_kernel");
+  if (wide && tc >= 8) return itemsize == 2 ? launch_tile_wide<uint16_t, false>(src, dst, batch, rows, cols, tr, tc, stream) : launch_tile_wide<uint32_t, false>(src, dst, batch, rows, cols, tr, tc, stream);
+  if (itemsize == 2) return launch_early("untilize_kernel", wide ? untilize_kernel<uint16_t, true> : untilize_kernel<uint16_t, false>, blocks, stream, as_ptr<uint16_t>(src), as_ptr<uint16_t>(dst), batch, rows, cols, tr, tc);
+  return launch_early("untilize_kernel", wide ? untilize_kernel<uint32_t, true> : untilize_kernel<uint32_t, false>, blocks, stream, as_ptr<uint32_t>(src), as_ptr<uint32_t>(dst), batch, rows, cols, tr, tc);
 }
 
 static int many(const char *what, bool tilize, int device, int itemsize, int n, const uint64_t *src, const uint64_t *dst, const int *rows, const int *cols,
@@ -657,16 +649,8 @@ static int many(const char *what, bool tilize, int device, int itemsize, int n, 
       BT_REQUIRE(a.first[k] + halves < (1ll << 31), "%s: too much for one launch: put large matrices through the single-matrix call", what);
       a.first[k + 1] = a.first[k] + (int)halves;
     }
-    const unsigned blocks = blocks_for((size_t)a.first[a.n]);
-    cudaStream_t st = as_stream(stream);
-    if (itemsize == 2) {
-      if (tilize) many_kernel<uint16_t, true><<<blocks, kThreads, 0, st>>>(a);
-      else many_kernel<uint16_t, false><<<blocks, kThreads, 0, st>>>(a);
-    } else {
-      if (tilize) many_kernel<uint32_t, true><<<blocks, kThreads, 0, st>>>(a);
-      else many_kernel<uint32_t, false><<<blocks, kThreads, 0, st>>>(a);
-    }
-    if (int s = launched("many_kernel")) return s;
+    const auto kernel = itemsize == 2 ? (tilize ? many_kernel<uint16_t, true> : many_kernel<uint16_t, false>) : tilize ? many_kernel<uint32_t, true> : many_kernel<uint32_t, false>;
+    if (int s = launch_early("many_kernel", kernel, blocks_for((size_t)a.first[a.n]), stream, a)) return s;
   }
   return BT_OK;
 }
@@ -682,8 +666,7 @@ int bt_untilize_many(int device, int itemsize, int n, const uint64_t *src, const
 int bt_round_bf16(int device, uint64_t src_f32, uint64_t dst_bf16, size_t count, uint64_t stream) {
   BT_REQUIRE(src_f32 && dst_bf16 && count, "bt_round_bf16: null device address or zero count");
   if (int s = use_device(device)) return s;
-  round_bf16_kernel<<<blocks_for(count), kThreads, 0, as_stream(stream)>>>(as_ptr<uint32_t>(src_f32), as_ptr<uint16_t>(dst_bf16), count);
-  return launched("round_bf16_kernel");
+  return launch_early("round_bf16_kernel", round_bf16_kernel, blocks_for(count), stream, as_ptr<uint32_t>(src_f32), as_ptr<uint16_t>(dst_bf16), count);
 }
 
 int bt_pack_bfp(int device, int fmt, uint64_t src, uint64_t dst, size_t ntiles, uint64_t stream) {
@@ -692,9 +675,7 @@ int bt_pack_bfp(int device, int fmt, uint64_t src, uint64_t dst, size_t ntiles, 
   BT_REQUIRE(src % 16 == 0 && dst % 16 == 0, "bt_pack_bfp: tiles must be 16-byte aligned");
   if (int s = use_device(device)) return s;
   size_t pairs = ntiles * 32;
-  if (fmt == BT_BFP8) pack_kernel<BT_BFP8><<<blocks_for(pairs), kThreads, 0, as_stream(stream)>>>(as_ptr<uint4>(src), as_ptr<uint8_t>(dst), pairs);
-  else pack_kernel<BT_BFP4><<<blocks_for(pairs), kThreads, 0, as_stream(stream)>>>(as_ptr<uint4>(src), as_ptr<uint8_t>(dst), pairs);
-  return launched("pack_kernel");
+  return launch_early("pack_kernel", fmt == BT_BFP8 ? pack_kernel<BT_BFP8> : pack_kernel<BT_BFP4>, blocks_for(pairs), stream, as_ptr<uint4>(src), as_ptr<uint8_t>(dst), pairs);
 }
 
 int bt_unpack_bfp(int device, int fmt, uint64_t src, uint64_t dst, size_t ntiles, uint64_t stream) {
@@ -719,13 +700,11 @@ int bt_put(int device, int fmt, uint64_t dst, uint64_t x, uint64_t ids, int batc
   uint8_t *d = as_ptr<uint8_t>(dst);
   const uint8_t *s8 = as_ptr<uint8_t>(x);
   const int *places = as_ptr<int>(ids);
-  cudaStream_t st = as_stream(stream);
   int *last = as_ptr<int>(scratch);
   if (last) {
     BT_REQUIRE(scratch % 4 == 0, "bt_put: the scratch holds ints");
-    BT_CUDA(cudaMemsetAsync(last, 0xFF, (size_t)dst_tr * 32 * sizeof(int), st));
-    put_last_kernel<<<blocks_for((size_t)n), kThreads, 0, st>>>(places, n, dst_tr, dst_rows == 1, last);
-    if (int s = launched("put_last_kernel")) return s;
+    BT_CUDA(cudaMemsetAsync(last, 0xFF, (size_t)dst_tr * 32 * sizeof(int), as_stream(stream)));
+    if (int s = launch_early("put_last_kernel", put_last_kernel, blocks_for((size_t)n), stream, places, n, dst_tr, (int)(dst_rows == 1), last)) return s;
   }
   const auto kernel = fmt == BT_BFP8 ? put_kernel<BT_BFP8> : fmt == BT_BFP4 ? put_kernel<BT_BFP4> : fmt == BT_BF16 ? put_kernel<-2> : put_kernel<-4>;
   return launch_early("put_kernel", kernel, blocks, stream, d, s8, places, batch, n, tc, dst_tr, x_tr, (int)(dst_rows == 1), last);
@@ -739,16 +718,12 @@ int bt_relayout(int device, int fmt, int to_stream, int tile_rows, int tile_cols
   BT_REQUIRE(runs <= 65535, "bt_relayout: at most %d tile columns in one launch, not %d", 65535 * kPanel, tile_cols);
   BT_REQUIRE(src && dst && src != dst && src % 16 == 0 && dst % 16 == 0, "bt_relayout: needs distinct 16-byte aligned buffers");
   if (int s = use_device(device)) return s;
-  cudaStream_t st = as_stream(stream);
   const uint8_t *s8 = as_ptr<uint8_t>(src);
   uint8_t *d8 = as_ptr<uint8_t>(dst);
   const unsigned long long units = (unsigned long long)tile_rows * min(kPanel, tile_cols) * (fmt == BT_BFP8 ? 8 : 4);
   const dim3 grid((unsigned)((units + 255) / 256), (unsigned)runs);
-  if (fmt == BT_BFP8 && to_stream) to_stream_kernel<BT_BFP8><<<grid, 256, 0, st>>>(s8, d8, tile_rows, tile_cols);
-  else if (to_stream) to_stream_kernel<BT_BFP4><<<grid, 256, 0, st>>>(s8, d8, tile_rows, tile_cols);
-  else if (fmt == BT_BFP8) from_stream_kernel<BT_BFP8><<<grid, 256, 0, st>>>(s8, d8, tile_rows, tile_cols);
-  else from_stream_kernel<BT_BFP4><<<grid, 256, 0, st>>>(s8, d8, tile_rows, tile_cols);
-  return launched(to_stream ? "to_stream_kernel" : "from_stream_kernel");
+  const auto kernel = to_stream ? (fmt == BT_BFP8 ? to_stream_kernel<BT_BFP8> : to_stream_kernel<BT_BFP4>) : fmt == BT_BFP8 ? from_stream_kernel<BT_BFP8> : from_stream_kernel<BT_BFP4>;
+  return launch_early(to_stream ? "to_stream_kernel" : "from_stream_kernel", kernel, grid, stream, s8, d8, tile_rows, tile_cols);
 }
 
 }  // extern "C"
