@@ -61,6 +61,7 @@ struct GemmParams {
   int row_blocks;            // blocks of 512 rows, or of 256 where `half`
   int half;                  // every pair takes 256 rows
   int splits;                // pairs of CTAs that share a block, each with its part of K; their sums meet in `part`
+  int weights_early;         // the launch before this one laid x out by rows
   float *part;               // [split][gate, up][tile_rows * 32][TC * 32] fp32, where splits > 1
   int whole;                 // pairs of CTAs that take a whole block of 512 rows x 256 MMA columns; the pairs after them
 };                           // take half a block (256 rows) each, so that the last wave of the grid is a short one
@@ -169,10 +170,13 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
   __syncthreads();
   cluster_sync();                                                   // the peer's barriers exist before anyone signals them
   tc_fence_after();
-  // All of that may happen while the launch before this one drains; what it wrote is read, and what it read written, from here
-  // on. The next launch may do the same (77 rows of 2048x5632, gate/up and down, 53.7 us without it).
+  // All of that may happen while the launch before this one drains. What that one writes is read, and what it reads written, only
+  // behind this wait: x, the addend, the result. Where it is the one that lays x out by rows, everything before it is
+  // complete (its blocks wait for that before they let this launch come up), so the weights need not wait, and the first
+  // of them are expanded by the time x is there.
+  auto in_turn = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
+  if (!p.weights_early) in_turn();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + 176);
 
   if (warp == 0) {
@@ -190,6 +194,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
           for (int j = 0; j < rows; j++) bulk_g2s(p_stage(ps) + j * kPanel * L::TB, src + (size_t)j * width * L::TB, width * L::TB, pfull0 + 8 * ps);
       };
       for (int i = 0; i < min(kbs, kStagesP - 1); i++) packed(i);
+      in_turn();
       for (int i = 0; i < kbs; i++) {
         if (i + kStagesP - 1 < kbs) packed(i + kStagesP - 1);
         const int s = i % kStagesAB;
@@ -230,6 +235,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
         mbar_arrive_cluster(leader_full0 + 8 * s);
       }
     }
+    in_turn();
     wait(acc_full, 0, 16);
     tc_fence_after();
     const int q = warp & 3, ch = d >> 2;                            // tensor-memory lane quarter; column half
@@ -392,7 +398,7 @@ int deal_blocks(GemmParams &p, int slots, size_t part_bytes) {
 
 // Argument checks and launches of both entry points.
 int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N, uint64_t a, uint64_t w, uint64_t w2, uint64_t add, int add_rows, float alpha,
-         uint64_t out, int out_dtype, uint64_t part, size_t part_bytes, uint64_t work, uint64_t stream) {
+         uint64_t out, int out_dtype, uint64_t part, size_t part_bytes, bool weights_early, uint64_t work, uint64_t stream) {
   BT_REQUIRE(fmt == BT_BFP8 || fmt == BT_BFP4, "%s: weights must be bfp8 (8) or bfp4 (4), not %d", who, fmt);
   BT_REQUIRE(epilogue >= BT_EPI_NONE && epilogue <= BT_EPI_GLU, "%s: the epilogue is none, relu, silu or glu, not %d", who, epilogue);
   const bool pair = epilogue == BT_EPI_GLU;
@@ -410,7 +416,7 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
   p.w[0] = as_ptr<uint8_t>(w), p.w[1] = as_ptr<uint8_t>(w2), p.add = as_ptr<uint16_t>(add), p.out = as_ptr<void>(out), p.error = as_ptr<int>(work);
   p.alpha = alpha, p.M = M, p.KT = K / 32, p.TC = (N + 31) / 32, p.epi = epilogue, p.out_fp32 = out_dtype == BT_FP32, p.pair = pair;
   p.add_row_stride = add && add_rows > 1 ? (size_t)p.TC * 1024 : 0;
-  p.part = as_ptr<float>(part);
+  p.part = as_ptr<float>(part), p.weights_early = weights_early;
   int sms = 0;
   BT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   const int pairs = deal_blocks(p, sms / 2 > 0 ? sms / 2 : 1, part_bytes);
@@ -452,7 +458,7 @@ extern "C" {
 
 int bt_gemm_bfp(int device, int fmt, int epilogue, int M, int K, int N, uint64_t a, uint64_t w, uint64_t w2, uint64_t add, int add_rows,
                 float alpha, uint64_t out, int out_dtype, uint64_t work, uint64_t stream) {
-  return gemm("bt_gemm_bfp", device, fmt, epilogue, M, K, N, a, w, w2, add, add_rows, alpha, out, out_dtype, 0, 0, work, stream);
+  return gemm("bt_gemm_bfp", device, fmt, epilogue, M, K, N, a, w, w2, add, add_rows, alpha, out, out_dtype, 0, 0, false, work, stream);
 }
 
 int bt_gemm_tiles(int device, int fmt, int epilogue, int M, int K, int N, uint64_t x, uint64_t w, uint64_t w2, uint64_t add, int add_rows,
@@ -461,7 +467,7 @@ int bt_gemm_tiles(int device, int fmt, int epilogue, int M, int K, int N, uint64
   const size_t rows = ((size_t)M * K * 2 + 255) / 256 * 256;
   BT_REQUIRE(x && x % 16 == 0 && scratch && scratch % 256 == 0 && scratch_bytes >= rows, "bt_gemm_tiles: needs x and at least %zu bytes of 256-byte aligned scratch, got %zu", rows, scratch_bytes);
   if (int s = bt_untilize(device, 2, x, scratch, 1, M, K, stream)) return s;
-  return gemm("bt_gemm_tiles", device, fmt, epilogue, M, K, N, scratch, w, w2, add, add_rows, alpha, out, out_dtype, scratch + rows, scratch_bytes - rows, work, stream);
+  return gemm("bt_gemm_tiles", device, fmt, epilogue, M, K, N, scratch, w, w2, add, add_rows, alpha, out, out_dtype, scratch + rows, scratch_bytes - rows, true, work, stream);
 }
 
 }  // extern "C"

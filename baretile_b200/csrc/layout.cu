@@ -27,8 +27,8 @@ int launch_early(const char *name, void (*kernel)(P...), dim3 grid, uint64_t str
 template <typename P> __device__ __forceinline__ void behind_wait(P &p) { asm volatile("" : "+l"(p)::"memory"); }
 template <typename... P>
 __device__ __forceinline__ void in_turn(P &...read) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // only now: whoever comes up finds all before this launch complete
   (behind_wait(read), ...);
 }
 
