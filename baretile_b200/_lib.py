@@ -4,7 +4,7 @@ The reference binds its device library the same way: ctypes.CDLL with explicit a
 (baretile/pci.py:52-63). Status codes become the exceptions the reference raises for the same conditions
 (docs/api.md:51-62): bad argument -> ValueError, device or state -> RuntimeError, timeout -> TimeoutError,
 out of memory -> MemoryError."""
-import ctypes, os, pathlib
+import ctypes, functools, os, pathlib, struct
 
 PATH = pathlib.Path(os.environ.get("BARETILE_B200_LIB") or pathlib.Path(__file__).resolve().parent / "libbaretile_b200.so")
 u64, i32, f32, size_t, vp = ctypes.c_uint64, ctypes.c_int, ctypes.c_float, ctypes.c_size_t, ctypes.c_void_p
@@ -22,6 +22,8 @@ class GemvOp(ctypes.Structure):
 
 
 SIGNATURES = {
+  "bt_packed_index": [ctypes.c_char_p, ctypes.POINTER(i32)],
+  "bt_packed_call": [ctypes.c_char_p],
   "bt_device_count": [ctypes.POINTER(i32)],
   "bt_device_info_get": [i32, ctypes.POINTER(DeviceInfo)],
   "bt_malloc": [i32, size_t, ctypes.POINTER(u64)],
@@ -82,12 +84,14 @@ SIGNATURES = {
 }
 
 ERRORS = {1: ValueError, 2: RuntimeError, 3: TimeoutError, 4: MemoryError}
+WORDS = {i32: "q", u64: "Q", size_t: "Q", vp: "Q", f32: "d"}
 _lib = None
+_packed, _packed_call = {}, None       # entry point -> its arguments as words, for bt_packed_call
 
 
 def lib():
   """The loaded library. Raises if it was not built: this backend has no other way to compute."""
-  global _lib
+  global _lib, _packed, _packed_call
   if _lib is None:
     if not PATH.exists():
       raise RuntimeError(f"{PATH} is missing: build it with `make -C {PATH.parent / 'csrc'}` (needs nvcc, sm_100a); "
@@ -97,6 +101,10 @@ def lib():
       f = getattr(loaded, name)
       f.argtypes, f.restype = argtypes, i32
     loaded.bt_last_error.argtypes, loaded.bt_last_error.restype = [], ctypes.c_char_p
+    index, _packed, _packed_call = i32(), {}, loaded.bt_packed_call
+    for name, argtypes in SIGNATURES.items():
+      loaded.bt_packed_index(name.encode(), ctypes.byref(index))
+      if index.value >= 0: _packed[name] = functools.partial(struct.Struct("=q" + "".join(WORDS[t] for t in argtypes)).pack, index.value)
     _lib = loaded
   return _lib
 
@@ -107,5 +115,14 @@ def check(status):
 
 
 def call(name, *args):
+  pack = _packed.get(name)
+  if pack is not None:
+    # numbers go across as one array (ctypes converts arguments one by one); what is not a number that fits goes the usual way
+    try: words = pack(*args)
+    except (struct.error, OverflowError, TypeError): pass
+    else:
+      status = _packed_call(words)
+      if status: check(status)
+      return
   status = getattr(_lib or lib(), name)(*args)
   if status: check(status)

@@ -40,7 +40,7 @@ class Tensor:
     if not (type(batch) is type(rows) is type(cols) is int and batch > 0 and rows > 0 and cols > 0): batch, rows, cols = _shape((batch, rows, cols))
     if dtype not in DTYPES: raise ValueError(f"unknown tensor dtype: {dtype}")
     if srcs and any(s.rt is not rt for s in srcs if isinstance(s, Tensor)): raise ValueError("tensor operands must use the same runtime")
-    if not rt.active: rt.check()
+    rt.check()
     self.rt, self.rows, self.cols, self.batch, self.op, self.srcs, self.dtype = rt, rows, cols, batch, op, srcs, dtype
     self.lead = (batch,)
     self.tr, self.tc = -(-rows // 32), -(-cols // 32)
@@ -281,7 +281,7 @@ class Tensor:
 
   def realize(self, into=None):
     """Compute an unrealized expression with one launch and keep the result (baretile/tensor.py:466-524)."""
-    if not self.rt.active: self.rt.check()
+    self.rt.check()
     if self.op is None: return self
     if into is not None: raise ValueError("realize(into=) is not on this backend's path")
     plan = _plan(self)

@@ -42,6 +42,12 @@ typedef struct bt_device_info {
 /* Text of the calling thread's last error. */
 const char *bt_last_error(void);
 
+/* An entry point with its arguments as one array of 8-byte words, for callers whose foreign-function layer pays for every
+ * argument: the first word is the entry point's index, the others its arguments in order, integers and addresses as they are, a
+ * float as a double. bt_packed_index gives the index of an entry point by name; -1 for those that are not called this way. */
+int bt_packed_index(const char *name, int *index);
+int bt_packed_call(const char *words);
+
 /* ---- device, memory, streams, events: stand in for pci.open_device / Chip / Runtime
  *      (baretile/pci.py:453-463, baretile/chip.py:75-83, baretile/runtime.py:543-923) ---- */
 int bt_device_count(int *count);                       /* pci.Sim.chips / find_cards */
