@@ -16,7 +16,8 @@
 //                        directly on the LEADER CTA's "full" barrier (a cta_group::2 load; the leader arms the barrier
 //                        for both CTAs' bytes), and bulk-copies its 8 packed weight tiles (one run of the streaming
 //                        layout, two tile rows) into a ring.
-//   warps 2-9 (dequant)  each takes one packed tile, expands it to exact bf16 in registers the way the decode kernel
+//   warps 2-9 (dequant)  (and 10-17, which take every other K block, where a pair has 256 rows: there a K block's expansion
+//                        takes longer than its MMAs) each takes one packed tile, expands it to exact bf16 in registers the way the decode kernel
 //                        does (a mask or byte permute, then a packed multiply-add with the face row's power of two),
 //                        and stores it into the B tile in the K-major 128-byte-swizzled layout the MMA reads. The
 //                        weights carry a factor 2^-64, undone in the epilogue. When its tile is stored and fenced
@@ -43,7 +44,7 @@ namespace {
 constexpr int kBK = 64;                                  // K block
 constexpr int kStagesAB = 3, kStagesP = 4;             // four stages of x and weights measured the same as three
 constexpr int kDequantWarps = 8;
-constexpr int kThreads = (2 + kDequantWarps) * 32;
+constexpr int threads_of(int groups) { return (2 + groups * kDequantWarps) * 32; }
 constexpr uint32_t kWaitLimit = 1u << 14;                // attempts of up to 100 us each
 
 constexpr int kABytes = 128 * 128;                       // one 128-row half of this CTA's x for a K block
@@ -130,8 +131,8 @@ __device__ __forceinline__ void expand_tile(uint32_t tile, uint32_t b, int c, in
 
 // SPLIT: the pairs share K. A kernel of its own, since whole blocks lose 2 % to the K block a pair starts at and the sums that
 // go out as they are.
-template <int FMT, bool SPLIT>
-__global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap) {
+template <int FMT, bool SPLIT, int GROUPS>
+__global__ void __launch_bounds__(threads_of(GROUPS), 1) gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap amap) {
   using L = Layout<FMT>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);   // swizzled tiles want 1024-byte alignment
@@ -220,9 +221,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
     }
   } else {
     // ---- dequant warps, then the epilogue ----
-    const int d = warp - 2, c = d & 3, j = d >> 2;                  // this warp's tile column and tile row in a K block
+    const int d = warp - 2, c = d & 3, j = d >> 2 & 1;                  // this warp's tile column and tile row in a K block
     const uint32_t leader_full0 = map_to_cta(full0, 0);
-    for (int i = 0; i < kbs; i++) {
+    for (int i = d / kDequantWarps; i < kbs; i += GROUPS) {
       const int ps = i % kStagesP, s = i % kStagesAB;
       if (width > 0) wait(pfull0 + 8 * ps, (i / kStagesP) & 1, 14);
       if (i >= kStagesAB) wait(empty0 + 8 * s, (i / kStagesAB - 1) & 1, 15);
@@ -240,77 +241,66 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kernel(const GemmParams p, c
     tc_fence_after();
     const int q = warp & 3, ch = d >> 2;                            // tensor-memory lane quarter; column half
     const float unscale = 18446744073709551616.f * p.alpha;         // 2^64: the weights were expanded times 2^-64
-    const int out_cols = p.pair ? 128 : 256, chunks = out_cols / 64;  // 32-column chunks for this warp
+    const int out_cols = p.pair ? 128 : 256, part = out_cols / (2 * GROUPS);   // this warp's columns
+    constexpr int COLS = GROUPS == 1 ? 32 : 16;                     // and how many at a time: 32 need more registers than 18 warps have
     const int tile_rows = (p.M + 31) / 32;
 #pragma unroll 1
     for (int mh = 0; mh < MH; mh++) {
       const int row = row0(mh) + 32 * q + lane, tr = row >> 5;
       if (tr >= tile_rows) continue;                                // the whole warp is past the tensor's tile rows
 #pragma unroll 1
-      for (int cc = 0; cc < chunks; cc++) {
-        const int col = ch * (out_cols / 2) + 32 * cc;              // first output column of the chunk, within the block
+      for (int col = ch * part; col < (ch + 1) * part; col += COLS) {   // first output column, within the block
         const int tcol = bc * (out_cols / 32) + (col >> 5);         // its tile column
         if (tcol >= p.TC) continue;
-        uint32_t v[32], u[32];
-        tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + mh * 256 + col, v);
-        if (p.pair) tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + mh * 256 + 128 + col, u);
+        uint32_t v[COLS], u[COLS];
+        tmem_ld(tmem + ((uint32_t)(32 * q) << 16) + mh * 256 + col, v);
+        if (p.pair) tmem_ld(tmem + ((uint32_t)(32 * q) << 16) + mh * 256 + 128 + col, u);
         tmem_ld_wait();
         if (SPLIT) {
           // sums of a part of K, as they are: reduce_kernel adds the parts
           if (row < p.M) {
             const size_t cols = (size_t)p.TC * 32, plane = (size_t)tile_rows * 32 * cols;
-            float *o = p.part + (size_t)split * (p.pair ? 2 : 1) * plane + (size_t)row * cols + tcol * 32;
+            float *o = p.part + (size_t)split * (p.pair ? 2 : 1) * plane + (size_t)row * cols + tcol * 32 + (col & 16);
 #pragma unroll
-            for (int i = 0; i < 8; i++) reinterpret_cast<uint4 *>(o)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            for (int i = 0; i < COLS / 4; i++) reinterpret_cast<uint4 *>(o)[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
             if (p.pair) {
 #pragma unroll
-              for (int i = 0; i < 8; i++) reinterpret_cast<uint4 *>(o + plane)[i] = make_uint4(u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
+              for (int i = 0; i < COLS / 4; i++) reinterpret_cast<uint4 *>(o + plane)[i] = make_uint4(u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
             }
           }
           continue;
         }
-        const int in_tile = ((row >> 4) & 1) * 512 + (row & 15) * 16;    // datum index of (row, 0) in the tile
-        float f[32];
+        const int in_tile = ((row >> 4) & 1) * 512 + (col & 16) * 16 + (row & 15) * 16;    // datum index of (row, col) in the tile
+        uint32_t w[COLS / 2] = {};
         if (p.add) {
-          const uint16_t *a = p.add + (size_t)tr * p.add_row_stride + (size_t)tcol * 1024 + (p.add_row_stride ? in_tile : 0);
+          const uint4 *a = reinterpret_cast<const uint4 *>(p.add + (size_t)tr * p.add_row_stride + (size_t)tcol * 1024 + (p.add_row_stride ? in_tile : (col & 16) * 16));
 #pragma unroll
-          for (int fcol = 0; fcol < 2; fcol++)
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-              const uint4 w4 = reinterpret_cast<const uint4 *>(a + fcol * 256)[i];
-              const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-              for (int k = 0; k < 4; k++) f[16 * fcol + 8 * i + 2 * k] = __uint_as_float(w[k] << 16), f[16 * fcol + 8 * i + 2 * k + 1] = __uint_as_float(w[k] & 0xFFFF0000u);
-            }
+          for (int i = 0; i < COLS / 8; i++) {
+            const uint4 a4 = a[i / 2 * 32 + i % 2];
+            w[4 * i] = a4.x, w[4 * i + 1] = a4.y, w[4 * i + 2] = a4.z, w[4 * i + 3] = a4.w;
+          }
         }
+        float f[COLS];
 #pragma unroll
-        for (int i = 0; i < 32; i++) {
+        for (int i = 0; i < COLS; i++) {
           float x = __uint_as_float(v[i]) * unscale;
-          if (p.add) x += f[i];
+          if (p.add) x += __uint_as_float(i % 2 ? w[i / 2] & 0xFFFF0000u : w[i / 2] << 16);
           if (p.pair) x = silu(x) * (__uint_as_float(u[i]) * unscale);
           else if (p.epi == BT_EPI_RELU) x = fmaxf(x, 0.f);
           else if (p.epi == BT_EPI_SILU) x = silu(x);
           f[i] = row < p.M ? x : 0.f;
         }
-        const size_t tile = (size_t)tr * p.TC + tcol;
+        const size_t at = ((size_t)tr * p.TC + tcol) * 1024 + in_tile;
         if (p.out_fp32) {
-          float *o = static_cast<float *>(p.out) + tile * 1024 + in_tile;
+          float4 *o = reinterpret_cast<float4 *>(static_cast<float *>(p.out) + at);
 #pragma unroll
-          for (int fcol = 0; fcol < 2; fcol++)
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-              reinterpret_cast<float4 *>(o + fcol * 256)[i] = make_float4(f[16 * fcol + 4 * i], f[16 * fcol + 4 * i + 1], f[16 * fcol + 4 * i + 2], f[16 * fcol + 4 * i + 3]);
+          for (int i = 0; i < COLS / 4; i++) o[i / 4 * 64 + i % 4] = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
         } else {
-          uint16_t *o = static_cast<uint16_t *>(p.out) + tile * 1024 + in_tile;
+          uint4 *o = reinterpret_cast<uint4 *>(static_cast<uint16_t *>(p.out) + at);
 #pragma unroll
-          for (int fcol = 0; fcol < 2; fcol++)
+          for (int k = 0; k < COLS / 2; k++) w[k] = bf16_half_up(f[2 * k]) | bf16_half_up(f[2 * k + 1]) << 16;
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
-              uint32_t w[4];
-#pragma unroll
-              for (int k = 0; k < 4; k++) w[k] = bf16_half_up(f[16 * fcol + 8 * i + 2 * k]) | bf16_half_up(f[16 * fcol + 8 * i + 2 * k + 1]) << 16;
-              reinterpret_cast<uint4 *>(o + fcol * 256)[i] = make_uint4(w[0], w[1], w[2], w[3]);
-            }
+          for (int i = 0; i < COLS / 8; i++) o[i / 2 * 32 + i % 2] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
         }
       }
     }
@@ -371,6 +361,11 @@ __global__ void __launch_bounds__(256) reduce_kernel(const GemmParams p) {
 // takes kBlockUs for a K block of 256 rows and kFixedUs for everything else; the parts move at 3 TB/s and cost another
 // launch. 2048 rows of 14336 x 4096 stay as they are (64 blocks), 77 rows of 5632 x 2048 (8 blocks of 88 K blocks) go in 9
 // parts.
+// Where every pair has 256 rows the MMAs of a K block take 512 cycles and its expansion, one warp's chain of waits, loads,
+// arithmetic and stores, 700, so two groups of warps expand K blocks in turn: 40 rows of 4096x14336, gate/up and down, 133 -> 118
+// us, 512 rows 202 -> 191. With 512 rows to a pair the MMAs take 1024, one group keeps up, and a second one only
+// gets in the way of the MMAs' operands (2048 rows 562 -> 665).
+bool two_groups(const GemmParams &p) { return p.half || p.M <= 256; }
 constexpr float kBlockUs = 0.42f, kFixedUs = 5.f, kReduceUs = 3.f, kPartBytesPerUs = 3e6f;
 int deal_blocks(GemmParams &p, int slots, size_t part_bytes) {
   const int runs = (p.TC + kPanel - 1) / kPanel, columns = p.pair ? runs : (runs + 1) / 2, KB = (p.KT + 1) / 2, tile_rows = (p.M + 31) / 32;
@@ -420,12 +415,14 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
   int sms = 0;
   BT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   const int pairs = deal_blocks(p, sms / 2 > 0 ? sms / 2 : 1, part_bytes);
+  using Kernel = void (*)(GemmParams, CUtensorMap);
+  static const Kernel kernels[2][2][2] = {{{gemm_kernel<BT_BFP8, false, 1>, gemm_kernel<BT_BFP8, false, 2>}, {gemm_kernel<BT_BFP8, true, 1>, gemm_kernel<BT_BFP8, true, 2>}},
+                                          {{gemm_kernel<BT_BFP4, false, 1>, gemm_kernel<BT_BFP4, false, 2>}, {gemm_kernel<BT_BFP4, true, 1>, gemm_kernel<BT_BFP4, true, 2>}}};
+  static const int bytes[2] = {Layout<BT_BFP8>::BYTES + 1024, Layout<BT_BFP4>::BYTES + 1024};
   static bool configured[64] = {};
   if (!configured[device & 63]) {
-    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP8>::BYTES + 1024));
-    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP8>::BYTES + 1024));
-    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP4>::BYTES + 1024));
-    BT_CUDA(cudaFuncSetAttribute(gemm_kernel<BT_BFP4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<BT_BFP4>::BYTES + 1024));
+    for (int f = 0; f < 2; f++)
+      for (int k = 0; k < 4; k++) BT_CUDA(cudaFuncSetAttribute(kernels[f][k / 2][k % 2], cudaFuncAttributeMaxDynamicSharedMemorySize, bytes[f]));
     configured[device & 63] = true;
   }
   cudaLaunchConfig_t cfg{};
@@ -433,15 +430,14 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
   cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = (fmt == BT_BFP8 ? Layout<BT_BFP8>::BYTES : Layout<BT_BFP4>::BYTES) + 1024;
+  const int groups = two_groups(p) ? 2 : 1;
+  cfg.blockDim = dim3(threads_of(groups));
+  cfg.dynamicSmemBytes = bytes[fmt == BT_BFP4];
   cfg.stream = as_stream(stream);
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr, cfg.numAttrs = 2;
-  const bool split = p.splits > 1;
-  if (fmt == BT_BFP8) BT_CUDA(split ? cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP8, true>, p, amap) : cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP8, false>, p, amap));
-  else BT_CUDA(split ? cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP4, true>, p, amap) : cudaLaunchKernelEx(&cfg, gemm_kernel<BT_BFP4, false>, p, amap));
+  BT_CUDA(cudaLaunchKernelEx(&cfg, kernels[fmt == BT_BFP4][p.splits > 1][groups - 1], p, amap));
   if (int s = launched("gemm_kernel")) return s;
   if (p.splits == 1) return BT_OK;
   // its blocks come up while the last of gemm_kernel drain, and wait there until that is complete
