@@ -17,9 +17,9 @@
 // layout). A unit is one tile row of one sub-panel. Units are numbered sub-panel by sub-panel and dealt out in
 // contiguous ranges to the CTAs, one per SM: equal shares of all CTAs, so every SM streams the same number of bytes
 // whatever the shape, or, for small matmuls, whole sub-panels. A sub-panel that several CTAs share is finished by the
-// CTA that holds its last tile row: the others write their fp32 partial sums to scratch and bump a counter; the owner,
-// which takes that sub-panel last, waits for the counter (with a limit), adds the partials in CTA order, so results do
-// not depend on timing, and runs the epilogue. Contributors never wait, so the owner's wait always ends; it is bounded
+// CTA that holds its last tile row: the others write their fp32 partial sums to scratch, where a word is zero until its
+// sum is there; the owner, which takes that sub-panel last, waits for the words (with a limit), adds them in CTA order, so
+// results do not depend on timing, and runs the epilogue. Contributors never wait, so the owner's wait always ends; it is bounded
 // all the same.
 //
 // Inside a CTA: two producer warps fill the ring, 16 consumer warps empty it. For one weight matrix a consumer warp has
@@ -905,8 +905,7 @@ int wait_for(const bt_gemv_op *ops, int i, int sets) {
 // with the least estimated time is taken, from the rates measured on 8192 x 28672 in steady state: HBM 6.3 TB/s, 50 GB/s
 // into one SM, and an SM's time for a tile row of four tiles (row_us). In ranges that straddle, a sub-panel shared by two or
 // three CTAs is handed over early: its contributors take it first. 4096 x 4096 is cut 4 ways (128 CTAs), 4096 x 14336 not
-// at all (112 CTAs), 576 x 1536 not at all, 1536 x 576 8 ways; a gate/up pair of 4096 x 14336 and 8192 x 28672 go in
-// equal shares. The choice depends on the shape only, never on a matmul's place in a queue: the way the sums are grouped,
+// at all (112 CTAs); a gate/up pair of 4096 x 14336 and 8192 x 28672 go in equal shares. The choice depends on the shape only, never on a matmul's place in a queue: the way the sums are grouped,
 // and with it the last bit of a result, must not change with how matmuls are batched.
 constexpr float kHbmBytesPerUs = 6.3e6f, kSmBytesPerUs = 50e3f, kHandOverUs = 2.f, kEarlyUs = 1.2f, kFourSlotsUs = 0.4f, kStraddleUs = 1.f;
 float row_us(int tg) { return tg == 1 ? 0.07f : tg == 2 ? 0.1f : 0.145f; }
