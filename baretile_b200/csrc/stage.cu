@@ -1,8 +1,13 @@
 // Large copies between pageable host memory and the device. A plain cudaMemcpyAsync from pageable memory moves a few
 // GB/s: one thread of the driver copies everything through a buffer of its own before the bus sees it. Here several
 // threads copy, each through two page-locked buffers of its own: while the bus moves one, the thread fills (or empties)
-// the other. Eight threads keep the bus busy; megabyte chunks stay in the cores' caches between the copy and the bus.
-// A staging object belongs to its creator (a Runtime): 16 MB of page-locked memory and 7 sleeping threads, made at the
+// the other. How many threads, and how much at a time, is measured (us, 16 cores):
+//   to the device   five threads keep the bus busy and more only contend for it; 2 MB at a time, or 512 KB where that would leave
+//                   threads with less than four chunks (6 MB 970 -> 590, 24 MB 2000 -> 1030, 112 MB 4740 -> 3890,
+//                   against eight threads and 1 MB)
+//   to the host     the pages written to are often fresh, and faulting them in is what takes the time: eight threads, 1 MB at a
+//                   time (112 MB 6800; five threads 9700)
+// A staging object belongs to its creator (a Runtime): 32 MB of page-locked memory and 7 sleeping threads, made at the
 // first large copy and given back by bt_stage_destroy. Calls on one object take turns.
 #include "common.cuh"
 #include <condition_variable>
@@ -15,8 +20,8 @@ using namespace bt;
 
 namespace {
 
-constexpr size_t kChunk = 1 << 20;
-constexpr int kMostThreads = 8;
+constexpr size_t kBuffer = 2 << 20;
+constexpr size_t kMostThreads = 8, kUpThreads = 5;
 
 struct Stage {
   struct Lane {                       // one thread's buffers and the events that say when each is free
@@ -34,7 +39,7 @@ struct Stage {
   // the copy at hand
   bool up = false;
   char *host = nullptr, *dev = nullptr;
-  size_t bytes = 0;
+  size_t bytes = 0, chunk = 0, active = 0;   // the lanes from `active` on sit this one out
   cudaStream_t stream = nullptr;
   std::atomic<size_t> next{0};
   std::atomic<int> failed{0};
@@ -44,13 +49,13 @@ struct Stage {
     for (int b = 0;; b ^= 1) {
       if (cudaError_t e = cudaEventSynchronize(l.free[b])) return e;
       if (n[b]) memcpy(host + at[b], l.buf[b], n[b]), n[b] = 0;
-      const size_t i = failed ? SIZE_MAX / kChunk : next++;
-      const size_t from = i * kChunk;
+      const size_t i = failed ? SIZE_MAX / kBuffer : next++;
+      const size_t from = i * chunk;
       if (from >= bytes) {
         if (n[b ^ 1]) continue;       // the other buffer still has one
         return cudaSuccess;
       }
-      const size_t size = bytes - from < kChunk ? bytes - from : kChunk;
+      const size_t size = bytes - from < chunk ? bytes - from : chunk;
       if (up) memcpy(l.buf[b], host + from, size);
       else at[b] = from, n[b] = size;
       if (cudaError_t e = up ? cudaMemcpyAsync(dev + from, l.buf[b], size, cudaMemcpyHostToDevice, stream) : cudaMemcpyAsync(l.buf[b], dev + from, size, cudaMemcpyDeviceToHost, stream)) return e;
@@ -68,6 +73,7 @@ struct Stage {
         wake.wait(hold, [&] { return stop || round != seen; });
         if (stop) return;
         seen = round;
+        if (lane >= active) continue;
       }
       work(lanes[lane]);
       std::lock_guard<std::mutex> hold(lock);
@@ -77,10 +83,12 @@ struct Stage {
   cudaError_t copy(bool up_, void *host_, uint64_t dev_, size_t bytes_, cudaStream_t stream_) {
     std::lock_guard<std::mutex> one(call);
     up = up_, host = static_cast<char *>(host_), dev = as_ptr<char>(dev_), bytes = bytes_, stream = stream_, next = 0, failed = 0;
-    const bool several = bytes > 2 * kChunk;
+    const size_t most = up && lanes.size() > kUpThreads ? kUpThreads : lanes.size();
+    chunk = !up ? kBuffer / 2 : bytes < 4 * kBuffer * most ? kBuffer / 4 : kBuffer;
+    const bool several = bytes > 2 * chunk && most > 1;
     if (several) {
       std::lock_guard<std::mutex> hold(lock);
-      round++, working = (int)threads.size();
+      round++, active = most, working = (int)most - 1;
       wake.notify_all();
     }
     work(lanes[0]);
@@ -119,7 +127,7 @@ int bt_stage_create(int device, uint64_t *stage) {
   cudaError_t e = cudaSuccess;
   for (auto &l : st->lanes)
     for (int b = 0; b < 2 && e == cudaSuccess; b++) {
-      e = cudaMallocHost(&l.buf[b], kChunk);
+      e = cudaMallocHost(&l.buf[b], kBuffer);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.free[b], cudaEventDisableTiming);
     }
   if (e != cudaSuccess) {
