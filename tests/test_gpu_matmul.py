@@ -462,3 +462,22 @@ def test_edges_of_stages_ranges_and_panels(rt, fmt, m, k, n):
   values, ids = (upload(rt, x) @ upload(rt, w).cast(fmt).columns()).topk(1)
   full = upload(rt, x).matmul(upload(rt, w).cast(fmt).columns(), dtype="fp32").numpy()
   assert np.array_equal(np.array(ids.tolist())[:, 0], o.argmax(full)) and np.array_equal(np.array(values.tolist())[:, 0], full.max(-1))
+
+
+@pytest.mark.parametrize("small", [False, True])
+@pytest.mark.parametrize("count", [8, 9])
+def test_lists_of_every_kind(rt, count, small):
+  # short and long lists, with and without a small matmul between large ones: the same bits as one launch per matmul
+  rng = np.random.default_rng(count)
+  big, little = (upload(rt, weights(rng, k, k)).cast("bfp8").columns() for k in (4096, 96))
+  x, y = upload(rt, acts(rng, 3, 4096)), upload(rt, acts(rng, 3, 96))
+  def both():
+    h, out = x, [(y @ little).realize()] if small else []
+    while len(out) < count:
+      h = (h @ big).silu().realize()
+      out.append(h)
+    return out
+  separate = [t.numpy() for t in both()]
+  with rt.queue(): queued = both()
+  rt.wait()
+  for got, want in zip(queued, separate): assert np.array_equal(got.numpy(), want)
