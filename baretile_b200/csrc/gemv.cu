@@ -8,10 +8,11 @@
 // unless the next weights are already on their way. The kernel therefore takes a list of matmuls (up to kQueueMax
 // per launch) and runs them in order with the same persistent CTAs. The weight warp of a CTA walks the whole list:
 // weight copies depend on nothing and go out as soon as the ring has room, across the boundary between two matmuls.
-// Only x waits: the x warp copies a matmul's activations once every sub-panel of the matmuls it depends on is
-// reported finished (a counter per matmul in global memory, read with acquire semantics; the host works out the dependences
-// from the buffer addresses, and matmuls that do not depend on one another overlap, two in flight at most). While
-// that report travels, the ring fills with the next weights: 190 KB per SM, 28 MB in all, over 4 us of HBM.
+// Only x waits: the x warp copies a matmul's activations once the last earlier matmul that this one depends on, and all
+// before that one, are complete: every sub-panel reported finished (a counter per matmul in global memory, read with acquire
+// semantics; see Gate on the host side, which works out the dependences from the buffer addresses). Matmuls that do not
+// depend on one another overlap, two in flight at most. While that report travels, the ring fills with the next weights:
+// 190 KB per SM, 28 MB in all, over 4 us of HBM.
 //
 // Decomposition ("stream-K"). A weight matrix is cut into sub-panels of 4 tile columns (one run of the streaming
 // layout). A unit is one tile row of one sub-panel. Units are numbered sub-panel by sub-panel and dealt out in
@@ -120,7 +121,8 @@ struct alignas(64) GemvParams {
   float alpha;
   int arg_base, M, KT, TC, epi, out_fp32;
   int fmt, pair, tg;
-  int wait_for, wait_panels;  // the matmul of the launch that must be complete before this one starts (-1: none), and its sub-panels
+  int wait_for, wait_panels;  // the last matmul of the launch that must be complete before this one starts (-1: none), and its sub-panels
+  int wait_also, also_panels; // the one before it, where its being complete does not follow (see Gate), and its sub-panels
   int turn;                   // CTA c takes the unit range (c + turn) % CTAs
   int lw, panels;             // tile columns of a sub-panel are 1 << lw, and there are so many sub-panels
   int tiled;                  // wmap is used
@@ -496,17 +498,21 @@ struct Ring {
 // its issuer and the copy engine the same whatever its size: with two plain copies of 256 bytes per tile the x
 // warp alone held an 8192 x 28672 bfp4 matmul at 46 us, with one of 1 KB at 35, where the weights take 31.
 // x may be the result of the launch before this one, or of an earlier matmul of this one: the host has worked out the
-// last matmul this one must see finished, all of its sub-panels. False: gave up.
+// last matmul of the launch that this one must see complete, and every one before that must be complete too (see Gate). A
+// whole warp waits, a lane for each of the two counters, so that their loads are in flight together. False: gave up.
 __device__ __forceinline__ bool await_turn(const QueueHead &q, const GemvParams &p, int pause_ns) {
   asm volatile("griddepcontrol.wait;" ::: "memory");     // returns when the previous launch is complete and visible
-  if (p.wait_for >= 0) {
+  const int lane = threadIdx.x & 31, op = lane == 0 ? p.wait_for : lane == 1 ? p.wait_also : -1;
+  bool ok = true;
+  if (op >= 0) {
+    const int panels = lane ? p.also_panels : p.wait_panels;
     uint32_t spins = 0;
-    while (ld_acquire_gpu(q.ops_done + p.wait_for) < p.wait_panels) {
-      if (++spins > kSpinLimit * 64) return false;
+    while (ld_acquire_gpu(q.ops_done + op) < panels) {
+      if (++spins > kSpinLimit * 64) { ok = false; break; }
       if (pause_ns) __nanosleep(pause_ns);
     }
   }
-  return true;
+  return __all_sync(0xFFFFFFFFu, ok);                    // what either lane acquired is visible to the whole warp
 }
 
 template <bool WEIGHTS, bool SMALL, class Q>
@@ -576,9 +582,7 @@ __device__ __forceinline__ void produce(const Q &q, uint8_t *smem, uint32_t sbas
           }
         } else {
           if (gate) {
-            int ok = 1;
-            if (lane == 0) ok = await_turn(q, p, 0);
-            if (!__shfl_sync(0xFFFFFFFFu, ok, 0) && lane == 0) atomicExch(q.error, 5);
+            if (!await_turn(q, p, 0) && lane == 0) atomicExch(q.error, 5);
             // x was written with ordinary stores (by other CTAs of this launch, or by the launch before) and is about to
             // be read by TMA copies: order what the acquire made visible before the asynchronous proxy's reads
             fence_proxy_async();
@@ -702,8 +706,7 @@ template <bool SMALL, class Q> __device__ __forceinline__ void carry(const Q &q,
     if (me < p.active) {
       walk.start(p, me);
       // the counters and the result are this matmul's only when the ones before it that it must not overtake are done
-      if (lane == 0 && !await_turn(q, p, 100)) atomicExch(q.error, 5);
-      __syncwarp();
+      if (!await_turn(q, p, 100) && lane == 0) atomicExch(q.error, 5);
     }
     while (walk.more()) {
       int sp, kt, rows;
@@ -747,7 +750,8 @@ template <bool SMALL, class Q> __device__ __forceinline__ void carry(const Q &q,
         __syncwarp();
       }
       // Report the sub-panel: its results are visible to the whole GPU before the count moves. A matmul is complete when all
-      // its sub-panels are: by then every CTA with a part in it has read its x, and is past its look at the counts. (Counting
+      // its sub-panels are: by then every CTA with a part in it has read its x, and is past its look at the counts. It says
+      // nothing about the matmul before it, of which this CTA may have no part: that is what Gate is about. (Counting
       // the CTAs instead, idle ones too, took 148 reports to one address where a small matmul has 5 sub-panels.) The last
       // report of the launch therefore finds nobody looking any more, and zeroes the counts for the next launch.
       if (lane == 0) {
@@ -898,6 +902,21 @@ int wait_for(const bt_gemv_op *ops, int i, int sets) {
   return w < 0 ? -1 : w;
 }
 
+// The matmuls whose counters matmul `i` looks at before it starts, so that `last` AND ALL BEFORE IT are complete: it may
+// depend on any of those, and any of them may still use its set of scratch. A matmul's counter speaks for that matmul
+// alone, since a CTA without a range in it passes it by. What follows from it: matmul j has started everywhere, so what j
+// itself waited for is complete, and (by induction over j) that is j's own `last` and all before it. `last` of every
+// matmul is at most kSets = 2 places back; so of the matmuls before w = `last`, all up to w - 2 are complete when w is, and
+// w - 1 is in doubt unless w waited for it. Then it is looked at too. In a chain it never is.
+static_assert(kSets == 2, "one more counter closes the gap that a last matmul two places back leaves");
+struct Gate {
+  int last, also;             // -1: none
+};
+Gate gate(const bt_gemv_op *ops, int i, int sets) {
+  const int w = wait_for(ops, i, sets);
+  return {w, w > 0 && wait_for(ops, w, sets) < w - 1 ? w - 1 : -1};
+}
+
 // The ranges of a matmul's units. Sharing a sub-panel costs a hand-over of partial sums, a range that straddles sub-panels
 // a second pass through a sub-panel's end, and fewer CTAs than SMs cost time only while the busy ones cannot take in what
 // HBM delivers. So the candidates are: every sub-panel cut into 1, 2, ... ranges, as many as there are SMs for; whole
@@ -1021,9 +1040,10 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       p.out = as_ptr<void>(o.out), p.arg_val = as_ptr<float>(o.arg_val), p.arg_idx = as_ptr<int>(o.arg_idx);
       p.alpha = o.alpha, p.arg_base = o.arg_base, p.M = o.M, p.KT = o.K / 32, p.TC = o.N / 32, p.epi = o.epilogue, p.out_fp32 = o.out_dtype == BT_FP32 ? 1 : o.out_dtype == BT_FP32_ROWS ? 2 : 0;
       p.fmt = o.fmt, p.pair = o.epilogue == BT_EPI_GLU, p.tg = o.M <= 8 ? 1 : o.M <= 16 ? 2 : 4;
-      p.wait_for = wait_for(ops + base, i, scratch.sets);
+      const Gate g = gate(ops + base, i, scratch.sets);
+      p.wait_for = g.last, p.wait_also = g.also;
       p.turn = (int)(((long long)(base + i) * 101) % ctas);
-      if (p.wait_for >= 0) p.wait_panels = q.op[p.wait_for].panels;
+      p.wait_panels = g.last >= 0 ? q.op[g.last].panels : 0, p.also_panels = g.also >= 0 ? q.op[g.also].panels : 0;
       deal_units(p, ctas);
       q.panels += p.panels;
       small |= p.small;
@@ -1110,6 +1130,18 @@ int bt_gemv_queue_plan(int n, const bt_gemv_op *ops, int *waits) {
   for (int i = 0; i < n; i++) {
     const int base = i / kQueueMax * kQueueMax, w = wait_for(ops + base, i - base, kSets);
     waits[i] = w < 0 ? -1 : base + w;
+  }
+  return BT_OK;
+}
+
+int bt_gemv_queue_gates(int n, const bt_gemv_op *ops, int *gates) {
+  BT_REQUIRE(n >= 1 && ops && gates, "bt_gemv_queue_gates: needs at least one matmul and somewhere for the answer");
+  for (int i = 0; i < n; i++)
+    if (int s = check_op("bt_gemv_queue_gates", i, ops[i])) return s;
+  for (int i = 0; i < n; i++) {
+    const int base = i / kQueueMax * kQueueMax;
+    const Gate g = gate(ops + base, i - base, kSets);
+    gates[2 * i] = g.last < 0 ? -1 : base + g.last, gates[2 * i + 1] = g.also < 0 ? -1 : base + g.also;
   }
   return BT_OK;
 }

@@ -175,12 +175,16 @@ typedef struct bt_gemv_op {
 } bt_gemv_op;
 int bt_gemv_queue(int device, int n, const bt_gemv_op *ops, uint64_t work, size_t work_bytes, uint64_t stream);
 /* What bt_gemv_queue would make each matmul wait for, without touching a device: waits[i] receives the index of the
- * last earlier matmul that ops[i] must see finished before it starts, or -1 when it only waits for the launch
- * before it. A matmul waits for the latest earlier one whose result it reads (x, add) or whose result buffers it
- * writes or that reads what it writes, and never runs more than two places ahead of a matmul still in flight; a
- * list longer than 32 is cut into launches of 32, and the first matmul of a launch waits for the whole launch
- * before it (-1). */
+ * last earlier matmul that ops[i] must see finished before it starts, it and all matmuls of the launch before it, or -1
+ * when it only waits for the launch before it. That is the latest earlier one whose result it reads (x, add) or whose result
+ * buffers it writes or that reads what it writes, or the one two places back where that comes later: a matmul never runs
+ * more than two places ahead of one still in flight. A list longer than 32 is cut into launches of 32, and the
+ * first matmul of a launch waits for the whole launch before it (-1). */
 int bt_gemv_queue_plan(int n, const bt_gemv_op *ops, int *waits);
+/* How it sees that: the matmuls whose own completion ops[i] looks at, gates[2 * i] = waits[i] and gates[2 * i + 1] the one
+ * before that where nothing else vouches for it (else -1). That everything up to waits[i] is finished follows from these
+ * two and from what they themselves had to see. For tests of that rule. */
+int bt_gemv_queue_gates(int n, const bt_gemv_op *ops, int *gates);
 /* ---- the matmul: fused_kernel's prefill grid (baretile/kernels.py:205-215, :470-506, grid_parts :18-39) ----
  * out[M, N] = epilogue(alpha * (a[M, K] @ W[K, N]) + add) for many rows, on the tcgen05 tensor cores with fp32
  * accumulators in tensor memory, two CTAs to an MMA. The weights are expanded from block float to exact bf16

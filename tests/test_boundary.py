@@ -1,6 +1,6 @@
 """The C-ABI boundary and the host-side mirror, without a GPU: the library loads and exports every symbol the header
 declares, the Python bindings agree with the header, and argument checks run before anything touches a device."""
-import ctypes, pathlib, re, subprocess, sys
+import ctypes, pathlib, random, re, subprocess, sys
 import pytest
 
 ROOT = pathlib.Path(__file__).resolve().parent.parent
@@ -115,6 +115,64 @@ def test_queue_plan_follows_the_addresses(built):
   waits = plan(many)
   assert waits[:3] == [-1, -1, 0] and waits[31] == 29 and waits[32] == -1 and waits[33] == -1
   with pytest.raises(ValueError, match="matmul 1: takes 1 to 32 rows"): plan([op(A, B), op(A, C, m=33)])
+
+
+def _gates(ops):
+  from baretile_b200 import _lib
+  arr, gates = (_lib.GemvOp * len(ops))(*ops), (ctypes.c_int * (2 * len(ops)))()
+  _lib.call("bt_gemv_queue_gates", len(ops), arr, gates)
+  return [tuple(gates[2 * i:2 * i + 2]) for i in range(len(ops))]
+
+
+def _complete(gates):
+  """For each matmul, the earlier ones of its launch that are complete when it starts: those it looks at, and whatever was
+  complete when those started. Nothing else: a matmul may be complete, or start, while one before it still runs."""
+  seen = []
+  for looks in gates: seen.append({j for g in looks if g >= 0 for j in (g, *seen[g])})
+  return seen
+
+
+def _must_be_complete(ops, i):
+  """The earlier matmuls of ops[i]'s launch (of 32) that it may not overlap: users of its scratch (two sets, taken in
+  turn) and those one of whose results it reads or overwrites, or that read what it writes."""
+  def reads(o): return {o.x, o.add} - {0}
+  def writes(o): return {o.arg_val, o.arg_idx} if o.epilogue == 4 else {o.out}
+  o, first = ops[i], i // 32 * 32
+  return {e for e in range(first, i) if (i - e) % 2 == 0 or writes(ops[e]) & (reads(o) | writes(o)) or reads(ops[e]) & writes(o)}
+
+
+def test_queue_waits_cover_every_dependence(built):
+  # a matmul looks at the counters of one or two earlier ones, each of which speaks for its own matmul only; what else must
+  # be complete has to follow from those
+  from baretile_b200 import _lib
+  def op(x, out, k=32, n=32, add=0, pick=False):
+    return _lib.GemvOp(fmt=8, epilogue=4 if pick else 0, M=1, K=k, N=n, out_dtype=0, alpha=1.0, x=x, w=0x100000, add=add, out=0 if pick else out,
+                       arg_val=out if pick else 0, arg_idx=out + 0x100000 if pick else 0)
+  A, B, C, D, E, F = (0x1000000 * i for i in range(1, 7))
+  lists = {
+    "a result read three places back": [op(A, B, k=8192), op(C, D), op(C, E), op(B, F)],
+    "two dependences": [op(A, B, k=8192), op(C, D), op(D, E, add=B)],
+    "scratch": [op(A, B, k=8192, pick=True), op(C, D), op(D, E, pick=True)],
+    "memory used again": [op(A, B, k=8192), op(C, D), op(C, E), op(C, A, n=8192)],
+  }
+  for name, ops in lists.items():
+    seen = _complete(_gates(ops))
+    for i in range(len(ops)): assert _must_be_complete(ops, i) <= seen[i], (name, i, _gates(ops))
+  # in a chain the one before it is all that a matmul looks at
+  assert _gates([op(A, B), op(B, C), op(C, D), op(D, E)]) == [(-1, -1), (0, -1), (1, -1), (2, -1)]
+  assert _gates([op(A, B), op(A, C), op(A, D), op(A, E)]) == [(-1, -1), (-1, -1), (0, -1), (1, 0)]
+  rng = random.Random(3)
+  for _ in range(300):
+    places = [0x1000000 * i for i in range(1, rng.choice([4, 8, 40]))]
+    ops = []
+    for _ in range(rng.randint(1, 70)):
+      x, out, add = (rng.choice(places) for _ in range(3))
+      ops.append(op(x, out, add=add if rng.random() < 0.3 else 0, pick=rng.random() < 0.2))
+    gates = _gates(ops)
+    seen = _complete(gates)
+    for i in range(len(ops)):
+      assert _must_be_complete(ops, i) <= seen[i], (i, gates)
+      assert all(g == -1 or i // 32 * 32 <= g < i for g in gates[i])     # the launch before it is complete as a whole
 
 
 def test_queue_collects_matmuls_and_flushes_in_order(monkeypatch):
