@@ -861,7 +861,8 @@ int check_op(const char *who, int index, const bt_gemv_op &o) {
   return BT_OK;
 }
 
-// The byte ranges a matmul reads (besides its weights, which no matmul writes) and writes.
+// The byte ranges a matmul reads and writes. No earlier matmul writes its weights, but a later one may write where they lay: in
+// the memory of weights that were freed behind their last use.
 struct Range {
   uint64_t a, b;
   bool meets(const Range &o) const { return a < o.b && o.a < b; }
@@ -870,6 +871,9 @@ int ranges_read(const bt_gemv_op &o, Range *r) {
   int n = 0;
   r[n++] = {o.x, o.x + (uint64_t)(o.K / 32) * 2048};
   if (o.add) r[n++] = {o.add, o.add + (uint64_t)(o.N / 32) * 2048};
+  const uint64_t weights = (uint64_t)(o.K / 32) * (o.N / 32) * tile_bytes(o.fmt);
+  r[n++] = {o.w, o.w + weights};
+  if (o.w2) r[n++] = {o.w2, o.w2 + weights};
   return n;
 }
 int ranges_written(const bt_gemv_op &o, Range *r) {
@@ -881,7 +885,7 @@ int ranges_written(const bt_gemv_op &o, Range *r) {
 }
 // `later` must not start before `earlier` is complete: it reads or writes what `earlier` writes, or writes what it reads.
 bool depends(const bt_gemv_op &later, const bt_gemv_op &earlier) {
-  Range lr[2], lw[2], er[2], ew[2];
+  Range lr[4], lw[2], er[4], ew[2];
   const int nlr = ranges_read(later, lr), nlw = ranges_written(later, lw), ner = ranges_read(earlier, er), new_ = ranges_written(earlier, ew);
   for (int i = 0; i < new_; i++) {
     for (int j = 0; j < nlr; j++) if (ew[i].meets(lr[j])) return true;

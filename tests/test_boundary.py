@@ -92,8 +92,8 @@ def test_hole_allocator_merges():
 def test_queue_plan_follows_the_addresses(built):
   # which earlier matmul each one of a queue waits for: worked out on the host from the buffers, no device needed
   from baretile_b200 import _lib
-  def op(x, out, m=8, k=512, n=1024, add=0, fmt=8, epilogue=0):
-    return _lib.GemvOp(fmt=fmt, epilogue=epilogue, M=m, K=k, N=n, out_dtype=0, alpha=1.0, x=x, w=0x100000, w2=0x200000 if epilogue == 3 else 0, add=add, out=out)
+  def op(x, out, m=8, k=512, n=1024, add=0, fmt=8, epilogue=0, w=0x100000, w2=0x200000):
+    return _lib.GemvOp(fmt=fmt, epilogue=epilogue, M=m, K=k, N=n, out_dtype=0, alpha=1.0, x=x, w=w, w2=w2 if epilogue == 3 else 0, add=add, out=out)
   def plan(ops):
     arr, waits = (_lib.GemvOp * len(ops))(*ops), (ctypes.c_int * len(ops))()
     _lib.call("bt_gemv_queue_plan", len(ops), arr, waits)
@@ -110,6 +110,11 @@ def test_queue_plan_follows_the_addresses(built):
   assert plan([op(A, B), op(A + 512 * 64, C, k=32)]) == [-1, -1]      # reads A's tiles past the first one's 16: no overlap with B
   assert plan([op(A, B), op(B + 2048 * 31, C, k=32)]) == [-1, 0]      # the last tile of B
   assert plan([op(A, B), op(B + 2048 * 32, C, k=32)]) == [-1, -1]     # just past B
+  # a result in memory that held an earlier matmul's weights, whose last byte still counts, and just past them
+  for fmt, size in ((8, 16 * 32 * 1088), (4, 16 * 32 * 576)):
+    assert plan([op(A, B, fmt=fmt, w=D), op(C, D + size - 256)]) == [-1, 0]
+    assert plan([op(A, B, fmt=fmt, w=D), op(C, D + size)]) == [-1, -1]
+    assert plan([op(A, B, fmt=fmt, epilogue=3, w2=D), op(C, D + size - 256)]) == [-1, 0]
   # a list longer than one launch: the 33rd matmul starts a new launch and waits for all of the first
   many = [op(A, B + 0x10000 * i) for i in range(34)]
   waits = plan(many)

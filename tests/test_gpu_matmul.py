@@ -249,19 +249,21 @@ def test_queue_random_programs(rt):
     for i, (got, want) in enumerate(zip(queued, separate)): assert np.array_equal(got.numpy(), want, equal_nan=True), (program, i, m, steps[i][0], steps[i][1][2])
 
 
-@pytest.mark.parametrize("case", ["read three places back", "two dependences", "picks share scratch", "sums share scratch", "memory used again"])
+@pytest.mark.parametrize("case", ["read three places back", "two dependences", "picks share scratch", "sums share scratch", "memory used again", "weights' memory used again"])
 def test_queue_that_is_neither_a_chain_nor_independent(rt, case):
   # one matmul takes long in a single CTA (256 tile rows of one tile), the others are done at once in CTAs that have no part in
   # it; what must wait for the long one does, and the bits are those of one launch per matmul
   rng = np.random.default_rng(23)
   def w(k, n, fmt="bfp8"): return upload(rt, weights(rng, k, n, stress=False) * 8).cast(fmt).columns()
   xl, xs, wl, w1, w2, w3 = acts(rng, 1, 8192), upload(rt, acts(rng, 1, 32)), w(8192, 32), w(32, 32), w(32, 32), w(32, 32)
-  wide, deep, w8 = w(32, 8192), w(4096, 4096), w(32, 4096)
+  wide, exact, deep, w8 = w(32, 8192), w(32, 4352), w(4096, 4096), w(32, 4096)       # a result of 4352 columns takes what wl takes
+  long = weights(rng, 8192, 32)
   x8, h8 = upload(rt, acts(rng, 8, 32)), upload(rt, acts(rng, 8, 4096))
   def pick(x, w, to):   # the entry point itself, since topk lays its answer out in a launch of its own
     rt.launch("bt_gemv_bfp", (8, 4, 1, w.rows, w.cols, x.addr, w.addr, 0, 0, 1.0, 0, 0, to, to + 256, 0, rt.work, rt.work_bytes))
   def run(queued):
     x, picks = upload(rt, xl), upload(rt, np.zeros((1, 32), np.float32), "fp32")
+    own = upload(rt, long).cast("bfp8").columns()
     with rt.queue() if queued else contextlib.nullcontext():
       if case == "sums share scratch":
         a, b = (h8 @ deep).realize(), (x8 @ w8).realize()
@@ -270,6 +272,11 @@ def test_queue_that_is_neither_a_chain_nor_independent(rt, case):
         pick(x, wl, picks.addr)
         outs = [(xs @ w1).realize(), picks]
         pick(outs[0], w2, picks.addr + 512)
+      elif case == "weights' memory used again":
+        at, a = own.addr, (x @ own).realize()
+        del own
+        outs = [a, (xs @ exact).realize()]
+        assert outs[1].addr == at
       else:
         a, b, at = (x @ wl).realize(), (xs @ w1).realize(), x.addr
         if case == "two dependences": outs = [a, b, ((b @ w2) + a).realize()]
