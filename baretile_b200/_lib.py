@@ -35,6 +35,7 @@ SIGNATURES = {
   "bt_stream_sync": [i32, u64, i32],
   "bt_stream_query": [i32, u64, ctypes.POINTER(i32)],
   "bt_h2d": [i32, u64, vp, size_t, u64],
+  "bt_upload": [i32, u64, vp, size_t, u64],
   "bt_d2h": [i32, vp, u64, size_t, u64],
   "bt_d2d": [i32, u64, u64, size_t, u64],
   "bt_memset": [i32, u64, i32, size_t, u64],

@@ -45,7 +45,7 @@ struct PackedEntry {
 const PackedEntry kPacked[] = {
     BT_PACKED(bt_gemv_bfp), BT_PACKED(bt_gemm_tiles), BT_PACKED(bt_gemm_bfp), BT_PACKED(bt_tilize), BT_PACKED(bt_untilize), BT_PACKED(bt_round_bf16),
     BT_PACKED(bt_pack_bfp), BT_PACKED(bt_unpack_bfp), BT_PACKED(bt_put), BT_PACKED(bt_relayout), BT_PACKED(bt_d2d), BT_PACKED(bt_memset),
-    BT_PACKED(bt_h2d), BT_PACKED(bt_d2h), BT_PACKED(bt_stage_upload), BT_PACKED(bt_stage_download), BT_PACKED(bt_stream_sync), BT_PACKED(bt_graph_launch),
+    BT_PACKED(bt_h2d), BT_PACKED(bt_upload), BT_PACKED(bt_d2h), BT_PACKED(bt_stage_upload), BT_PACKED(bt_stage_download), BT_PACKED(bt_stream_sync), BT_PACKED(bt_graph_launch),
 };
 #undef BT_PACKED
 }  // namespace
@@ -172,6 +172,25 @@ int bt_stream_sync(int device, uint64_t stream, int timeout_ms) {
 int bt_h2d(int device, uint64_t dst, const void *src, size_t bytes, uint64_t stream) {
   if (int s = use_device(device)) return s;
   BT_CUDA(cudaMemcpyAsync(as_ptr<void>(dst), src, bytes, cudaMemcpyHostToDevice, as_stream(stream)));
+  return BT_OK;
+}
+
+// From pageable memory a queued copy has staged its bytes by the time it returns; from page-locked (or managed, or device)
+// memory it is still to read them. Asking which it is takes a fraction of a microsecond, a synchronisation several, and as
+// long as everything queued before it.
+int bt_upload(int device, uint64_t dst, const void *src, size_t bytes, uint64_t stream) {
+  BT_REQUIRE(dst && src && bytes, "bt_upload: null address, or no bytes");
+  if (int s = use_device(device)) return s;
+  auto pageable = [](const char *p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+  };
+  const char *first = static_cast<const char *>(src);
+  const bool staged = pageable(first) && pageable(first + bytes - 1);
+  BT_CUDA(cudaMemcpyAsync(as_ptr<void>(dst), src, bytes, cudaMemcpyHostToDevice, as_stream(stream)));
+  if (!staged) BT_CUDA(cudaStreamSynchronize(as_stream(stream)));
   return BT_OK;
 }
 

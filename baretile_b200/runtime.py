@@ -493,7 +493,7 @@ class Runtime:
     try:
       self.flush()
       if src.len >= LARGE: _lib.call("bt_stage_upload", self._staging(), addr, src.buf, src.len, self.stream)
-      elif src.len: _lib.call("bt_h2d", self.device, addr, src.buf, src.len, self.stream)   # from pageable memory: returns when it has been read
+      elif src.len: _lib.call("bt_upload", self.device, addr, src.buf, src.len, self.stream)
     finally: src.release()
 
   def download(self, addr, n):

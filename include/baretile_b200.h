@@ -61,6 +61,9 @@ int bt_stream_destroy(int device, uint64_t stream);
 int bt_stream_sync(int device, uint64_t stream, int timeout_ms); /* Runtime.wait(timeout) (runtime.py:858-880) */
 int bt_stream_query(int device, uint64_t stream, int *done);     /* Runtime.finished (runtime.py:837) */
 int bt_h2d(int device, uint64_t dst, const void *src, size_t bytes, uint64_t stream); /* Chip.write / upload_kernel */
+/* bt_h2d that returns when src has been read, whatever memory it lies in: bt_h2d has staged the bytes by then where src is
+ * pageable, but from page-locked memory it still has them to read. Not for recording. */
+int bt_upload(int device, uint64_t dst, const void *src, size_t bytes, uint64_t stream);
 int bt_d2h(int device, void *dst, uint64_t src, size_t bytes, uint64_t stream);       /* Chip.read / readback_kernel */
 int bt_d2d(int device, uint64_t dst, uint64_t src, size_t bytes, uint64_t stream);    /* copy_kernel (kernels.py:1051) */
 int bt_memset(int device, uint64_t dst, int value, size_t bytes, uint64_t stream);    /* zeros_kernel (kernels.py:1439) */

@@ -256,6 +256,22 @@ def test_beside_blocks_fork_from_the_stream_and_join_it_again(monkeypatch):
     with pytest.raises(RuntimeError, match="inside a beside block"): rt.join()
 
 
+@pytest.mark.parametrize("size", [1, 4096, (256 << 10) - 1, 256 << 10])
+def test_upload_returns_when_its_source_has_been_read(monkeypatch, size):
+  # a copy that is only queued may still have page-locked memory to read: uploads go through the two entry points that
+  # return when they have read it, whatever memory it is
+  from baretile_b200 import _lib, runtime
+  calls = []
+  monkeypatch.setattr(_lib, "call", lambda name, *args: calls.append((name, args)))
+  rt = runtime.Runtime.__new__(runtime.Runtime)
+  rt.active, rt.device, rt.stream, rt.pending, rt.recording, rt.stage = False, 0, 7, None, None, 99
+  rt.check = lambda: None
+  for data in (bytes(size), bytearray(size), memoryview(bytearray(size + 1))[1:], (ctypes.c_char * size)()):
+    rt.upload(4096, data)
+    name, args = calls.pop()
+    assert (name, args[0], args[1], args[3:]) == (("bt_upload", 0, 4096, (size, 7)) if size < 256 << 10 else ("bt_stage_upload", 99, 4096, (size, 7))) and not calls
+
+
 def test_newer_entry_points_refuse_bad_arguments_before_any_device_work(built):
   """Argument checks come first in every entry point: they raise ValueError on a box without a GPU too."""
   import ctypes
@@ -271,6 +287,7 @@ def test_newer_entry_points_refuse_bad_arguments_before_any_device_work(built):
   # the streaming layout: one launch takes up to 65535 runs of 4 tile columns; and an event to wait for must exist
   with pytest.raises(ValueError, match="tile columns in one launch"): _lib.call("bt_relayout", 0, 8, 1, 1, 4 * 65535 + 1, 256, 512, 0)
   with pytest.raises(ValueError, match="null event"): _lib.call("bt_stream_wait_event", 0, 0, 0)
+  with pytest.raises(ValueError, match="no bytes"): _lib.call("bt_upload", 0, 256, 256, 0, 0)
   # many small matrices: a table is needed
   with pytest.raises(ValueError, match="no matrices"): _lib.call("bt_tilize_many", 0, 2, 0, None, None, None, None, 0)
   with pytest.raises(ValueError, match="itemsize"): _lib.call("bt_untilize_many", 0, 3, 1, None, None, None, None, 0)

@@ -258,6 +258,24 @@ def test_copies_beside_a_recorded_step(rt):
     for addr in stage_in + stage_out: rt.dram_free(addr)
 
 
+@pytest.mark.parametrize("size", [1, 4096, (256 << 10) - 1, 256 << 10, 3 << 20])
+@pytest.mark.parametrize("at", [0, 1])
+def test_upload_has_read_page_locked_memory_when_it_returns(rt, size, at):
+  # behind work that takes far longer than the call: what the caller writes into its buffer afterwards is not seen
+  rng = np.random.default_rng(size + at)
+  buf, junk, addr = rt.host_alloc(size + at), rt.dram_alloc(2 << 30), rt.dram_alloc(size)
+  host = np.frombuffer(buf, np.uint8)[at:]
+  want = rng.integers(1, 256, size, dtype=np.uint8)
+  try:
+    host[:] = want
+    for _ in range(4): rt.launch("bt_memset", (junk, 0, 2 << 30), name="zeros")
+    rt.upload(addr, host)
+    host[:] = 0
+    assert rt.download(addr, size) == want.tobytes()
+  finally:
+    for a in (junk, addr): rt.dram_free(a)
+
+
 @pytest.mark.parametrize("size", [1, 255, (256 << 10) - 1, 256 << 10, (1 << 20) + 1, (2 << 20) + 7, 16 << 20, (37 << 20) - 3])
 def test_host_copies_of_every_size(rt, size):
   # below and above where copies go through the staging buffers, one thread's chunk and more, a ragged last chunk; any
