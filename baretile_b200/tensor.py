@@ -393,9 +393,13 @@ def _launch_matmul(rt, e, epilogue, out, rows, arg=(0, 0), arg_base=0):
     if rows > 32: raise ValueError("the fused pick takes up to 32 rows")
   out_dtype = FMT_CODE[out.dtype] if out is not None else 0
   if rows > 32:
-    # many rows: the tensor-core kernel, which lays x out by rows in scratch lent to it, and adds up parts of K there
+    # many rows: the tensor-core kernel, which lays x out by rows in scratch lent to it, and adds up parts of K there. It
+    # needs the rows only: on a nearly full device it does without the parts
     size = 2 * rows * K + 256 + min(PARTS, 16 * 4 * out.tiles * 1024 * (2 if w2 else 1))
-    scratch = rt.dram_alloc(size)
+    try: scratch = rt.dram_alloc(size)
+    except MemoryError:
+      size = -(-2 * rows * K // 256) * 256
+      scratch = rt.dram_alloc(size)
     try:
       rt.launch("bt_gemm_tiles", (fmt, code, rows, K, w.cols, x.addr, w.addr, w2.addr if w2 else 0, add.addr if add else 0,
                                   add.rows if add else 0, alpha, out.addr, out_dtype, scratch, size, rt.work), name=f"prefill {w.dtype} {epilogue}")

@@ -82,6 +82,46 @@ print("all raised")
   assert run.returncode == 0 and run.stdout.strip() == "all raised", run.stdout + run.stderr
 
 
+class TightRuntime:
+  """A runtime without a device that hands out addresses while there is room, and notes what is launched."""
+  active, work, work_bytes, room = True, 1 << 40, 1 << 30, 1 << 62
+  def __init__(self): self.used, self.launched, self.asked = {}, [], []
+  def check(self):
+    if not self.active: raise RuntimeError("runtime is closed or was replaced by an overlapping runtime")
+  def dram_alloc(self, size):
+    self.asked.append(size)
+    if sum(self.used.values()) + size > self.room: raise MemoryError(f"no {size} bytes free in DRAM")
+    addr = 1 << 20 | len(self.asked) << 32
+    self.used[addr] = size
+    return addr
+  def dram_free(self, addr): del self.used[addr]
+  def launch(self, kernel, args=(), units=None, name=""): self.launched.append((kernel, args))
+
+
+def _many_rows(rt):
+  from baretile_b200.tensor import Tensor
+  x, w = Tensor(rt, 77, 2048), Tensor(rt, 2048, 544, dtype="bfp8")
+  w.runs = (5, 64, 0)
+  return x, w
+
+
+def test_many_rows_run_without_room_for_parts_of_k():
+  # scratch for x by rows is all that a matmul of many rows needs: with no room for parts of K beside it, it does without
+  rt = TightRuntime()
+  x, w = _many_rows(rt)
+  y = (x @ w).realize()
+  kernel, args = rt.launched.pop()
+  assert kernel == "bt_gemm_tiles" and args[-2] > 2 * 77 * 2048 + 77 * 544 * 4 and len(rt.used) == 3
+  rt.room = sum(rt.used.values()) + 3 * 17 * 2048 + 2 * 77 * 2048
+  z = (x @ w).realize()
+  kernel, args = rt.launched.pop()
+  assert kernel == "bt_gemm_tiles" and args[-2] == 2 * 77 * 2048 and len(rt.used) == 4
+  del z
+  rt.room -= 1
+  with pytest.raises(MemoryError, match="bytes free"): (x @ w).realize()
+  assert not rt.launched
+
+
 def test_hole_allocator_merges():
   from baretile_b200.runtime import _merge_holes
   holes = [(512, 256), (0, 256), (256, 256), (2048, 64)]

@@ -113,6 +113,31 @@ def test_shapes_that_are_not_whole_blocks(rt, fmt, k, n):
   check_matmul(got, x, None, ref, 1e-2)
 
 
+@pytest.mark.parametrize("epilogue", ["none", "glu"])
+def test_without_room_for_parts_of_k(rt, monkeypatch, epilogue):
+  # a device with room for x by rows but not for the parts: the matmul runs all the same, and one that has no room for x by
+  # rows either says so
+  rng = np.random.default_rng(5)
+  m, k, n = 77, 2048, 544
+  x, w, w2 = acts(rng, m, k), weights(rng, k, n), weights(rng, k, n)
+  tx, tw, tw2 = upload(rt, x), upload(rt, w).cast("bfp8").columns(), upload(rt, w2).cast("bfp8").columns()
+  asked, alloc = [], rt.dram_alloc
+  def tight(size, limit=2 * m * k):
+    asked.append(size)
+    if size > limit: raise MemoryError(f"no {size} bytes free in DRAM")
+    return alloc(size)
+  def expression(): return (tx @ tw) if epilogue == "none" else (tx @ tw).silu() * (tx @ tw2)
+  monkeypatch.setattr(rt, "dram_alloc", tight)
+  y = expression().realize()
+  assert asked[-2] > asked[-1] == 2 * m * k
+  monkeypatch.setattr(rt, "dram_alloc", lambda size: tight(size, 2 * m * k - 1))
+  with pytest.raises(MemoryError, match="bytes free"): expression().realize()
+  monkeypatch.undo()
+  ref = x @ o.dequant(w, "bfp8")
+  if epilogue == "glu": ref = o.silu(ref) * (x @ o.dequant(w2, "bfp8"))
+  check_matmul(y.numpy(), x, o.dequant(w, "bfp8") if epilogue == "none" else None, ref, 1e-2)
+
+
 def test_results_stay_inside_their_tiles(rt):
   # the tensors either side of a result in device memory keep their bytes (ragged rows and columns included)
   from baretile_b200.tensor import Tensor
