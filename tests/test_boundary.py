@@ -122,6 +122,20 @@ def test_many_rows_run_without_room_for_parts_of_k():
   assert not rt.launched
 
 
+def test_expressions_on_a_closed_runtime_raise():
+  # at once, as anything else on it does, not first when a result is asked for
+  from baretile_b200.tensor import Tensor
+  rt = TightRuntime()
+  x, w = Tensor(rt, 4, 64), Tensor(rt, 64, 64, dtype="bfp8")
+  y = x @ w
+  rt.active = False
+  for late in (lambda: x @ w, lambda: x.matmul(w, dtype="fp32"), lambda: y.relu(), lambda: y.silu(), lambda: y * 2, lambda: 0.5 * y, lambda: y * y,
+               lambda: y + y, lambda: y.realize(), lambda: Tensor(rt, 1, 1)):
+    with pytest.raises(RuntimeError, match="closed"): late()
+  rt.active = True
+  (x @ w).relu()
+
+
 def test_hole_allocator_merges():
   from baretile_b200.runtime import _merge_holes
   holes = [(512, 256), (0, 256), (256, 256), (2048, 64)]
