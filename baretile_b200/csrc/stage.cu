@@ -12,6 +12,8 @@
 #include "common.cuh"
 #include <condition_variable>
 #include <cstring>
+#include <exception>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -121,23 +123,26 @@ int bt_stage_create(int device, uint64_t *stage) {
   BT_REQUIRE(stage, "bt_stage_create: null result");
   if (int s = use_device(device)) return s;
   const unsigned cores = std::thread::hardware_concurrency();
-  Stage *st = new Stage;
-  st->device = device;
-  st->lanes.resize(cores < 2 ? 1 : cores < kMostThreads ? cores : kMostThreads);
-  cudaError_t e = cudaSuccess;
-  for (auto &l : st->lanes)
-    for (int b = 0; b < 2 && e == cudaSuccess; b++) {
-      e = cudaMallocHost(&l.buf[b], kBuffer);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.free[b], cudaEventDisableTiming);
-    }
-  if (e != cudaSuccess) {
-    delete st;
-    cudaGetLastError();
-    return fail(BT_NO_MEMORY, "no page-locked memory for a staging object: %s", cudaGetErrorString(e));
+  try {                                // memory, and threads where a process may have only so many
+    auto st = std::make_unique<Stage>();
+    st->device = device;
+    st->lanes.resize(cores < 2 ? 1 : cores < kMostThreads ? cores : kMostThreads);
+    for (auto &l : st->lanes)
+      for (int b = 0; b < 2; b++) {
+        cudaError_t e = cudaMallocHost(&l.buf[b], kBuffer);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.free[b], cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+          cudaGetLastError();
+          return fail(BT_NO_MEMORY, "no page-locked memory for a staging object: %s", cudaGetErrorString(e));
+        }
+      }
+    st->threads.reserve(st->lanes.size());
+    for (size_t i = 1; i < st->lanes.size(); i++) st->threads.emplace_back(&Stage::run, st.get(), i);
+    *stage = reinterpret_cast<uint64_t>(st.release());
+    return BT_OK;
+  } catch (const std::exception &e) {
+    return fail(BT_NO_MEMORY, "no memory or threads for a staging object: %s", e.what());
   }
-  for (size_t i = 1; i < st->lanes.size(); i++) st->threads.emplace_back([st, i] { st->run(i); });
-  *stage = reinterpret_cast<uint64_t>(st);
-  return BT_OK;
 }
 
 int bt_stage_destroy(uint64_t stage) {

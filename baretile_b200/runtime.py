@@ -492,7 +492,8 @@ class Runtime:
     except (TypeError, ValueError, BufferError): src = _Buffer(bytes(data))
     try:
       self.flush()
-      if src.len >= LARGE: _lib.call("bt_stage_upload", self._staging(), addr, src.buf, src.len, self.stream)
+      stage = self._staging() if src.len >= LARGE else 0
+      if stage: _lib.call("bt_stage_upload", stage, addr, src.buf, src.len, self.stream)
       elif src.len: _lib.call("bt_upload", self.device, addr, src.buf, src.len, self.stream)
     finally: src.release()
 
@@ -502,16 +503,19 @@ class Runtime:
     if self.recording is not None: raise RuntimeError("a read-back cannot be recorded: use download_async into page-locked memory")
     out = _new_bytes(None, n)
     self.flush()
-    if n >= LARGE: _lib.call("bt_stage_download", self._staging(), _bytes_at(out), addr, n, self.stream)
+    stage = self._staging() if n >= LARGE else 0
+    if stage: _lib.call("bt_stage_download", stage, _bytes_at(out), addr, n, self.stream)
     else:
       _lib.call("bt_d2h", self.device, _bytes_at(out), addr, n, self.stream)
       _lib.call("bt_stream_sync", self.device, self.stream, -1)
     return out
 
   def _staging(self):
-    """The runtime's page-locked staging buffers, made at the first large copy and kept until close()."""
+    """The runtime's page-locked staging buffers, made at the first large copy and kept until close(). 0 where the host has
+    no memory or threads for them: the copy then goes as a small one does."""
     if not self.stage:
       stage = ctypes.c_uint64()
-      _lib.call("bt_stage_create", self.device, ctypes.byref(stage))
+      try: _lib.call("bt_stage_create", self.device, ctypes.byref(stage))
+      except MemoryError: return 0
       self.stage = stage.value
     return self.stage

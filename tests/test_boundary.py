@@ -326,6 +326,22 @@ def test_upload_returns_when_its_source_has_been_read(monkeypatch, size):
     assert (name, args[0], args[1], args[3:]) == (("bt_upload", 0, 4096, (size, 7)) if size < 256 << 10 else ("bt_stage_upload", 99, 4096, (size, 7))) and not calls
 
 
+def test_large_copies_without_staging_buffers(monkeypatch):
+  # a host with no page-locked memory or threads to spare still copies, as it does what is small
+  from baretile_b200 import _lib, runtime
+  calls = []
+  def fake_call(name, *args):
+    calls.append(name)
+    if name == "bt_stage_create": raise MemoryError("no memory or threads for a staging object")
+  monkeypatch.setattr(_lib, "call", fake_call)
+  rt = runtime.Runtime.__new__(runtime.Runtime)
+  rt.active, rt.device, rt.stream, rt.pending, rt.recording, rt.stage = False, 0, 7, None, None, 0
+  rt.check = lambda: None
+  rt.upload(4096, bytes(1 << 20))
+  assert len(rt.download(4096, 1 << 20)) == 1 << 20
+  assert calls == ["bt_stage_create", "bt_upload", "bt_stage_create", "bt_d2h", "bt_stream_sync"]
+
+
 def test_newer_entry_points_refuse_bad_arguments_before_any_device_work(built):
   """Argument checks come first in every entry point: they raise ValueError on a box without a GPU too."""
   import ctypes
