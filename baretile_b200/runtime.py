@@ -3,8 +3,9 @@
 The reference's Runtime owns a rectangle of workers, a command ring in host memory, a DRAM hole allocator with
 deferred frees, and per-launch timing records. Here one CUDA stream plays the ring (launches run in order,
 asynchronously; `wait` blocks), device memory comes from arenas carved by the same first-fit hole allocator
-(64-byte granularity there, 256 here), and timing records are CUDA events. Frees need no deferral: every access
-to device memory is queued on the runtime's stream, so memory released now is reused only by work queued later.
+(64-byte granularity there, 256 here), and timing records are CUDA events. Frees need no deferral while every access
+to device memory is queued on the runtime's own stream, since memory released now is reused only by work queued later.
+Behind a beside block, whose stream the own one does not wait for, what is released meanwhile is kept until they join.
 """
 import bisect, collections, ctypes, time
 from baretile_b200 import _lib
@@ -237,6 +238,7 @@ class Runtime:
   """Run kernels on one CUDA device, in order. A new Runtime on a chip closes the chip's older runtime, as an
   overlapping rectangle does in the reference (baretile/runtime.py:593-598). Close a runtime to release its
   memory; a closed runtime cannot be reused."""
+  late = ()                # (address, size) of memory freed while beside blocks were open or not yet joined
   def __init__(self, chip, start=None, end=None, ring=1 << 20, timing=False):
     if ring < 64 or ring & (ring - 1): raise ValueError("ring size must be a power of two, at least 64 bytes")
     self.chip, self.device, self.launches = chip, chip.device, 0
@@ -297,7 +299,7 @@ class Runtime:
     for ptr in getattr(self, "pinned", []): _lib.lib().bt_host_free(ptr)
     self.pinned = []
     for addr, _ in self.arenas: _lib.lib().bt_free(self.device, addr)
-    self.arenas, self.holes, self.kept, self.kept_count = [], [], {}, 0
+    self.arenas, self.holes, self.kept, self.kept_count, self.late = [], [], {}, 0, ()
     self.used.clear()
     _lib.lib().bt_stream_destroy(self.device, self.stream)
     self.chip.taken.pop(id(self), None)
@@ -362,6 +364,7 @@ class Runtime:
     if self.side is not None: raise RuntimeError("join inside a beside block")
     done, self.unjoined = self.unjoined, []
     for e in done: _lib.call("bt_stream_wait_event", self.device, self.stream, e)
+    if self.late: self._free_late()
 
   def flush(self):
     """Send the matmuls collected so far as one queue launch."""
@@ -427,23 +430,39 @@ class Runtime:
       if attempt: break
       arena, addr = max(size, ARENA), ctypes.c_uint64()
       try: _lib.call("bt_malloc", self.device, arena, ctypes.byref(addr))
-      except MemoryError: raise MemoryError(f"no {size} bytes free in DRAM") from None
+      except MemoryError:
+        if not self.late: raise MemoryError(f"no {size} bytes free in DRAM") from None
+        for stream, _, _ in self.sides: _lib.call("bt_stream_sync", self.device, stream, -1)     # then nothing beside uses it any more
+        self._free_late()
+        return self.dram_alloc(size)
       self.arenas.append((addr.value, arena))
       _add_hole(self.holes, addr.value, arena, self.arenas)
     raise MemoryError(f"no {size} bytes free in DRAM")
 
   def dram_free(self, addr):
     """Release an allocation (baretile/runtime.py:814-820). Work already queued may still use it; work queued
-    later may reuse it, which the stream's ordering makes safe."""
+    later may reuse it, which the stream's ordering makes safe. Beside blocks have other streams: what is freed in one, or
+    before one is joined, is reused only behind the join."""
     if not self.active: return
     size = self.used.pop(addr, None)
     if size is None: return
     if self.recording is not None:   # a replay will use this memory again
       self.recording.held.append((addr, size))
       return
+    if self.unjoined or self.side is not None:
+      if not self.late: self.late = []
+      self.late.append((addr, size))
+      return
+    self._keep(addr, size)
+
+  def _keep(self, addr, size):
     self.kept.setdefault(size, []).append(addr)
     self.kept_count += 1
     if self.kept_count > KEPT: self._join_kept()
+
+  def _free_late(self):
+    late, self.late = self.late, ()
+    for addr, size in late: self._keep(addr, size)
 
   def _join_kept(self):
     for size, addrs in self.kept.items():

@@ -310,6 +310,48 @@ def test_beside_blocks_fork_from_the_stream_and_join_it_again(monkeypatch):
     with pytest.raises(RuntimeError, match="inside a beside block"): rt.join()
 
 
+def test_memory_freed_behind_a_beside_block_is_not_reused_before_the_join(monkeypatch):
+  # the block's stream may still read it, and the runtime's own stream, or another block's, does not wait for that
+  from baretile_b200 import _lib, runtime
+  calls, room, next_arena = [], [1], 1 << 32
+  made = iter(range(100, 200))
+  def fake_call(name, *args):
+    nonlocal next_arena
+    calls.append((name, args))
+    if name in ("bt_stream_create", "bt_event_create"): args[-1]._obj.value = next(made)
+    if name == "bt_malloc":
+      if not room: raise MemoryError("no bytes free")
+      room.pop()
+      args[-1]._obj.value, next_arena = next_arena, next_arena + (1 << 40)
+  monkeypatch.setattr(_lib, "call", fake_call)
+  rt = runtime.Runtime.__new__(runtime.Runtime)
+  rt.active, rt.device, rt.stream, rt.recording, rt.pending, rt.log, rt.sent, rt.launches, rt.timing = True, 0, 7, None, None, None, {}, 0, False
+  rt.sides, rt.unjoined, rt.side, rt.holes, rt.used, rt.arenas, rt.kept, rt.kept_count = [], [], None, [], {}, [], {}, 0
+  a = rt.dram_alloc(4096)
+  rt.dram_free(a)
+  assert rt.dram_alloc(4096) == a                                     # nothing beside: reused at once
+  with rt.beside():
+    rt.dram_free(a)                                                   # what the block has queued may still use it
+    b = rt.dram_alloc(4096)
+    assert b != a
+  rt.dram_free(b)
+  c = rt.dram_alloc(4096)
+  assert c not in (a, b)
+  with rt.beside(): assert rt.dram_alloc(4096) not in (a, b, c)
+  rt.join()
+  assert {rt.dram_alloc(4096), rt.dram_alloc(4096)} == {a, b}
+  # with no other memory left the host waits for the blocks' streams instead of giving up
+  with rt.beside(): pass
+  rest = rt.dram_alloc(rt.holes[0][1])
+  rt.dram_free(c)
+  calls.clear()
+  assert rt.dram_alloc(4096) == c and [n for n, _ in calls] == ["bt_malloc", "bt_stream_sync", "bt_stream_sync"]
+  assert {args[1] for n, args in calls if n == "bt_stream_sync"} == {s for s, _, _ in rt.sides}
+  with pytest.raises(MemoryError, match="no 8192 bytes free"): rt.dram_alloc(8192)
+  rt.dram_free(rest)
+  rt.active = False
+
+
 @pytest.mark.parametrize("size", [1, 4096, (256 << 10) - 1, 256 << 10])
 def test_upload_returns_when_its_source_has_been_read(monkeypatch, size):
   # a copy that is only queued may still have page-locked memory to read: uploads go through the two entry points that
