@@ -133,6 +133,7 @@ class Recording:
     if self.graph is None: raise RuntimeError("nothing was recorded")
     if self.rt.recording is not None: raise RuntimeError("cannot replay while recording on the same runtime")
     if not binding:
+      self.rt.flush()
       _lib.call("bt_graph_launch", self.rt.device, self.graph, self.rt.stream)
       self.rt.launches += self.count
       return

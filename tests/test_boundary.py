@@ -310,6 +310,22 @@ def test_beside_blocks_fork_from_the_stream_and_join_it_again(monkeypatch):
     with pytest.raises(RuntimeError, match="inside a beside block"): rt.join()
 
 
+def test_replay_runs_behind_the_matmuls_collected_before_it(monkeypatch):
+  from baretile_b200 import _lib, runtime
+  calls = []
+  monkeypatch.setattr(_lib, "call", lambda name, *args: calls.append(name))
+  rt = runtime.Runtime.__new__(runtime.Runtime)
+  rt.active, rt.device, rt.stream, rt.launches, rt.sent, rt.log, rt.pending, rt.timing, rt.work, rt.work_bytes = True, 0, 7, 0, {}, None, None, False, 4096, 1 << 20
+  rt.sides, rt.unjoined, rt.side, rt.recording = [], [], None, None
+  step = runtime.Recording(rt)
+  step.graph, step.count = 5, 3
+  with rt.queue():
+    rt.launch("bt_gemv_bfp", (8, 0, 4, 512, 1024, 0x10, 0x1000, 0, 0, 1.0, 0x20, 0, 0, 0, 0, rt.work, rt.work_bytes))
+    step.replay()
+  assert calls == ["bt_gemv_queue", "bt_graph_launch"]
+  rt.active = False
+
+
 def test_memory_freed_behind_a_beside_block_is_not_reused_before_the_join(monkeypatch):
   # the block's stream may still read it, and the runtime's own stream, or another block's, does not wait for that
   from baretile_b200 import _lib, runtime
