@@ -132,6 +132,7 @@ class Recording:
     self.rt.check()
     if self.graph is None: raise RuntimeError("nothing was recorded")
     if self.rt.recording is not None: raise RuntimeError("cannot replay while recording on the same runtime")
+    if self.rt.side is not None and any(kernel in MATMULS for kernel, *_ in self.launches): raise RuntimeError(BESIDE)
     if not binding:
       self.rt.flush()
       _lib.call("bt_graph_launch", self.rt.device, self.graph, self.rt.stream)
@@ -199,6 +200,7 @@ class Queue:
       if self.outer is None: self.rt.pending = None
 
 
+MATMULS, BESIDE = ("bt_gemv_bfp", "bt_gemv_queue", "bt_gemm_bfp", "bt_gemm_tiles"), "a matmul uses the runtime's scratch and runs on its own stream, not in a beside block"
 SIDES = 4   # streams a runtime keeps for work that runs beside its own
 
 
@@ -320,8 +322,7 @@ class Runtime:
     is accepted for parity; the entry point sizes its own grid."""
     if not self.active: self.check()
     if units is not None and not 1 <= int(units) < 2**32: raise ValueError("launch units must be in [1, 2**32 - 1]")
-    if self.side is not None and kernel in ("bt_gemv_bfp", "bt_gemv_queue", "bt_gemm_bfp", "bt_gemm_tiles"):
-      raise RuntimeError("a matmul uses the runtime's scratch and runs on its own stream, not in a beside block")
+    if self.side is not None and kernel in MATMULS: raise RuntimeError(BESIDE)
     if self.log is not None: self.log.append((kernel, args, units, name))
     if self.pending is not None and kernel == "bt_gemv_bfp":
       self.pending.append(args)

@@ -318,11 +318,17 @@ def test_replay_runs_behind_the_matmuls_collected_before_it(monkeypatch):
   rt.active, rt.device, rt.stream, rt.launches, rt.sent, rt.log, rt.pending, rt.timing, rt.work, rt.work_bytes = True, 0, 7, 0, {}, None, None, False, 4096, 1 << 20
   rt.sides, rt.unjoined, rt.side, rt.recording = [], [], None, None
   step = runtime.Recording(rt)
-  step.graph, step.count = 5, 3
+  step.graph, step.count, step.launches = 5, 3, [("bt_untilize", (2, 0x30, 0x40, 1, 4, 1024), None, "readback")]
   with rt.queue():
     rt.launch("bt_gemv_bfp", (8, 0, 4, 512, 1024, 0x10, 0x1000, 0, 0, 1.0, 0x20, 0, 0, 0, 0, rt.work, rt.work_bytes))
     step.replay()
   assert calls == ["bt_gemv_queue", "bt_graph_launch"]
+  # and a recorded matmul stays out of beside blocks, as any other does
+  rt.side, rt.stream = 7, 9
+  step.replay()
+  step.launches.append(("bt_gemm_tiles", (), None, ""))
+  with pytest.raises(RuntimeError, match="own stream"): step.replay()
+  assert calls == ["bt_gemv_queue", "bt_graph_launch", "bt_graph_launch"]
   rt.active = False
 
 
