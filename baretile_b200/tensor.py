@@ -291,7 +291,11 @@ class Tensor:
       raise ValueError(f"this backend runs act(alpha * (x @ W) + addend) and (x @ Wg).silu() * (x @ Wu); got {_describe(self)}")
     epilogue, e = plan
     self.addr = self._alloc()
-    _launch_matmul(self.rt, e, epilogue, self, self.rows)
+    try: _launch_matmul(self.rt, e, epilogue, self, self.rows)
+    except BaseException:                 # still an expression: asked for again it allocates again
+      addr, self.addr = self.addr, None
+      self.rt.dram_free(addr)
+      raise
     self.op, self.srcs = None, ()
     return self
 

@@ -118,8 +118,12 @@ def test_many_rows_run_without_room_for_parts_of_k():
   assert kernel == "bt_gemm_tiles" and args[-2] == 2 * 77 * 2048 and len(rt.used) == 4
   del z
   rt.room -= 1
-  with pytest.raises(MemoryError, match="bytes free"): (x @ w).realize()
-  assert not rt.launched
+  z = x @ w
+  for _ in range(2):
+    with pytest.raises(MemoryError, match="bytes free"): z.realize()
+    assert not rt.launched and z.addr is None and len(rt.used) == 3     # an attempt that fails keeps nothing
+  rt.room += 1
+  assert z.realize().addr in rt.used
 
 
 def test_expressions_on_a_closed_runtime_raise():
