@@ -48,7 +48,7 @@ constexpr int kCW = 16;                     // consumer warps of the CTA; an SM 
 constexpr int kConsumers = kCW * 32;
 constexpr int kThreads = (kCW + 3) * 32;    // plus two producer warps and a messenger
 constexpr int kBars = 16;                   // stages in the ring at most: mbarriers that go round with the stages
-constexpr int kMaxCtas = 320;
+constexpr int kMaxCtas = 160;               // one CTA per SM; a B200 has 148
 constexpr int kMaxSubPanels = 16384;
 constexpr int kQueueMax = 32;               // matmuls per launch; longer lists take several launches
 constexpr uint32_t kSpinLimit = 1u << 14;   // attempts of up to 100 us each (mbarriers) or polls x 64 (counters)
@@ -133,8 +133,9 @@ struct alignas(64) GemvParams {
   int share, extra;           // range b then starts at b * share + min(b, extra), and the last one ends at units
 };
 
-// The kernel exists twice: for lists with a small matmul in them, and for lists without one, which is spared all that sub-panels
-// of other widths than four take (as one kernel it cost lists of large matmuls 2-3 %).
+// The kernel exists for lists with a small matmul in them and for lists without one, which is spared all that sub-panels
+// of other widths than four take (as one kernel it cost lists of large matmuls 2-3 %); each for short and for long lists (see
+// kQueueShort).
 template <bool SMALL> __device__ __forceinline__ int lw_of(const GemvParams &p) { return SMALL ? p.lw : 2; }
 
 // Where sub-panel `sp` lies: 1 << lw tile columns from `col` on, fewer at the end of a matrix, part of a run of `run_width`.
@@ -1104,12 +1105,12 @@ QueueHead workspace_scratch(uint64_t work) {
 // at reduced limits: up to 8 rows of x, up to kStaticSubPanels sub-panels of 4 tile columns.
 namespace {
 constexpr int kStaticSubPanels = 4096;                                  // N <= 4096 * 4 * 32 = 524288 columns
-constexpr size_t kStaticSlotFloats = 8 * 8 * 32;                        // 8 warps, 8 accumulators per lane
+constexpr size_t kStaticSlotFloats = 8 * 2 * 128;                       // 8 tokens x up to two matrices x 128 channels
 constexpr size_t kStKeys = 256;
 constexpr size_t kStCounters = 512;
 constexpr size_t kStControlBytes = kStCounters + 4 * (size_t)kStaticSubPanels;   // what must be zero when a call starts
 constexpr size_t kStPartials = kStControlBytes;
-constexpr size_t kStaticBytes = kStPartials + (size_t)kMaxCtas * kStaticSlotFloats * 4;   // about 2.6 MB
+constexpr size_t kStaticBytes = kStPartials + (size_t)kMaxCtas * kStaticSlotFloats * 4;   // about 1.3 MB
 }  // namespace
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticBytes];
 

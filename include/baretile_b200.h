@@ -68,7 +68,7 @@ int bt_d2h(int device, void *dst, uint64_t src, size_t bytes, uint64_t stream); 
 int bt_d2d(int device, uint64_t dst, uint64_t src, size_t bytes, uint64_t stream);    /* copy_kernel (kernels.py:1051) */
 int bt_memset(int device, uint64_t dst, int value, size_t bytes, uint64_t stream);    /* zeros_kernel (kernels.py:1439) */
 /* Large copies from and to pageable host memory: several threads copy through page-locked buffers while the bus moves
- * the others' (host DMA pages, runtime.py:548-600). A staging object holds up to 16 MB of page-locked memory and 7
+ * the others' (host DMA pages, runtime.py:548-600). A staging object holds up to 32 MB of page-locked memory and 7
  * threads until it is destroyed; calls on one object take turns. bt_stage_upload returns when src has been read (the
  * copy itself is queued on the stream like bt_h2d), bt_stage_download when dst is complete. Not for recording. */
 int bt_stage_create(int device, uint64_t *stage);
@@ -211,7 +211,7 @@ int bt_gemm_tiles(int device, int fmt, int epilogue, int M, int K, int N, uint64
  * Some embedders of this library run where cudaMalloc is off limits -- inside another framework's capture or
  * allocator-owned region, in a process whose memory budget was handed out in full at start-up, or in a plug-in
  * that is only ever given its input and output buffers. For them the scratch that bt_gemv_bfp takes from the
- * caller sits in a fixed array inside the library's device image (about 2.6 MB on every GPU that loads the
+ * caller sits in a fixed array inside the library's device image (about 1.3 MB on every GPU that loads the
  * library, held until the process exits). The call allocates and frees nothing, on the host side either.
  * Limits, rejected with BT_BAD_ARGUMENT: M <= 8 rows of x, N <= 524288 columns. Inputs and outputs are the
  * caller's, exactly as for bt_gemv_bfp. The first call on a device looks the array's address up (one runtime

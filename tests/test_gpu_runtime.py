@@ -119,8 +119,8 @@ def test_wait_times_out_and_the_runtime_stays_usable(rt):
 def test_bounded_wait_for_an_earlier_matmul_reports_instead_of_hanging(rt):
   # A wait inside the matmul kernel that cannot be met gives up after its limit and sets the error word, which
   # Runtime.wait turns into RuntimeError; the kernel ends normally and the runtime keeps working. The wait is made
-  # unmeetable on the host: a matmul of a queue takes its x only when every CTA has reported the matmul two places
-  # before it finished, and that count (one int per matmul of a launch, from byte 8 of the workspace: kWsOpsDone in
+  # unmeetable on the host: a matmul of a queue takes its x only when every sub-panel of the matmul two places
+  # before it is reported finished, and that count (one int per matmul of a launch, from byte 8 of the workspace: kWsOpsDone in
   # csrc/gemv.cu) starts far below zero for the first matmul, so the third one's x warp never sees it complete.
   from helpers import acts, upload, weights
   from oracle import bfp_oracle as o
