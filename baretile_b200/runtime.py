@@ -455,16 +455,13 @@ class Runtime:
       if not self.late: self.late = []
       self.late.append((addr, size))
       return
-    self._keep(addr, size)
-
-  def _keep(self, addr, size):
     self.kept.setdefault(size, []).append(addr)
     self.kept_count += 1
     if self.kept_count > KEPT: self._join_kept()
 
   def _free_late(self):
     late, self.late = self.late, ()
-    for addr, size in late: self._keep(addr, size)
+    for addr, size in late: _add_hole(self.holes, addr, size, self.arenas)
 
   def _join_kept(self):
     for size, addrs in self.kept.items():

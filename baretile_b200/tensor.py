@@ -225,7 +225,7 @@ class Tensor:
     # an expression's shape and operands are its sources', which were checked when they were made; most expressions are
     # only parts of others, so what storage they would take is worked out when it is asked for (__getattr__). A runtime can
     # have been closed since
-    self.rt.check()
+    if not self.rt.active: self.rt.check()
     t = Tensor.__new__(Tensor)
     t.__dict__ = {"rt": self.rt, "rows": rows or self.rows, "cols": cols or self.cols, "batch": self.batch, "op": op, "srcs": srcs, "dtype": dtype or self.dtype}
     return t
