@@ -4,6 +4,9 @@
 // The work is bound by HBM: every packed weight byte is read once, by a bulk (TMA) copy into a ring of
 // shared-memory stages, and dequantised in registers on its way into a bf16 MMA with fp32 accumulators.
 //
+// Lists of small matmuls for a few tokens, where the way from one result to the next is all that counts, have a kernel of
+// their own at the end of this file (chain_kernel). All others run in gemv_queue_kernel:
+//
 // A queue. In decode one matmul's result is the next one's x, so between two of them the GPU has nothing to read
 // unless the next weights are already on their way. The kernel therefore takes a list of matmuls (up to kQueueMax
 // per launch) and runs them in order with the same persistent CTAs. The weight warp of a CTA walks the whole list:
@@ -57,12 +60,15 @@ constexpr uint32_t kSpinLimit = 1u << 14;   // attempts of up to 100 us each (mb
 constexpr int kSmFull = 0, kSmEmpty = 128;  // mbarriers: a stage's weights and x have landed; it is free again
 constexpr int kSmHeld = 256;                // uint32[2][kBars]: ring bytes of each stage in the ring, as each producer warp noted them
 constexpr int kSmDead = 384;                // int: a wait on a stage gave up; nobody in this CTA waits for the ring any more
+constexpr int kSmEpoch = 388;               // chains: uint32, the launch's number
+constexpr int kSmReady = 392, kSmGo = 400, kSmDone = 416;   // chains: mbarriers: the launch's number is there; [2] a matmul may start; [2] its results are stored
 constexpr int kSmStages = 512;              // Stage[kBars]: what the weight warp tells the consumers about each stage
 constexpr int kSmSums = 1024;               // float[k groups x matrices, or tile rows x matrices][tokens][channels of a sub-panel + 4]
 // Floats from one token's channels to the next: 4 past the channels, so that the fragment stores meet no bank twice.
 __host__ __device__ constexpr int sum_stride(int lw) { return (32 << lw) + 4; }
 constexpr int sums_bytes(int tg) { return 4 * 8 * tg * sum_stride(2) * 4; }
 constexpr int kSmallSums = 84 * 1024;       // bytes at most that the sums of a small matmul's tile rows take of the ring
+__host__ __device__ constexpr int small_groups(int lw, bool pair) { return kCW >> lw >> (pair ? 1 : 0); }   // warps that share a column (of a matrix)
 constexpr int kSmemBytes = 227 * 1024;
 
 // Scratch layout (byte offsets into the caller's workspace). Two matmuls of a queue may be in flight at once, so
@@ -70,6 +76,7 @@ constexpr int kSmemBytes = 227 * 1024;
 constexpr size_t kWsError = 0;                                   // int: set to nonzero when a wait gave up
 constexpr size_t kWsOpsDone = 8;                                 // int[kQueueMax]: finished sub-panels of each matmul of the launch
 constexpr size_t kWsAllDone = 144;                               // int: and of all of them
+constexpr size_t kWsEpoch = 148;                                 // uint32: launches of chains that used this workspace so far, modulo kEpochs
 constexpr size_t kWsSets = 256;                                  // the sets start here
 constexpr size_t kSetPanelsDone = 0;                             // int: sub-panels finished (argmax epilogue)
 constexpr size_t kSetKeys = 256;                                 // u64[32]: per token the best (value, column) so far (argmax epilogue)
@@ -78,7 +85,11 @@ constexpr size_t kSetPartials = kSetCounters + 4 * kMaxSubPanels;
 constexpr size_t kSlotFloatsMax = 32 * 2 * 128;                  // 32 tokens x up to two matrices x 128 channels
 constexpr size_t kSetBytes = kSetPartials + (size_t)kMaxCtas * kSlotFloatsMax * 4;
 constexpr int kSets = 2;                                         // matmuls of a queue in flight at most
-constexpr size_t kWsBytes = kWsSets + kSets * kSetBytes;
+constexpr size_t kWsExchange = (kWsSets + kSets * kSetBytes + 255) / 256 * 256;   // kExchanges results on their way to the next matmul of a chain
+constexpr int kExchanges = 3, kChainRows = 8;                    // chains are for up to 8 tokens
+constexpr size_t kExchangeBytes = (size_t)kMaxCtas * kWC * 2 * kChainRows * 64;
+constexpr size_t kWsBytes = kWsExchange + kExchanges * kExchangeBytes;
+constexpr uint32_t kEpochs = 1u << 26;
 
 // The shape of a stage for one kind of matmul: format, one matrix or a gate/up pair, token groups of 8 rows, columns of a
 // sub-panel (1 << lw).
@@ -114,6 +125,7 @@ struct alignas(64) GemvParams {
   CUtensorMap xmap;           // x as (16-datum face rows of the staged tokens, faces, tile columns)
   CUtensorMap wmap[2];        // for sub-panels narrower than a run: the weights as (a tile's bytes, the four tiles of a run's tile row, tile rows)
   const uint8_t *w[2];
+  const uint16_t *x;          // chains read it themselves, where it does not come from an exchange
   const uint16_t *add;
   void *out;
   float *arg_val;
@@ -123,6 +135,11 @@ struct alignas(64) GemvParams {
   int fmt, pair, tg;
   int wait_for, wait_panels;  // the last matmul of the launch that must be complete before this one starts (-1: none), and its sub-panels
   int wait_also, also_panels; // the one before it, where its being complete does not follow (see Gate), and its sub-panels
+  int from;                   // chains: x is the result of the matmul before this one and comes from its exchange
+  int add_from;               // so does the addend
+  int to;                     // chains: the matmul after this one reads the exchange
+  int early, early_panels;    // with `from`: what must be complete before this one stores anything, as wait_for and
+  int early_also, early_also_panels;   // wait_also without it
   int turn;                   // CTA c takes the unit range (c + turn) % CTAs
   int lw, panels;             // tile columns of a sub-panel are 1 << lw, and there are so many sub-panels
   int tiled;                  // wmap is used
@@ -174,6 +191,8 @@ struct QueueHead {
   int n;
   int sets;                   // kSets: matmuls take the sets in turn, and as many may be in flight; 1: one after the other
   int *error, *ops_done, *all_done;
+  uint32_t *epoch;            // the launch's number, with `exchange`
+  uint8_t *exchange;          // or null
   int panels;                 // sub-panels of all matmuls
   Scratch set[kSets];
   int slot_floats;            // floats between two CTAs' slots of partial sums
@@ -322,26 +341,49 @@ template <bool SMALL> __device__ __forceinline__ void zero_rows(const GemvParams
     for (int i = max(M - (face & 2) * 8, 0) * per_row + lane; i < 16 * per_row; i += 32) rows[i] = make_uint4(0, 0, 0, 0);
   }
 }
+// Where the pair of channels `pr` of a sub-panel, in tile column `tcol`, has row r in the result's tiles: a datum's index, as in an addend's.
+__device__ __forceinline__ int pair_place(int tcol, int pr, int r) { return tcol * 1024 + ((r >> 4) * 2 + (pr >> 3 & 1)) * 256 + (r & 15) * 16 + (2 * pr & 15); }
+// A pair of neighbouring channels of one token to the result. Neighbouring lanes have neighbouring pairs of the same token.
+__device__ __forceinline__ void store_pair(const GemvParams &p, int tcol, int pr, int row, bool live, float2 v) {
+  const uint32_t both = bf16_half_up(v.x) | bf16_half_up(v.y) << 16;
+  char *out = static_cast<char *>(p.out);
+  if (p.out_fp32 == 2) {
+    // row-major fp32, only the rows there are: partial sums on their way to an all-reduce
+    if (live) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + tcol * 32 + (2 * pr & 31))) = v;
+  } else if (p.M > 1) {
+    if (live && p.out_fp32) *reinterpret_cast<float2 *>(out + 4 * (size_t)pair_place(tcol, pr, row)) = v;
+    else if (live) *reinterpret_cast<uint32_t *>(out + 2 * (size_t)pair_place(tcol, pr, row)) = both;
+  } else if (p.out_fp32) {
+    // a one-row result repeats across its tile
+    for (int r = 0; live && r < 32; r++) *reinterpret_cast<float2 *>(out + 4 * (size_t)pair_place(tcol, pr, r)) = v;
+  } else {
+    // the same: four lanes put half a face row together, and each of them writes it to eight of the rows
+    uint4 half;
+    half.x = __shfl_sync(0xFFFFFFFFu, both, 0, 4), half.y = __shfl_sync(0xFFFFFFFFu, both, 1, 4);
+    half.z = __shfl_sync(0xFFFFFFFFu, both, 2, 4), half.w = __shfl_sync(0xFFFFFFFFu, both, 3, 4);
+    if (live) {
+#pragma unroll
+      for (int r = 0; r < 32; r += 4) *reinterpret_cast<uint4 *>(out + 2 * (size_t)(pair_place(tcol, pr, r + (pr & 3)) - 2 * (pr & 3))) = half;
+    }
+  }
+}
 template <bool SMALL> __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc, uint32_t smem, int *error) {
   const Columns<SMALL> at(p, pc.sp);
-  const int lw = lw_of<SMALL>(p), pairs = 16 << lw, pr = threadIdx.x & (pairs - 1), M = p.M, epi = p.epi, fp32 = p.out_fp32;
+  const int lw = lw_of<SMALL>(p), pairs = 16 << lw, pr = threadIdx.x & (pairs - 1), M = p.M, epi = p.epi;
   const bool pair = p.pair, owner = pc.me == pc.last;
   const int others = owner ? pc.last - pc.first : 0;                                  // contributors whose sums are to be added
   const int tcol = at.col + (pr >> 4), n0 = at.col * 32 + 2 * pr;                     // tile column and first channel of the pair
   const bool inside = (pr >> 4) < at.width;
   const float unscale = unscale_of(p.tg) * p.alpha;
   const uint16_t *add = owner && inside ? p.add : nullptr;
-  char *out = static_cast<char *>(p.out);
   float *slots = sc.partials + (size_t)(owner ? pc.first : pc.me) * slot_floats + 2 * pr;
   const int rows = kConsumers >> (4 + lw), mine = threadIdx.x >> (4 + lw);            // rows at a time, and this thread's among them
-  // datum index of (row, channel pair) in the result's tiles, and in an addend's
-  auto place = [&](int r) { return tcol * 1024 + ((r >> 4) * 2 + ((pr >> 3) & 1)) * 256 + (r & 15) * 16 + (2 * pr & 15); };
-  auto addend = [&](int r) { return add && r < M ? __ldcg(reinterpret_cast<const uint32_t *>(add + place(r))) : 0u; };
+  auto addend = [&](int r) { return add && r < M ? __ldcg(reinterpret_cast<const uint32_t *>(add + pair_place(tcol, pr, r))) : 0u; };
   uint32_t a = addend(mine);
   // what the barrier is waited with is worked out and fetched already
   int KT = p.KT, next = M * sum_stride(lw) * (pair ? 2 : 1);
   float scale = unscale;
-  asm volatile("" : "+r"(KT), "+r"(next), "+f"(scale), "+l"(out), "+l"(slots) :: "memory");
+  asm volatile("" : "+r"(KT), "+r"(next), "+f"(scale), "+l"(slots) :: "memory");
   named_barrier(1, kConsumers);                                                       // every warp's sums are in place
   uint32_t patience = others && lds32(smem + kSmDead) ? 1 : kSpinLimit * 64;
   for (int row0 = 0; row0 < M; row0 += rows) {
@@ -418,26 +460,7 @@ template <bool SMALL> __device__ __forceinline__ void end_piece(const GemvParams
       if ((threadIdx.x & (min(pairs, 32) - 1)) == 0 && key) atomicMax(sc.keys + row, key);
       continue;
     }
-    const uint32_t both = bf16_half_up(v.x) | bf16_half_up(v.y) << 16;
-    if (fp32 == 2) {
-      // row-major fp32, only the rows there are: partial sums on their way to an all-reduce
-      if (inside && live) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + n0)) = v;
-    } else if (M > 1) {
-      if (inside && live && fp32) *reinterpret_cast<float2 *>(out + 4 * (size_t)place(row)) = v;
-      else if (inside && live) *reinterpret_cast<uint32_t *>(out + 2 * (size_t)place(row)) = both;
-    } else if (fp32) {
-      // a one-row result repeats across its tile
-      for (int r = 0; inside && live && r < 32; r++) *reinterpret_cast<float2 *>(out + 4 * (size_t)place(r)) = v;
-    } else {
-      // the same: four lanes put half a face row together, and each of them writes it to eight of the rows
-      uint4 half;
-      half.x = __shfl_sync(0xFFFFFFFFu, both, 0, 4), half.y = __shfl_sync(0xFFFFFFFFu, both, 1, 4);
-      half.z = __shfl_sync(0xFFFFFFFFu, both, 2, 4), half.w = __shfl_sync(0xFFFFFFFFu, both, 3, 4);
-      if (inside && live) {
-#pragma unroll
-        for (int r = 0; r < 32; r += 4) *reinterpret_cast<uint4 *>(out + 2 * (size_t)(place(r + (pr & 3)) - 2 * (pr & 3))) = half;
-      }
-    }
+    store_pair(p, tcol, pr, row, inside && live, v);
   }
   if (!patience) {
     sts32(smem + kSmDead, 1);
@@ -501,12 +524,12 @@ struct Ring {
 // x may be the result of the launch before this one, or of an earlier matmul of this one: the host has worked out the
 // last matmul of the launch that this one must see complete, and every one before that must be complete too (see Gate). A
 // whole warp waits, a lane for each of the two counters, so that their loads are in flight together. False: gave up.
-__device__ __forceinline__ bool await_turn(const QueueHead &q, const GemvParams &p, int pause_ns) {
+__device__ __forceinline__ bool await_turn(const QueueHead &q, int wait_for, int wait_panels, int wait_also, int also_panels, int pause_ns) {
   asm volatile("griddepcontrol.wait;" ::: "memory");     // returns when the previous launch is complete and visible
-  const int lane = threadIdx.x & 31, op = lane == 0 ? p.wait_for : lane == 1 ? p.wait_also : -1;
+  const int lane = threadIdx.x & 31, op = lane == 0 ? wait_for : lane == 1 ? wait_also : -1;
   bool ok = true;
   if (op >= 0) {
-    const int panels = lane ? p.also_panels : p.wait_panels;
+    const int panels = lane ? also_panels : wait_panels;
     uint32_t spins = 0;
     while (ld_acquire_gpu(q.ops_done + op) < panels) {
       if (++spins > kSpinLimit * 64) { ok = false; break; }
@@ -515,8 +538,9 @@ __device__ __forceinline__ bool await_turn(const QueueHead &q, const GemvParams 
   }
   return __all_sync(0xFFFFFFFFu, ok);                    // what either lane acquired is visible to the whole warp
 }
+__device__ __forceinline__ bool await_turn(const QueueHead &q, const GemvParams &p, int pause_ns) { return await_turn(q, p.wait_for, p.wait_panels, p.wait_also, p.also_panels, pause_ns); }
 
-template <bool WEIGHTS, bool SMALL, class Q>
+template <bool WEIGHTS, bool SMALL, bool CHAIN, class Q>
 __device__ __forceinline__ void produce(const Q &q, uint8_t *smem, uint32_t sbase, int cta, int ctas) {
   const uint32_t full0 = sbase + kSmFull, empty0 = sbase + kSmEmpty, ring0 = sbase + q.ring, ring_bytes = q.ring_bytes;
   volatile uint32_t *held = reinterpret_cast<volatile uint32_t *>(smem + kSmHeld) + (WEIGHTS ? 0 : kBars);   // ring bytes of each stage in the ring
@@ -530,7 +554,8 @@ __device__ __forceinline__ void produce(const Q &q, uint8_t *smem, uint32_t sbas
   uint32_t count = 0, oldest = 0, used = 0;   // stages placed; first stage not yet known to be free; ring bytes held from there on
   for (int i = 0; i < q.n; i++) {
     const GemvParams &p = q.op[i];
-    const Geometry g = geometry(p.fmt, p.pair != 0, p.tg, lw_of<SMALL>(p));
+    Geometry g = geometry(p.fmt, p.pair != 0, p.tg, lw_of<SMALL>(p));
+    if (CHAIN) g.stage = g.w_bytes;                          // x goes straight to registers
     const int me = (cta + p.turn) % ctas;                    // the range this CTA takes in this matmul
     if (me >= p.active) continue;
     const int KT = p.KT, nw = p.pair ? 2 : 1;
@@ -697,6 +722,29 @@ __device__ __forceinline__ uint4 stream_small(Place &w, float *sums, int *error,
 // ---- the messenger: one warp tells other CTAs and hears from them ------------------------------------------------
 // It goes through the CTA's pieces beside the consumers and meets them when they have stored what they had. A release
 // takes 1000 to 3000 cycles under load; a consumer warp that did it was that much behind the others at the next barrier.
+// Report a sub-panel: its results are visible to the whole GPU before the count moves. A matmul is complete when all
+// its sub-panels are: by then every CTA with a part in it has read its x, and is past its look at the counts. It says
+// nothing about the matmul before it, of which this CTA may have no part: that is what Gate is about. (Counting
+// the CTAs instead, idle ones too, took 148 reports to one address where a small matmul has 5 sub-panels.) The last
+// report of the launch therefore finds nobody looking any more, and zeroes the counts for the next launch.
+__device__ __forceinline__ void report(const QueueHead &q, int i) {
+  const int lane = threadIdx.x & 31;
+  int end = 0;
+  if (lane == 0) {
+    red_release_gpu(q.ops_done + i, 1);
+    if (atom_add_acq_rel_gpu(q.all_done, 1) == q.panels - 1) {
+      for (int j = 0; j < q.n; j++) q.ops_done[j] = 0;
+      *q.all_done = 0;
+      if (q.exchange) {
+        const uint32_t next = (*q.epoch + 1) % kEpochs;
+        *q.epoch = next, end = next == 0;
+      }
+    }
+  }
+  if (__shfl_sync(0xFFFFFFFFu, end, 0))          // the tags start over
+    for (size_t at = lane; at < kExchanges * kExchangeBytes / 16; at += 32) reinterpret_cast<uint4 *>(q.exchange)[at] = make_uint4(0, 0, 0, 0);
+}
+
 template <bool SMALL, class Q> __device__ __forceinline__ void carry(const Q &q, int cta, int ctas) {
   const int lane = threadIdx.x & 31;
   for (int i = 0; i < q.n; i++) {
@@ -750,18 +798,7 @@ template <bool SMALL, class Q> __device__ __forceinline__ void carry(const Q &q,
         }
         __syncwarp();
       }
-      // Report the sub-panel: its results are visible to the whole GPU before the count moves. A matmul is complete when all
-      // its sub-panels are: by then every CTA with a part in it has read its x, and is past its look at the counts. It says
-      // nothing about the matmul before it, of which this CTA may have no part: that is what Gate is about. (Counting
-      // the CTAs instead, idle ones too, took 148 reports to one address where a small matmul has 5 sub-panels.) The last
-      // report of the launch therefore finds nobody looking any more, and zeroes the counts for the next launch.
-      if (lane == 0) {
-        red_release_gpu(q.ops_done + i, 1);
-        if (atom_add_acq_rel_gpu(q.all_done, 1) == q.panels - 1) {
-          for (int j = 0; j < q.n; j++) q.ops_done[j] = 0;
-          *q.all_done = 0;
-        }
-      }
+      report(q, i);
       __syncwarp();
     }
   }
@@ -794,8 +831,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
   }
   __syncthreads();
   if (warp >= kCW) {
-    if (warp == kCW) produce<true, SMALL>(q, smem, sbase, cta, ctas);
-    else if (warp == kCW + 1) produce<false, SMALL>(q, smem, sbase, cta, ctas);
+    if (warp == kCW) produce<true, SMALL, false>(q, smem, sbase, cta, ctas);
+    else if (warp == kCW + 1) produce<false, SMALL, false>(q, smem, sbase, cta, ctas);
     else carry<SMALL>(q, cta, ctas);
     return;
   }
@@ -842,6 +879,270 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
       end_piece<SMALL>(p, sc, q.slot_floats, sums, pc, sbase, q.error);
       named_barrier(2, kConsumers + 32);       // the messenger may tell; the sums may be overwritten
     }
+  }
+}
+
+// ---- chains of small matmuls --------------------------------------------------------------------------------------
+// In a small model's decode step every matmul is small (a sub-panel to a CTA, whole) and reads the one before it. What such a matmul
+// costs is the way from one's result to the next one's. In the general kernel that is 4.9 us: the stores have to be acknowledged before the
+// report (0.7), the report is seen by polling (0.7-1.0), then the copy of x starts (0.8), and from x to the result there are some 2.7 us of
+// instructions, most of them fetched anew for every matmul. So lists of small matmuls with up to 8 tokens have a kernel of their own:
+//  * A result also goes to an exchange where every word (two bf16 values) travels with a tag: the launch's number and the matmul's
+//    place in it. What has the right tag is there: no report, no copy. A consumer lane fetches the words of its own
+//    MMA fragments, straight into registers.
+//  * Weights are expanded, scale and all, while x is still on its way, and wait in shared memory as the MMAs take them.
+//  * The next matmul runs on other CTAs, which have had the time for that.
+// 2.0-2.2 us a matmul for one token (1.0 until x is seen, 0.4 to the sums, 0.6 to add them and publish), 3 for eight, whose words and
+// tags are 36 KB to a CTA of a gate/up pair. 30 layers of 576 x 1536 with host values in and out: one token 500 -> 279 us, eight 507 -> 390.
+//
+// What makes it safe to start before the matmul before is known to be complete: of that matmul only x (and the addend, where it is the
+// same tensor) is read, from the exchange. Whatever this one overwrites that the matmul before reads has been
+// read by then: a word is published after the values that go into it were read, and every word this matmul stores depends on all of
+// its x. (The zero rows, which do not, wait for the counter: the messenger writes them.) Everything else waits for the counters of the
+// matmuls before that one (early), and so does every store. kExchanges = 3: matmul i + 3 stores when i + 1, which reads exchange i, is complete.
+// A tag comes up once in kEpochs launches, and then the exchanges are cleared.
+//
+// An exchange: [tile column][left, right face][row < M][8 words with their tags].
+__device__ __forceinline__ uint32_t tag_of(uint32_t epoch, int i) { return epoch * 64 + i + 1; }
+
+// A tile's weights as the registers of its four MMAs, [h][fs], exactly: the codes as integers times 2^-6, times 2^(e - 127).
+template <int FMT> __device__ __forceinline__ void expand_tile(uint32_t tile, uint32_t ex, uint32_t (&a)[2][2][4]) {
+  const uint4 ev = lds128(ex);
+  const uint32_t ee[4] = {ev.x, ev.y, ev.z, ev.w};
+  uint4 wv[2];
+  wv[0] = lds128(tile + 64);
+  if (FMT == BT_BFP8) wv[1] = lds128(tile + 64 + 512);
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int fs = 0; fs < 2; fs++) {
+      const uint32_t e = ee[2 * h + fs], s01 = (e << 7) & 0x7F807F80u, s23 = (e >> 1) & 0x7F807F80u;
+      uint32_t c0, c1, c2, c3, o0, o1;     // codes of rows g and g + 8, first and second k pair, and their offsets
+      if (FMT == BT_BFP8) {
+        const uint32_t w0 = fs ? wv[h].z : wv[h].x, w1 = fs ? wv[h].w : wv[h].y;
+        c0 = w0 & kByteLanes, c1 = w1 & kByteLanes, c2 = prmt(w0, 0u, kOddBytes), c3 = prmt(w1, 0u, kOddBytes), o0 = kOff128, o1 = kOff128;
+      } else {
+        const uint32_t w = h ? (fs ? wv[0].w : wv[0].z) : (fs ? wv[0].y : wv[0].x);
+        c0 = w & kByteLanes, c1 = w & kNibbleLanes, c2 = prmt(w, 0u, kOddBytes), c3 = c2 & kNibbleLanes, o0 = kOff136, o1 = kOff8;
+      }
+      a[h][fs][0] = mul_bf16x2(fma_bf16x2(c0, kTo6, o0), s01), a[h][fs][1] = mul_bf16x2(fma_bf16x2(c1, kTo6, o1), s01);
+      a[h][fs][2] = mul_bf16x2(fma_bf16x2(c2, kTo6, o0), s23), a[h][fs][3] = mul_bf16x2(fma_bf16x2(c3, kTo6, o1), s23);
+    }
+}
+
+// One matmul's part of a consumer warp: its tile rows, every `groups`-th from ck on. x is asked for kAhead tile rows ahead.
+constexpr int kAhead = 3;                            // 48 tile rows of one column: K = 1536
+constexpr int kAheadBytes = kAhead * kCW * 2048;     // expanded weights of so many tile rows per warp
+struct Link {
+  uint32_t smem, count, turn;        // shared memory; stages, and matmuls of this CTA, so far
+  int warp, lane;
+};
+template <int FMT> __device__ __forceinline__ void chain_matmul(const GemvParams &p, const QueueHead &q, int index, int me, Link &w, float *sums, uint32_t expanded) {
+  constexpr int TB = tile_bytes(FMT);
+  const int lane = w.lane, t = lane & 3, token = lane >> 2, M = p.M, lw = p.lw, KT = p.KT, thread = threadIdx.x;
+  const bool from = p.from, pair = p.pair;
+  const int rest = w.warp >> lw, cc = w.warp & ((1 << lw) - 1), mat = pair ? rest & 1 : 0, ck = pair ? rest >> 1 : rest, groups = small_groups(lw, pair);
+  uint32_t tag = tag_of(lds32(w.smem + kSmEpoch), index) - 1;        // of the matmul before
+  // this thread's place in the result: a pair of channels of one token
+  const Columns<true> at(p, me);
+  const int pr = thread & ((16 << lw) - 1), row = thread >> (4 + lw), tcol = at.col + (pr >> 4);
+  const bool live = row < M && (pr >> 4) < at.width;
+  const int before = (index + kExchanges - 1) % kExchanges, word = ((tcol * 2 + (pr >> 3 & 1)) * M + row) * 64 + (pr & 7) * 8;
+  const uint8_t *x = from ? q.exchange + before * kExchangeBytes + token * 64 + t * 16 : reinterpret_cast<const uint8_t *>(p.x) + token * 32 + t * 8;
+  const uint8_t *addend = p.add_from ? q.exchange + before * kExchangeBytes + word : reinterpret_cast<const uint8_t *>(p.add + pair_place(tcol, pr, row));
+  const bool add_from = p.add_from && live, add = p.add && !p.add_from && live;
+  uint8_t *to = p.to && live ? q.exchange + index % kExchanges * kExchangeBytes + word : nullptr;
+  float alpha = p.alpha;
+  int epi = p.epi;
+  // what the end needs is fetched here, not when it is waited for
+  asm volatile("" : "+f"(alpha), "+r"(epi), "+l"(to), "+l"(addend), "+l"(x), "+r"(tag));
+  const uint32_t go = w.smem + kSmGo + 8 * (w.turn & 1);
+  if (!from) stage_wait(w.smem, go, w.turn >> 1 & 1, q.error);
+  const int steps = (KT + groups - 1) / groups, per_stage = stage_rows_per_warp(FMT, 1, lw);
+  const uint32_t matrix = (uint32_t)mat * geometry(FMT, pair, 1, lw).matrix;
+  expanded += w.warp * 2048 + lane * 16;
+  uint32_t patience = kSpinLimit * 64;
+  uint2 a = make_uint2(0, tag);
+  const int stride = sum_stride(lw), slab = M * stride;
+  for (int k0 = 0, in_stage = 0; k0 < steps; k0 += kAhead) {
+    const int n = min(steps - k0, kAhead);
+    // the weights of up to kAhead tile rows, as the MMAs take them
+    uint4 stage = make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+    for (int j = 0; j < n; j++) {
+      const uint32_t slot = w.count & (kBars - 1);
+      if (in_stage == 0 || j == 0) {
+        const bool ok = stage_wait(w.smem, w.smem + kSmFull + 8 * slot, w.count / kBars & 1, q.error);
+        stage = __all_sync(0xFFFFFFFFu, ok) ? lds128(w.smem + kSmStages + 32 * slot) : make_uint4(0, 0, 0, 0);
+      }
+      const int r = ck + in_stage * groups;
+      uint32_t m[2][2][4] = {};
+      if (cc < (int)stage.z && r < (int)stage.y) {
+        const uint32_t tile = stage.x + matrix + (r * stage.z + cc) * TB;
+        expand_tile<FMT>(tile + lane * 16, tile + t * 16, m);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) sts128(expanded + j * (kCW * 2048) + i * 512, make_uint4(m[i / 2][i % 2][0], m[i / 2][i % 2][1], m[i / 2][i % 2][2], m[i / 2][i % 2][3]));
+      if (++in_stage == per_stage || k0 + j == steps - 1) {
+        in_stage = 0, w.count++;
+        __syncwarp();
+        mbar_arrive_if(w.smem + kSmEmpty + 8 * slot, lane == 0);
+      }
+    }
+    // their x: upper and lower half of each, what this lane's token has there
+    uint4 v[kAhead][2];
+#pragma unroll
+    for (int j = 0; j < kAhead; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int r = ck + (k0 + j) * groups;
+        v[j][h] = make_uint4(0, tag, 0, tag);
+        if (token < M && r < KT) {
+          if (from) v[j][h].y = ~tag;
+          else {
+            const uint2 u = __ldcg(reinterpret_cast<const uint2 *>(x + r * 2048 + h * 512));
+            v[j][h].x = u.x, v[j][h].z = u.y;
+          }
+        }
+      }
+    if (k0 == 0) {
+      if (from) stage_wait(w.smem, go, w.turn >> 1 & 1, q.error);
+      __syncwarp();
+      if (add) a.x = __ldcg(reinterpret_cast<const uint32_t *>(addend));
+      if (add_from) a.y = ~tag;
+    }
+    if (from) {
+      bool missing;
+      do {
+        if (lds32(w.smem + kSmDead)) patience = 1;
+#pragma unroll
+        for (int j = 0; j < kAhead; j++)
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+            if (v[j][h].y != tag || v[j][h].w != tag) v[j][h] = ld_relaxed4(x + ((ck + (k0 + j) * groups) * 2 + h) * M * 64);
+        if (a.y != tag) a = ld_relaxed64(addend);
+        missing = a.y != tag;
+#pragma unroll
+        for (int j = 0; j < kAhead; j++) missing |= v[j][0].y != tag || v[j][0].w != tag || v[j][1].y != tag || v[j][1].w != tag;
+      } while (__any_sync(0xFFFFFFFFu, missing) && --patience);
+    }
+    // the sums of the matmul before have been read
+    if (k0 == 0 && w.turn) stage_wait(w.smem, w.smem + kSmDone + 8 * ((w.turn - 1) & 1), (w.turn - 1) >> 1 & 1, q.error);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < kAhead; j++)
+      if (ck + (k0 + j) * groups < KT) {
+        float acc[2][1][4];
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[i / 4][0][i % 4] = 0.f;
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int fs = 0; fs < 2; fs++) {
+            const uint4 m = lds128(expanded + j * (kCW * 2048) + (2 * h + fs) * 512);
+            mma_bf16(acc[fs][0], m.x, m.y, m.z, m.w, v[j][h].x, v[j][h].z);
+          }
+        leave_sums<FMT, 1>(acc, sums + ((ck + (k0 + j) * groups) * (pair ? 2 : 1) + mat) * slab, stride, M, cc, lane);
+      }
+  }
+  if (!patience) {
+    sts32(w.smem + kSmDead, 1);
+    atomicExch(q.error, 6);
+  }
+  // the last tile row's sums, then the others' in order: as in the general kernel, and with the same last bit
+  const int next = pair ? 2 * slab : slab;
+  const float *from_sum = sums + row * stride + 2 * pr, *last_sum = from_sum + (KT - 1) * next;
+  int rows = KT - 1;
+  asm volatile("" : "+l"(from_sum), "+l"(last_sum), "+r"(rows) :: "memory");
+  named_barrier(1, kConsumers);
+  // from here on a pair of channels of a token to a thread
+  if (row - (lane >> min(4 + lw, 5)) < M) {                          // (whole warps)
+    float2 s = make_float2(0.f, 0.f), u = s;
+    if (row < M) {
+      s = *reinterpret_cast<const float2 *>(last_sum);
+      if (!pair) {
+#pragma unroll 8
+        for (int i = 0; i < rows; i++, from_sum += next) {
+          const float2 y = *reinterpret_cast<const float2 *>(from_sum);
+          s.x += y.x, s.y += y.y;
+        }
+      } else {
+        u = *reinterpret_cast<const float2 *>(last_sum + slab);
+#pragma unroll 4
+        for (int i = 0; i < rows; i++, from_sum += next) {
+          const float2 y = *reinterpret_cast<const float2 *>(from_sum), z = *reinterpret_cast<const float2 *>(from_sum + slab);
+          s.x += y.x, s.y += y.y, u.x += z.x, u.y += z.y;
+        }
+      }
+    }
+    s.x = s.x * alpha + __uint_as_float(a.x << 16), s.y = s.y * alpha + __uint_as_float(a.x & 0xFFFF0000u);
+    if (epi == BT_EPI_RELU) s.x = fmaxf(s.x, 0.f), s.y = fmaxf(s.y, 0.f);
+    if (epi == BT_EPI_SILU || pair) s.x = silu(s.x), s.y = silu(s.y);
+    if (pair) s.x *= (u.x + 0.f) * alpha, s.y *= (u.y + 0.f) * alpha;
+    if (to) st_relaxed64(to, make_uint2(bf16_half_up(s.x) | bf16_half_up(s.y) << 16, tag + 1));
+    store_pair(p, tcol, pr, row, live, s);
+  }
+  __syncwarp();
+  mbar_arrive_if(w.smem + kSmDone + 8 * (w.turn & 1), lane == 0);
+  w.turn++;
+}
+
+template <int OPS>
+__global__ void __launch_bounds__(kThreads, 1) chain_kernel(const __grid_constant__ Queue<OPS> q) {
+  extern __shared__ __align__(128) uint8_t smem[];
+  const uint32_t sbase = smem_u32(smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, cta = blockIdx.x, ctas = gridDim.x;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (threadIdx.x == 0) {
+    sts32(sbase + kSmDead, 0);
+    for (int s = 0; s < kBars; s++) mbar_init(sbase + kSmFull + 8 * s, 1), mbar_init(sbase + kSmEmpty + 8 * s, kCW);
+    mbar_init(sbase + kSmReady, 1);
+    for (int s = 0; s < 2; s++) mbar_init(sbase + kSmGo + 8 * s, 1), mbar_init(sbase + kSmDone + 8 * s, kCW);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  if (warp == kCW) return produce<true, true, true>(q, smem, sbase, cta, ctas);
+  if (warp < kCW) {
+    Link w = {sbase, 0, 0, warp, lane};
+    stage_wait(sbase, sbase + kSmReady, 0, q.error);
+    for (int i = 0; i < q.n; i++) {
+      const GemvParams &p = q.op[i];
+      const int me = (cta + p.turn) % ctas;
+      if (me >= p.active) continue;
+      if (p.fmt == BT_BFP8) chain_matmul<BT_BFP8>(p, q, i, me, w, reinterpret_cast<float *>(smem + kSmSums + kAheadBytes), sbase + kSmSums);
+      else chain_matmul<BT_BFP4>(p, q, i, me, w, reinterpret_cast<float *>(smem + kSmSums + kAheadBytes), sbase + kSmSums);
+    }
+    return;
+  }
+  // one warp lets the consumers go ahead, one, the messenger, reports what they have done
+  const bool messenger = warp == kCW + 2;
+  if (!messenger) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (lane == 0) {
+      if (q.exchange) sts32(sbase + kSmEpoch, *reinterpret_cast<volatile int *>(q.epoch));
+      mbar_arrive(sbase + kSmReady);
+    }
+    __syncwarp();
+  }
+  uint32_t turn = 0;
+  for (int i = 0; i < q.n; i++) {
+    const GemvParams &p = q.op[i];
+    const int me = (cta + p.turn) % ctas;
+    if (me >= p.active) continue;
+    const bool early = !messenger && p.from;
+    if (!await_turn(q, early ? p.early : p.wait_for, early ? p.early_panels : p.wait_panels, early ? p.early_also : p.wait_also, early ? p.early_also_panels : p.also_panels, messenger ? 100 : 0) &&
+        lane == 0)
+      atomicExch(q.error, 5);
+    __syncwarp();
+    if (!messenger) mbar_arrive_if(sbase + kSmGo + 8 * (turn & 1), lane == 0);
+    else {
+      zero_rows<true>(p, me);
+      stage_wait(sbase, sbase + kSmDone + 8 * (turn & 1), turn >> 1 & 1, q.error);
+      __syncwarp();
+      report(q, i);
+      __syncwarp();
+    }
+    turn++;
   }
 }
 
@@ -920,6 +1221,23 @@ struct Gate {
 Gate gate(const bt_gemv_op *ops, int i, int sets) {
   const int w = wait_for(ops, i, sets);
   return {w, w > 0 && wait_for(ops, w, sets) < w - 1 ? w - 1 : -1};
+}
+
+// Whether matmul `i` of a chain takes its x from the exchange of matmul i - 1: x is that one's result, all of it, and nothing
+// else stands between them than what the exchange takes care of.
+bool exchanged(const bt_gemv_op *ops, int i) {
+  if (i < 1) return false;
+  const bt_gemv_op &o = ops[i], &e = ops[i - 1];
+  if (o.x != e.out || e.out_dtype != BT_BF16 || o.M != e.M || o.K != e.N) return false;
+  Range lr[4], lw[2], ew[2];
+  ranges_read(o, lr), ranges_written(o, lw), ranges_written(e, ew);
+  return !lw[0].meets(ew[0]) && (!o.add || o.add == e.out || !lr[1].meets(ew[0]));
+}
+// Lists that chain_kernel takes: every matmul small, a sub-panel to a CTA, up to 8 tokens, no pick and no rows for an all-reduce.
+bool chain(const QueueHead &q, const GemvParams *op) {
+  for (int i = 0; i < q.n; i++)
+    if (!op[i].small || op[i].M > kChainRows || op[i].epi == BT_EPI_ARGMAX || op[i].out_fp32 == 2 || op[i].share != op[i].KT || op[i].extra) return false;
+  return true;
 }
 
 // The ranges of a matmul's units. Sharing a sub-panel costs a hand-over of partial sums, a range that straddles sub-panels
@@ -1024,6 +1342,8 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       if (per_sm < 1) return fail(BT_DEVICE, "%s: the matmul kernel does not fit an SM of device %d", who, device);
       return BT_OK;
     };
+    if (int s = fits(chain_kernel<kQueueShort>)) return s;
+    if (int s = fits(chain_kernel<kQueueMax>)) return s;
     if (int s = fits(gemv_queue_kernel<true, kQueueShort>)) return s;
     if (int s = fits(gemv_queue_kernel<true, kQueueMax>)) return s;
     if (int s = fits(gemv_queue_kernel<false, kQueueShort>)) return s;
@@ -1049,11 +1369,26 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       p.wait_for = g.last, p.wait_also = g.also;
       p.turn = (int)(((long long)(base + i) * 101) % ctas);
       p.wait_panels = g.last >= 0 ? q.op[g.last].panels : 0, p.also_panels = g.also >= 0 ? q.op[g.also].panels : 0;
+      p.x = as_ptr<uint16_t>(o.x);
+      p.from = p.to = p.add_from = 0;
       deal_units(p, ctas);
       q.panels += p.panels;
       small |= p.small;
       if (int s = make_maps(p, o.x)) return s;
       sums = max(sums, p.small ? p.KT * (p.pair ? 2 : 1) * p.M * sum_stride(p.lw) * 4 : sums_bytes(p.tg));
+    }
+    const bool chained = chain(q, q.op);
+    if (chained) {
+      sums += kAheadBytes;
+      // the next matmul goes to other CTAs: they have its weights at hand when its x comes
+      for (int i = 0, start = 0; i < q.n; start = (start + q.op[i++].active) % ctas) q.op[i].turn = (ctas - start) % ctas;
+      for (int i = 1; i < q.n && scratch.exchange; i++) {
+        GemvParams &p = q.op[i];
+        if (!exchanged(ops + base, i)) continue;
+        const int w = i - scratch.sets, v = w > 0 && wait_for(ops + base, w, scratch.sets) < w - 1 ? w - 1 : -1;
+        p.from = q.op[i - 1].to = 1, p.add_from = p.add && ops[base + i].add == ops[base + i].x;
+        p.early = w < 0 ? -1 : w, p.early_panels = w >= 0 ? q.op[w].panels : 0, p.early_also = v, p.early_also_panels = v >= 0 ? q.op[v].panels : 0;
+      }
     }
     q.ring = kSmSums + (sums + 127) / 128 * 128, q.ring_bytes = (kSmemBytes - q.ring) / 128 * 128;
     // Programmatic dependent launch: this grid may begin while the previous launch of the stream is still finishing.
@@ -1071,8 +1406,8 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       Queue<kQueueShort> s;
       static_cast<QueueHead &>(s) = q;
       std::copy(q.op, q.op + q.n, s.op);
-      BT_CUDA(small ? cudaLaunchKernelEx(&cfg, gemv_queue_kernel<true, kQueueShort>, s) : cudaLaunchKernelEx(&cfg, gemv_queue_kernel<false, kQueueShort>, s));
-    } else BT_CUDA(small ? cudaLaunchKernelEx(&cfg, gemv_queue_kernel<true, kQueueMax>, q) : cudaLaunchKernelEx(&cfg, gemv_queue_kernel<false, kQueueMax>, q));
+      BT_CUDA(chained ? cudaLaunchKernelEx(&cfg, chain_kernel<kQueueShort>, s) : small ? cudaLaunchKernelEx(&cfg, gemv_queue_kernel<true, kQueueShort>, s) : cudaLaunchKernelEx(&cfg, gemv_queue_kernel<false, kQueueShort>, s));
+    } else BT_CUDA(chained ? cudaLaunchKernelEx(&cfg, chain_kernel<kQueueMax>, q) : small ? cudaLaunchKernelEx(&cfg, gemv_queue_kernel<true, kQueueMax>, q) : cudaLaunchKernelEx(&cfg, gemv_queue_kernel<false, kQueueMax>, q));
     if (int st = launched("gemv_queue_kernel")) return st;
   }
   return BT_OK;
@@ -1093,6 +1428,7 @@ QueueHead workspace_scratch(uint64_t work) {
   q.sets = kSets;
   for (int s = 0; s < kSets; s++) q.set[s] = scratch_at(base + kWsSets + s * kSetBytes);
   q.slot_floats = (int)kSlotFloatsMax;
+  q.epoch = reinterpret_cast<uint32_t *>(base + kWsEpoch), q.exchange = base + kWsExchange;
   return q;
 }
 

@@ -178,6 +178,9 @@ __device__ __forceinline__ void tmem_ld(uint32_t addr, uint32_t (&v)[32]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+__device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
@@ -211,6 +214,23 @@ __device__ __forceinline__ uint2 ld_relaxed2(const void *p) {
 }
 __device__ __forceinline__ void st_relaxed2(void *p, uint2 v) {
   asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1, %2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
+}
+// Two words that travel as one, and two such pairs, each whole on its own.
+__device__ __forceinline__ void st_relaxed64(void *p, uint2 v) {
+  asm volatile("{\n\t.reg .b64 t;\n\tmov.b64 t, {%1, %2};\n\tst.relaxed.gpu.global.b64 [%0], t;\n\t}" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
+}
+__device__ __forceinline__ uint2 ld_relaxed64(const void *p) {
+  uint2 v;
+  asm volatile("{\n\t.reg .b64 t;\n\tld.relaxed.gpu.global.b64 t, [%2];\n\tmov.b64 {%0, %1}, t;\n\t}" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 ld_relaxed4(const void *p) {
+  uint4 v;
+  asm volatile("{\n\t.reg .b64 t, u;\n\tld.relaxed.gpu.global.v2.b64 {t, u}, [%4];\n\tmov.b64 {%0, %1}, t;\n\tmov.b64 {%2, %3}, u;\n\t}"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
 }
 // Orders this thread's earlier (observed) generic-proxy accesses before its later asynchronous-proxy ones (TMA and
 // bulk copies), here: global data another CTA wrote, about to be fetched by a bulk copy.
