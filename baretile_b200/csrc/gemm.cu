@@ -33,7 +33,7 @@
 // before either frees its tensor memory or exits, so neither signals a barrier of a CTA that has gone.
 #include "common.cuh"
 #include "ptx.cuh"
-#include "stream_layout.cuh"
+#include "expand.cuh"
 #include "tmap.cuh"
 #include <cstring>
 
@@ -83,50 +83,24 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
 // Instruction descriptor: fp32 accumulator, bf16 A and B, both K-major, N = 256, M = 256 (128 rows in each CTA).
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 
-__device__ __forceinline__ float silu(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
-__device__ __forceinline__ uint32_t bf16_half_up(float v) { return (__float_as_uint(v) + 0x8000u) >> 16; }
-
 // Expand one packed tile (streaming layout, shared address `tile`) to bf16 and store it as rows [32 c, 32 c + 32) and
 // K columns [32 j, 32 j + 32) of the B tile at shared address `b` (K-major, 128-byte rows, 128-byte swizzle: the
-// 16-byte chunk index of a row is XORed with the row's index modulo 8). Weights are stored in offset binary: a byte
-// (or a masked nibble) zero-extended into a 16-bit lane is the bf16 number code * 2^-133, and one packed fused
-// multiply-add with the face row's power of two, minus the offset times it, makes it the exact signed weight
-// times 2^(e - 197). A nibble q is worth 16 q: a high nibble stays where it is in its byte (16 * code), a low nibble
-// takes 16 times the scale.
+// 16-byte chunk index of a row is XORed with the row's index modulo 8).
 template <int FMT>
 __device__ __forceinline__ void expand_tile(uint32_t tile, uint32_t b, int c, int j, int lane) {
   const int g = lane >> 2, t = lane & 3;
-  const uint4 ev = lds128(tile + t * 16);
-  const uint32_t ee[4] = {ev.x, ev.y, ev.z, ev.w};
-  uint4 wv[2];
-  if (FMT == BT_BFP8) wv[0] = lds128(tile + 64 + lane * 16), wv[1] = lds128(tile + 64 + 512 + lane * 16);
-  else wv[0] = lds128(tile + 64 + lane * 16), wv[1] = wv[0];
+  uint32_t a[2][2][4];
+  expand_weights<FMT>(packed_lane<FMT>(tile, lane), a);
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
+  for (int h = 0; h < 2; h++)
 #pragma unroll
     for (int fs = 0; fs < 2; fs++) {
-      const uint32_t ew = ee[2 * h + fs];
-      const uint32_t s01 = scale_pair<0>(ew), s23 = scale_pair<1>(ew);
-      uint32_t a0, a1, a2, a3;   // channels 2g (a0, a2) and 2g + 1 (a1, a3), four consecutive k each
-      if (FMT == BT_BFP8) {
-        const uint32_t w0 = fs ? wv[h].z : wv[h].x, w1 = fs ? wv[h].w : wv[h].y;
-        const uint32_t n01 = mul_bf16x2(s01, 0x80808080u), n23 = mul_bf16x2(s23, 0x80808080u);   // -128 * 2^-133 * scale
-        a0 = fma_bf16x2(w0 & 0x00FF00FFu, s01, n01), a1 = fma_bf16x2(w1 & 0x00FF00FFu, s01, n01);
-        a2 = fma_bf16x2(prmt(w0, 0u, 0x4341u), s23, n23), a3 = fma_bf16x2(prmt(w1, 0u, 0x4341u), s23, n23);
-      } else {
-        const uint32_t wb = h ? (fs ? wv[0].w : wv[0].z) : (fs ? wv[0].y : wv[0].x), wo = prmt(wb, 0u, 0x4341u);
-        const uint32_t t01 = mul_bf16x2(s01, 0x41804180u), t23 = mul_bf16x2(s23, 0x41804180u);   // 16 * scale: a nibble q is worth 16 q
-        const uint32_t n01 = mul_bf16x2(t01, 0x80088008u), n23 = mul_bf16x2(t23, 0x80088008u);   // -8 * 2^-133 * 16 * scale
-        a0 = fma_bf16x2(wb & 0x000F000Fu, t01, n01), a1 = fma_bf16x2(wb & 0x00F000F0u, s01, n01);
-        a2 = fma_bf16x2(wo & 0x000F000Fu, t23, n23), a3 = fma_bf16x2(wo & 0x00F000F0u, s23, n23);
-      }
       const int n0 = 32 * c + 16 * fs + 2 * g;                       // even, so n0 and n0 + 1 share an 8-row group
       const int chunk = 4 * j + 2 * h + (t >> 1);                    // 16-byte chunk of k = 32 j + 16 h + 4 t
       const uint32_t group = b + (n0 >> 3) * 1024 + (t & 1) * 8;
-      sts64(group + (n0 & 7) * 128 + ((chunk ^ (n0 & 7)) << 4), a0, a2);
-      sts64(group + ((n0 + 1) & 7) * 128 + ((chunk ^ ((n0 + 1) & 7)) << 4), a1, a3);
+      sts64(group + (n0 & 7) * 128 + ((chunk ^ (n0 & 7)) << 4), a[h][fs][0], a[h][fs][2]);
+      sts64(group + ((n0 + 1) & 7) * 128 + ((chunk ^ ((n0 + 1) & 7)) << 4), a[h][fs][1], a[h][fs][3]);
     }
-  }
 }
 
 // SPLIT: the pairs share K. A kernel of its own, since whole blocks lose 2 % to the K block a pair starts at and the sums that
@@ -240,7 +214,7 @@ __global__ void __launch_bounds__(threads_of(GROUPS), 1) gemm_kernel(const GemmP
     wait(acc_full, 0, 16);
     tc_fence_after();
     const int q = warp & 3, ch = d >> 2;                            // tensor-memory lane quarter; column half
-    const float unscale = 18446744073709551616.f * p.alpha;         // 2^64: the weights were expanded times 2^-64
+    const float unscale = kExpandedUnscale * p.alpha;
     const int out_cols = p.pair ? 128 : 256, part = out_cols / (2 * GROUPS);   // this warp's columns
     constexpr int COLS = GROUPS == 1 ? 32 : 16;                     // and how many at a time: 32 need more registers than 18 warps have
     const int tile_rows = (p.M + 31) / 32;
@@ -321,7 +295,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const GemmParams p) {
   if (i >= (unsigned)tile_rows * 32 * quads) return;
   const int row = i / quads, col = (i - row * quads) * 4, tcol = col >> 5, tr = row >> 5;
   const size_t cols = (size_t)p.TC * 32, plane = (size_t)tile_rows * 32 * cols;
-  const float unscale = 18446744073709551616.f * p.alpha;           // 2^64: the weights were expanded times 2^-64
+  const float unscale = kExpandedUnscale * p.alpha;
   float f[4] = {0.f, 0.f, 0.f, 0.f}, g[4] = {0.f, 0.f, 0.f, 0.f};
   const int at = ((row >> 4) & 1) * 512 + (row & 15) * 16 + ((col >> 4) & 1) * 256 + (col & 15);   // datum index in the tile
   if (row < p.M) {
@@ -391,17 +365,22 @@ int deal_blocks(GemmParams &p, int slots, size_t part_bytes) {
   return pairs;
 }
 
-// Argument checks and launches of both entry points.
-int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N, uint64_t a, uint64_t w, uint64_t w2, uint64_t add, int add_rows, float alpha,
-         uint64_t out, int out_dtype, uint64_t part, size_t part_bytes, bool weights_early, uint64_t work, uint64_t stream) {
+// Argument checks of both entry points.
+int check(const char *who, int fmt, int epilogue, int M, int K, int N, uint64_t a, uint64_t w, uint64_t w2, uint64_t add, int add_rows, uint64_t out, int out_dtype, uint64_t work) {
   BT_REQUIRE(fmt == BT_BFP8 || fmt == BT_BFP4, "%s: weights must be bfp8 (8) or bfp4 (4), not %d", who, fmt);
   BT_REQUIRE(epilogue >= BT_EPI_NONE && epilogue <= BT_EPI_GLU, "%s: the epilogue is none, relu, silu or glu, not %d", who, epilogue);
-  const bool pair = epilogue == BT_EPI_GLU;
   BT_REQUIRE(M >= 1 && K > 0 && N > 0 && K % 32 == 0, "%s: needs M >= 1, N >= 1 and K a positive multiple of 32: %d x %d x %d", who, M, K, N);
   BT_REQUIRE(a && w && out && work && a % 16 == 0 && w % 16 == 0 && out % 16 == 0, "%s: needs 16-byte aligned device addresses", who);
-  BT_REQUIRE(pair == (w2 != 0) && w2 % 16 == 0, "%s: w2 goes with the GLU epilogue, and only with it", who);
+  BT_REQUIRE((epilogue == BT_EPI_GLU) == (w2 != 0) && w2 % 16 == 0, "%s: w2 goes with the GLU epilogue, and only with it", who);
   BT_REQUIRE(add % 16 == 0 && (!add || add_rows == 1 || add_rows == M), "%s: the addend is 16-byte aligned and has 1 or M rows, not %d", who, add_rows);
   BT_REQUIRE(out_dtype == BT_BF16 || out_dtype == BT_FP32, "%s: results are bf16 or fp32", who);
+  return BT_OK;
+}
+// Their launches.
+int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N, uint64_t a, uint64_t w, uint64_t w2, uint64_t add, int add_rows, float alpha,
+         uint64_t out, int out_dtype, uint64_t part, size_t part_bytes, bool weights_early, uint64_t work, uint64_t stream) {
+  const bool pair = epilogue == BT_EPI_GLU;
+  if (int s = check(who, fmt, epilogue, M, K, N, a, w, w2, add, add_rows, out, out_dtype, work)) return s;
   if (int s = use_device(device)) return s;
   alignas(64) CUtensorMap amap;
   const uint64_t dims[2] = {(uint64_t)K, (uint64_t)M}, strides[1] = {(uint64_t)K * 2};
@@ -448,6 +427,10 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
   return launched("reduce_kernel");
 }
 
+// Up to so many rows gemm_few.cu is the faster one (its sums of 128 tokens of a pair and the expanded weights fill tensor memory): 128 rows of
+// 4096 x 14336, gate/up and down, 58 us against 120, 33 rows 47 against 113.
+constexpr int kFewRows = 128;
+
 }  // namespace
 
 extern "C" {
@@ -462,6 +445,11 @@ int bt_gemm_tiles(int device, int fmt, int epilogue, int M, int K, int N, uint64
   BT_REQUIRE(M >= 1 && K > 0 && K % 32 == 0, "bt_gemm_tiles: needs M >= 1 and K a positive multiple of 32: %d x %d", M, K);
   const size_t rows = ((size_t)M * K * 2 + 255) / 256 * 256;
   BT_REQUIRE(x && x % 16 == 0 && scratch && scratch % 256 == 0 && scratch_bytes >= rows, "bt_gemm_tiles: needs x and at least %zu bytes of 256-byte aligned scratch, got %zu", rows, scratch_bytes);
+  if (M > 32 && M <= kFewRows) {
+    if (int s = check("bt_gemm_tiles", fmt, epilogue, M, K, N, x, w, w2, add, add_rows, out, out_dtype, work)) return s;
+    if (int s = use_device(device)) return s;
+    return gemm_few(device, fmt, epilogue, M, K, N, x, w, w2, add, add_rows, alpha, out, out_dtype, work, stream);
+  }
   if (int s = bt_untilize(device, 2, x, scratch, 1, M, K, stream)) return s;
   return gemm("bt_gemm_tiles", device, fmt, epilogue, M, K, N, scratch, w, w2, add, add_rows, alpha, out, out_dtype, scratch + rows, scratch_bytes - rows, true, work, stream);
 }

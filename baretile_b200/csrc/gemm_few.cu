@@ -1,0 +1,339 @@
+// Prefill matmul for 33 to 128 token rows (a short prompt, a large speculative or decode batch): out = epilogue(alpha * x @ W + add),
+// W block-float in streaming layout, x in tiles as Tensor holds it.
+//
+// With so few rows every weight is used a few dozen times and the work is bound by the stream of packed weights: by
+// HBM (an SM's share of it is a tile in 43 cycles in bfp8, 23 in bfp4), by their expansion (25 cycles a tile) and by what a launch
+// costs. MMAs with the rows of x as their M would be mostly padding, and expanded weights as a B operand would cross shared memory
+// twice (2 KB a tile each way, of 128 bytes a cycle). So the operands change places: the 128 output channels of a sub-panel are the MMA's M,
+// the tokens its N (only as many as there are, in sixteens), and the expanded weights go from registers to TENSOR MEMORY, from
+// where tcgen05.mma takes its A operand; a lane's registers are 16x256b store fragments as they come.
+//
+// A CTA has a sub-panel of 4 tile columns (of both matrices of a gate/up pair) and all rows; where sub-panels are fewer than SMs a
+// cluster of up to 8 CTAs shares one, each with a part of K. At the end the CTAs' fp32 sums are added through distributed shared memory,
+// in order, and each CTA of the cluster runs the epilogue for its share of the rows: one launch, no scratch, x not laid out anew.
+//
+// Per stage of up to 4 tile rows (K = 128):
+//   warps 0-15   expand packed tiles into tensor memory, two groups of eight that take the stages in turn (as one group all warps computed at
+//                the same time and waited at the same time: 33 rows of 4096 x 14336 52 us against 46); then the epilogue
+//   warp 16      copies the packed tiles (a bulk copy per matrix)
+//   warp 17      issues the MMAs (128 channels x tokens x 16 each); a commit frees x and the tensor memory of the stage
+//   warps 18-21  copy x, a tile row each: 16 tokens x 16 k of a tile are 512 consecutive bytes, a warp's one cp.async, which lands
+//                in the 32-byte swizzle
+// Gate/up pair and down projection, against the kernel of gemm.cu with its x laid out by rows and its parts of K added up by another launch:
+// 77 rows of 2048 x 5632 (bfp4, bfp8) 43.7 -> 22.5 us, 33 rows of 512 x 1024 23.8 -> 11.1, 33 rows of 4096 x 14336 113 -> 47, 128 rows 120 -> 58.
+// A launch costs 5 to 10 us beside its stages: setting up and the first weights and x 3, the sums' way through the cluster and the epilogue 3.
+// Every wait is bounded and reports through the error word.
+#include "common.cuh"
+#include "expand.cuh"
+#include <algorithm>
+
+namespace bt {
+namespace {
+
+constexpr int kRows = 4;                            // tile rows of a stage
+constexpr int kExpandWarps = 16, kWeightWarp = 16, kMmaWarp = 17, kXWarp = 18, kXWarps = kRows;
+constexpr int kGroups = 2, kGroupWarps = kExpandWarps / kGroups;   // groups of warps that take the stages in turn
+constexpr int kThreads = (kXWarp + kXWarps) * 32;
+constexpr int kMaxStages = 8, kMaxBufs = 4, kMaxSplits = 8;
+constexpr uint32_t kLimit = 1u << 14;               // attempts of up to 100 us each
+
+// Shared memory: mbarriers, then the ring (packed weights of a stage, its x), over which the sums go in the end.
+constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kRing = 1024;
+constexpr int kSmem = 227 * 1024;
+constexpr int kSumStride = 132;                     // floats from one token's 128 channels to the next
+
+struct FewParams {
+  const uint8_t *w[2];
+  const uint8_t *x;
+  const uint16_t *add;
+  size_t add_row_stride;     // datums from one tile row of the addend to the next; 0 when the addend is one row
+  void *out;
+  int *error;
+  float alpha;
+  int M, KT, TC, epi, out_fp32;
+  int splits;                // CTAs of a cluster, which share a sub-panel
+  int stages, bufs;          // of the ring, and of expanded weights in tensor memory
+  int tokens;                // rows of x in sixteens: the MMAs' N
+  int weights_early;         // the launch before this one does not write weights
+};
+
+// Shared-memory descriptor of x: K-major rows of 32 bytes, 32-byte swizzle, 8-row groups 256 bytes apart.
+__device__ __forceinline__ uint64_t x_desc(uint32_t addr) { return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) | (6ull << 61); }
+
+template <int FMT, bool PAIR>
+__global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_constant__ FewParams p) {
+  constexpr int TB = tile_bytes(FMT), MATS = PAIR ? 2 : 1, W_STAGE = MATS * kRows * kPanel * TB, BUF = MATS * kRows * 16;   // BUF: tensor-memory columns of a stage's weights
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t sb = smem_u32(smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = p.splits > 1 ? (int)cluster_ctarank() : 0, panel = blockIdx.x / p.splits;
+  const int k0 = p.KT * rank / p.splits, kn = p.KT * (rank + 1) / p.splits - k0, steps = (kn + kRows - 1) / kRows;   // this CTA's tile rows
+  const int width = min(kPanel, p.TC - panel * kPanel), N = p.tokens, stages = p.stages, bufs = p.bufs;
+  const int x_row = N * 64, w_stage = W_STAGE, stage_bytes = W_STAGE + kRows * x_row;
+  auto wait = [&](uint32_t bar, uint32_t parity, int code) {
+    if (!mbar_wait(bar, parity, kLimit)) atomicExch(p.error, code);
+  };
+  if (warp == 0) {                                  // a lane to a place of the rings
+    if (lane < kMaxStages) {
+      mbar_init(sb + kWFull + 8 * lane, 1), mbar_init(sb + kWEmpty + 8 * lane, kGroupWarps);
+      mbar_init(sb + kXFull + 8 * lane, kXWarps), mbar_init(sb + kXEmpty + 8 * lane, 1);
+    }
+    if (lane < kMaxBufs) mbar_init(sb + kReady + 8 * lane, kGroupWarps), mbar_init(sb + kFree + 8 * lane, 1);
+    if (lane == 0) mbar_init(sb + kDone, 1);
+    mbar_fence_init();
+  }
+  if (warp == kMmaWarp) tmem_alloc(sb + kTmem, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  // All of that, and the first weights where the launch before writes none, may happen while that launch drains. x, the addend and
+  // the result wait.
+  auto in_turn = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
+  if (!p.weights_early) in_turn();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + kTmem), weights0 = tmem + 512 - bufs * BUF;
+
+  // Every role is one warp's chain of dependent instructions, about 5 cycles each, so what is worked out per stage counts: places in
+  // the ring go round by themselves (divisions by a number of stages known only at run time took 400 cycles of 2400 a stage).
+  struct Turn {                                      // of a ring of n: the place, and the parity of its round
+    int at = 0;
+    uint32_t parity = 0;
+    __device__ __forceinline__ void next(int n) {
+      if (++at == n) at = 0, parity ^= 1;
+    }
+  };
+  if (warp == kWeightWarp) {
+    const uint8_t *from = p.w[lane < MATS ? lane : 0] + ((size_t)panel * kPanel * p.KT + (size_t)k0 * width) * TB;
+    const uint32_t stage = kRows * width * TB;
+    Turn t;
+    for (int i = 0; i < steps; i++, t.next(stages), from += stage) {
+      if (i >= stages) wait(sb + kWEmpty + 8 * t.at, t.parity ^ 1, 21);
+      const uint32_t bytes = min(kRows, kn - i * kRows) * width * TB, bar = sb + kWFull + 8 * t.at;
+      if (lane == 0) mbar_expect_tx(bar, MATS * bytes);
+      __syncwarp();
+      if (lane < MATS) bulk_g2s(sb + kRing + t.at * stage_bytes + lane * (kRows * kPanel * TB), from, bytes, bar);
+    }
+  } else if (warp == kMmaWarp) {
+    {
+      const uint32_t leader = elect_one();
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+      const uint64_t x0 = x_desc(sb + kRing + w_stage);
+      const uint32_t row = x_row >> 4, half = N * 2, stage = stage_bytes >> 4;   // descriptors count 16 bytes
+      auto mmas = [&](uint64_t x, uint32_t a, int r, uint32_t more) {
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+          for (int m = 0; m < MATS; m++) umma_bf16_ts(tmem + m * N, a + m * (kRows * 16) + r * 16 + h * 8, x + h * half, idesc, h ? 1u : more, leader);
+      };
+      Turn t, u;
+      for (int i = 0; i < steps; i++, t.next(stages), u.next(bufs)) {
+        const int n = min(kRows, kn - i * kRows);
+        wait(sb + kXFull + 8 * t.at, t.parity, 22);
+        wait(sb + kReady + 8 * u.at, u.parity, 23);
+        tc_fence_after();
+        const uint64_t x = x0 + t.at * stage;
+        const uint32_t a = weights0 + u.at * BUF;
+        mmas(x, a, 0, i != 0);
+        if (n == kRows) {
+#pragma unroll
+          for (int r = 1; r < kRows; r++) mmas(x + r * row, a, r, 1u);
+        } else
+          for (int r = 1; r < n; r++) mmas(x + r * row, a, r, 1u);
+        umma_commit_if(sb + kXEmpty + 8 * t.at, leader);
+        umma_commit_if(sb + kFree + 8 * u.at, leader);
+      }
+      umma_commit_if(sb + kDone, leader);
+    }
+  } else if (warp >= kXWarp) {
+    in_turn();
+    const int me = warp - kXWarp;
+    const uint32_t place = (lane >> 1) * 32 + (((lane & 1) ^ (lane >> 3 & 1)) << 4);
+    Turn t, seen;
+    auto landed = [&] {                              // everything this lane copied for the stage is there, and the tensor core may look
+      fence_async_shared();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(sb + kXFull + 8 * seen.at);
+      seen.next(stages);
+    };
+    // a warp copies its tile row of the stage. A stage is reported when the two after it have been asked for, as far as there is
+    // room for them, and the first one when the next has: everything waits for that one
+    const uint8_t *from = p.x + ((size_t)k0 + me) * 2048 + lane * 16;
+    const bool ahead = stages > 3;
+    for (int i = 0; i < steps; i++, t.next(stages), from += kRows * 2048) {
+      if (i >= stages) wait(sb + kXEmpty + 8 * t.at, t.parity ^ 1, 24);
+      if (me < kn - i * kRows) {
+        uint32_t to = sb + kRing + t.at * stage_bytes + w_stage + place + me * x_row;
+        const uint8_t *src = from;
+        for (int tb = 0; tb < N / 16; tb += 2, to += 1024, src += (size_t)p.KT * 2048) {
+          cp_async16(to, src), cp_async16(to + N * 32, src + 512);
+          if (tb + 1 < N / 16) cp_async16(to + 512, src + 1024), cp_async16(to + N * 32 + 512, src + 1536);
+        }
+      }
+      cp_async_commit();
+      if (!ahead || i == 1) {
+        if (i >= 1) cp_async_wait<1>(), landed();
+      } else if (i >= 3) cp_async_wait<2>(), landed();
+    }
+    cp_async_wait<0>();
+    landed();
+    if (ahead && steps > 2) landed();
+  } else {
+    const int cc = warp & 3, group = warp / kGroupWarps, row = warp % kGroupWarps >> 2;
+    const uint32_t lanes = (uint32_t)(32 * cc) << 16, tile0 = sb + kRing + (row * width + cc) * TB, a0 = weights0 + lanes + row * 16;
+    Turn t, u;
+    for (int i = 0; i < group; i++) t.next(stages), u.next(bufs);
+    for (int i = group; i < steps; i += kGroups) {
+      wait(sb + kWFull + 8 * t.at, t.parity, 25);
+      if (i >= bufs) wait(sb + kFree + 8 * u.at, u.parity ^ 1, 26);
+      tc_fence_after();
+      if (cc < width) {
+#pragma unroll
+        for (int r = 0; r < kRows; r += kGroupWarps / 4)
+#pragma unroll
+          for (int m = 0; m < MATS; m++) {           // (rows past a last stage: what lies there, which no MMA takes)
+            uint32_t a[2][2][4];
+            expand_weights<FMT>(packed_lane<FMT>(tile0 + t.at * stage_bytes + m * (kRows * kPanel * TB) + r * width * TB, lane), a);
+            // a lane's two pairs of k are two neighbouring 32-bit columns of rows g and g + 8
+#pragma unroll
+            for (int fs = 0; fs < 2; fs++) {
+              const uint32_t v[8] = {a[0][fs][0], a[0][fs][2], a[0][fs][1], a[0][fs][3], a[1][fs][0], a[1][fs][2], a[1][fs][1], a[1][fs][3]};
+              tmem_st_16x256b(a0 + ((uint32_t)(16 * fs) << 16) + u.at * BUF + m * (kRows * 16) + r * 16, v);
+            }
+          }
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(sb + kWEmpty + 8 * t.at), mbar_arrive(sb + kReady + 8 * u.at);
+      for (int g = 0; g < kGroups; g++) t.next(stages), u.next(bufs);
+    }
+    wait(sb + kDone, 0, 27);
+    tc_fence_after();
+    // the sums go over the ring: every stage has been used
+    const int t0 = 32 * (warp >> 2), ch = 32 * cc + (lane & 16) + 2 * (lane & 7) + (lane >> 3 & 1);
+    if (t0 < p.M) {
+#pragma unroll
+      for (int m = 0; m < MATS; m++) {
+        uint32_t v[32];
+        tmem_ld(tmem + lanes + m * N + t0, v);
+        tmem_ld_wait();
+        float *to = reinterpret_cast<float *>(smem + kRing) + (m * p.M + t0) * kSumStride + ch;
+#pragma unroll
+        for (int j = 0; j < 32; j++)
+          if (t0 + j < p.M) to[j * kSumStride] = __uint_as_float(v[j]);
+      }
+    }
+  }
+  in_turn();
+  __syncwarp();
+  tc_fence_before();
+  if (p.splits > 1) cluster_sync();
+  else __syncthreads();
+  tc_fence_after();
+  if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
+  // a warp to a row of 128 channels, a lane to four of them
+  const int tile_rows = (p.M + 31) / 32, first = tile_rows * 32 * rank / p.splits, end = tile_rows * 32 * (rank + 1) / p.splits;
+  const int tcol = panel * kPanel + (lane >> 3), in_face = (lane & 4) * 64 + (lane & 3) * 4;   // datum of the lane's first channel in a tile's row 0
+  if (lane >> 3 < width) {
+    const float unscale = kExpandedUnscale * p.alpha;
+    for (int row = first + warp; row < end; row += kThreads / 32) {
+      float f[4] = {0.f, 0.f, 0.f, 0.f}, g[4] = {0.f, 0.f, 0.f, 0.f};
+      const int tr = row >> 5, at = in_face + (row >> 4 & 1) * 512 + (row & 15) * 16;
+      if (row < p.M) {
+        uint2 a = make_uint2(0, 0);
+        if (p.add) a = __ldcg(reinterpret_cast<const uint2 *>(p.add + (size_t)tr * p.add_row_stride + (size_t)tcol * 1024 + (p.add_row_stride ? at : in_face)));
+        const float *own = reinterpret_cast<const float *>(smem + kRing) + row * kSumStride + lane * 4;
+        for (int c = 0; c < p.splits; c += 4) {      // of up to four CTAs in flight together; the way between SMs is narrow, so not this one's own
+          float4 v[4], u[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            v[j] = u[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (c + j == rank) {
+              v[j] = *reinterpret_cast<const float4 *>(own);
+              if (PAIR) u[j] = *reinterpret_cast<const float4 *>(own + p.M * kSumStride);
+            } else if (c + j < p.splits) {
+              const uint32_t from = map_to_cta(smem_u32(own), c + j);
+              v[j] = ld_cluster4(from);
+              if (PAIR) u[j] = ld_cluster4(from + p.M * kSumStride * 4);
+            }
+          }
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            f[0] += v[j].x, f[1] += v[j].y, f[2] += v[j].z, f[3] += v[j].w;
+            if (PAIR) g[0] += u[j].x, g[1] += u[j].y, g[2] += u[j].z, g[3] += u[j].w;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint32_t w = k < 2 ? a.x : a.y;
+          float y = f[k] * unscale;
+          if (p.add) y += __uint_as_float(k % 2 ? w & 0xFFFF0000u : w << 16);
+          if (PAIR) y = silu(y) * (g[k] * unscale);
+          else if (p.epi == BT_EPI_RELU) y = fmaxf(y, 0.f);
+          else if (p.epi == BT_EPI_SILU) y = silu(y);
+          f[k] = y;
+        }
+      }
+      const size_t o = ((size_t)tr * p.TC + tcol) * 1024 + at;
+      if (p.out_fp32) *reinterpret_cast<float4 *>(static_cast<float *>(p.out) + o) = make_float4(f[0], f[1], f[2], f[3]);
+      else *reinterpret_cast<uint2 *>(static_cast<uint16_t *>(p.out) + o) = make_uint2(bf16_half_up(f[0]) | bf16_half_up(f[1]) << 16, bf16_half_up(f[2]) | bf16_half_up(f[3]) << 16);
+    }
+  }
+  __syncwarp();
+  if (p.splits > 1) cluster_sync();                // nobody leaves while others read its sums
+}
+
+constexpr float kFixedUs = 4.f, kTileUs = 0.0125f;   // a wave's start and end; an SM's time for a packed tile
+
+}  // namespace
+
+int gemm_few(int device, int fmt, int epilogue, int M, int K, int N, uint64_t x, uint64_t w, uint64_t w2, uint64_t add, int add_rows, float alpha, uint64_t out,
+             int out_dtype, uint64_t work, uint64_t stream) {
+  const bool pair = epilogue == BT_EPI_GLU;
+  FewParams p{};
+  p.w[0] = as_ptr<uint8_t>(w), p.w[1] = as_ptr<uint8_t>(w2), p.x = as_ptr<uint8_t>(x), p.add = as_ptr<uint16_t>(add), p.out = as_ptr<void>(out), p.error = as_ptr<int>(work);
+  p.alpha = alpha, p.M = M, p.KT = K / 32, p.TC = (N + 31) / 32, p.epi = epilogue, p.out_fp32 = out_dtype == BT_FP32;
+  p.add_row_stride = add && add_rows > 1 ? (size_t)p.TC * 1024 : 0;
+  p.tokens = (M + 15) / 16 * 16;
+  const int mats = pair ? 2 : 1, stage = kRows * (mats * kPanel * tile_bytes(fmt) + p.tokens * 64);
+  p.stages = std::min(kMaxStages, (kSmem - kRing) / stage), p.bufs = std::min(kMaxBufs, (512 - mats * p.tokens) / (mats * kRows * 16));
+  p.weights_early = follows_matmul(stream);
+
+  using Kernel = void (*)(FewParams);
+  static const Kernel kernels[2][2] = {{few_rows_kernel<BT_BFP8, false>, few_rows_kernel<BT_BFP8, true>}, {few_rows_kernel<BT_BFP4, false>, few_rows_kernel<BT_BFP4, true>}};
+  const Kernel kernel = kernels[fmt == BT_BFP4][pair];
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(kThreads), cfg.dynamicSmemBytes = kSmem, cfg.stream = as_stream(stream), cfg.attrs = attr;
+  // how many clusters of each size fit on the GPU at once: all four kernels take the same room
+  static int clusters[64][kMaxSplits + 1] = {};
+  int *fit = clusters[device & 63];
+  if (!fit[1]) {
+    for (int k = 0; k < 4; k++) BT_CUDA(cudaFuncSetAttribute(kernels[k / 2][k % 2], cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+    for (int s = kMaxSplits; s >= 1; s--) {
+      int n = 0;
+      attr[1].val.clusterDim.x = s, cfg.gridDim = dim3(s), cfg.numAttrs = 2;
+      BT_CUDA(cudaOccupancyMaxActiveClusters(&n, kernels[0][0], &cfg));
+      fit[s] = std::max(n, 1);
+    }
+  }
+  // The split with the least estimated time: waves of CTAs, each with its start and end and its tiles. As many CTAs as fit at once, in
+  // short: 77 rows of 2048 x 5632 (44 sub-panels, pair) 16.9, 12.7, 12.5, 21 us in 1, 2, 3 and 4 parts, 5632 x 2048 (16)
+  // 15.5, 10.4, 10.3, 16.3 in 2, 4, 6 and 8.
+  const int panels = (p.TC + kPanel - 1) / kPanel;
+  float best = 1e30f;
+  for (int s = 1; s <= std::min(kMaxSplits, p.KT); s++) {
+    const int waves = (panels + fit[s] - 1) / fit[s];
+    const float us = waves * (kFixedUs + (p.KT + s - 1) / s * kPanel * mats * kTileUs) + (s > 1 ? 0.5f + 0.1f * s : 0.f);
+    if (us < best) best = us, p.splits = s;
+  }
+  cfg.gridDim = dim3(panels * p.splits), attr[1].val.clusterDim.x = p.splits, cfg.numAttrs = p.splits > 1 ? 2 : 1;
+  BT_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+  return launched("few_rows_kernel");
+}
+
+}  // namespace bt

@@ -1306,9 +1306,10 @@ int make_maps(GemvParams &p, uint64_t x) {
   return BT_OK;
 }
 
-// Whether the last thing this library queued, on any stream, before the current entry-point call was a matmul launch
-// on `stream`; and the note that one is being queued now. Entry points stamp g_calls when they select their device.
-bool follows_matmul(uint64_t stream) {
+}  // namespace
+
+// Entry points stamp g_calls when they select their device.
+bool bt::follows_matmul(uint64_t stream) {
   static std::mutex lock;
   static struct { uint64_t stream, stamp; } last[64] = {};
   std::lock_guard<std::mutex> hold(lock);
@@ -1323,6 +1324,8 @@ bool follows_matmul(uint64_t stream) {
   last[slot].stream = stream, last[slot].stamp = now;
   return yes;
 }
+
+namespace {
 
 // Argument checks and the launches shared by the entry points. `scratch` carries the scratch pointers.
 int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const QueueHead &scratch, uint64_t stream) {

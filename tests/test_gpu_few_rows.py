@@ -1,0 +1,68 @@
+"""The tensor-core matmul for 33 to 128 rows (weights expanded into tensor memory): edges of its token groups, of sub-panels of
+fewer than four tile columns, of stages and of the clusters that share K, against the oracle's dequantised weights."""
+import numpy as np
+import pytest
+from oracle import bfp_oracle as o
+from helpers import acts, bf16, check_matmul, upload, weights
+from test_gpu_prefill import run
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+@pytest.mark.parametrize("m,k,n", [(33, 32, 32), (48, 64, 96), (49, 96, 128), (64, 128, 160), (65, 160, 320), (80, 1120, 64), (96, 288, 544), (97, 2048, 256),
+                                   (112, 4128, 416), (113, 544, 1504), (127, 256, 2400), (128, 992, 4896), (128, 352, 9600), (129, 352, 544)])
+def test_edges(rt, fmt, m, k, n):
+  # small integers are exact in both formats and in fp32 sums, whatever the order: any misplaced row, column or k shows up. 129 rows
+  # take the other kernel
+  rng = np.random.default_rng(m * 131 + k + n)
+  xi, wi, vi = rng.integers(-2, 3, (m, k)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32)
+  add = rng.integers(-9, 10, (m, n)).astype(np.float32)
+  got, _ = run(rt, xi, wi, fmt, dtype="fp32")
+  assert np.array_equal(got, xi @ wi)
+  got, _ = run(rt, xi, wi, fmt, "relu", add=add, alpha=0.5, dtype="fp32")
+  assert np.array_equal(got, np.maximum((xi @ wi) * 0.5 + add, 0))
+  got, ref = run(rt, xi, wi, fmt, "glu", vi, dtype="fp32")
+  check_matmul(got, xi, None, ref, 1e-4)
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+@pytest.mark.parametrize("m", [40, 128])
+def test_same_bits_every_time(rt, fmt, m):
+  # sums of parts of K are added in order: a result does not depend on timing, nor on what ran before it
+  rng = np.random.default_rng(m)
+  x, w, w2 = acts(rng, m, 1536), weights(rng, 1536, 640), weights(rng, 1536, 640)
+  tx, tw, tw2 = upload(rt, x), upload(rt, w).cast(fmt).columns(), upload(rt, w2).cast(fmt).columns()
+  first = ((tx @ tw).silu() * (tx @ tw2)).numpy()
+  for _ in range(20):
+    ys = [((tx @ tw).silu() * (tx @ tw2)).realize() for _ in range(3)]
+    assert all(np.array_equal(y.numpy(), first) for y in ys)
+  assert o.rel_err(first, o.silu(x @ o.dequant(w, fmt)) * (x @ o.dequant(w2, fmt))) <= 1e-2
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+def test_fp32_sums_are_no_further_from_64_bits(rt, fmt):
+  # fp32 accumulation over K = 4096: an error of the sums of products within that of adding them one after the other,
+  # K * 2^-24 of the sum of magnitudes (a bound; what is seen is a hundredth of it)
+  rng = np.random.default_rng(11)
+  x, w = acts(rng, 100, 4096), weights(rng, 4096, 256)
+  got, _ = run(rt, x, w, fmt, dtype="fp32")
+  wd = o.dequant(w, fmt).astype(np.float64)
+  assert (np.abs(got - x.astype(np.float64) @ wd) <= 4096 * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(wd))).all()
+
+
+def test_chain_and_recording(rt):
+  # a gate/up pair and the matmul on its result back to back, live and replayed, between decode matmuls that read and write the same tensors
+  rng = np.random.default_rng(3)
+  x = upload(rt, acts(rng, 77, 512))
+  wg, wu, wd = (upload(rt, weights(rng, *s)).cast("bfp8").columns() for s in ((512, 1408), (512, 1408), (1408, 512)))
+  def mlp(x): return (((((x @ wg).silu() * (x @ wu)).realize() @ wd) + x).realize())
+  want = mlp(mlp(x)).numpy()
+  held = []
+  with rt.record() as step:
+    held.append(mlp(x)), held.append(mlp(held[-1]))
+  for _ in range(3):
+    step.replay()
+    rt.wait()
+    assert np.array_equal(held[-1].numpy(), want)
+  step.close()
