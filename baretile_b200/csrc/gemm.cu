@@ -428,7 +428,7 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
 }
 
 // Up to so many rows gemm_few.cu is the faster one (its sums of 128 tokens of a pair and the expanded weights fill tensor memory): 128 rows of
-// 4096 x 14336, gate/up and down, 58 us against 120, 33 rows 47 against 113.
+// 4096 x 14336, gate/up and down, 55 us against 120, 33 rows 44 against 113.
 constexpr int kFewRows = 128;
 
 }  // namespace

@@ -18,9 +18,9 @@
 //   warp 16      copies the packed tiles (a bulk copy per matrix)
 //   warp 17      issues the MMAs (128 channels x tokens x 16 each); a commit frees x and the tensor memory of the stage
 //   warps 18-21  copy x, a tile row each: 16 tokens x 16 k of a tile are 512 consecutive bytes, a warp's one cp.async, which lands
-//                in the 32-byte swizzle
+//                in the 32-byte swizzle, and tells the stage's barrier itself when it has (warps that waited for their copies: 128 rows 58 us against 55)
 // Gate/up pair and down projection, against the kernel of gemm.cu with its x laid out by rows and its parts of K added up by another launch:
-// 77 rows of 2048 x 5632 (bfp4, bfp8) 43.7 -> 22.5 us, 33 rows of 512 x 1024 23.8 -> 11.1, 33 rows of 4096 x 14336 113 -> 47, 128 rows 120 -> 58.
+// 77 rows of 2048 x 5632 (bfp4, bfp8) 43.7 -> 22.1 us, 33 rows of 512 x 1024 23.8 -> 10.6, 33 rows of 4096 x 14336 113 -> 44, 128 rows 120 -> 55.
 // A launch costs 5 to 10 us beside its stages: setting up and the first weights and x 3, the sums' way through the cluster and the epilogue 3.
 // Every wait is bounded and reports through the error word.
 #include "common.cuh"
@@ -38,7 +38,7 @@ constexpr int kMaxStages = 8, kMaxBufs = 4, kMaxSplits = 8;
 constexpr uint32_t kLimit = 1u << 14;               // attempts of up to 100 us each
 
 // Shared memory: mbarriers, then the ring (packed weights of a stage, its x), over which the sums go in the end.
-constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kRing = 1024;
+constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kAllocated = 336, kRing = 1024;
 constexpr int kSmem = 227 * 1024;
 constexpr int kSumStride = 132;                     // floats from one token's 128 channels to the next
 
@@ -76,22 +76,18 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   if (warp == 0) {                                  // a lane to a place of the rings
     if (lane < kMaxStages) {
       mbar_init(sb + kWFull + 8 * lane, 1), mbar_init(sb + kWEmpty + 8 * lane, kGroupWarps);
-      mbar_init(sb + kXFull + 8 * lane, kXWarps), mbar_init(sb + kXEmpty + 8 * lane, 1);
+      mbar_init(sb + kXFull + 8 * lane, kXWarps * 32), mbar_init(sb + kXEmpty + 8 * lane, 1);
     }
     if (lane < kMaxBufs) mbar_init(sb + kReady + 8 * lane, kGroupWarps), mbar_init(sb + kFree + 8 * lane, 1);
-    if (lane == 0) mbar_init(sb + kDone, 1);
+    if (lane == 0) mbar_init(sb + kDone, 1), mbar_init(sb + kAllocated, 1);
     mbar_fence_init();
   }
-  if (warp == kMmaWarp) tmem_alloc(sb + kTmem, 512);
-  tc_fence_before();
   __syncthreads();
-  tc_fence_after();
   // All of that, and the first weights where the launch before writes none, may happen while that launch drains. x, the addend and
   // the result wait.
   auto in_turn = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
   if (!p.weights_early) in_turn();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + kTmem), weights0 = tmem + 512 - bufs * BUF;
 
   // Every role is one warp's chain of dependent instructions, about 5 cycles each, so what is worked out per stage counts: places in
   // the ring go round by themselves (divisions by a number of stages known only at run time took 400 cycles of 2400 a stage).
@@ -115,7 +111,11 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     }
   } else if (warp == kMmaWarp) {
     {
-      const uint32_t leader = elect_one();
+      // the copies need not wait for tensor memory
+      tmem_alloc(sb + kTmem, 512);
+      tc_fence_before();
+      mbar_arrive_if(sb + kAllocated, lane == 0);
+      const uint32_t tmem = lds32(sb + kTmem), weights0 = tmem + 512 - bufs * BUF, leader = elect_one();
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       const uint64_t x0 = x_desc(sb + kRing + w_stage);
       const uint32_t row = x_row >> 4, half = N * 2, stage = stage_bytes >> 4;   // descriptors count 16 bytes
@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
         const int n = min(kRows, kn - i * kRows);
         wait(sb + kXFull + 8 * t.at, t.parity, 22);
         wait(sb + kReady + 8 * u.at, u.parity, 23);
+        fence_async_shared();                        // x came with copies of the generic proxy
         tc_fence_after();
         const uint64_t x = x0 + t.at * stage;
         const uint32_t a = weights0 + u.at * BUF;
@@ -148,17 +149,9 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     in_turn();
     const int me = warp - kXWarp;
     const uint32_t place = (lane >> 1) * 32 + (((lane & 1) ^ (lane >> 3 & 1)) << 4);
-    Turn t, seen;
-    auto landed = [&] {                              // everything this lane copied for the stage is there, and the tensor core may look
-      fence_async_shared();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(sb + kXFull + 8 * seen.at);
-      seen.next(stages);
-    };
-    // a warp copies its tile row of the stage. A stage is reported when the two after it have been asked for, as far as there is
-    // room for them, and the first one when the next has: everything waits for that one
+    Turn t;
+    // a warp copies its tile row of the stage, whose barrier hears from every lane when its copies have landed
     const uint8_t *from = p.x + ((size_t)k0 + me) * 2048 + lane * 16;
-    const bool ahead = stages > 3;
     for (int i = 0; i < steps; i++, t.next(stages), from += kRows * 2048) {
       if (i >= stages) wait(sb + kXEmpty + 8 * t.at, t.parity ^ 1, 24);
       if (me < kn - i * kRows) {
@@ -169,17 +162,15 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
           if (tb + 1 < N / 16) cp_async16(to + 512, src + 1024), cp_async16(to + N * 32 + 512, src + 1536);
         }
       }
-      cp_async_commit();
-      if (!ahead || i == 1) {
-        if (i >= 1) cp_async_wait<1>(), landed();
-      } else if (i >= 3) cp_async_wait<2>(), landed();
+      cp_async_arrive(sb + kXFull + 8 * t.at);
     }
-    cp_async_wait<0>();
-    landed();
-    if (ahead && steps > 2) landed();
+    cp_async_wait_all();
   } else {
     const int cc = warp & 3, group = warp / kGroupWarps, row = warp % kGroupWarps >> 2;
-    const uint32_t lanes = (uint32_t)(32 * cc) << 16, tile0 = sb + kRing + (row * width + cc) * TB, a0 = weights0 + lanes + row * 16;
+    wait(sb + kAllocated, 0, 28);
+    __syncwarp();
+    tc_fence_after();
+    const uint32_t tmem = lds32(sb + kTmem), weights0 = tmem + 512 - bufs * BUF, lanes = (uint32_t)(32 * cc) << 16, tile0 = sb + kRing + (row * width + cc) * TB, a0 = weights0 + lanes + row * 16;
     Turn t, u;
     for (int i = 0; i < group; i++) t.next(stages), u.next(bufs);
     for (int i = group; i < steps; i += kGroups) {
@@ -230,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   if (p.splits > 1) cluster_sync();
   else __syncthreads();
   tc_fence_after();
-  if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
+  if (warp == kMmaWarp) tmem_dealloc(lds32(sb + kTmem), 512);
   // a warp to a row of 128 channels, a lane to four of them
   const int tile_rows = (p.M + 31) / 32, first = tile_rows * 32 * rank / p.splits, end = tile_rows * 32 * (rank + 1) / p.splits;
   const int tcol = panel * kPanel + (lane >> 3), in_face = (lane & 4) * 64 + (lane & 3) * 4;   // datum of the lane's first channel in a tile's row 0
