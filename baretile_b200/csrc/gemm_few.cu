@@ -38,7 +38,7 @@ constexpr int kMaxStages = 8, kMaxBufs = 4, kMaxSplits = 8;
 constexpr uint32_t kLimit = 1u << 14;               // attempts of up to 100 us each
 
 // Shared memory: mbarriers, then the ring (packed weights of a stage, its x), over which the sums go in the end.
-constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kAllocated = 336, kRing = 1024;
+constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kRing = 1024;
 constexpr int kSmem = 227 * 1024;
 constexpr int kSumStride = 132;                     // floats from one token's 128 channels to the next
 
@@ -72,6 +72,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   const int x_row = N * 64, w_stage = W_STAGE, stage_bytes = W_STAGE + kRows * x_row;
   auto wait = [&](uint32_t bar, uint32_t parity, int code) {
     if (!mbar_wait(bar, parity, kLimit)) atomicExch(p.error, code);
+    __syncwarp();                                   // whole warps wait, and the tensor-memory instructions that follow want them in step
   };
   if (warp == 0) {                                  // a lane to a place of the rings
     if (lane < kMaxStages) {
@@ -79,15 +80,19 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
       mbar_init(sb + kXFull + 8 * lane, kXWarps * 32), mbar_init(sb + kXEmpty + 8 * lane, 1);
     }
     if (lane < kMaxBufs) mbar_init(sb + kReady + 8 * lane, kGroupWarps), mbar_init(sb + kFree + 8 * lane, 1);
-    if (lane == 0) mbar_init(sb + kDone, 1), mbar_init(sb + kAllocated, 1);
+    if (lane == 0) mbar_init(sb + kDone, 1);
     mbar_fence_init();
   }
-  __syncthreads();
+  if (warp == kMmaWarp) tmem_alloc(sb + kTmem, 512);
+  tc_fence_before();
+  __syncthreads();                                  // the barriers are set up, and the allocation's answer is there for everyone, the warp that asked included
+  tc_fence_after();
   // All of that, and the first weights where the launch before writes none, may happen while that launch drains. x, the addend and
   // the result wait.
   auto in_turn = [] { asm volatile("griddepcontrol.wait;" ::: "memory"); };
   if (!p.weights_early) in_turn();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + kTmem), weights0 = tmem + 512 - bufs * BUF;
 
   // Every role is one warp's chain of dependent instructions, about 5 cycles each, so what is worked out per stage counts: places in
   // the ring go round by themselves (divisions by a number of stages known only at run time took 400 cycles of 2400 a stage).
@@ -111,11 +116,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     }
   } else if (warp == kMmaWarp) {
     {
-      // the copies need not wait for tensor memory
-      tmem_alloc(sb + kTmem, 512);
-      tc_fence_before();
-      mbar_arrive_if(sb + kAllocated, lane == 0);
-      const uint32_t tmem = lds32(sb + kTmem), weights0 = tmem + 512 - bufs * BUF, leader = elect_one();
+      const uint32_t leader = elect_one();
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
       const uint64_t x0 = x_desc(sb + kRing + w_stage);
       const uint32_t row = x_row >> 4, half = N * 2, stage = stage_bytes >> 4;   // descriptors count 16 bytes
@@ -167,23 +168,20 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     cp_async_wait_all();
   } else {
     const int cc = warp & 3, group = warp / kGroupWarps, row = warp % kGroupWarps >> 2;
-    wait(sb + kAllocated, 0, 28);
-    __syncwarp();
-    tc_fence_after();
-    const uint32_t tmem = lds32(sb + kTmem), weights0 = tmem + 512 - bufs * BUF, lanes = (uint32_t)(32 * cc) << 16, tile0 = sb + kRing + (row * width + cc) * TB, a0 = weights0 + lanes + row * 16;
+    const uint32_t lanes = (uint32_t)(32 * cc) << 16, tile0 = sb + kRing + (row * width + cc) * TB, a0 = weights0 + lanes + row * 16;
     Turn t, u;
     for (int i = 0; i < group; i++) t.next(stages), u.next(bufs);
     for (int i = group; i < steps; i += kGroups) {
       wait(sb + kWFull + 8 * t.at, t.parity, 25);
       if (i >= bufs) wait(sb + kFree + 8 * u.at, u.parity ^ 1, 26);
       tc_fence_after();
-      if (cc < width) {
+      {
 #pragma unroll
         for (int r = 0; r < kRows; r += kGroupWarps / 4)
 #pragma unroll
           for (int m = 0; m < MATS; m++) {           // (rows past a last stage: what lies there, which no MMA takes)
-            uint32_t a[2][2][4];
-            expand_weights<FMT>(packed_lane<FMT>(tile0 + t.at * stage_bytes + m * (kRows * kPanel * TB) + r * width * TB, lane), a);
+            uint32_t a[2][2][4] = {};                // of a column that the matrix does not have: zeros
+            if (cc < width) expand_weights<FMT>(packed_lane<FMT>(tile0 + t.at * stage_bytes + m * (kRows * kPanel * TB) + r * width * TB, lane), a);
             // a lane's two pairs of k are two neighbouring 32-bit columns of rows g and g + 8
 #pragma unroll
             for (int fs = 0; fs < 2; fs++) {
@@ -205,13 +203,17 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     if (t0 < p.M) {
 #pragma unroll
       for (int m = 0; m < MATS; m++) {
-        uint32_t v[32];
-        tmem_ld(tmem + lanes + m * N + t0, v);
-        tmem_ld_wait();
         float *to = reinterpret_cast<float *>(smem + kRing) + (m * p.M + t0) * kSumStride + ch;
 #pragma unroll
-        for (int j = 0; j < 32; j++)
-          if (t0 + j < p.M) to[j * kSumStride] = __uint_as_float(v[j]);
+        for (int c = 0; c < 32; c += 16)
+          if (t0 + c < N) {
+            uint32_t v[16];
+            tmem_ld(tmem + lanes + m * N + t0 + c, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; j++)
+              if (t0 + c + j < p.M) to[(c + j) * kSumStride] = __uint_as_float(v[j]);
+          }
       }
     }
   }
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   if (p.splits > 1) cluster_sync();
   else __syncthreads();
   tc_fence_after();
-  if (warp == kMmaWarp) tmem_dealloc(lds32(sb + kTmem), 512);
+  if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
   // a warp to a row of 128 channels, a lane to four of them
   const int tile_rows = (p.M + 31) / 32, first = tile_rows * 32 * rank / p.splits, end = tile_rows * 32 * (rank + 1) / p.splits;
   const int tcol = panel * kPanel + (lane >> 3), in_face = (lane & 4) * 64 + (lane & 3) * 4;   // datum of the lane's first channel in a tile's row 0
