@@ -32,12 +32,18 @@ namespace {
 
 constexpr int kRows = 4;                            // tile rows of a stage
 constexpr int kExpandWarps = 16, kWeightWarp = 16, kMmaWarp = 17, kXWarp = 18, kXWarps = kRows;
-constexpr int kGroups = 2, kGroupWarps = kExpandWarps / kGroups;   // groups of warps that take the stages in turn
+// Groups of warps that take the stages in turn. An mbarrier's parity tells a phase only from its neighbours, so whoever waits for one has to know that the
+// phase before is over. A place of the weights' ring therefore belongs to one group: the ring has a multiple of kGroups places. (With three, a group came to a
+// place where the other group's weights had not landed yet, and took the phase before that for its own: garbage, and in the end a launch
+// failure.) A buffer in tensor memory may go from group to group, up to 4 of them: its phases end in order, and a group has waited for one of the stages
+// before.
+constexpr int kGroups = 2, kGroupWarps = kExpandWarps / kGroups;
 constexpr int kThreads = (kXWarp + kXWarps) * 32;
 constexpr int kMaxStages = 8, kMaxBufs = 4, kMaxSplits = 8;
+static_assert(kMaxStages % kGroups == 0, "places of the ring belong to groups");
 constexpr uint32_t kLimit = 1u << 14;               // attempts of up to 100 us each
 
-// Shared memory: mbarriers, then the ring (packed weights of a stage, its x), over which the sums go in the end.
+// Shared memory: mbarriers, then the rings of packed weights and of x, over which the sums go in the end.
 constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kRing = 1024;
 constexpr int kSmem = 227 * 1024;
 constexpr int kSumStride = 132;                     // floats from one token's 128 channels to the next
@@ -52,7 +58,7 @@ struct FewParams {
   float alpha;
   int M, KT, TC, epi, out_fp32;
   int splits;                // CTAs of a cluster, which share a sub-panel
-  int stages, bufs;          // of the ring, and of expanded weights in tensor memory
+  int stages, x_stages, bufs;   // of the rings of packed weights and of x, and of expanded weights in tensor memory
   int tokens;                // rows of x in sixteens: the MMAs' N
   int weights_early;         // the launch before this one does not write weights
 };
@@ -68,8 +74,9 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = p.splits > 1 ? (int)cluster_ctarank() : 0, panel = blockIdx.x / p.splits;
   const int k0 = p.KT * rank / p.splits, kn = p.KT * (rank + 1) / p.splits - k0, steps = (kn + kRows - 1) / kRows;   // this CTA's tile rows
-  const int width = min(kPanel, p.TC - panel * kPanel), N = p.tokens, stages = p.stages, bufs = p.bufs;
-  const int x_row = N * 64, w_stage = W_STAGE, stage_bytes = W_STAGE + kRows * x_row;
+  const int width = min(kPanel, p.TC - panel * kPanel), N = p.tokens, stages = p.stages, x_stages = p.x_stages, bufs = p.bufs;
+  const int x_row = N * 64, x_stage = kRows * x_row;
+  const uint32_t x_ring = sb + kRing + stages * W_STAGE;
   auto wait = [&](uint32_t bar, uint32_t parity, int code) {
     if (!mbar_wait(bar, parity, kLimit)) atomicExch(p.error, code);
     __syncwarp();                                   // whole warps wait, and the tensor-memory instructions that follow want them in step
@@ -112,14 +119,14 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
       const uint32_t bytes = min(kRows, kn - i * kRows) * width * TB, bar = sb + kWFull + 8 * t.at;
       if (lane == 0) mbar_expect_tx(bar, MATS * bytes);
       __syncwarp();
-      if (lane < MATS) bulk_g2s(sb + kRing + t.at * stage_bytes + lane * (kRows * kPanel * TB), from, bytes, bar);
+      if (lane < MATS) bulk_g2s(sb + kRing + t.at * W_STAGE + lane * (kRows * kPanel * TB), from, bytes, bar);
     }
   } else if (warp == kMmaWarp) {
     {
       const uint32_t leader = elect_one();
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-      const uint64_t x0 = x_desc(sb + kRing + w_stage);
-      const uint32_t row = x_row >> 4, half = N * 2, stage = stage_bytes >> 4;   // descriptors count 16 bytes
+      const uint64_t x0 = x_desc(x_ring);
+      const uint32_t row = x_row >> 4, half = N * 2, stage = x_stage >> 4;   // descriptors count 16 bytes
       auto mmas = [&](uint64_t x, uint32_t a, int r, uint32_t more) {
 #pragma unroll
         for (int h = 0; h < 2; h++)
@@ -127,7 +134,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
           for (int m = 0; m < MATS; m++) umma_bf16_ts(tmem + m * N, a + m * (kRows * 16) + r * 16 + h * 8, x + h * half, idesc, h ? 1u : more, leader);
       };
       Turn t, u;
-      for (int i = 0; i < steps; i++, t.next(stages), u.next(bufs)) {
+      for (int i = 0; i < steps; i++, t.next(x_stages), u.next(bufs)) {
         const int n = min(kRows, kn - i * kRows);
         wait(sb + kXFull + 8 * t.at, t.parity, 22);
         wait(sb + kReady + 8 * u.at, u.parity, 23);
@@ -153,10 +160,10 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     Turn t;
     // a warp copies its tile row of the stage, whose barrier hears from every lane when its copies have landed
     const uint8_t *from = p.x + ((size_t)k0 + me) * 2048 + lane * 16;
-    for (int i = 0; i < steps; i++, t.next(stages), from += kRows * 2048) {
-      if (i >= stages) wait(sb + kXEmpty + 8 * t.at, t.parity ^ 1, 24);
+    for (int i = 0; i < steps; i++, t.next(x_stages), from += kRows * 2048) {
+      if (i >= x_stages) wait(sb + kXEmpty + 8 * t.at, t.parity ^ 1, 24);
       if (me < kn - i * kRows) {
-        uint32_t to = sb + kRing + t.at * stage_bytes + w_stage + place + me * x_row;
+        uint32_t to = x_ring + t.at * x_stage + place + me * x_row;
         const uint8_t *src = from;
         for (int tb = 0; tb < N / 16; tb += 2, to += 1024, src += (size_t)p.KT * 2048) {
           cp_async16(to, src), cp_async16(to + N * 32, src + 512);
@@ -181,7 +188,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
 #pragma unroll
           for (int m = 0; m < MATS; m++) {           // (rows past a last stage: what lies there, which no MMA takes)
             uint32_t a[2][2][4] = {};                // of a column that the matrix does not have: zeros
-            if (cc < width) expand_weights<FMT>(packed_lane<FMT>(tile0 + t.at * stage_bytes + m * (kRows * kPanel * TB) + r * width * TB, lane), a);
+            if (cc < width) expand_weights<FMT>(packed_lane<FMT>(tile0 + t.at * W_STAGE + m * (kRows * kPanel * TB) + r * width * TB, lane), a);
             // a lane's two pairs of k are two neighbouring 32-bit columns of rows g and g + 8
 #pragma unroll
             for (int fs = 0; fs < 2; fs++) {
@@ -288,8 +295,11 @@ int gemm_few(int device, int fmt, int epilogue, int M, int K, int N, uint64_t x,
   p.alpha = alpha, p.M = M, p.KT = K / 32, p.TC = (N + 31) / 32, p.epi = epilogue, p.out_fp32 = out_dtype == BT_FP32;
   p.add_row_stride = add && add_rows > 1 ? (size_t)p.TC * 1024 : 0;
   p.tokens = (M + 15) / 16 * 16;
-  const int mats = pair ? 2 : 1, stage = kRows * (mats * kPanel * tile_bytes(fmt) + p.tokens * 64);
-  p.stages = std::min(kMaxStages, (kSmem - kRing) / stage), p.bufs = std::min(kMaxBufs, (512 - mats * p.tokens) / (mats * kRows * 16));
+  const int mats = pair ? 2 : 1, w_stage = kRows * mats * kPanel * tile_bytes(fmt), x_stage = kRows * p.tokens * 64;
+  // as many places for x as leave four for the weights (128 tokens and a pair in bfp8: two)
+  for (p.x_stages = kMaxStages; p.x_stages > 2 && (kSmem - kRing - p.x_stages * x_stage) / w_stage < 4; p.x_stages--);
+  p.stages = std::min(kMaxStages, (kSmem - kRing - p.x_stages * x_stage) / w_stage) / kGroups * kGroups;
+  p.bufs = std::min(kMaxBufs, (512 - mats * p.tokens) / (mats * kRows * 16));
   p.weights_early = follows_matmul(stream);
 
   using Kernel = void (*)(FewParams);
