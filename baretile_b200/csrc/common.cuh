@@ -58,9 +58,9 @@ inline int launched(const char *name) {
 // Whether the last thing this library queued, on any stream, before the current entry-point call was a matmul launch on `stream`
 // (which writes no weights); and the note that one is being queued now (gemv.cu).
 bool follows_matmul(uint64_t stream);
-// The prefill matmul for 33 to 128 rows (gemm_few.cu); arguments as checked by bt_gemm_tiles.
+// The prefill matmul for few rows (gemm_few.cu); arguments as checked by bt_gemm_tiles. Runs, and says so, if it expects to take less than beat_us.
 int gemm_few(int device, int fmt, int epilogue, int M, int K, int N, uint64_t x, uint64_t w, uint64_t w2, uint64_t add, int add_rows, float alpha, uint64_t out,
-             int out_dtype, uint64_t work, uint64_t stream);
+             int out_dtype, float beat_us, bool *taken, uint64_t work, uint64_t stream);
 
 inline cudaStream_t as_stream(uint64_t s) { return reinterpret_cast<cudaStream_t>(s); }
 template <class T> inline T *as_ptr(uint64_t p) { return reinterpret_cast<T *>(p); }

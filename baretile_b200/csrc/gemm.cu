@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(256) reduce_kernel(const GemmParams p) {
 // gets in the way of the MMAs' operands (2048 rows 562 -> 665).
 bool two_groups(const GemmParams &p) { return p.half || p.M <= 256; }
 constexpr float kBlockUs = 0.42f, kFixedUs = 5.f, kReduceUs = 3.f, kPartBytesPerUs = 3e6f;
-int deal_blocks(GemmParams &p, int slots, size_t part_bytes) {
+int deal_blocks(GemmParams &p, int slots, size_t part_bytes, float *expected_us) {
   const int runs = (p.TC + kPanel - 1) / kPanel, columns = p.pair ? runs : (runs + 1) / 2, KB = (p.KT + 1) / 2, tile_rows = (p.M + 31) / 32;
   p.row_blocks = (p.M + 511) / 512, p.half = 0, p.splits = 1;
   const int blocks = p.row_blocks * columns;
@@ -349,6 +349,7 @@ int deal_blocks(GemmParams &p, int slots, size_t part_bytes) {
   if (blocks >= slots) {
     const int last = blocks % slots;
     if (last > 0 && 2 * last <= slots && p.M > 256) p.whole = blocks - last;
+    *expected_us = (p.whole < blocks ? blocks / slots + 0.5f : (float)((blocks + slots - 1) / slots)) * (kFixedUs + KB * kBlockUs * (p.M > 256 ? 2 : 1));
     return p.whole + 2 * (blocks - p.whole);
   }
   float best = 1e30f;
@@ -362,6 +363,7 @@ int deal_blocks(GemmParams &p, int slots, size_t part_bytes) {
       if (us < best) best = us, pairs = b * splits, p.half = half, p.splits = splits, p.row_blocks = rows, p.whole = b;
     }
   }
+  *expected_us = best;
   return pairs;
 }
 
@@ -393,7 +395,8 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
   p.part = as_ptr<float>(part), p.weights_early = weights_early;
   int sms = 0;
   BT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  const int pairs = deal_blocks(p, sms / 2 > 0 ? sms / 2 : 1, part_bytes);
+  float expected_us;
+  const int pairs = deal_blocks(p, sms / 2 > 0 ? sms / 2 : 1, part_bytes, &expected_us);
   using Kernel = void (*)(GemmParams, CUtensorMap);
   static const Kernel kernels[2][2][2] = {{{gemm_kernel<BT_BFP8, false, 1>, gemm_kernel<BT_BFP8, false, 2>}, {gemm_kernel<BT_BFP8, true, 1>, gemm_kernel<BT_BFP8, true, 2>}},
                                           {{gemm_kernel<BT_BFP4, false, 1>, gemm_kernel<BT_BFP4, false, 2>}, {gemm_kernel<BT_BFP4, true, 1>, gemm_kernel<BT_BFP4, true, 2>}}};
@@ -427,9 +430,17 @@ int gemm(const char *who, int device, int fmt, int epilogue, int M, int K, int N
   return launched("reduce_kernel");
 }
 
-// Up to so many rows gemm_few.cu is the faster one (its sums of 128 tokens of a pair and the expanded weights fill tensor memory): 128 rows of
-// 4096 x 14336, gate/up and down, 55 us against 120, 33 rows 44 against 113.
-constexpr int kFewRows = 128;
+// What this kernel is expected to take for x in tiles, laid out by rows first (2.5 us, and x read and written at 5 TB/s).
+int expected(int device, int epilogue, int M, int K, int N, size_t part_bytes, float *us) {
+  int sms = 0;
+  BT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  GemmParams p{};
+  p.M = M, p.KT = K / 32, p.TC = (N + 31) / 32, p.pair = epilogue == BT_EPI_GLU;
+  deal_blocks(p, sms / 2 > 0 ? sms / 2 : 1, part_bytes, us);
+  if (M <= 256) *us *= 1.1f;                      // one half of 256 rows at a time: a tenth slower than the estimate has it (128 rows of 4096 x 14336 120 us, not 108)
+  *us += 2.5f + 4.f * M * K / 5e6f;
+  return BT_OK;
+}
 
 }  // namespace
 
@@ -445,10 +456,17 @@ int bt_gemm_tiles(int device, int fmt, int epilogue, int M, int K, int N, uint64
   BT_REQUIRE(M >= 1 && K > 0 && K % 32 == 0, "bt_gemm_tiles: needs M >= 1 and K a positive multiple of 32: %d x %d", M, K);
   const size_t rows = ((size_t)M * K * 2 + 255) / 256 * 256;
   BT_REQUIRE(x && x % 16 == 0 && scratch && scratch % 256 == 0 && scratch_bytes >= rows, "bt_gemm_tiles: needs x and at least %zu bytes of 256-byte aligned scratch, got %zu", rows, scratch_bytes);
-  if (M > 32 && M <= kFewRows) {
+  // The kernel of gemm_few.cu where its estimate is the lower one by 8 % (what the estimates are good for). Gate/up and down together, this kernel and that one: 128 rows of 4096 x 14336 120 and 55 us, 640
+  // rows 287 and 228, 1024 rows 333 and 348, 2048 rows 569 and 695; 1024 rows of 2048 x 5632 104 and 89, 1400 rows 127 and 135; 2048 rows of
+  // 1024 x 3000 78 and 63. Blocks of 128 x 128 waste less of a last wave and need no parts of K in memory; blocks of 512 x 256 expand a weight a fourth as often.
+  if (M > 32) {
     if (int s = check("bt_gemm_tiles", fmt, epilogue, M, K, N, x, w, w2, add, add_rows, out, out_dtype, work)) return s;
     if (int s = use_device(device)) return s;
-    return gemm_few(device, fmt, epilogue, M, K, N, x, w, w2, add, add_rows, alpha, out, out_dtype, work, stream);
+    float us;
+    bool taken;
+    if (int s = expected(device, epilogue, M, K, N, scratch_bytes - rows, &us)) return s;
+    if (int s = gemm_few(device, fmt, epilogue, M, K, N, x, w, w2, add, add_rows, alpha, out, out_dtype, 0.92f * us, &taken, work, stream)) return s;
+    if (taken) return BT_OK;
   }
   if (int s = bt_untilize(device, 2, x, scratch, 1, M, K, stream)) return s;
   return gemm("bt_gemm_tiles", device, fmt, epilogue, M, K, N, scratch, w, w2, add, add_rows, alpha, out, out_dtype, scratch + rows, scratch_bytes - rows, true, work, stream);

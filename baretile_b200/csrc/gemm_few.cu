@@ -1,14 +1,14 @@
-// Prefill matmul for 33 to 128 token rows (a short prompt, a large speculative or decode batch): out = epilogue(alpha * x @ W + add),
+// Prefill matmul for prompts of up to some hundred rows (and longer ones on few columns; see bt_gemm_tiles): out = epilogue(alpha * x @ W + add),
 // W block-float in streaming layout, x in tiles as Tensor holds it.
 //
-// With so few rows every weight is used a few dozen times and the work is bound by the stream of packed weights: by
+// With few rows every weight is used a few dozen times and the work is bound by the stream of packed weights: by
 // HBM (an SM's share of it is a tile in 43 cycles in bfp8, 23 in bfp4), by their expansion (25 cycles a tile) and by what a launch
 // costs. MMAs with the rows of x as their M would be mostly padding, and expanded weights as a B operand would cross shared memory
 // twice (2 KB a tile each way, of 128 bytes a cycle). So the operands change places: the 128 output channels of a sub-panel are the MMA's M,
-// the tokens its N (only as many as there are, in sixteens), and the expanded weights go from registers to TENSOR MEMORY, from
+// the tokens its N (only as many as there are, in sixteens, up to 128), and the expanded weights go from registers to TENSOR MEMORY, from
 // where tcgen05.mma takes its A operand; a lane's registers are 16x256b store fragments as they come.
 //
-// A CTA has a sub-panel of 4 tile columns (of both matrices of a gate/up pair) and all rows; where sub-panels are fewer than SMs a
+// A CTA has a sub-panel of 4 tile columns (of both matrices of a gate/up pair) and a block of up to 128 rows; where these are fewer than SMs a
 // cluster of up to 8 CTAs shares one, each with a part of K. At the end the CTAs' fp32 sums are added through distributed shared memory,
 // in order, and each CTA of the cluster runs the epilogue for its share of the rows: one launch, no scratch, x not laid out anew.
 //
@@ -20,7 +20,8 @@
 //   warps 18-21  copy x, a tile row each: 16 tokens x 16 k of a tile are 512 consecutive bytes, a warp's one cp.async, which lands
 //                in the 32-byte swizzle, and tells the stage's barrier itself when it has (warps that waited for their copies: 128 rows 58 us against 55)
 // Gate/up pair and down projection, against the kernel of gemm.cu with its x laid out by rows and its parts of K added up by another launch:
-// 77 rows of 2048 x 5632 (bfp4, bfp8) 43.7 -> 22.1 us, 33 rows of 512 x 1024 23.8 -> 10.6, 33 rows of 4096 x 14336 113 -> 44, 128 rows 120 -> 55.
+// 77 rows of 2048 x 5632 (bfp4, bfp8) 43.7 -> 22.1 us, 33 rows of 512 x 1024 23.8 -> 10.6, 33 rows of 4096 x 14336 113 -> 44, 128 rows 120 -> 55,
+// 256 rows 126 -> 100, 640 rows 287 -> 228; 512 rows of 1024 x 3000 38 -> 25.
 // A launch costs 5 to 10 us beside its stages: setting up and the first weights and x 3, the sums' way through the cluster and the epilogue 3.
 // Every wait is bounded and reports through the error word.
 #include "common.cuh"
@@ -46,6 +47,7 @@ constexpr uint32_t kLimit = 1u << 14;               // attempts of up to 100 us 
 // Shared memory: mbarriers, then the rings of packed weights and of x, over which the sums go in the end.
 constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kRing = 1024;
 constexpr int kSmem = 227 * 1024;
+constexpr int kBlockRows = 4;                       // tile rows of a CTA at most: the sums of 128 tokens of a pair and the expanded weights fill tensor memory
 constexpr int kSumStride = 132;                     // floats from one token's 128 channels to the next
 
 struct FewParams {
@@ -59,7 +61,8 @@ struct FewParams {
   int M, KT, TC, epi, out_fp32;
   int splits;                // CTAs of a cluster, which share a sub-panel
   int stages, x_stages, bufs;   // of the rings of packed weights and of x, and of expanded weights in tensor memory
-  int tokens;                // rows of x in sixteens: the MMAs' N
+  int blocks, block_rows;    // blocks of rows, and tile rows of each but the last
+  int tokens;                // rows of a block in sixteens: the MMAs' N
   int weights_early;         // the launch before this one does not write weights
 };
 
@@ -72,10 +75,11 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sb = smem_u32(smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = p.splits > 1 ? (int)cluster_ctarank() : 0, panel = blockIdx.x / p.splits;
+  const int rank = p.splits > 1 ? (int)cluster_ctarank() : 0, panel = blockIdx.x / (p.splits * p.blocks);
+  const int tr0 = blockIdx.x / p.splits % p.blocks * p.block_rows, M = min(p.M - tr0 * 32, p.block_rows * 32);   // first tile row, and rows
   const int k0 = p.KT * rank / p.splits, kn = p.KT * (rank + 1) / p.splits - k0, steps = (kn + kRows - 1) / kRows;   // this CTA's tile rows
-  const int width = min(kPanel, p.TC - panel * kPanel), N = p.tokens, stages = p.stages, x_stages = p.x_stages, bufs = p.bufs;
-  const int x_row = N * 64, x_stage = kRows * x_row;
+  const int width = min(kPanel, p.TC - panel * kPanel), N = (M + 15) / 16 * 16, stages = p.stages, x_stages = p.x_stages, bufs = p.bufs;
+  const int x_row = N * 64, x_stage = kRows * p.tokens * 64;
   const uint32_t x_ring = sb + kRing + stages * W_STAGE;
   auto wait = [&](uint32_t bar, uint32_t parity, int code) {
     if (!mbar_wait(bar, parity, kLimit)) atomicExch(p.error, code);
@@ -159,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     const uint32_t place = (lane >> 1) * 32 + (((lane & 1) ^ (lane >> 3 & 1)) << 4);
     Turn t;
     // a warp copies its tile row of the stage, whose barrier hears from every lane when its copies have landed
-    const uint8_t *from = p.x + ((size_t)k0 + me) * 2048 + lane * 16;
+    const uint8_t *from = p.x + ((size_t)tr0 * p.KT + k0 + me) * 2048 + lane * 16;
     for (int i = 0; i < steps; i++, t.next(x_stages), from += kRows * 2048) {
       if (i >= x_stages) wait(sb + kXEmpty + 8 * t.at, t.parity ^ 1, 24);
       if (me < kn - i * kRows) {
@@ -207,10 +211,10 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     tc_fence_after();
     // the sums go over the ring: every stage has been used
     const int t0 = 32 * (warp >> 2), ch = 32 * cc + (lane & 16) + 2 * (lane & 7) + (lane >> 3 & 1);
-    if (t0 < p.M) {
+    if (t0 < M) {
 #pragma unroll
       for (int m = 0; m < MATS; m++) {
-        float *to = reinterpret_cast<float *>(smem + kRing) + (m * p.M + t0) * kSumStride + ch;
+        float *to = reinterpret_cast<float *>(smem + kRing) + (m * M + t0) * kSumStride + ch;
 #pragma unroll
         for (int c = 0; c < 32; c += 16)
           if (t0 + c < N) {
@@ -219,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; j++)
-              if (t0 + c + j < p.M) to[(c + j) * kSumStride] = __uint_as_float(v[j]);
+              if (t0 + c + j < M) to[(c + j) * kSumStride] = __uint_as_float(v[j]);
           }
       }
     }
@@ -232,14 +236,14 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   tc_fence_after();
   if (warp == kMmaWarp) tmem_dealloc(tmem, 512);
   // a warp to a row of 128 channels, a lane to four of them
-  const int tile_rows = (p.M + 31) / 32, first = tile_rows * 32 * rank / p.splits, end = tile_rows * 32 * (rank + 1) / p.splits;
+  const int tile_rows = (M + 31) / 32, first = tile_rows * 32 * rank / p.splits, end = tile_rows * 32 * (rank + 1) / p.splits;
   const int tcol = panel * kPanel + (lane >> 3), in_face = (lane & 4) * 64 + (lane & 3) * 4;   // datum of the lane's first channel in a tile's row 0
   if (lane >> 3 < width) {
     const float unscale = kExpandedUnscale * p.alpha;
     for (int row = first + warp; row < end; row += kThreads / 32) {
       float f[4] = {0.f, 0.f, 0.f, 0.f}, g[4] = {0.f, 0.f, 0.f, 0.f};
-      const int tr = row >> 5, at = in_face + (row >> 4 & 1) * 512 + (row & 15) * 16;
-      if (row < p.M) {
+      const int tr = tr0 + (row >> 5), at = in_face + (row >> 4 & 1) * 512 + (row & 15) * 16;
+      if (row < M) {
         uint2 a = make_uint2(0, 0);
         if (p.add) a = __ldcg(reinterpret_cast<const uint2 *>(p.add + (size_t)tr * p.add_row_stride + (size_t)tcol * 1024 + (p.add_row_stride ? at : in_face)));
         const float *own = reinterpret_cast<const float *>(smem + kRing) + row * kSumStride + lane * 4;
@@ -250,11 +254,11 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
             v[j] = u[j] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (c + j == rank) {
               v[j] = *reinterpret_cast<const float4 *>(own);
-              if (PAIR) u[j] = *reinterpret_cast<const float4 *>(own + p.M * kSumStride);
+              if (PAIR) u[j] = *reinterpret_cast<const float4 *>(own + M * kSumStride);
             } else if (c + j < p.splits) {
               const uint32_t from = map_to_cta(smem_u32(own), c + j);
               v[j] = ld_cluster4(from);
-              if (PAIR) u[j] = ld_cluster4(from + p.M * kSumStride * 4);
+              if (PAIR) u[j] = ld_cluster4(from + M * kSumStride * 4);
             }
           }
 #pragma unroll
@@ -283,24 +287,26 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   if (p.splits > 1) cluster_sync();                // nobody leaves while others read its sums
 }
 
-constexpr float kFixedUs = 4.f, kTileUs = 0.0125f;   // a wave's start and end; an SM's time for a packed tile
+constexpr float kStartUs = 2.f, kFixedUs = 4.f;     // a launch's start, a wave's start and end
+float tile_us(int tokens) { return 0.02f + 0.0001f * tokens; }   // an SM's time for a packed tile: 0.024 with 48 tokens, 0.032 with 128
 
 }  // namespace
 
 int gemm_few(int device, int fmt, int epilogue, int M, int K, int N, uint64_t x, uint64_t w, uint64_t w2, uint64_t add, int add_rows, float alpha, uint64_t out,
-             int out_dtype, uint64_t work, uint64_t stream) {
+             int out_dtype, float beat_us, bool *taken, uint64_t work, uint64_t stream) {
   const bool pair = epilogue == BT_EPI_GLU;
   FewParams p{};
   p.w[0] = as_ptr<uint8_t>(w), p.w[1] = as_ptr<uint8_t>(w2), p.x = as_ptr<uint8_t>(x), p.add = as_ptr<uint16_t>(add), p.out = as_ptr<void>(out), p.error = as_ptr<int>(work);
   p.alpha = alpha, p.M = M, p.KT = K / 32, p.TC = (N + 31) / 32, p.epi = epilogue, p.out_fp32 = out_dtype == BT_FP32;
   p.add_row_stride = add && add_rows > 1 ? (size_t)p.TC * 1024 : 0;
-  p.tokens = (M + 15) / 16 * 16;
+  const int tile_rows = (M + 31) / 32;
+  p.blocks = (tile_rows + kBlockRows - 1) / kBlockRows, p.block_rows = (tile_rows + p.blocks - 1) / p.blocks;
+  p.tokens = (std::min(M, p.block_rows * 32) + 15) / 16 * 16;
   const int mats = pair ? 2 : 1, w_stage = kRows * mats * kPanel * tile_bytes(fmt), x_stage = kRows * p.tokens * 64;
   // as many places for x as leave four for the weights (128 tokens and a pair in bfp8: two)
   for (p.x_stages = kMaxStages; p.x_stages > 2 && (kSmem - kRing - p.x_stages * x_stage) / w_stage < 4; p.x_stages--);
   p.stages = std::min(kMaxStages, (kSmem - kRing - p.x_stages * x_stage) / w_stage) / kGroups * kGroups;
   p.bufs = std::min(kMaxBufs, (512 - mats * p.tokens) / (mats * kRows * 16));
-  p.weights_early = follows_matmul(stream);
 
   using Kernel = void (*)(FewParams);
   static const Kernel kernels[2][2] = {{few_rows_kernel<BT_BFP8, false>, few_rows_kernel<BT_BFP8, true>}, {few_rows_kernel<BT_BFP4, false>, few_rows_kernel<BT_BFP4, true>}};
@@ -329,12 +335,17 @@ int gemm_few(int device, int fmt, int epilogue, int M, int K, int N, uint64_t x,
   // 15.5, 10.4, 10.3, 16.3 in 2, 4, 6 and 8.
   const int panels = (p.TC + kPanel - 1) / kPanel;
   float best = 1e30f;
+  int rounds = 1;
   for (int s = 1; s <= std::min(kMaxSplits, p.KT); s++) {
-    const int waves = (panels + fit[s] - 1) / fit[s];
-    const float us = waves * (kFixedUs + (p.KT + s - 1) / s * kPanel * mats * kTileUs) + (s > 1 ? 0.5f + 0.1f * s : 0.f);
-    if (us < best) best = us, p.splits = s;
+    const int waves = (panels * p.blocks + fit[s] - 1) / fit[s];
+    const float us = kStartUs + waves * (kFixedUs + (p.KT + s - 1) / s * kPanel * mats * tile_us(p.tokens)) + (s > 1 ? 0.5f + 0.1f * s : 0.f);
+    if (us < best) best = us, p.splits = s, rounds = waves;
   }
-  cfg.gridDim = dim3(panels * p.splits), attr[1].val.clusterDim.x = p.splits, cfg.numAttrs = p.splits > 1 ? 2 : 1;
+  // many waves of 128 x 128 draw more power than the estimate knows of: 2048 rows of 3000 x 8000 291 us where it had 250, the other kernel 278
+  *taken = best < (rounds > 2 ? 0.87f : 1.f) * beat_us;
+  if (!*taken) return BT_OK;
+  p.weights_early = follows_matmul(stream);
+  cfg.gridDim = dim3(panels * p.blocks * p.splits), attr[1].val.clusterDim.x = p.splits, cfg.numAttrs = p.splits > 1 ? 2 : 1;
   BT_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
   return launched("few_rows_kernel");
 }

@@ -203,7 +203,8 @@ int bt_gemm_bfp(int device, int fmt, int epilogue, int M, int K, int N, uint64_t
                 int add_rows, float alpha, uint64_t out, int out_dtype, uint64_t work, uint64_t stream);
 /* The same with x as Tensor holds it, bf16 tiles, and scratch for it: 2 * M * K bytes (rounded up to 256) for x by rows,
  * and what is left for sums of parts of K in fp32, which keep the GPU busy when rows and columns are few (as many parts as
- * there is room for; 0 bytes left: one). 33 to 128 rows take a kernel that reads x as it is and leaves the scratch alone.
+ * there is room for; 0 bytes left: one). Prompts of up to some hundred rows mostly take a kernel
+ * that reads x as it is and leaves the scratch alone.
  * The scratch is free again when the work queued here is done. */
 int bt_gemm_tiles(int device, int fmt, int epilogue, int M, int K, int N, uint64_t x, uint64_t w, uint64_t w2, uint64_t add, int add_rows,
                   float alpha, uint64_t out, int out_dtype, uint64_t scratch, size_t scratch_bytes, uint64_t work, uint64_t stream);

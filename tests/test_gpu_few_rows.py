@@ -1,5 +1,6 @@
-"""The tensor-core matmul for 33 to 128 rows (weights expanded into tensor memory): edges of its token groups, of sub-panels of
-fewer than four tile columns, of stages and of the clusters that share K, against the oracle's dequantised weights."""
+"""The tensor-core matmul for few rows (weights expanded into tensor memory): edges of its token groups and blocks of rows, of sub-panels
+of fewer than four tile columns, of stages and of the clusters that share K, against the oracle's dequantised weights; and the
+rule that chooses it against the kernel for many rows."""
 import numpy as np
 import pytest
 from oracle import bfp_oracle as o
@@ -11,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
 @pytest.mark.parametrize("m,k,n", [(33, 32, 32), (48, 64, 96), (49, 96, 128), (64, 128, 160), (65, 160, 320), (80, 1120, 64), (96, 288, 544), (97, 2048, 256),
-                                   (112, 4128, 416), (113, 544, 1504), (127, 256, 2400), (128, 992, 4896), (128, 352, 9600), (129, 352, 544)])
+                                   (112, 4128, 416), (113, 544, 1504), (127, 256, 2400), (128, 992, 4896), (128, 352, 9600), (129, 352, 544), (160, 1120, 96), (161, 544, 1504), (255, 96, 128), (256, 2080, 416)])
 def test_edges(rt, fmt, m, k, n):
   # small integers are exact in both formats and in fp32 sums, whatever the order: any misplaced row, column or k shows up. 129 rows
   # take the other kernel
@@ -66,6 +67,31 @@ def test_chain_and_recording(rt):
     rt.wait()
     assert np.array_equal(held[-1].numpy(), want)
   step.close()
+
+
+@pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
+@pytest.mark.parametrize("m,k,n", [(33, 96, 130), (129, 544, 1000), (300, 4128, 96), (520, 352, 2080), (1000, 256, 4128), (2050, 1056, 9000)])
+def test_the_same_as_the_kernel_for_many_rows(rt, fmt, m, k, n):
+  # whichever kernel the rule takes: every epilogue, addend and result type, exactly as the other kernel has it on small integers
+  from baretile_b200.tensor import FMT_CODE, Tensor
+  rng = np.random.default_rng(m + k + n)
+  x, w, v = rng.integers(-2, 3, (m, k)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32)
+  tx, tw, tv = upload(rt, x), upload(rt, w).cast(fmt).columns(), upload(rt, v).cast(fmt).columns()
+  adds = {0: None, 1: upload(rt, rng.integers(-9, 10, (1, n)).astype(np.float32)), m: upload(rt, rng.integers(-9, 10, (m, n)).astype(np.float32))}
+  K = tx.tc * 32
+  rows = rt.dram_alloc(2 * m * K)
+  rt.launch("bt_untilize", (2, tx.addr, rows, 1, m, K), name="rows")
+  for epilogue, add, dtype in (("none", 0, "fp32"), ("relu", m, "bf16"), ("none", 1, "bf16"), ("relu", 1, "fp32")):
+    y = tx.matmul(tw, dtype=dtype)
+    if add: y = y + adds[add]
+    if epilogue == "relu": y = y.relu()
+    want = Tensor(rt, m, n, dtype=dtype)
+    a = adds[add]
+    rt.launch("bt_gemm_bfp", (FMT_CODE[fmt], 1 if epilogue == "relu" else 0, m, K, n, rows, tw.addr, 0, a.addr if a is not None else 0, add, 1.0, want.addr, FMT_CODE[dtype], rt.work), name="many rows")
+    assert np.array_equal(y.numpy(), want.numpy()), (epilogue, add, dtype)
+  got = (tx.matmul(tw).silu() * tx.matmul(tv)).numpy()
+  check_matmul(got, x, None, o.silu(x @ w) * (x @ v), 1e-2)
+  rt.dram_free(rows)
 
 
 @pytest.mark.parametrize("fmt,m", [("bfp8", 96), ("bfp8", 112), ("bfp4", 100)])
