@@ -1231,11 +1231,12 @@ bool exchanged(const bt_gemv_op *ops, int i) {
   if (o.x != e.out || e.out_dtype != BT_BF16 || o.M != e.M || o.K != e.N) return false;
   Range lr[4], lw[2], ew[2];
   ranges_read(o, lr), ranges_written(o, lw), ranges_written(e, ew);
-  return !lw[0].meets(ew[0]) && (!o.add || o.add == e.out || !lr[1].meets(ew[0]));
+  // an addend that is the same tensor comes from the exchange too, which has no more columns than the matmul before
+  return !lw[0].meets(ew[0]) && (!o.add || (o.add == e.out ? o.N <= e.N : !lr[1].meets(ew[0])));
 }
 // Lists that chain_kernel takes: every matmul small, a sub-panel to a CTA, up to 8 tokens, no pick and no rows for an all-reduce.
-bool chain(const QueueHead &q, const GemvParams *op) {
-  for (int i = 0; i < q.n; i++)
+bool chain(int n, const GemvParams *op) {
+  for (int i = 0; i < n; i++)
     if (!op[i].small || op[i].M > kChainRows || op[i].epi == BT_EPI_ARGMAX || op[i].out_fp32 == 2 || op[i].share != op[i].KT || op[i].extra) return false;
   return true;
 }
@@ -1285,6 +1286,26 @@ void deal_units(GemvParams &p, int ctas) {
   for (int parts = 2; parts <= p.KT && parts * panels <= ctas; parts++) {
     const float t = stream((float)((p.KT + parts - 1) / parts)) + shared(parts);
     if (t < best) best = t, p.parts = parts, p.active = parts * panels;
+  }
+}
+
+// A matmul but for its place in a list and its tensor maps.
+void describe(GemvParams &p, const bt_gemv_op &o, int ctas) {
+  p.x = as_ptr<uint16_t>(o.x), p.w[0] = as_ptr<uint8_t>(o.w), p.w[1] = as_ptr<uint8_t>(o.w2), p.add = as_ptr<uint16_t>(o.add);
+  p.out = as_ptr<void>(o.out), p.arg_val = as_ptr<float>(o.arg_val), p.arg_idx = as_ptr<int>(o.arg_idx);
+  p.alpha = o.alpha, p.arg_base = o.arg_base, p.M = o.M, p.KT = o.K / 32, p.TC = o.N / 32, p.epi = o.epilogue, p.out_fp32 = o.out_dtype == BT_FP32 ? 1 : o.out_dtype == BT_FP32_ROWS ? 2 : 0;
+  p.fmt = o.fmt, p.pair = o.epilogue == BT_EPI_GLU, p.tg = o.M <= 8 ? 1 : o.M <= 16 ? 2 : 4;
+  p.from = p.to = p.add_from = 0;
+  deal_units(p, ctas);
+}
+// Which matmuls of a chain take x from the exchange, and what those wait for.
+void link(int n, GemvParams *op, const bt_gemv_op *ops, int sets) {
+  for (int i = 1; i < n; i++) {
+    GemvParams &p = op[i];
+    if (!exchanged(ops, i)) continue;
+    const int w = i - sets, v = w > 0 && wait_for(ops, w, sets) < w - 1 ? w - 1 : -1;
+    p.from = op[i - 1].to = 1, p.add_from = p.add && ops[i].add == ops[i].x;
+    p.early = w < 0 ? -1 : w, p.early_panels = w >= 0 ? op[w].panels : 0, p.early_also = v, p.early_also_panels = v >= 0 ? op[v].panels : 0;
   }
 }
 
@@ -1364,34 +1385,22 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
     for (int i = 0; i < q.n; i++) {
       const bt_gemv_op &o = ops[base + i];
       GemvParams &p = q.op[i];
-      p.w[0] = as_ptr<uint8_t>(o.w), p.w[1] = as_ptr<uint8_t>(o.w2), p.add = as_ptr<uint16_t>(o.add);
-      p.out = as_ptr<void>(o.out), p.arg_val = as_ptr<float>(o.arg_val), p.arg_idx = as_ptr<int>(o.arg_idx);
-      p.alpha = o.alpha, p.arg_base = o.arg_base, p.M = o.M, p.KT = o.K / 32, p.TC = o.N / 32, p.epi = o.epilogue, p.out_fp32 = o.out_dtype == BT_FP32 ? 1 : o.out_dtype == BT_FP32_ROWS ? 2 : 0;
-      p.fmt = o.fmt, p.pair = o.epilogue == BT_EPI_GLU, p.tg = o.M <= 8 ? 1 : o.M <= 16 ? 2 : 4;
+      describe(p, o, ctas);
       const Gate g = gate(ops + base, i, scratch.sets);
       p.wait_for = g.last, p.wait_also = g.also;
       p.turn = (int)(((long long)(base + i) * 101) % ctas);
       p.wait_panels = g.last >= 0 ? q.op[g.last].panels : 0, p.also_panels = g.also >= 0 ? q.op[g.also].panels : 0;
-      p.x = as_ptr<uint16_t>(o.x);
-      p.from = p.to = p.add_from = 0;
-      deal_units(p, ctas);
       q.panels += p.panels;
       small |= p.small;
       if (int s = make_maps(p, o.x)) return s;
       sums = max(sums, p.small ? p.KT * (p.pair ? 2 : 1) * p.M * sum_stride(p.lw) * 4 : sums_bytes(p.tg));
     }
-    const bool chained = chain(q, q.op);
+    const bool chained = chain(q.n, q.op);
     if (chained) {
       sums += kAheadBytes;
       // the next matmul goes to other CTAs: they have its weights at hand when its x comes
       for (int i = 0, start = 0; i < q.n; start = (start + q.op[i++].active) % ctas) q.op[i].turn = (ctas - start) % ctas;
-      for (int i = 1; i < q.n && scratch.exchange; i++) {
-        GemvParams &p = q.op[i];
-        if (!exchanged(ops + base, i)) continue;
-        const int w = i - scratch.sets, v = w > 0 && wait_for(ops + base, w, scratch.sets) < w - 1 ? w - 1 : -1;
-        p.from = q.op[i - 1].to = 1, p.add_from = p.add && ops[base + i].add == ops[base + i].x;
-        p.early = w < 0 ? -1 : w, p.early_panels = w >= 0 ? q.op[w].panels : 0, p.early_also = v, p.early_also_panels = v >= 0 ? q.op[v].panels : 0;
-      }
+      if (scratch.exchange) link(q.n, q.op, ops + base, scratch.sets);
     }
     q.ring = kSmSums + (sums + 127) / 128 * 128, q.ring_bytes = (kSmemBytes - q.ring) / 128 * 128;
     // Programmatic dependent launch: this grid may begin while the previous launch of the stream is still finishing.
@@ -1486,6 +1495,21 @@ int bt_gemv_queue_gates(int n, const bt_gemv_op *ops, int *gates) {
     const int base = i / kQueueMax * kQueueMax;
     const Gate g = gate(ops + base, i - base, kSets);
     gates[2 * i] = g.last < 0 ? -1 : base + g.last, gates[2 * i + 1] = g.also < 0 ? -1 : base + g.also;
+  }
+  return BT_OK;
+}
+
+int bt_gemv_queue_links(int sms, int n, const bt_gemv_op *ops, int *links) {
+  BT_REQUIRE(sms >= 1 && n >= 1 && ops && links, "bt_gemv_queue_links: needs a GPU's number of SMs, at least one matmul and somewhere for the answer");
+  for (int i = 0; i < n; i++)
+    if (int s = check_op("bt_gemv_queue_links", i, ops[i])) return s;
+  for (int base = 0; base < n; base += kQueueMax) {
+    GemvParams op[kQueueMax];
+    const int count = min(kQueueMax, n - base);
+    for (int i = 0; i < count; i++) describe(op[i], ops[base + i], min(sms, kMaxCtas));
+    const bool chained = chain(count, op);
+    if (chained) link(count, op, ops + base, kSets);
+    for (int i = 0; i < count; i++) links[base + i] = chained ? op[i].from : -1;
   }
   return BT_OK;
 }

@@ -188,6 +188,10 @@ int bt_gemv_queue_plan(int n, const bt_gemv_op *ops, int *waits);
  * before that where nothing else vouches for it (else -1). That everything up to waits[i] is finished follows from these
  * two and from what they themselves had to see. For tests of that rule. */
 int bt_gemv_queue_gates(int n, const bt_gemv_op *ops, int *gates);
+/* Which kernel the launches take on a GPU of so many SMs, and where x comes from: links[i] is -1 in a launch of the general kernel, and in one
+ * of the kernel for chains of small matmuls 1 where ops[i] takes its x (and an addend that is the same tensor) from the matmul before it while that
+ * one still runs, 0 where it reads x from memory. For tests of that rule. */
+int bt_gemv_queue_links(int sms, int n, const bt_gemv_op *ops, int *links);
 /* ---- the matmul: fused_kernel's prefill grid (baretile/kernels.py:205-215, :470-506, grid_parts :18-39) ----
  * out[M, N] = epilogue(alpha * (a[M, K] @ W[K, N]) + add) for many rows, on the tcgen05 tensor cores with fp32
  * accumulators in tensor memory, two CTAs to an MMA. The weights are expanded from block float to exact bf16

@@ -187,6 +187,32 @@ def _gates(ops):
   return [tuple(gates[2 * i:2 * i + 2]) for i in range(len(ops))]
 
 
+def _links(ops, sms=148):
+  from baretile_b200 import _lib
+  arr, links = (_lib.GemvOp * len(ops))(*ops), (ctypes.c_int * len(ops))()
+  _lib.call("bt_gemv_queue_links", sms, len(ops), arr, links)
+  return list(links)
+
+
+def test_chain_takes_from_the_matmul_before_what_that_one_has(built):
+  from baretile_b200 import _lib
+  def op(x, out, k=64, n=64, add=0, m=2, fp32=False):
+    return _lib.GemvOp(fmt=8, epilogue=0, M=m, K=k, N=n, out_dtype=int(fp32), alpha=1.0, x=x, w=0x100000, add=add, out=out)
+  A, B, C, D = (0x1000000 * i for i in range(1, 5))
+  assert _links([op(A, B), op(B, C), op(C, D)]) == [0, 1, 1]
+  assert _links([op(A, B), op(B, C, add=B)]) == [0, 1]
+  assert _links([op(A, B), op(B, C, n=32, add=B)]) == [0, 1]
+  # an addend of more columns than the matmul before has results: the columns past those come from memory
+  assert _links([op(A, B), op(B, C, n=96, add=B)]) == [0, 0]
+  assert _links([op(A, B), op(B, C, n=8192, add=B)]) == [0, 0]
+  assert _links([op(A, B), op(B, C, n=96, add=D)]) == [0, 1]
+  # another width or number of rows, an addend or a result that overlaps the result before, and fp32 results
+  assert _links([op(A, B, n=96), op(B, C)]) == [0, 0] and _links([op(A, B), op(B, C, m=1)]) == [0, 0] and _links([op(A, B, fp32=True), op(B, C)]) == [0, 0]
+  assert _links([op(A, B), op(B, C, add=B + 2048)]) == [0, 0] and _links([op(A, B), op(B, B + 2048)]) == [0, 0]
+  # a matmul that is not small, or more rows: the general kernel
+  assert _links([op(A, B), op(B, C, n=32768)]) == [-1, -1] and _links([op(A, B, m=9), op(B, C, m=9)]) == [-1, -1]
+
+
 def _complete(gates):
   """For each matmul, the earlier ones of its launch that are complete when it starts: those it looks at, and whatever was
   complete when those started. Nothing else: a matmul may be complete, or start, while one before it still runs."""

@@ -106,3 +106,20 @@ def test_exact_weights(rt):
     x = bf16(np.random.default_rng(6).integers(-3, 4, (2, 64)))
     got = upload(rt, x).matmul(upload(rt, w).cast("bfp8").columns(), dtype="fp32").numpy()
     assert np.array_equal(got.astype(np.float64), x.astype(np.float64) @ o.dequant(w, "bfp8").astype(np.float64))
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 64, 96), (3, 96, 64), (8, 64, 4096)])
+def test_addend_wider_than_the_matmul_before(rt, m, k, n):
+  """x and the addend start at the same place, and the addend goes on past what the matmul before has written there."""
+  from baretile_b200 import _lib
+  from baretile_b200.tensor import Tensor
+  rng = np.random.default_rng(m + n)
+  w, v = (upload(rt, weights(rng, k, c, stress=False)).cast("bfp8").columns() for c in (k, n))
+  x, wide = upload(rt, acts(rng, m, k)), acts(rng, m, max(k, n))
+  def run(queued):
+    y, z = upload(rt, wide), Tensor(rt, m, n)
+    ops = [_lib.GemvOp(fmt=8, epilogue=0, M=m, K=k, N=c, out_dtype=0, alpha=1.0, x=a, w=b.addr, add=add, out=to)
+           for c, a, b, add, to in ((k, x.addr, w, 0, y.addr), (n, y.addr, v, y.addr, z.addr))]
+    for some in ([ops] if queued else [[o] for o in ops]): _lib.call("bt_gemv_queue", rt.device, len(some), (_lib.GemvOp * len(some))(*some), rt.work, rt.work_bytes, rt.stream)
+    return z.numpy()
+  assert np.array_equal(run(True), run(False))
