@@ -1024,7 +1024,7 @@ template <int FMT> __device__ __forceinline__ void chain_matmul(const GemvParams
         missing = a.y != tag;
 #pragma unroll
         for (int j = 0; j < kAhead; j++) missing |= v[j][0].y != tag || v[j][0].w != tag || v[j][1].y != tag || v[j][1].w != tag;
-      } while (__any_sync(0xFFFFFFFFu, missing) && --patience);
+      } while (__any_sync(0xFFFFFFFFu, missing && patience && --patience));   // the vote keeps the warp together; a lane that has given up stays that way
     }
     // the sums of the matmul before have been read
     if (k0 == 0 && w.turn) stage_wait(w.smem, w.smem + kSmDone + 8 * ((w.turn - 1) & 1), (w.turn - 1) >> 1 & 1, q.error);

@@ -141,6 +141,29 @@ def test_bounded_wait_for_an_earlier_matmul_reports_instead_of_hanging(rt):
   del ys
 
 
+def test_bounded_wait_of_a_chain_reports_instead_of_hanging(rt):
+  # The same for a list that runs as a chain of small matmuls: the count of the first one's finished sub-panels starts far
+  # below zero, so neither the warp that lets the third one go ahead nor the messengers behind it see what they wait for. The last one has
+  # more tile rows (64) than a warp asks for at a time (16 warps, 3 each), so its lanes go on to a second batch.
+  from helpers import acts, upload, weights
+  rng = np.random.default_rng(6)
+  x, (w, up, down) = upload(rt, acts(rng, 4, 64)), (upload(rt, weights(rng, *s, stress=False) * 8).cast("bfp8").columns() for s in ((64, 64), (64, 2048), (2048, 64)))
+  def four():
+    with rt.queue():
+      a = (x @ w).realize()
+      b = (a @ w).realize()
+      c = (b @ up).realize()
+      return [a, b, c, (c @ down).realize()]
+  good = [y.numpy() for y in four()]
+  rt.wait()
+  rt.upload(rt.work + 8, bytes((ctypes.c_int * 1)(-1000)))
+  ys = four()
+  with pytest.raises(RuntimeError, match="gave up on a bounded wait"): rt.wait()
+  rt.wait()                                                        # the flag was read and cleared, the counts and the exchanges reset
+  for _ in range(2): assert all(np.array_equal(y.numpy(), g) for y, g in zip(four(), good))
+  del ys
+
+
 def test_bounded_wait_for_partial_sums_reports_instead_of_hanging(rt):
   # A wait inside the matmul kernel that cannot be met gives up after its limit and sets the error word, which
   # Runtime.wait turns into RuntimeError; the kernel ends normally and the runtime keeps working. The wait is made
