@@ -343,25 +343,27 @@ template <bool SMALL> __device__ __forceinline__ void zero_rows(const GemvParams
 }
 // Where the pair of channels `pr` of a sub-panel, in tile column `tcol`, has row r in the result's tiles: a datum's index, as in an addend's.
 __device__ __forceinline__ int pair_place(int tcol, int pr, int r) { return tcol * 1024 + ((r >> 4) * 2 + (pr >> 3 & 1)) * 256 + (r & 15) * 16 + (2 * pr & 15); }
-// A pair of neighbouring channels of one token to the result. Neighbouring lanes have neighbouring pairs of the same token.
-__device__ __forceinline__ void store_pair(const GemvParams &p, int tcol, int pr, int row, bool live, float2 v) {
+// A pair of neighbouring channels of one token to the result; n0 is the first of them. Neighbouring lanes have neighbouring pairs of the same token.
+// end_piece is on the way from one matmul to the next, where code and parameters are fetched anew every time, so what it has at hand comes
+// as it is: `live` as an expression for every use of it, n0, the pointer. With one flag worked out before and the rest taken from the parameters
+// behind the barrier the way between two small matmuls took 0.5 us more (3 rows of 8192 x 64 and back, 6.3 us a matmul against 5.8).
+template <class Live> __device__ __forceinline__ void store_pair(const GemvParams &p, char *out, int fp32, int M, int tcol, int pr, int n0, int row, Live live, float2 v) {
   const uint32_t both = bf16_half_up(v.x) | bf16_half_up(v.y) << 16;
-  char *out = static_cast<char *>(p.out);
-  if (p.out_fp32 == 2) {
+  if (fp32 == 2) {
     // row-major fp32, only the rows there are: partial sums on their way to an all-reduce
-    if (live) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + tcol * 32 + (2 * pr & 31))) = v;
-  } else if (p.M > 1) {
-    if (live && p.out_fp32) *reinterpret_cast<float2 *>(out + 4 * (size_t)pair_place(tcol, pr, row)) = v;
-    else if (live) *reinterpret_cast<uint32_t *>(out + 2 * (size_t)pair_place(tcol, pr, row)) = both;
-  } else if (p.out_fp32) {
+    if (live()) *reinterpret_cast<float2 *>(out + 4 * ((size_t)row * (p.TC * 32) + n0)) = v;
+  } else if (M > 1) {
+    if (live() && fp32) *reinterpret_cast<float2 *>(out + 4 * (size_t)pair_place(tcol, pr, row)) = v;
+    else if (live()) *reinterpret_cast<uint32_t *>(out + 2 * (size_t)pair_place(tcol, pr, row)) = both;
+  } else if (fp32) {
     // a one-row result repeats across its tile
-    for (int r = 0; live && r < 32; r++) *reinterpret_cast<float2 *>(out + 4 * (size_t)pair_place(tcol, pr, r)) = v;
+    for (int r = 0; live() && r < 32; r++) *reinterpret_cast<float2 *>(out + 4 * (size_t)pair_place(tcol, pr, r)) = v;
   } else {
     // the same: four lanes put half a face row together, and each of them writes it to eight of the rows
     uint4 half;
     half.x = __shfl_sync(0xFFFFFFFFu, both, 0, 4), half.y = __shfl_sync(0xFFFFFFFFu, both, 1, 4);
     half.z = __shfl_sync(0xFFFFFFFFu, both, 2, 4), half.w = __shfl_sync(0xFFFFFFFFu, both, 3, 4);
-    if (live) {
+    if (live()) {
 #pragma unroll
       for (int r = 0; r < 32; r += 4) *reinterpret_cast<uint4 *>(out + 2 * (size_t)(pair_place(tcol, pr, r + (pr & 3)) - 2 * (pr & 3))) = half;
     }
@@ -369,13 +371,14 @@ __device__ __forceinline__ void store_pair(const GemvParams &p, int tcol, int pr
 }
 template <bool SMALL> __device__ __forceinline__ void end_piece(const GemvParams &p, const Scratch &sc, int slot_floats, const float *sums, const Piece &pc, uint32_t smem, int *error) {
   const Columns<SMALL> at(p, pc.sp);
-  const int lw = lw_of<SMALL>(p), pairs = 16 << lw, pr = threadIdx.x & (pairs - 1), M = p.M, epi = p.epi;
+  const int lw = lw_of<SMALL>(p), pairs = 16 << lw, pr = threadIdx.x & (pairs - 1), M = p.M, epi = p.epi, fp32 = p.out_fp32;
   const bool pair = p.pair, owner = pc.me == pc.last;
   const int others = owner ? pc.last - pc.first : 0;                                  // contributors whose sums are to be added
   const int tcol = at.col + (pr >> 4), n0 = at.col * 32 + 2 * pr;                     // tile column and first channel of the pair
   const bool inside = (pr >> 4) < at.width;
   const float unscale = unscale_of(p.tg) * p.alpha;
   const uint16_t *add = owner && inside ? p.add : nullptr;
+  char *out = static_cast<char *>(p.out);
   float *slots = sc.partials + (size_t)(owner ? pc.first : pc.me) * slot_floats + 2 * pr;
   const int rows = kConsumers >> (4 + lw), mine = threadIdx.x >> (4 + lw);            // rows at a time, and this thread's among them
   auto addend = [&](int r) { return add && r < M ? __ldcg(reinterpret_cast<const uint32_t *>(add + pair_place(tcol, pr, r))) : 0u; };
@@ -383,7 +386,7 @@ template <bool SMALL> __device__ __forceinline__ void end_piece(const GemvParams
   // what the barrier is waited with is worked out and fetched already
   int KT = p.KT, next = M * sum_stride(lw) * (pair ? 2 : 1);
   float scale = unscale;
-  asm volatile("" : "+r"(KT), "+r"(next), "+f"(scale), "+l"(slots) :: "memory");
+  asm volatile("" : "+r"(KT), "+r"(next), "+f"(scale), "+l"(out), "+l"(slots) :: "memory");
   named_barrier(1, kConsumers);                                                       // every warp's sums are in place
   uint32_t patience = others && lds32(smem + kSmDead) ? 1 : kSpinLimit * 64;
   for (int row0 = 0; row0 < M; row0 += rows) {
@@ -460,7 +463,7 @@ template <bool SMALL> __device__ __forceinline__ void end_piece(const GemvParams
       if ((threadIdx.x & (min(pairs, 32) - 1)) == 0 && key) atomicMax(sc.keys + row, key);
       continue;
     }
-    store_pair(p, tcol, pr, row, inside && live, v);
+    store_pair(p, out, fp32, M, tcol, pr, n0, row, [&] { return inside && live; }, v);
   }
   if (!patience) {
     sts32(smem + kSmDead, 1);
@@ -726,8 +729,9 @@ __device__ __forceinline__ uint4 stream_small(Place &w, float *sums, int *error,
 // its sub-panels are: by then every CTA with a part in it has read its x, and is past its look at the counts. It says
 // nothing about the matmul before it, of which this CTA may have no part: that is what Gate is about. (Counting
 // the CTAs instead, idle ones too, took 148 reports to one address where a small matmul has 5 sub-panels.) The last
-// report of the launch therefore finds nobody looking any more, and zeroes the counts for the next launch.
-__device__ __forceinline__ void report(const QueueHead &q, int i) {
+// report of the launch therefore finds nobody looking any more, and zeroes the counts for the next launch (and counts a launch of chains:
+// reading and writing that number at the end of every launch took 0.35 us).
+template <bool CHAIN> __device__ __forceinline__ void report(const QueueHead &q, int i) {
   const int lane = threadIdx.x & 31;
   int end = 0;
   if (lane == 0) {
@@ -735,13 +739,13 @@ __device__ __forceinline__ void report(const QueueHead &q, int i) {
     if (atom_add_acq_rel_gpu(q.all_done, 1) == q.panels - 1) {
       for (int j = 0; j < q.n; j++) q.ops_done[j] = 0;
       *q.all_done = 0;
-      if (q.exchange) {
+      if (CHAIN && q.exchange) {
         const uint32_t next = (*q.epoch + 1) % kEpochs;
         *q.epoch = next, end = next == 0;
       }
     }
   }
-  if (__shfl_sync(0xFFFFFFFFu, end, 0))          // the tags start over
+  if (CHAIN && __shfl_sync(0xFFFFFFFFu, end, 0))          // the tags start over
     for (size_t at = lane; at < kExchanges * kExchangeBytes / 16; at += 32) reinterpret_cast<uint4 *>(q.exchange)[at] = make_uint4(0, 0, 0, 0);
 }
 
@@ -798,7 +802,7 @@ template <bool SMALL, class Q> __device__ __forceinline__ void carry(const Q &q,
         }
         __syncwarp();
       }
-      report(q, i);
+      report<false>(q, i);
       __syncwarp();
     }
   }
@@ -1080,7 +1084,7 @@ template <int FMT> __device__ __forceinline__ void chain_matmul(const GemvParams
     if (epi == BT_EPI_SILU || pair) s.x = silu(s.x), s.y = silu(s.y);
     if (pair) s.x *= (u.x + 0.f) * alpha, s.y *= (u.y + 0.f) * alpha;
     if (to) st_relaxed64(to, make_uint2(bf16_half_up(s.x) | bf16_half_up(s.y) << 16, tag + 1));
-    store_pair(p, tcol, pr, row, live, s);
+    store_pair(p, static_cast<char *>(p.out), p.out_fp32, M, tcol, pr, at.col * 32 + 2 * pr, row, [&] { return live; }, s);
   }
   __syncwarp();
   mbar_arrive_if(w.smem + kSmDone + 8 * (w.turn & 1), lane == 0);
@@ -1139,7 +1143,7 @@ __global__ void __launch_bounds__(kThreads, 1) chain_kernel(const __grid_constan
       zero_rows<true>(p, me);
       stage_wait(sbase, sbase + kSmDone + 8 * (turn & 1), turn >> 1 & 1, q.error);
       __syncwarp();
-      report(q, i);
+      report<true>(q, i);
       __syncwarp();
     }
     turn++;
