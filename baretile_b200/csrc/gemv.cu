@@ -890,7 +890,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
 // In a small model's decode step every matmul is small (a sub-panel to a CTA, whole) and reads the one before it. What such a matmul
 // costs is the way from one's result to the next one's. In the general kernel that is 4.9 us: the stores have to be acknowledged before the
 // report (0.7), the report is seen by polling (0.7-1.0), then the copy of x starts (0.8), and from x to the result there are some 2.7 us of
-// instructions, most of them fetched anew for every matmul. So lists of small matmuls with up to 8 tokens have a kernel of their own:
+// instructions, most of them fetched anew for every matmul. So lists of small matmuls with up to 8 tokens have a kernel of their own (where it is the faster one: see chain):
 //  * A result also goes to an exchange where every word (two bf16 values) travels with a tag: the launch's number and the matmul's
 //    place in it. What has the right tag is there: no report, no copy. A consumer lane fetches the words of its own
 //    MMA fragments, straight into registers.
@@ -1238,11 +1238,25 @@ bool exchanged(const bt_gemv_op *ops, int i) {
   // an addend that is the same tensor comes from the exchange too, which has no more columns than the matmul before
   return !lw[0].meets(ew[0]) && (!o.add || (o.add == e.out ? o.N <= e.N : !lr[1].meets(ew[0])));
 }
-// Lists that chain_kernel takes: every matmul small, a sub-panel to a CTA, up to 8 tokens, no pick and no rows for an all-reduce.
-bool chain(int n, const GemvParams *op) {
-  for (int i = 0; i < n; i++)
+// Lists that chain_kernel takes: every matmul small, a sub-panel to a CTA, up to 8 tokens, no pick and no rows for an all-reduce; and it has to be
+// the faster kernel. What it gains is the way from one result to the next. A matmul that reads x from memory gains little, and with many tile rows
+// it loses, since x is then fetched batch by batch, each behind the weights it goes with; and a launch costs more. us, general kernel and this one (tokens):
+//   chains of 24, a matmul: 576 x 1536 and back 5.1 and 2.7 (1), 5.2 and 3.9 (8); 4096 x 256 6.4 and 5.3 (1), 5.4 (3); 8192 x 64 10.9 and 10.4 (1), 11.4 and 13.7 (2); 9000 x 100 8.7 and 10.0 (1)
+//   a launch of two: 576 x 576 9.3 and 7.9 (1), 9.0 (3); 2048 x 256 and back 10.5 and 10.3 (1), 11.4 (3), 12.4 (8); of three 15.9 and 13.7 (1), 14.2 (3)
+//   not dependent, 24, a matmul: 576 x 576 2.4 and 2.3; 576 x 1536 3.1 and 2.5; 1024 x 768 2.6 and 2.7; 2048 x 512 3.3 and 3.6 (1), 3.4 and 4.5 (8); 4096 x 256 4.1 and 5.0; 100 x 9000 4.6 and 3.2
+//   and a few: one of 576 x 1536 5.2 and 5.9, of 100 x 9000 6.6 and 6.3, three of 576 x 576 9.3 and 10.2, four of 576 x 1536 14.4 and 11.6
+constexpr float kChainStartUs = 1.f;
+float chain_gain_us(const GemvParams &p, bool linked) {
+  if (linked) return p.M == 1 ? 2.4f - 0.017f * p.KT : 1.5f - 0.01f * p.KT - 0.03f * max(p.KT - 128, 0);
+  return p.KT > 24 ? -0.0175f * p.KT : p.panels >= 32 ? 1.05f - 0.035f * p.KT : 0.1f;
+}
+bool chain(int n, const GemvParams *op, const bt_gemv_op *ops) {
+  float gain = -kChainStartUs;
+  for (int i = 0; i < n; i++) {
     if (!op[i].small || op[i].M > kChainRows || op[i].epi == BT_EPI_ARGMAX || op[i].out_fp32 == 2 || op[i].share != op[i].KT || op[i].extra) return false;
-  return true;
+    gain += chain_gain_us(op[i], exchanged(ops, i));
+  }
+  return gain > 0.f;
 }
 
 // The ranges of a matmul's units. Sharing a sub-panel costs a hand-over of partial sums, a range that straddles sub-panels
@@ -1399,12 +1413,12 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       if (int s = make_maps(p, o.x)) return s;
       sums = max(sums, p.small ? p.KT * (p.pair ? 2 : 1) * p.M * sum_stride(p.lw) * 4 : sums_bytes(p.tg));
     }
-    const bool chained = chain(q.n, q.op);
+    const bool chained = scratch.exchange && chain(q.n, q.op, ops + base);
     if (chained) {
       sums += kAheadBytes;
       // the next matmul goes to other CTAs: they have its weights at hand when its x comes
       for (int i = 0, start = 0; i < q.n; start = (start + q.op[i++].active) % ctas) q.op[i].turn = (ctas - start) % ctas;
-      if (scratch.exchange) link(q.n, q.op, ops + base, scratch.sets);
+      link(q.n, q.op, ops + base, scratch.sets);
     }
     q.ring = kSmSums + (sums + 127) / 128 * 128, q.ring_bytes = (kSmemBytes - q.ring) / 128 * 128;
     // Programmatic dependent launch: this grid may begin while the previous launch of the stream is still finishing.
@@ -1511,7 +1525,7 @@ int bt_gemv_queue_links(int sms, int n, const bt_gemv_op *ops, int *links) {
     GemvParams op[kQueueMax];
     const int count = min(kQueueMax, n - base);
     for (int i = 0; i < count; i++) describe(op[i], ops[base + i], min(sms, kMaxCtas));
-    const bool chained = chain(count, op);
+    const bool chained = chain(count, op, ops + base);
     if (chained) link(count, op, ops + base, kSets);
     for (int i = 0; i < count; i++) links[base + i] = chained ? op[i].from : -1;
   }

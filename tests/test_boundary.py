@@ -198,19 +198,47 @@ def test_chain_takes_from_the_matmul_before_what_that_one_has(built):
   from baretile_b200 import _lib
   def op(x, out, k=64, n=64, add=0, m=2, fp32=False):
     return _lib.GemvOp(fmt=8, epilogue=0, M=m, K=k, N=n, out_dtype=int(fp32), alpha=1.0, x=x, w=0x100000, add=add, out=out)
-  A, B, C, D = (0x1000000 * i for i in range(1, 5))
-  assert _links([op(A, B), op(B, C), op(C, D)]) == [0, 1, 1]
-  assert _links([op(A, B), op(B, C, add=B)]) == [0, 1]
-  assert _links([op(A, B), op(B, C, n=32, add=B)]) == [0, 1]
+  A, B, C, D, *more = (0x1000000 * i for i in range(1, 12))
+  def links(*ops):           # behind a chain of some matmuls, so that the list is one whatever these are
+    m = ops[0].M
+    lead = [op(a, b, m=m) for a, b in zip(more, more[1:])]
+    got = _links(lead + list(ops))
+    assert got[:len(lead)] in ([0] + [1] * (len(lead) - 1), [-1] * len(lead))
+    return got[len(lead):]
+  assert links(op(A, B), op(B, C), op(C, D)) == [0, 1, 1]
+  assert links(op(A, B), op(B, C, add=B)) == [0, 1]
+  assert links(op(A, B), op(B, C, n=32, add=B)) == [0, 1]
   # an addend of more columns than the matmul before has results: the columns past those come from memory
-  assert _links([op(A, B), op(B, C, n=96, add=B)]) == [0, 0]
-  assert _links([op(A, B), op(B, C, n=8192, add=B)]) == [0, 0]
-  assert _links([op(A, B), op(B, C, n=96, add=D)]) == [0, 1]
+  assert links(op(A, B), op(B, C, n=96, add=B)) == [0, 0]
+  assert links(op(A, B), op(B, C, n=8192, add=B)) == [0, 0]
+  assert links(op(A, B), op(B, C, n=96, add=D)) == [0, 1]
   # another width or number of rows, an addend or a result that overlaps the result before, and fp32 results
-  assert _links([op(A, B, n=96), op(B, C)]) == [0, 0] and _links([op(A, B), op(B, C, m=1)]) == [0, 0] and _links([op(A, B, fp32=True), op(B, C)]) == [0, 0]
-  assert _links([op(A, B), op(B, C, add=B + 2048)]) == [0, 0] and _links([op(A, B), op(B, B + 2048)]) == [0, 0]
+  assert links(op(A, B, n=96), op(B, C)) == [0, 0] and links(op(A, B), op(B, C, m=1)) == [0, 0] and links(op(A, B, fp32=True), op(B, C)) == [0, 0]
+  assert links(op(A, B), op(B, C, add=B + 2048)) == [0, 0] and links(op(A, B), op(B, B + 2048)) == [0, 0]
   # a matmul that is not small, or more rows: the general kernel
-  assert _links([op(A, B), op(B, C, n=32768)]) == [-1, -1] and _links([op(A, B, m=9), op(B, C, m=9)]) == [-1, -1]
+  assert links(op(A, B), op(B, C, n=32768)) == [-1, -1] and links(op(A, B, m=9), op(B, C, m=9)) == [-1, -1]
+
+
+def test_chain_kernel_takes_lists_that_gain_by_it(built):
+  # (k, n) of each matmul, read from the one before ("chain") or from inputs of their own ("apart")
+  from baretile_b200 import _lib
+  def takes(how, m, *shapes):
+    at = [0x1000000 * (i + 1) for i in range(2 * len(shapes) + 1)]
+    ops = [_lib.GemvOp(fmt=8, epilogue=0, M=m, K=-(-k // 32) * 32, N=-(-n // 32) * 32, out_dtype=0, alpha=1.0, w=0x100000, out=at[2 * i + 1],
+                       x=at[2 * i - 1] if i and how == "chain" else at[2 * i]) for i, (k, n) in enumerate(shapes)]
+    links = _links(ops)
+    assert links[0] in (0, -1) and len(set(links[1:])) <= 1
+    return links[0] == 0
+  def back_and_forth(a, b, count): return [(a, b), (b, a)] * (count // 2) + [(a, b)] * (count % 2)
+  for m in (1, 3, 8):
+    assert takes("chain", m, *back_and_forth(576, 1536, 24)) and takes("chain", m, (576, 576), (576, 576)) and takes("chain", m, *back_and_forth(2048, 512, 24))
+    assert takes("apart", m, *[(576, 1536)] * 4) and takes("apart", m, *[(576, 576)] * 24) and takes("apart", m, *[(100, 9000)] * 2)
+    # one alone, some narrow ones, and many tile rows: the general kernel
+    assert not takes("apart", m, (576, 1536)) and not takes("apart", m, *[(576, 576)] * 3)
+    for k, n in ((1024, 768), (2048, 512), (4096, 256)): assert not takes("apart", m, *[(k, n)] * 24) and not takes("apart", m, (k, n))
+    assert takes("chain", m, (2048, 256), (256, 2048)) == (m == 1) and not takes("chain", m, (4096, 256), (256, 4096)) and not takes("chain", m, (256, 4096), (4096, 256))
+    assert takes("chain", m, *back_and_forth(8192, 64, 24)) == (m == 1) and not takes("chain", m, *back_and_forth(100, 9000, 24))
+  assert takes("chain", 1, *back_and_forth(4096, 256, 24)) and takes("chain", 3, *back_and_forth(4096, 256, 24))
 
 
 def _complete(gates):
