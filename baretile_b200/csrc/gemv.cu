@@ -125,7 +125,6 @@ struct alignas(64) GemvParams {
   CUtensorMap xmap;           // x as (16-datum face rows of the staged tokens, faces, tile columns)
   CUtensorMap wmap[2];        // for sub-panels narrower than a run: the weights as (a tile's bytes, the four tiles of a run's tile row, tile rows)
   const uint8_t *w[2];
-  const uint16_t *x;          // chains read it themselves, where it does not come from an exchange
   const uint16_t *add;
   void *out;
   float *arg_val;
@@ -135,11 +134,6 @@ struct alignas(64) GemvParams {
   int fmt, pair, tg;
   int wait_for, wait_panels;  // the last matmul of the launch that must be complete before this one starts (-1: none), and its sub-panels
   int wait_also, also_panels; // the one before it, where its being complete does not follow (see Gate), and its sub-panels
-  int from;                   // chains: x is the result of the matmul before this one and comes from its exchange
-  int add_from;               // so does the addend
-  int to;                     // chains: the matmul after this one reads the exchange
-  int early, early_panels;    // with `from`: what must be complete before this one stores anything, as wait_for and
-  int early_also, early_also_panels;   // wait_also without it
   int turn;                   // CTA c takes the unit range (c + turn) % CTAs
   int lw, panels;             // tile columns of a sub-panel are 1 << lw, and there are so many sub-panels
   int tiled;                  // wmap is used
@@ -148,6 +142,13 @@ struct alignas(64) GemvParams {
   int active;                 // CTAs with a range
   int parts;                  // > 0: every sub-panel is cut into so many ranges; 0: ranges of equal size whatever they straddle,
   int share, extra;           // range b then starts at b * share + min(b, extra), and the last one ends at units
+  // what chains have beside it, behind what the general kernel reads (between its fields these cost independent small matmuls 2 %: 2.66 us each for 2.60)
+  const uint16_t *x;          // chains read it themselves, where it does not come from an exchange
+  int from;                   // chains: x is the result of the matmul before this one and comes from its exchange
+  int add_from;               // so does the addend
+  int to;                     // chains: the matmul after this one reads the exchange
+  int early, early_panels;    // with `from`: what must be complete before this one stores anything, as wait_for and
+  int early_also, early_also_panels;   // wait_also without it
 };
 
 // The kernel exists for lists with a small matmul in them and for lists without one, which is spared all that sub-panels
