@@ -14,8 +14,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("m,k,n", [(33, 32, 32), (48, 64, 96), (49, 96, 128), (64, 128, 160), (65, 160, 320), (80, 1120, 64), (96, 288, 544), (97, 2048, 256),
                                    (112, 4128, 416), (113, 544, 1504), (127, 256, 2400), (128, 992, 4896), (128, 352, 9600), (129, 352, 544), (160, 1120, 96), (161, 544, 1504), (255, 96, 128), (256, 2080, 416)])
 def test_edges(rt, fmt, m, k, n):
-  # small integers are exact in both formats and in fp32 sums, whatever the order: any misplaced row, column or k shows up. 129 rows
-  # take the other kernel
+  # small integers are exact in both formats and in fp32 sums, whatever the order: any misplaced row, column or k shows up.
+  # (All of these go to the kernel for few rows; `run` compares the other one with it.)
   rng = np.random.default_rng(m * 131 + k + n)
   xi, wi, vi = rng.integers(-2, 3, (m, k)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32)
   add = rng.integers(-9, 10, (m, n)).astype(np.float32)

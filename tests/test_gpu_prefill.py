@@ -1,5 +1,6 @@
 """The tensor-core (tcgen05) matmul for many rows against the oracle's fp32 NumPy matmul over the same dequantised
 weights: max relative error 1e-2 for bf16 results, 1e-4 for fp32 results (relative error as in docs/workload.md:141)."""
+import ctypes
 import numpy as np
 import pytest
 from oracle import bfp_oracle as o
@@ -14,23 +15,40 @@ def deq(w, fmt):
   return o.dequant(np.pad(w, ((0, 0), (0, pad))), fmt)[:, :w.shape[1]]
 
 
+def many_rows(rt, tx, tw, tw2, add, epilogue, alpha, dtype):
+  """The kernel for many rows (bt_gemm_bfp, x laid out by rows for it), whatever Tensor's rule would take."""
+  from baretile_b200.tensor import EPILOGUE, FMT_CODE, Tensor
+  m, k = tx.rows, tx.tc * 32
+  rows, out = rt.dram_alloc(2 * m * k), Tensor(rt, m, tw.cols, dtype=dtype or "bf16")
+  rt.launch("bt_untilize", (2, tx.addr, rows, 1, m, k), name="rows")
+  rt.launch("bt_gemm_bfp", (FMT_CODE[tw.dtype], EPILOGUE[epilogue], m, k, tw.cols, rows, tw.addr, tw2.addr if tw2 is not None else 0, add.addr if add is not None else 0,
+                            add.rows if add is not None else 0, 1.0 if alpha is None else alpha, out.addr, FMT_CODE[out.dtype], rt.work), name="many rows")
+  rt.dram_free(rows)
+  return out.numpy()
+
+
 def run(rt, x, w, fmt, epilogue="none", w2=None, dtype=None, add=None, alpha=None):
-  tx, tw = upload(rt, x), upload(rt, w).cast(fmt).columns()
+  """The matmul as an expression, which takes the kernel that the rule expects to be the faster one, and by the kernel for many rows beside it:
+  both within the bounds, and both exact where the one is."""
+  tx, tw, tadd = upload(rt, x), upload(rt, w).cast(fmt).columns(), upload(rt, add) if add is not None else None
+  tw2 = upload(rt, w2).cast(fmt).columns() if w2 is not None else None
   y, ref = tx.matmul(tw, dtype=dtype), x.astype(np.float32) @ deq(w, fmt)
   if alpha is not None: y, ref = y * alpha, ref * np.float32(alpha)
-  if add is not None: y, ref = y + upload(rt, add), ref + add
+  if add is not None: y, ref = y + tadd, ref + add
   if epilogue == "relu": y, ref = y.relu(), np.maximum(ref, 0)
   elif epilogue == "silu": y, ref = y.silu(), o.silu(ref)
-  elif epilogue == "glu":
-    y, ref = y.silu() * tx.matmul(upload(rt, w2).cast(fmt).columns(), dtype=dtype), o.silu(ref) * (x.astype(np.float32) @ deq(w2, fmt))
+  elif epilogue == "glu": y, ref = y.silu() * tx.matmul(tw2, dtype=dtype), o.silu(ref) * (x.astype(np.float32) @ deq(w2, fmt))
   rt.log = []
   got = y.realize()
   rt.wait()
   names, rt.log = [n for *_, n in rt.log], None
-  assert sum(n.startswith("prefill") for n in names) == 1, names    # the tensor-core kernel ran, once, not the decode loop
-  out = got.numpy()
-  if epilogue in ("none", "relu"):   # every element within 2^-8 of sum |x||w| (+ |addend|): the reference's per-element bound
-    check_matmul(out, x, deq(w, fmt), ref, 1e-2 if dtype != "fp32" else 1e-4, addend=add, alpha=alpha if alpha is not None else 1.0)
+  assert sum(n.startswith("prefill") for n in names) == 1, names    # a tensor-core kernel ran, once, not the decode loop
+  out, many, tol = got.numpy(), many_rows(rt, tx, tw, tw2, tadd, epilogue, alpha, dtype), 1e-2 if dtype != "fp32" else 1e-4
+  for result in (out, many):
+    # every element of a linear or ReLU result within 2^-8 of sum |x||w| (+ |addend|): the reference's per-element bound
+    linear = epilogue in ("none", "relu")
+    check_matmul(result, x, deq(w, fmt) if linear else None, ref, tol, addend=add if linear else None, alpha=alpha if alpha is not None else 1.0)
+  if np.array_equal(out, ref): assert np.array_equal(many, ref)
   return out, ref
 
 
@@ -173,3 +191,53 @@ def test_shared_k_and_half_blocks(rt, fmt, m, k, n):
   check_matmul(got, x, None, ref, 1e-4)
   got, ref = run(rt, x, w, fmt, "glu", w2)
   check_matmul(got, x, None, ref, 1e-2)
+
+
+@pytest.mark.parametrize("fmt,m,k,n,pair", [("bfp8", 33, 18784, 70, True), ("bfp4", 300, 18016, 100, True), ("bfp8", 330, 23968, 58, True),
+                                            ("bfp4", 400, 8992, 2900, False), ("bfp8", 300, 11040, 4000, False), ("bfp4", 1442, 12096, 1935, False)])
+def test_parts_of_k_in_memory(rt, monkeypatch, fmt, m, k, n, pair):
+  """Sizes at which pairs of CTAs share K through memory (gemm_kernel and reduce_kernel, after a launch that lays x out by rows): blocks of 256 and 512 rows, 2 to 16
+  parts, an odd last tile row in the last part. And the same without room for the parts, and without any."""
+  from baretile_b200 import _lib
+  rng = np.random.default_rng(m + k + n)
+  def launches():
+    count = ctypes.c_uint64()
+    _lib.call("bt_launch_count", ctypes.byref(count))
+    return count.value
+  def ints(a, b, *shape): return rng.integers(a, b, shape).astype(np.float32)
+  w, v = ints(-1, 2, k, n), ints(-1, 2, k, n) if pair else None
+  tw, tv = upload(rt, w).cast(fmt).columns(), upload(rt, v).cast(fmt).columns() if pair else None
+  def split(expression):
+    before = launches()
+    y = expression.realize()
+    assert launches() - before == 3
+    return y.numpy()
+  # small integers: fp32 sums are exact in any order, and so is a wide scale; values for the activations
+  xi, x = ints(-2, 3, m, k), bf16(rng.normal(0, 1 / np.sqrt(k), (m, k)))
+  ti, tx = upload(rt, xi), upload(rt, x)
+  if pair:
+    ref = o.silu(x @ w) * (x @ v)
+    check_matmul(split(tx.matmul(tw, dtype="fp32").silu() * tx.matmul(tv, dtype="fp32")), x, None, ref, 1e-4)
+    expression = lambda: (tx @ tw).silu() * (tx @ tv)
+    check_matmul(split(expression()), x, None, ref, 1e-2)
+  else:
+    exact, bias, resid = xi @ w, ints(-9, 10, 1, n), ints(-9, 10, m, n)
+    tb, tr = upload(rt, bias), upload(rt, resid)
+    assert np.array_equal(split(ti.matmul(tw, dtype="fp32")), exact)
+    assert np.array_equal(split((ti.matmul(tw, dtype="fp32") * 0.5 + tr).relu()), np.maximum(exact * 0.5 + resid, 0))
+    assert np.array_equal(split(ti.matmul(tw, dtype="fp32") + tb), exact + bias)
+    ref = o.silu(x @ w + bias)
+    expression = lambda: ((tx @ tw) + tb).silu()
+    check_matmul(split(expression()), x, None, ref, 1e-2)
+  alloc = rt.dram_alloc
+  def tight(size, limit=-(-2 * m * k // 256) * 256):
+    if size > limit: raise MemoryError(f"no {size} bytes free in DRAM")
+    return alloc(size)
+  monkeypatch.setattr(rt, "dram_alloc", tight)
+  before = launches()
+  y = expression().realize()
+  assert launches() - before <= 2
+  monkeypatch.setattr(rt, "dram_alloc", lambda size: tight(size, 2 * m * k - 1))
+  with pytest.raises(MemoryError, match="bytes free"): expression().realize()
+  monkeypatch.undo()
+  check_matmul(y.numpy(), x, None, ref, 1e-2)
