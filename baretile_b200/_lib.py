@@ -71,6 +71,7 @@ SIGNATURES = {
   "bt_gemv_queue_plan": [i32, ctypes.POINTER(GemvOp), ctypes.POINTER(i32)],
   "bt_gemv_queue_gates": [i32, ctypes.POINTER(GemvOp), ctypes.POINTER(i32)],
   "bt_gemv_queue_links": [i32, i32, ctypes.POINTER(GemvOp), ctypes.POINTER(i32)],
+  "bt_gemv_queue_rooms": [i32, i32, ctypes.POINTER(GemvOp), ctypes.POINTER(i32)],
   "bt_comm_unique_id": [vp, size_t],
   "bt_comm_init": [i32, i32, i32, vp, ctypes.POINTER(u64)],
   "bt_comm_destroy": [u64],

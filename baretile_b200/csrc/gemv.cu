@@ -508,7 +508,14 @@ struct Walk {
 // stage that would run past the end starts over at 0).
 struct Ring {
   uint32_t off;     // where the next stage would start
-  __device__ __forceinline__ uint32_t place(uint32_t bytes, uint32_t ring_bytes) {       // byte offset of the next stage
+  // The room that the next stage takes: its bytes plus what is skipped when it starts over. Together these may be more than a ring has which
+  // is shorter than two stages (a chain's, whose stages may differ in size). Such a stage waits until it is alone in the ring, and then skips nothing.
+  template <bool SHORT> __host__ __device__ __forceinline__ uint32_t room(uint32_t bytes, uint32_t ring_bytes, bool *alone) const {
+    const uint32_t skipped = off + bytes > ring_bytes ? ring_bytes - off : 0;
+    *alone = SHORT && bytes + skipped > ring_bytes;
+    return *alone ? bytes : bytes + skipped;
+  }
+  __host__ __device__ __forceinline__ uint32_t place(uint32_t bytes, uint32_t ring_bytes) {       // byte offset of the next stage
     if (off + bytes > ring_bytes) off = 0;
     const uint32_t at = off;
     off += bytes;
@@ -575,9 +582,9 @@ __device__ __forceinline__ void produce(const Q &q, uint8_t *smem, uint32_t sbas
       const int first = WEIGHTS ? cta_of(p, sp * KT) : 0, end = WEIGHTS ? cta_of(p, (sp + 1) * KT - 1) : 0;
       for (; rows > 0; rows -= g.ups, kt += g.ups) {
         const int n = min(g.ups, rows);
-        // room: the stage's bytes plus what is skipped when it starts over at the ring's beginning
-        const uint32_t need = g.stage + (ring.off + g.stage > ring_bytes ? ring_bytes - ring.off : 0);
-        while (used + need > ring_bytes || count - oldest == kBars) {
+        bool alone;
+        const uint32_t need = ring.room<CHAIN>(g.stage, ring_bytes, &alone);
+        while (used + need > ring_bytes || count - oldest == kBars || (alone && used)) {
           // asleep in the instruction: a polling loop takes issue slots from the consumers, and the ring is deep enough to
           // hide a late wake-up
           if (!stage_wait(sbase, empty0 + 8 * (oldest % kBars), (oldest / kBars) & 1, q.error)) {
@@ -1328,6 +1335,29 @@ void link(int n, GemvParams *op, const bt_gemv_op *ops, int sets) {
   }
 }
 
+// The stages that a launch holds: every stage has to fit a chain's ring, and two of them any other's (see Ring).
+constexpr int largest_stage(bool chain) {
+  int most = 0;
+  for (int fmt : {BT_BFP8, BT_BFP4})
+    for (int tg = 1; tg <= (chain ? 1 : 4); tg *= 2)
+      for (int lw = 0; lw <= 2; lw++)
+        for (bool pair : {false, true}) most = std::max(most, chain ? geometry(fmt, pair, tg, lw).w_bytes : geometry(fmt, pair, tg, lw).stage);
+  return most;
+}
+static_assert(kSmSums + kSmallSums + kAheadBytes + largest_stage(true) + 256 <= kSmemBytes, "a chain's ring has room for a stage");
+static_assert(kSmSums + std::max(kSmallSums, sums_bytes(4)) + 2 * largest_stage(false) + 256 <= kSmemBytes, "the general kernel's ring has room for two stages");
+
+// What a matmul's sums take of shared memory, and the ring of a launch behind them.
+int sums_of(const GemvParams &p) { return p.small ? p.KT * (p.pair ? 2 : 1) * p.M * sum_stride(p.lw) * 4 : sums_bytes(p.tg); }
+void lay_out(QueueHead &q, int sums, bool chained) {
+  if (chained) sums += kAheadBytes;
+  q.ring = kSmSums + (sums + 127) / 128 * 128, q.ring_bytes = (kSmemBytes - q.ring) / 128 * 128;
+}
+// Where a chain's matmuls run: the next one on other CTAs, which have its weights at hand when its x comes.
+void take_turns(int n, GemvParams *op, int ctas) {
+  for (int i = 0, start = 0; i < n; start = (start + op[i++].active) % ctas) op[i].turn = (ctas - start) % ctas;
+}
+
 // The tensor map of a matmul's x (one tile row of bf16 tiles): the staged token rows of each face are contiguous, a tile
 // has its faces 512 bytes apart, and a copy takes the tile columns of one stage. And those of its weights, if sub-panels are
 // narrower than the runs of the streaming layout.
@@ -1412,16 +1442,14 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       q.panels += p.panels;
       small |= p.small;
       if (int s = make_maps(p, o.x)) return s;
-      sums = max(sums, p.small ? p.KT * (p.pair ? 2 : 1) * p.M * sum_stride(p.lw) * 4 : sums_bytes(p.tg));
+      sums = max(sums, sums_of(p));
     }
     const bool chained = scratch.exchange && chain(q.n, q.op, ops + base);
     if (chained) {
-      sums += kAheadBytes;
-      // the next matmul goes to other CTAs: they have its weights at hand when its x comes
-      for (int i = 0, start = 0; i < q.n; start = (start + q.op[i++].active) % ctas) q.op[i].turn = (ctas - start) % ctas;
+      take_turns(q.n, q.op, ctas);
       link(q.n, q.op, ops + base, scratch.sets);
     }
-    q.ring = kSmSums + (sums + 127) / 128 * 128, q.ring_bytes = (kSmemBytes - q.ring) / 128 * 128;
+    lay_out(q, sums, chained);
     // Programmatic dependent launch: this grid may begin while the previous launch of the stream is still finishing.
     // It only sets up and prefetches weights until its x warps pass griddepcontrol.wait. Weights read that early must
     // be in place, so the launch overlaps its predecessor only when that was a matmul launch of this file too (which
@@ -1529,6 +1557,36 @@ int bt_gemv_queue_links(int sms, int n, const bt_gemv_op *ops, int *links) {
     const bool chained = chain(count, op, ops + base);
     if (chained) link(count, op, ops + base, kSets);
     for (int i = 0; i < count; i++) links[base + i] = chained ? op[i].from : -1;
+  }
+  return BT_OK;
+}
+
+int bt_gemv_queue_rooms(int sms, int n, const bt_gemv_op *ops, int *rooms) {
+  BT_REQUIRE(sms >= 1 && n >= 1 && ops && rooms, "bt_gemv_queue_rooms: needs a GPU's number of SMs, at least one matmul and somewhere for the answer");
+  for (int i = 0; i < n; i++)
+    if (int s = check_op("bt_gemv_queue_rooms", i, ops[i])) return s;
+  const int ctas = min(sms, kMaxCtas);
+  for (int base = 0; base < n; base += kQueueMax) {
+    GemvParams op[kQueueMax];
+    QueueHead q{};
+    const int count = min(kQueueMax, n - base);
+    int sums = 0;
+    for (int i = 0; i < count; i++) describe(op[i], ops[base + i], ctas), sums = max(sums, sums_of(op[i])), rooms[2 * (base + i)] = rooms[2 * (base + i) + 1] = 0;
+    if (!chain(count, op, ops + base)) continue;
+    lay_out(q, sums, true), take_turns(count, op, ctas);
+    for (int cta = 0; cta < ctas; cta++) {
+      Ring ring{0};
+      for (int i = 0; i < count; i++) {
+        rooms[2 * (base + i)] = q.ring_bytes;
+        if ((cta + op[i].turn) % ctas >= op[i].active) continue;
+        const Geometry g = geometry(op[i].fmt, op[i].pair != 0, op[i].tg, op[i].lw);
+        for (int k = 0; k < op[i].KT; k += g.ups) {              // (a whole sub-panel: see chain)
+          bool alone;
+          rooms[2 * (base + i) + 1] = max(rooms[2 * (base + i) + 1], (int)ring.room<true>(g.w_bytes, q.ring_bytes, &alone));
+          ring.place(g.w_bytes, q.ring_bytes);
+        }
+      }
+    }
   }
   return BT_OK;
 }

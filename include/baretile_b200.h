@@ -192,6 +192,10 @@ int bt_gemv_queue_gates(int n, const bt_gemv_op *ops, int *gates);
  * of the kernel for chains of small matmuls 1 where ops[i] takes its x (and an addend that is the same tensor) from the matmul before it while that
  * one still runs, 0 where it reads x from memory. For tests of that rule. */
 int bt_gemv_queue_links(int sms, int n, const bt_gemv_op *ops, int *links);
+/* The ring through which a launch of the kernel for chains streams its weights on a GPU of so many SMs: rooms[2i] is its bytes, rooms[2i + 1] the
+ * most room that a stage of ops[i] asks of it on any of them, which has to be there once the ring is empty. 0 and 0 for launches of the
+ * general kernel. For tests of that rule. */
+int bt_gemv_queue_rooms(int sms, int n, const bt_gemv_op *ops, int *rooms);
 /* ---- the matmul: fused_kernel's prefill grid (baretile/kernels.py:205-215, :470-506, grid_parts :18-39) ----
  * out[M, N] = epilogue(alpha * (a[M, K] @ W[K, N]) + add) for many rows, on the tcgen05 tensor cores with fp32
  * accumulators in tensor memory, two CTAs to an MMA. The weights are expanded from block float to exact bf16

@@ -241,6 +241,39 @@ def test_chain_kernel_takes_lists_that_gain_by_it(built):
   assert takes("chain", 1, *back_and_forth(4096, 256, 24)) and takes("chain", 3, *back_and_forth(4096, 256, 24))
 
 
+def test_chain_ring_takes_every_stage(built):
+  """A chain's ring may be shorter than two stages. Whatever stood in it before, a stage asks for no more than an empty ring has: on no CTA
+  would its copy wait for room that nobody frees."""
+  from baretile_b200 import _lib
+  def rooms(m, layers, *matmuls):
+    """layers of (format, k, n, gate/up pair) matmuls, each reading the one before where that has k columns."""
+    ops, out, columns = [], 0x1000000, 0
+    for i in range(layers):
+      for fmt, k, n, pair in matmuls:
+        k, n, x = -(-k // 32) * 32, -(-n // 32) * 32, out
+        if k != columns: x = 0x1000
+        out, columns = out + 0x1000000, n
+        ops.append(_lib.GemvOp(fmt=fmt, epilogue=3 if pair else 0, M=m, K=k, N=n, out_dtype=0, alpha=1.0, x=x, w=0x100000, w2=0x200000 if pair else 0, out=out))
+    arr, got = (_lib.GemvOp * len(ops))(*ops), (ctypes.c_int * (2 * len(ops)))()
+    _lib.call("bt_gemv_queue_rooms", 148, len(ops), arr, got)
+    return [tuple(got[2 * i:2 * i + 2]) for i in range(len(ops))]
+  short = 0
+  def check(got):
+    nonlocal short
+    for ring, most in got:
+      assert 0 < most <= ring or ring == most == 0
+      short += 0 < ring < 2 * 34816
+  for up, down in ((8, 8), (4, 8), (8, 4), (4, 4)):
+    for m in (1, 3, 8):
+      for d in (32, 96, 320, 576, 1024, 1152, 1344):
+        for f in (64, 576, 1024, 1152, 1536, 3072, 9600):
+          check(rooms(m, 8, (up, d, f, True), (down, f, d, False)))
+        check(rooms(m, 8, (4, 96, 9600, False), (up, d, 1024, True), (down, 1024, d, False)))
+  assert short
+  # stages of 18432 and 34816 bytes in a ring of 50176: CTAs 20 to 31 take one of each
+  assert rooms(8, 3, (4, 1152, 1024, True), (8, 1024, 1152, False))[5] == (50176, 50176)
+
+
 def _complete(gates):
   """For each matmul, the earlier ones of its launch that are complete when it starts: those it looks at, and whatever was
   complete when those started. Nothing else: a matmul may be complete, or start, while one before it still runs."""

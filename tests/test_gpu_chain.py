@@ -80,6 +80,28 @@ def test_chain_results_reuse_memory(rt):
   assert np.array_equal(got.numpy(), want)
 
 
+@pytest.mark.parametrize("m,d,f,up,down,wide", [(8, 1152, 1024, "bfp4", "bfp8", 0), (8, 1152, 1024, "bfp8", "bfp4", 0), (8, 1152, 1024, "bfp4", "bfp4", 9600),
+                                                (8, 1344, 1024, "bfp4", "bfp8", 0), (3, 576, 1536, "bfp4", "bfp8", 9600), (1, 1152, 1024, "bfp8", "bfp4", 9500)])
+def test_chain_of_stages_that_differ(rt, m, d, f, up, down, wide):
+  """Both formats in a list, and sub-panels of four tile columns (`wide`) among narrow ones: stages of 18, 34 and 36 KB in a ring that may have no
+  room for two of them."""
+  rng = np.random.default_rng(m + d + wide)
+  gate, lift, back, side = (upload(rt, weights(rng, *s, stress=False)).cast(fmt).columns() for s, fmt in (((d, f), up), ((d, f), up), ((f, d), down), ((96, wide or 32), "bfp4")))
+  x, z = upload(rt, acts(rng, m, d)), upload(rt, acts(rng, m, 96))
+  def run():
+    y, out = x, []
+    for _ in range(5):
+      if wide: out.append((z @ side).realize())
+      h = ((y @ gate).silu() * (y @ lift)).realize()
+      y = ((h @ back) + y).realize()
+      out += [h, y]
+    return out
+  separate = [t.numpy() for t in run()]
+  with rt.queue(): queued = run()
+  rt.wait()
+  for got, want in zip(queued, separate): assert np.array_equal(got.numpy(), want)
+
+
 def test_tags_start_over(rt):
   """The launch's number, a word of the workspace (kWsEpoch in csrc/gemv.cu), at its last value: the exchanges are cleared and it starts over."""
   rng = np.random.default_rng(4)
