@@ -23,7 +23,8 @@
 // 77 rows of 2048 x 5632 (bfp4, bfp8) 43.7 -> 22.1 us, 33 rows of 512 x 1024 23.8 -> 10.6, 33 rows of 4096 x 14336 113 -> 44, 128 rows 120 -> 55,
 // 256 rows 126 -> 110, 640 rows 287 -> 264; 512 rows of 1024 x 3000 38 -> 27.
 // A launch costs 5 to 10 us beside its stages: setting up and the first weights and x 3, the sums' way through the cluster and the epilogue 3.
-// Every wait is bounded and reports through the error word.
+// Every wait on an mbarrier is bounded and reports through the error word; the first that gives up ends the waiting of its CTA. The cluster's two barriers,
+// which every CTA reaches that way, have no limit of their own.
 #include "common.cuh"
 #include "expand.cuh"
 #include <algorithm>
@@ -45,7 +46,7 @@ static_assert(kMaxStages % kGroups == 0, "places of the ring belong to groups");
 constexpr uint32_t kLimit = 1u << 14;               // attempts of up to 100 us each
 
 // Shared memory: mbarriers, then the rings of packed weights and of x, over which the sums go in the end.
-constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kRing = 1024;
+constexpr int kWFull = 0, kWEmpty = 64, kXFull = 128, kXEmpty = 192, kReady = 256, kFree = 288, kDone = 320, kTmem = 328, kDead = 332, kRing = 1024;
 constexpr int kSmem = 227 * 1024;
 constexpr int kBlockRows = 4;                       // tile rows of a CTA at most: the sums of 128 tokens of a pair and the expanded weights fill tensor memory
 constexpr int kSumStride = 132;                     // floats from one token's 128 channels to the next
@@ -81,9 +82,14 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
   const int width = min(kPanel, p.TC - panel * kPanel), N = (M + 15) / 16 * 16, stages = p.stages, x_stages = p.x_stages, bufs = p.bufs;
   const int x_row = N * 64, x_stage = kRows * p.tokens * 64;
   const uint32_t x_ring = sb + kRing + stages * W_STAGE;
+  // A wait that gives up marks the CTA: from there on its sums are worthless, and every wait takes one attempt, so that the CTA ends in some
+  // milliseconds (with a full limit to each of up to 112 stages it held the GPU for minutes).
   auto wait = [&](uint32_t bar, uint32_t parity, int code) {
-    if (!mbar_wait(bar, parity, kLimit)) atomicExch(p.error, code);
+    bool ok = mbar_try_wait(bar, parity, 100000u);
+    for (uint32_t i = 1; !ok && i < kLimit && !lds32(sb + kDead); i++) ok = mbar_try_wait(bar, parity, 100000u);
+    if (!ok) sts32(sb + kDead, 1), atomicExch(p.error, code);
     __syncwarp();                                   // whole warps wait, and the tensor-memory instructions that follow want them in step
+    return ok;
   };
   if (warp == 0) {                                  // a lane to a place of the rings
     if (lane < kMaxStages) {
@@ -91,7 +97,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
       mbar_init(sb + kXFull + 8 * lane, kXWarps * 32), mbar_init(sb + kXEmpty + 8 * lane, 1);
     }
     if (lane < kMaxBufs) mbar_init(sb + kReady + 8 * lane, kGroupWarps), mbar_init(sb + kFree + 8 * lane, 1);
-    if (lane == 0) mbar_init(sb + kDone, 1);
+    if (lane == 0) mbar_init(sb + kDone, 1), sts32(sb + kDead, 0);
     mbar_fence_init();
   }
   if (warp == kMmaWarp) tmem_alloc(sb + kTmem, 512);
@@ -119,12 +125,14 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
     const uint32_t stage = kRows * width * TB;
     Turn t;
     for (int i = 0; i < steps; i++, t.next(stages), from += stage) {
-      if (i >= stages) wait(sb + kWEmpty + 8 * t.at, t.parity ^ 1, 21);
+      if (i >= stages && !__all_sync(0xFFFFFFFFu, wait(sb + kWEmpty + 8 * t.at, t.parity ^ 1, 21))) break;
       const uint32_t bytes = min(kRows, kn - i * kRows) * width * TB, bar = sb + kWFull + 8 * t.at;
       if (lane == 0) mbar_expect_tx(bar, MATS * bytes);
       __syncwarp();
       if (lane < MATS) bulk_g2s(sb + kRing + t.at * W_STAGE + lane * (kRows * kPanel * TB), from, bytes, bar);
     }
+    if (lds32(sb + kDead))                           // nobody may be waiting for the copies in flight any more; they land before the CTA ends
+      for (int i = 0; i < stages; i++, t.next(stages)) mbar_wait(sb + kWFull + 8 * t.at, t.parity ^ 1, 100);
   } else if (warp == kMmaWarp) {
     {
       const uint32_t leader = elect_one();
@@ -156,6 +164,7 @@ __global__ void __launch_bounds__(kThreads, 1) few_rows_kernel(const __grid_cons
         umma_commit_if(sb + kFree + 8 * u.at, leader);
       }
       umma_commit_if(sb + kDone, leader);
+      wait(sb + kDone, 0, 28);                       // tensor memory is given back by this warp
     }
   } else if (warp >= kXWarp) {
     in_turn();
