@@ -333,8 +333,8 @@ __global__ void __launch_bounds__(256) reduce_kernel(const GemmParams p) {
 // fewer, which is what prompts of some hundred rows and few columns have, blocks of 256 rows and blocks whose K is shared
 // by several pairs keep more of the GPU busy, at the price of fp32 parts written and read once more. The estimate: a pair
 // takes kBlockUs for a K block of 256 rows and kFixedUs for everything else; the parts move at 3 TB/s and cost another
-// launch. 2048 rows of 14336 x 4096 stay as they are (64 blocks), 77 rows of 5632 x 2048 (8 blocks of 88 K blocks) go in 8
-// parts.
+// launch. 2048 rows of 14336 x 4096 stay as they are (64 blocks), 400 rows of 8992 x 2900 (12 blocks of 141 K blocks) go in parts. (Most
+// sizes that want parts are the few-rows kernel's by bt_gemm_tiles' rule.)
 // Where every pair has 256 rows the MMAs of a K block take 512 cycles and its expansion, one warp's chain of waits, loads,
 // arithmetic and stores, 700, so two groups of warps expand K blocks in turn: 40 rows of 4096x14336, gate/up and down, 133 -> 118
 // us, 512 rows 202 -> 191. With 512 rows to a pair the MMAs take 1024, one group keeps up, and a second one only

@@ -21,7 +21,7 @@
 //                in the 32-byte swizzle, and tells the stage's barrier itself when it has (warps that waited for their copies: 128 rows 58 us against 55)
 // Gate/up pair and down projection, against the kernel of gemm.cu with its x laid out by rows and its parts of K added up by another launch:
 // 77 rows of 2048 x 5632 (bfp4, bfp8) 43.7 -> 22.1 us, 33 rows of 512 x 1024 23.8 -> 10.6, 33 rows of 4096 x 14336 113 -> 44, 128 rows 120 -> 55,
-// 256 rows 126 -> 110, 640 rows 287 -> 264; 512 rows of 1024 x 3000 38 -> 27.
+// 256 rows 124 -> 110, 640 rows 287 -> 228; 512 rows of 1024 x 3000 37.9 -> 24.7.
 // A launch costs 5 to 10 us beside its stages: setting up and the first weights and x 3, the sums' way through the cluster and the epilogue 3.
 // Every wait on an mbarrier is bounded and reports through the error word; the first that gives up ends the waiting of its CTA. The cluster's two barriers,
 // which every CTA reaches that way, have no limit of their own.

@@ -35,8 +35,7 @@
 // channels as its K and up to 8 tokens as its columns. The 16 weights of a face row share an exponent e; how the
 // packed bytes become weights is described at tile_mma.
 #include "common.cuh"
-#include "ptx.cuh"
-#include "stream_layout.cuh"
+#include "expand.cuh"
 #include "tmap.cuh"
 #include <algorithm>
 #include <cstring>
@@ -298,8 +297,6 @@ __device__ __forceinline__ void tile_mma(uint32_t tile, uint32_t ex, uint32_t xs
   }
 }
 
-__device__ __forceinline__ float silu(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
-__device__ __forceinline__ uint32_t bf16_half_up(float v) { return (__float_as_uint(v) + 0x8000u) >> 16; }
 // (value, column) as one number whose order is the pick's: larger value first, of equal values (-0 equals 0) the lower
 // column. Zero is "nothing": a NaN, which never wins, maps to it, and no other value does (-inf maps to 0x007FFFFF in
 // the upper half).
@@ -905,7 +902,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemv_queue_kernel(const __grid_co
 //  * Weights are expanded, scale and all, while x is still on its way, and wait in shared memory as the MMAs take them.
 //  * The next matmul runs on other CTAs, which have had the time for that.
 // 2.0-2.2 us a matmul for one token (1.0 until x is seen, 0.4 to the sums, 0.6 to add them and publish), 3 for eight, whose words and
-// tags are 36 KB to a CTA of a gate/up pair. 30 layers of 576 x 1536 with host values in and out: one token 500 -> 279 us, eight 507 -> 390.
+// tags are 36 KB to a CTA of a gate/up pair. 30 layers of 576 x 1536 with host values in and out: one token 500 -> 276 us, eight 507 -> 390.
 //
 // What makes it safe to start before the matmul before is known to be complete: of that matmul only x (and the addend, where it is the
 // same tensor) is read, from the exchange. Whatever this one overwrites that the matmul before reads has been
@@ -1467,7 +1464,7 @@ int enqueue(const char *who, int device, int n, const bt_gemv_op *ops, const Que
       std::copy(q.op, q.op + q.n, s.op);
       BT_CUDA(chained ? cudaLaunchKernelEx(&cfg, chain_kernel<kQueueShort>, s) : small ? cudaLaunchKernelEx(&cfg, gemv_queue_kernel<true, kQueueShort>, s) : cudaLaunchKernelEx(&cfg, gemv_queue_kernel<false, kQueueShort>, s));
     } else BT_CUDA(chained ? cudaLaunchKernelEx(&cfg, chain_kernel<kQueueMax>, q) : small ? cudaLaunchKernelEx(&cfg, gemv_queue_kernel<true, kQueueMax>, q) : cudaLaunchKernelEx(&cfg, gemv_queue_kernel<false, kQueueMax>, q));
-    if (int st = launched("gemv_queue_kernel")) return st;
+    if (int st = launched(chained ? "chain_kernel" : "gemv_queue_kernel")) return st;
   }
   return BT_OK;
 }

@@ -168,7 +168,8 @@ int bt_gemv_bfp(int device, int fmt, int epilogue, int M, int K, int N, uint64_t
  * step where each result feeds the next, and the library works out from the addresses which earlier matmuls each
  * one has to wait for (bt_gemv_queue_plan shows the answer). Between two matmuls the GPU keeps streaming: the
  * weights of the next ones are fetched while the previous one finishes, only x waits, and matmuls that do not
- * depend on one another overlap (two in flight at most). The weights (w, w2) must not be written by an earlier
+ * depend on one another overlap (two in flight at most). In a chain of small matmuls for up to 8 tokens x goes on to the next matmul
+ * word by word while the one before still runs (bt_gemv_queue_links); the results are the same, to the last bit. The weights (w, w2) must not be written by an earlier
  * matmul of the same call or by the launch right before it in the stream. The fields of bt_gemv_op are
  * bt_gemv_bfp's arguments of the same names. */
 typedef struct bt_gemv_op {
@@ -178,7 +179,8 @@ typedef struct bt_gemv_op {
 } bt_gemv_op;
 int bt_gemv_queue(int device, int n, const bt_gemv_op *ops, uint64_t work, size_t work_bytes, uint64_t stream);
 /* What bt_gemv_queue would make each matmul wait for, without touching a device: waits[i] receives the index of the
- * last earlier matmul that ops[i] must see finished before it starts, it and all matmuls of the launch before it, or -1
+ * last earlier matmul that ops[i] must see finished before it reads x from memory or stores anything (a matmul that bt_gemv_queue_links names
+ * takes x from that one word by word instead, and needs nothing else of it), it and all matmuls of the launch before it, or -1
  * when it only waits for the launch before it. That is the latest earlier one whose result it reads (x, add) or whose result
  * buffers it writes or that reads what it writes, or the one two places back where that comes later: a matmul never runs
  * more than two places ahead of one still in flight. A list longer than 32 is cut into launches of 32, and the

@@ -134,7 +134,7 @@ def test_shapes_that_are_not_whole_blocks(rt, fmt, k, n):
 @pytest.mark.parametrize("epilogue", ["none", "glu"])
 def test_without_room_for_parts_of_k(rt, monkeypatch, epilogue):
   # a device with room for x by rows but not for the parts: the matmul runs all the same, and one that has no room for x by
-  # rows either says so
+  # rows either says so. (The kernel for few rows, which this size takes, uses neither; test_parts_of_k_in_memory does the same where both are used.)
   rng = np.random.default_rng(5)
   m, k, n = 77, 2048, 544
   x, w, w2 = acts(rng, m, k), weights(rng, k, n), weights(rng, k, n)
@@ -177,8 +177,8 @@ def test_results_stay_inside_their_tiles(rt):
 @pytest.mark.parametrize("fmt", ["bfp8", "bfp4"])
 @pytest.mark.parametrize("m,k,n", [(33, 64, 32), (33, 4096, 64), (77, 2080, 330), (256, 1024, 128), (257, 2112, 96), (300, 8192, 288), (520, 1536, 1000)])
 def test_shared_k_and_half_blocks(rt, fmt, m, k, n):
-  # few blocks: their K is shared by several pairs of CTAs (one K block each at the least, an odd last tile row in the last
-  # part), blocks of 256 rows; every epilogue of the kernel that adds the parts up
+  # few blocks of 256 rows and an odd last tile row, every epilogue. The expression takes the kernel for few rows, whose clusters share K; `run` gives
+  # the kernel for many rows no room for parts of K (test_parts_of_k_in_memory has sizes that take them)
   rng = np.random.default_rng(m + k + n)
   xi, wi = rng.integers(-2, 3, (m, k)).astype(np.float32), rng.integers(-1, 2, (k, n)).astype(np.float32)
   got, _ = run(rt, xi, wi, fmt, dtype="fp32")
